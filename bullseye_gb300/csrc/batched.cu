@@ -400,55 +400,50 @@ __global__ void __launch_bounds__(kRecordWarps * 32) record_kernel(
 struct Variant {
   int J = 0;
   bool wide = false;
-  int regs = 0;  // register cap of the build
-  int NT = 0, V = 0, grid = 0;
-  size_t smem = 0;
+  int NT = 0, grid = 0;
+  ChunkShape chunk{0, 0, 0};
 };
 
 template <int NC, bool WPROJ, bool COMP>
 using SegKernel = void (*)(const GridArgs, const int);
 
+// Launches from visibility records (the tuner's candidates).
 template <int NC, bool WPROJ, bool COMP, bool WIDE>
-SegKernel<NC, WPROJ, COMP> seg_kernel_of(int J, int regs) {
-  if (J == 8) return romein_segment_kernel<NC, WPROJ, 8, COMP, WIDE>;
+SegKernel<NC, WPROJ, COMP> seg_kernel_of(int J) {
+  if (J == 8) return romein_segment_kernel<NC, WPROJ, 8, COMP, WIDE, true>;
 #if defined(BULLSEYE_SINGLE)
   if constexpr (NC == 4 && WPROJ) {
-    if (J == 6) return romein_segment_kernel<NC, WPROJ, 6, COMP, WIDE, kSegRegs6>;
+    if (J == 6) return romein_segment_kernel<NC, WPROJ, 6, COMP, WIDE, true>;
   }
 #endif
-  if constexpr (NC == 4 && WPROJ) {
-    if (regs == 64) return romein_segment_kernel<NC, WPROJ, 4, COMP, WIDE, 64>;
-    if (regs == 72) return romein_segment_kernel<NC, WPROJ, 4, COMP, WIDE, 72>;
-  }
-  return romein_segment_kernel<NC, WPROJ, 4, COMP, WIDE>;
+  return romein_segment_kernel<NC, WPROJ, 4, COMP, WIDE, true>;
 }
 
 template <int NC, bool WPROJ, bool COMP>
-SegKernel<NC, WPROJ, COMP> seg_kernel(int J, bool wide, int regs) {
-  return wide ? seg_kernel_of<NC, WPROJ, COMP, true>(J, regs) : seg_kernel_of<NC, WPROJ, COMP, false>(J, regs);
+SegKernel<NC, WPROJ, COMP> seg_kernel(int J, bool wide) {
+  return wide ? seg_kernel_of<NC, WPROJ, COMP, true>(J) : seg_kernel_of<NC, WPROJ, COMP, false>(J);
 }
 
-// Register caps the tuner tries for a layout.
-template <int NC, bool WPROJ>
-std::vector<int> reg_caps(int J) {
-  if (J == 8) return {kSegRegs<8>};
-  if (J == 6) return {kSegRegs6};
-  if (NC == 4 && WPROJ) return {kSegRegs<4>, 72, 64};
-  return {kSegRegs<4>};
+// Launches that prepare their visibilities in place (no records, or past the record budget).
+template <int NC, bool WPROJ, bool COMP>
+SegKernel<NC, WPROJ, COMP> inplace_kernel(int J, bool wide) {
+  if (wide) return romein_segment_kernel<NC, WPROJ, 8, COMP, true, false>;
+  return J == 8 ? romein_segment_kernel<NC, WPROJ, 8, COMP, false, false>
+                : romein_segment_kernel<NC, WPROJ, 4, COMP, false, false>;
 }
 
+constexpr int seg_regs(int J) { return J == 4 ? kSegRegs<4> : J == 6 ? kSegRegs<6> : kSegRegs<8>; }
+
 template <int NC, bool WPROJ>
-bool make_variant(int W, int J, bool wide, int regs, Variant &v) {
+bool make_variant(int W, int J, bool wide, Variant &v) {
   const int cols = ((W + 31) / 32) * 32;
   if (wide && (cols - W) * 8 > W) return false;
   const int owners = wide ? cols * ((W + J - 1) / J) : W * ((W + J - 1) / J);
   v.J = J;
   v.wide = wide;
-  v.regs = regs;
   v.NT = std::max(32, ((owners + 31) / 32) * 32);
   if (v.NT > 512) return false;
-  v.V = grid_chunk_size<NC, WPROJ>(W, v.NT, J, regs);
-  v.smem = grid_smem_bytes<NC, WPROJ>(v.V, W, v.NT, J);
+  v.chunk = chunk_shape<NC, WPROJ>(W, v.NT, J, seg_regs(J));
   return true;
 }
 
@@ -470,7 +465,7 @@ struct BatchedState {
   int conv_w_stride = 0;
   size_t rows_cap = 0, tracks_cap = 0, segs_cap = 0;
   // tuning decisions, by (class width, NC, WPROJ, COMP)
-  std::map<std::tuple<int, int, int, int>, std::tuple<int, int, int>> tuned;  // -> (J, wide, regs)
+  std::map<std::tuple<int, int, int, int>, std::tuple<int, int>> tuned;  // -> (J, wide)
   // captured graphs, by launch arguments (two slots: the reference's exports alternate between
   // the visibilities and the sampling function); least recently used is replaced
   struct GraphSlot {
@@ -733,11 +728,12 @@ bool launch_records(const GridArgs &base, int nfacets, cudaStream_t st, GridArgs
 }
 
 template <int NC, bool WPROJ, bool COMP>
-bool launch_class(const GridArgs &base, int k, const Variant &v, int nfacets, const int *count, int *next,
+bool launch_build(const GridArgs &base, int k, const Variant &v, bool inplace, int nfacets, const int *count, int *next,
                   cudaStream_t st) {
   GridArgs a = base;
   a.W = g_bs.cls[k].width;
-  a.V = v.V;
+  a.V = v.chunk.V;
+  a.GB = v.chunk.GB;
   a.plane_lo = g_bs.plane_lo.ptr;
   a.conv_w = g_bs.conv_w.ptr;
   a.conv_w_stride = g_bs.conv_w_stride;
@@ -750,28 +746,52 @@ bool launch_class(const GridArgs &base, int k, const Variant &v, int nfacets, co
     bz_record_error(BZ_ERR_CUDA, "batched: no layout chosen for support class %d", a.W);
     return false;
   }
-  auto kern = seg_kernel<NC, WPROJ, COMP>(v.J, v.wide, v.regs);
+  auto kern = inplace ? inplace_kernel<NC, WPROJ, COMP>(v.J, v.wide) : seg_kernel<NC, WPROJ, COMP>(v.J, v.wide);
   if (!open_smem(kern)) {
     bz_record_error(BZ_ERR_CUDA, "batched: cudaFuncSetAttribute failed");
     return false;
   }
   BZ_CUDA_TRY_RET(cudaMemsetAsync(next, 0, sizeof(int), st), false);
-  kern<<<v.grid, v.NT, v.smem, st>>>(a, nfacets);
+  kern<<<v.grid, v.NT, v.chunk.smem, st>>>(a, nfacets);
   g_ctx.launches++;
   BZ_CUDA_TRY_RET(cudaGetLastError(), false);
   return true;
 }
 
 template <int NC, bool WPROJ, bool COMP>
-bool finish_variant(Variant &v) {
-  auto kern = seg_kernel<NC, WPROJ, COMP>(v.J, v.wide, v.regs);
+bool finish_variant(Variant &v, bool inplace = false) {
+  auto kern = inplace ? inplace_kernel<NC, WPROJ, COMP>(v.J, v.wide) : seg_kernel<NC, WPROJ, COMP>(v.J, v.wide);
   if (!open_smem(kern)) return false;
   int per_sm = 0, dev = 0, sms = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, v.NT, v.smem) != cudaSuccess || per_sm < 1) return false;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, v.NT, v.chunk.smem) != cudaSuccess || per_sm < 1) return false;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   v.grid = per_sm * sms;
   return true;
+}
+
+// The layout of launches that prepare in place: J = 4 (J = 8 where the J = 4 layout needs more than 512
+// threads).
+template <int NC, bool WPROJ, bool COMP>
+bool inplace_variant(int W, Variant &v) {
+  for (int J : {4, 8})
+    if (make_variant<NC, WPROJ>(W, J, false, v) && finish_variant<NC, WPROJ, COMP>(v, true)) return true;
+  return make_variant<NC, WPROJ>(W, 8, true, v) && finish_variant<NC, WPROJ, COMP>(v, true);
+}
+
+// One support class: from records, and in place where there are none or they may not hold every item.
+template <int NC, bool WPROJ, bool COMP>
+bool launch_class(const GridArgs &base, int k, const Variant &v, int nfacets, const int *count, int *next,
+                  cudaStream_t st) {
+  const bool all = base.records && (double)base.nrows * base.nchan * nfacets <= (double)base.rec_capacity;
+  if (base.records && !launch_build<NC, WPROJ, COMP>(base, k, v, false, nfacets, count, next, st)) return false;
+  if (all) return true;
+  Variant in;
+  if (!inplace_variant<NC, WPROJ, COMP>(g_bs.cls[k].width, in)) {
+    bz_record_error(BZ_ERR_UNSUPPORTED, "batched: no layout for support class %d", g_bs.cls[k].width);
+    return false;
+  }
+  return launch_build<NC, WPROJ, COMP>(base, k, in, true, nfacets, count, next, st);
 }
 
 // Autotuner: time every valid layout of a class on a sample of its own work items, gridding into
@@ -788,26 +808,25 @@ bool tune_class(const GridArgs &base, int k, int nfacets, Variant &out, int host
   // column tap shared by 6 rows
   const bool six = BZ_PRECISION_BITS == 32 && NC == 4 && WPROJ;
   for (int J : {8, 6, 4})
-    for (bool wide : {true, false})
-      for (int regs : reg_caps<NC, WPROJ>(J)) {
-        if (J == 6 && !six) continue;
-        Variant v;
-        if (make_variant<NC, WPROJ>(W, J, wide, regs, v) && finish_variant<NC, WPROJ, COMP>(v)) cands.push_back(v);
-      }
+    for (bool wide : {true, false}) {
+      if (J == 6 && !six) continue;
+      Variant v;
+      if (make_variant<NC, WPROJ>(W, J, wide, v) && finish_variant<NC, WPROJ, COMP>(v)) cands.push_back(v);
+    }
   if (cands.empty()) {
     bz_record_error(BZ_ERR_UNSUPPORTED, "batched: no layout for support class %d", W);
     return false;
   }
   if (it != b.tuned.end()) {
     for (auto &v : cands)
-      if (v.J == std::get<0>(it->second) && (int)v.wide == std::get<1>(it->second) && v.regs == std::get<2>(it->second)) {
+      if (v.J == std::get<0>(it->second) && (int)v.wide == std::get<1>(it->second)) {
         out = v;
         return true;
       }
   }
   if (cands.size() == 1 || host_count == 0) {
     out = cands[0];
-    b.tuned[key] = std::make_tuple(out.J, (int)out.wide, out.regs);
+    b.tuned[key] = std::make_tuple(out.J, (int)out.wide);
     return true;
   }
   // Each candidate grids a quarter of the class's runs (at least 4096, when there are that many)
@@ -843,7 +862,7 @@ bool tune_class(const GridArgs &base, int k, int nfacets, Variant &out, int host
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   BZ_CUDA_TRY_RET(cudaMemsetAsync(c.scratch.ptr, 0, sizeof(vis_complex) * c.scratch.n, c.stream), false);
-  b.tuned[key] = std::make_tuple(out.J, (int)out.wide, out.regs);
+  b.tuned[key] = std::make_tuple(out.J, (int)out.wide);
   return bz_error_code() == BZ_OK;
 }
 
@@ -903,7 +922,7 @@ bool launch_all(const GridArgs &base_in, int nfacets, bool sampling, cudaStream_
       cudaEventElapsedTime(&ms, e0, e1);
       cudaEventDestroy(e0);
       cudaEventDestroy(e1);
-      b.records.push_back({b.cls[k].width, NC, v.J, (int)v.wide | (v.regs << 1), counts ? (*counts)[k] * nfacets : 0, ms});
+      b.records.push_back({b.cls[k].width, NC, v.J, (int)v.wide | (seg_regs(v.J) << 1), counts ? (*counts)[k] * nfacets : 0, ms});
     }
     if (!ok) return false;
   }
@@ -1499,19 +1518,10 @@ SupportWs support_ws_layout(long long R, int nchan, int nslots, int P, int os, i
   return l;
 }
 
-// Thread layout of one support class of the workspace form: J = 4 (J = 8 where the J = 4 layout
-// needs more than 512 threads), fixed so that concurrent calls share no tuning state.
-template <bool WPROJ, bool COMP>
-bool support_aware_variant(int W, Variant &v) {
-  for (int J : {4, 8})
-    if (make_variant<4, WPROJ>(W, J, false, kSegRegs<4>, v) && finish_variant<4, WPROJ, COMP>(v)) return true;
-  return make_variant<4, WPROJ>(W, 8, true, kSegRegs<8>, v) && finish_variant<4, WPROJ, COMP>(v);
-}
-
 template <bool WPROJ, bool COMP>
 bool support_aware_layouts(const ClassList &cl, Variant *vs) {
   for (int k = 0; k < cl.n; ++k)
-    if (!support_aware_variant<WPROJ, COMP>(cl.w[k], vs[k])) {
+    if (!inplace_variant<4, WPROJ, COMP>(cl.w[k], vs[k])) {
       bz_record_error(BZ_ERR_UNSUPPORTED, "support-aware gridding: no layout for class width %d", cl.w[k]);
       return false;
     }
@@ -1534,13 +1544,14 @@ bool support_aware_launches(const GridArgs &a, const ClassList &cl, const Varian
     const Variant &v = vs[k];
     GridArgs ak = a;
     ak.W = cl.w[k];
-    ak.V = v.V;
+    ak.V = v.chunk.V;
+    ak.GB = v.chunk.GB;
     ak.segment_base = class_off + k;
     ak.work_count = class_count + k;
     ak.work_next = work_next + k;
-    auto kern = seg_kernel<4, WPROJ, COMP>(v.J, v.wide, v.regs);
+    auto kern = inplace_kernel<4, WPROJ, COMP>(v.J, v.wide);
     if (cudaMemsetAsync(work_next + k, 0, sizeof(int), st) != cudaSuccess) return false;
-    kern<<<v.grid, v.NT, v.smem, st>>>(ak, nfacets);
+    kern<<<v.grid, v.NT, v.chunk.smem, st>>>(ak, nfacets);
     if (cudaGetLastError() != cudaSuccess) return false;
   }
   return true;

@@ -14,13 +14,12 @@
 // reference GPU kernel instead binds each thread to a fixed footprint offset
 // (bullseye/mo/gpu_algorithm/templated_gridder.h:59-69), which flushes on every cell move.
 //
-// Per-visibility work (the prologue) is done once per CTA, not once per thread: V threads each
+// Per-visibility work (the prologue) is done once per CTA, not once per thread: threads each
 // prepare one visibility (correlation selection, weights x flags, Jones J_p^-1 V J_q^-H, facet
-// phase rotation, planar uv transform, cell and tap-offset selection) into shared memory, the
-// CTA then stages the 2W + J - 1 taps of each staged visibility (in the persistent batched
-// kernel: two TMA bulk copies per visibility from the support-window table, completed on an
-// mbarrier; otherwise per-tap asynchronous copies from the ABI's table), and all threads grid
-// the staged chunk.
+// phase rotation, planar uv transform, cell and tap-offset selection) into shared memory (the
+// persistent batched kernel stages records that the record kernel prepared, by TMA bulk copies).
+// The staged chunk is then merged into groups of visibilities with a common tap row, and the
+// owner threads add each group to their cells (see "merged gridding" below).
 //
 // Numerics (matching the reference CPU library, bullseye/mo/cpu_algorithm/*):
 //  * uvw / lambda, the phase argument 2 pi (u dl + v dm + w dn), the uv transform and the
@@ -120,7 +119,7 @@ struct GridArgs {
   int mode;                      // CorrMode
   int phase, uvx;                // faceting phase rotation / planar uv transform
   int nslots, seg;               // track slots (baselines or fixed segments), segment length
-  int V;                         // visibilities staged per chunk
+  int V, GB;                     // visibilities staged per chunk, groups merged at a time
   const int *plane_lo;           // per w plane: first tap of its nonzero window (support-aware), or null
   const int4 *segments;          // persistent mode: {row_begin, row_end, channel, -} per segment, or null
   const int *work_count;         // persistent mode: number of segments of this launch (device)
@@ -221,14 +220,12 @@ __device__ __forceinline__ cplx phase_factor(double x) {
 }
 #endif
 
-// Flush one owned cell's register accumulator into the grid.  Compensated mode adds with
+// Flush one owned cell's register accumulator into the grid (cell: the grid element of correlation 0).  Compensated mode adds with
 // atomics that return the previous value, then recovers each addition's rounding error exactly
 // (TwoSum: s = a + b, e = (a - (s - (s - a))) + (b - (s - a))) and adds it to the lo grid; the
 // final grid is hi + lo.  The NC atomics of a cell are issued before any result is consumed.
 template <int NC, bool COMP>
-__device__ __forceinline__ void flush_cell(const GridArgs &a, long long base, long long nxy, int nx, int x, int y,
-                                           cplx (&acc)[NC]) {
-  const long long cell = base + (long long)y * nx + x;
+__device__ __forceinline__ void flush_cell(const GridArgs &a, long long cell, long long nxy, cplx (&acc)[NC]) {
 #if defined(BULLSEYE_SINGLE)
   if (COMP) {
     float2 old[NC];
@@ -272,7 +269,7 @@ constexpr int kDrainAt = 32;
 
 template <int NC>
 struct FlushRec {
-  long long cell;        // grid element of correlation 0 (base + y * nx + x)
+  long long cell;        // grid element of correlation 0
   float2 v[NC];
 };
 
@@ -308,20 +305,20 @@ __device__ __forceinline__ void drain_queue(const GridArgs &a, long long nxy, Fl
 
 // Queue one owned cell's accumulator (falls back to a direct flush when the queue is full).
 template <int NC>
-__device__ __forceinline__ void queue_cell(const GridArgs &a, long long base, long long nxy, int nx, int x, int y,
-                                           cplx (&acc)[NC], FlushRec<NC> *q, int *qn) {
+__device__ __forceinline__ void queue_cell(const GridArgs &a, long long cell, long long nxy, cplx (&acc)[NC],
+                                           FlushRec<NC> *q, int *qn) {
 #if defined(BULLSEYE_SINGLE)
   const int slot = atomicAdd(qn, 1);
   if (slot < kFlushQueueCap) {
     FlushRec<NC> r;
-    r.cell = base + (long long)y * nx + x;
+    r.cell = cell;
 #pragma unroll
     for (int k = 0; k < NC; ++k) r.v[k] = make_float2(acc[k].re, acc[k].im);
     q[slot] = r;
 #pragma unroll
     for (int k = 0; k < NC; ++k) { acc[k].re = 0; acc[k].im = 0; }
   } else {
-    flush_cell<NC, true>(a, base, nxy, nx, x, y, acc);
+    flush_cell<NC, true>(a, cell, nxy, acc);
   }
 #endif
 }
@@ -860,6 +857,10 @@ __device__ __forceinline__ void facet_record(const GridArgs &a, int f_local, int
     const int Wfull = a.W_full ? a.W_full : a.W;
     rec.fu = (int)(((long long)plane * a.tap_f + cell.fu) * Wfull + lo);
     rec.fv = (int)(((long long)plane * a.tap_f + cell.fv) * Wfull + lo);
+  } else {
+    // index of the first tap in the ABI's table
+    rec.fu += (int)(plane * a.K);
+    rec.fv += (int)(plane * a.K);
   }
   rec.plane = (int)plane;
   rec.u0 = du;
@@ -1006,6 +1007,10 @@ __device__ __forceinline__ void prologue(const GridArgs &a, int f_local, int cha
     const int Wfull = a.W_full ? a.W_full : a.W;
     rec.fu = (int)(((long long)plane * a.tap_f + cell.fu) * Wfull + lo);
     rec.fv = (int)(((long long)plane * a.tap_f + cell.fv) * Wfull + lo);
+  } else {
+    // index of the first tap in the ABI's table
+    rec.fu += (int)(plane * a.K);
+    rec.fv += (int)(plane * a.K);
   }
   rec.plane = (int)plane;
   rec.u0 = du;
@@ -1018,7 +1023,29 @@ __device__ __forceinline__ void prologue(const GridArgs &a, int f_local, int cha
   rec.valid = 1;
 }
 
-// Shared-memory bytes for a launch with V staged visibilities.
+// ------------------------------------------------------------------ merged gridding of staged chunks
+//
+// Taps are products: footprint cell (a, b) of a visibility gets vis x ka(a) x kb(b).  Consecutive
+// visibilities of a track sit a fraction of an oversampling step apart, so a stretch of them often
+// shares the footprint corner and one of the two tap rows.  Such a *group* is summed along the other
+// axis first,
+//     T(a) = sum over the group of vis x ka(a)            (W multiply-adds per visibility)
+//     cell(a, b) += T(a) x kb(b)                            (W^2 multiply-adds per group, not per visibility)
+// which is the same sum with its common factor taken out.  On Earth-rotation tracks sampled every 14 s
+// (27 EVLA antennas, 1024-cell grids 1.4 degrees wide, oversampling 15) groups hold 4.6 visibilities
+// on average when each work item merges along the axis on which its track moves less in tap steps;
+// fixed to one axis they hold 2.3 (u) or 3.9 (v), and merging only identical footprints gives 1.9.
+//
+// What the merge and the split of the builds measured (GB300, 27 antennas x 100 times x 64 channels,
+// 16 facets, whole batched call with copy-back): 36.5 -> 27.3 ms in single precision; 64-bit library,
+// 40 times x 16 channels x 4 facets: 28.2 -> 8.1 ms (its FP64 pipe bounded the multiply-adds).
+//
+// A chunk of V records in shared memory is taken in two steps, in batches of GB groups:
+//   merge_groups  thread (a, part) forms T(a) of every nparts-th group of the batch, reading ka from
+//                 the kernel table through L1, and copies the group's kb row;
+//   grid_groups   the Romein owner threads add T(a) x kb(b) to their J cells per column.
+// The item's axes are (a, b) = (u, v), or (v, u) when it merges along v ("swapped").
+
 // Per-warp flush queues (compensated single precision only): nwarps record arrays, then one
 // 16-byte counter slot per warp.
 template <int NC>
@@ -1031,65 +1058,72 @@ __host__ __device__ inline size_t flush_queue_bytes(int nwarps) {
 #endif
 }
 
-// Row taps are stored W + J - 1 long per visibility: the first J - 1 taps are repeated after the
-// last, so a thread's J consecutive owned rows read J consecutive taps without a wrap.
+// Most records of a chunk: group lists are built from 64-bit masks.
+constexpr int kMaxChunk = 64;
 
-// Staged tap rows per visibility: W column taps, then W + J - 1 row taps (the first J - 1 repeated
-// after the last), each row padded to a multiple of 16 bytes so that it can be one bulk copy.
-template <bool WPROJ>
-__host__ __device__ inline int tap_row_u(int W) {
-  constexpr int E = (int)(16 / sizeof(typename TapT<WPROJ>::type));
-  return (W + E - 1) / E * E;
-}
-template <bool WPROJ>
-__host__ __device__ inline int tap_row_v(int W, int J) {
-  constexpr int E = (int)(16 / sizeof(typename TapT<WPROJ>::type));
-  return (W + J - 1 + E - 1) / E * E;
-}
-
-// Bytes before the tap arrays, rounded up to 16: computed in place, V staged records, their
-// normalisation state (partial sums, grid group) and the V + 1 run starts of the chunk; from
-// precomputed records, two buffers of V GridRecs (one filled while the other is gridded) and the
-// run starts.  A launch reserves the larger, so each work item may take either form.
+// Merged values are stored as 16-byte vectors [group][NC / N][column], so that a warp's columns read
+// consecutive 16-byte words (no bank conflicts).
 template <int NC>
-__host__ __device__ inline size_t stage_head_per_vis() {
-  const size_t own = sizeof(VisRec<NC>) + sizeof(NormAcc) * NC + 2 * sizeof(int);
-  const size_t pre = 2 * sizeof(GridRec<NC>) + sizeof(int);
-  return own > pre ? own : pre;
-}
+struct MergeVec {
+  static constexpr int N = NC * sizeof(cplx) >= 16 ? (int)(16 / sizeof(cplx)) : NC;
+  static constexpr int H = NC / N;
+  struct __align__(N * sizeof(cplx)) type {
+    cplx v[N];
+  };
+};
+
+// Bytes before the merged values, rounded up to 16: computed in place, V staged records and their
+// normalisation state (partial sums, grid group); from precomputed records, two buffers of V GridRecs
+// (one filled while the other is gridded).  A launch reserves the larger, so each work item may take
+// either form.
 template <int NC>
 __host__ __device__ inline size_t stage_head_bytes(int V) {
-  return (stage_head_per_vis<NC>() * (size_t)V + sizeof(int) + 15) / 16 * 16;
+  const size_t own = sizeof(VisRec<NC>) + sizeof(NormAcc) * NC + sizeof(int);
+  const size_t pre = 2 * sizeof(GridRec<NC>);
+  return ((own > pre ? own : pre) * (size_t)V + 15) / 16 * 16;
 }
-
+// Merged values and the second axis' tap row (W + J - 1 taps: the first J - 1 repeated after the last,
+// so a thread's J consecutive owned rows read J consecutive taps without a wrap) of one group.
 template <int NC, bool WPROJ>
-__host__ __device__ inline size_t grid_smem_bytes(int V, int W, int nthreads, int J) {
-  size_t taps = sizeof(typename TapT<WPROJ>::type) * (size_t)V * (tap_row_u<WPROJ>(W) + tap_row_v<WPROJ>(W, J));
-  return stage_head_bytes<NC>(V) + taps + flush_queue_bytes<NC>((nthreads + 31) / 32) + 64;
+__host__ __device__ inline size_t merge_group_bytes(int W, int J) {
+  return sizeof(cplx) * NC * (size_t)W + sizeof(typename TapT<WPROJ>::type) * (size_t)(W + J - 1);
 }
+// One group list per warp.
+__host__ __device__ inline size_t group_list_bytes(int nwarps) { return (size_t)nwarps * kMaxChunk * sizeof(unsigned short); }
 
-// Staged-chunk size V for a CTA of nthreads: one visibility per thread at most, and shared memory
-// small enough that the CTAs the register file allows (regs registers per thread) fit on an SM.
+// Staged records V, groups per batch GB and dynamic shared memory of a launch.
+struct ChunkShape {
+  int V, GB;
+  size_t smem;
+};
+
+// The chunk shape for CTAs of nthreads with regs registers per thread: as many CTAs per SM as the
+// register file allows, with about 28 KB of the SM left to L1 for the kernel table, fewer when a batch
+// of six groups does not fit.  64 records per chunk where they take at most half of the CTA's share (a
+// chunk's end also ends a group), 32 otherwise.
 template <int NC, bool WPROJ>
-__host__ inline int grid_chunk_size(int W, int nthreads, int J, int regs = 128) {
-  const int ctas = std::max(1, std::min(8, 65536 / (nthreads * regs)));
-  const size_t smem_sm = 227 * 1024;
-  size_t budget = std::min<size_t>(200 * 1024, smem_sm / ctas - 1024);
-  const size_t fixed = flush_queue_bytes<NC>((nthreads + 31) / 32) + 64 + sizeof(int) + 15;
-  budget = budget > fixed ? budget - fixed : 0;
-  const size_t per = stage_head_per_vis<NC>() +
-                     sizeof(typename TapT<WPROJ>::type) * (size_t)(tap_row_u<WPROJ>(W) + tap_row_v<WPROJ>(W, J));
-  return std::max(1, (int)std::min<size_t>(nthreads, budget / per));
+__host__ inline ChunkShape chunk_shape(int W, int nthreads, int J, int regs = 128) {
+  const int nwarps = (nthreads + 31) / 32;
+  const size_t fixed = flush_queue_bytes<NC>(nwarps) + group_list_bytes(nwarps) + 64;
+  const size_t per = merge_group_bytes<NC, WPROJ>(W, J);
+  ChunkShape s{32, 1, 0};
+  for (int ctas = std::max(1, std::min(24, 65536 / (nthreads * regs)));; --ctas) {
+    const size_t budget = std::min<size_t>(200 * 1024, (size_t)(227 - 28) * 1024 / ctas - 1024);
+    for (int V : {64, 32}) {
+      const size_t head = stage_head_bytes<NC>(V) + fixed;
+      if (V > 32 && 2 * head > budget) continue;
+      const int gb = budget > head ? (int)std::min<size_t>((size_t)V, (budget - head) / per) : 0;
+      if (gb >= 6 || ctas == 1) {
+        s.V = V;
+        s.GB = std::max(1, gb);
+        s.smem = head + per * s.GB;
+        return s;
+      }
+    }
+  }
 }
 
 // premultiplied visibility times the column tap
-__device__ __forceinline__ cplx premul(cplx v, acc_real t) {
-  cplx r;
-  r.re = v.re * t;
-  r.im = v.im * t;
-  return r;
-}
-__device__ __forceinline__ cplx premul(cplx v, cplx t) { return cmul(v, t); }
 __device__ __forceinline__ void mac(cplx &acc, cplx a, acc_real t) {
   acc.re = fma(a.re, t, acc.re);
   acc.im = fma(a.im, t, acc.im);
@@ -1120,14 +1154,29 @@ __device__ __forceinline__ void owner_map(int tid, int W, int J, int &du, int &s
 }
 
 // Register state of a Romein owner thread: the accumulators of its J cells and the footprint they
-// belong to.  For the last footprint corner (pu0, pv0) the owned cells are
-// (pu0 + ou, pv0 + wrap(ov0 + j)), wrap(i) = i - W when i >= W.
+// belong to.  For the last footprint corner (pa0, pb0) the owned cells are
+// (pa0 + oa, pb0 + wrap(ob0 + j)), wrap(i) = i - W when i >= W.
 template <int NC, int J>
 struct OwnerState {
   cplx acc[J][NC];
   unsigned dirty;
-  int cg, pu0, pv0, ou, ov0;
+  int cg, pa0, pb0, oa, ob0;
 };
+
+template <int NC, int J>
+__device__ __forceinline__ void owner_reset(OwnerState<NC, J> &st) {
+#pragma unroll
+  for (int j = 0; j < J; ++j) {
+#pragma unroll
+    for (int k = 0; k < NC; ++k) { st.acc[j][k].re = 0; st.acc[j][k].im = 0; }
+  }
+  st.dirty = 0;
+  st.cg = -1;
+  st.pa0 = -1;
+  st.pb0 = -1;
+  st.oa = 0;
+  st.ob0 = 0;
+}
 
 // Prologue of one staging slot: the visibility of `row` staged into recs[slot].
 template <int NC, bool WPROJ>
@@ -1140,8 +1189,6 @@ __device__ __forceinline__ void stage_slot(const GridArgs &a, int f_local, int c
 
 // Normalisation term of a staged visibility from the precomputed kernel row sums, added to its
 // slot's running sums (which go to the global normalisation when the slot's grid group changes).
-// Runs after the chunk's records are published, so its table loads overlap the tap copies instead
-// of lengthening the prologue.
 template <int NC>
 __device__ __forceinline__ void norm_slot(const GridArgs &a, const VisRec<NC> &rec, int slot, NormAcc *s_nacc,
                                           int *s_ng, long long fslice) {
@@ -1164,94 +1211,46 @@ __device__ __forceinline__ void norm_slot(const GridArgs &a, const VisRec<NC> &r
   for (int k = 0; k < NC; ++k) norm_add(na[k], (NormTerm)rec.cw[k] * nt);
 }
 
-// Runs of a staged chunk, found by one warp: maximal stretches of valid staged visibilities with
-// one footprint corner and grid group (a Romein thread keeps its cells across a run); an invalid
-// slot is a run of its own.  runs[0..n) are the first slots of the runs, runs[n] = nv.
-template <class Rec>
-__device__ __forceinline__ void find_runs(const Rec *recs, int nv, int *runs, int *nruns) {
-  const int lane = threadIdx.x & 31;
-  int count = 0;
-  for (int b = 0; b < nv; b += 32) {
-    const int t = b + lane;
-    bool start = false;
-    if (t < nv) {
-      const int4 c0 = *reinterpret_cast<const int4 *>(&recs[t].u0);
-      const int4 c1 = *reinterpret_cast<const int4 *>(&recs[t].g);
-      start = !c1.y || t == 0;
-      if (!start) {
-        const int4 p0 = *reinterpret_cast<const int4 *>(&recs[t - 1].u0);
-        const int4 p1 = *reinterpret_cast<const int4 *>(&recs[t - 1].g);
-        start = !p1.y || p0.x != c0.x || p0.y != c0.y || p1.x != c1.x;
-      }
-    }
-    const unsigned m = __ballot_sync(0xffffffffu, start);
-    if (start) runs[count + __popc(m & ((1u << lane) - 1u))] = t;
-    count += __popc(m);
+// The kernel table that a staged record's fu and fv index: the support-window table or the table
+// regrouped by tap offset (taps of a row adjacent), or the ABI's own (taps os elements apart).  The
+// table is read one tap per lane, a row's taps by consecutive lanes.  A caller-owned ABI table may
+// start at any element part: it is read in parts then.
+template <bool WPROJ>
+struct TapTable {
+  const void *p;
+  int step;
+  bool whole;
+};
+template <bool WPROJ>
+__device__ __forceinline__ TapTable<WPROJ> tap_table(const GridArgs &a) {
+  TapTable<WPROJ> t;
+  t.p = a.conv_w ? a.conv_w : a.conv_t ? a.conv_t : a.conv;
+  t.step = a.conv_w || a.conv_t ? 1 : a.os;
+  t.whole = (reinterpret_cast<uintptr_t>(t.p) & (sizeof(typename TapT<WPROJ>::type) - 1)) == 0;
+  return t;
+}
+__device__ __forceinline__ acc_real read_tap(const TapTable<false> &t, int first, int j) {
+  return __ldg(reinterpret_cast<const acc_real *>(t.p) + first + j * t.step);
+}
+__device__ __forceinline__ cplx read_tap(const TapTable<true> &t, int first, int j) {
+  const int at = first + j * t.step;
+  cplx r;
+  if (t.whole) {
+#if defined(BULLSEYE_SINGLE)
+    const float2 v = __ldg(reinterpret_cast<const float2 *>(t.p) + at);
+#else
+    const double2 v = __ldg(reinterpret_cast<const double2 *>(t.p) + at);
+#endif
+    r.re = v.x;
+    r.im = v.y;
+  } else {
+    r.re = __ldg(reinterpret_cast<const acc_real *>(t.p) + 2 * (long long)at);
+    r.im = __ldg(reinterpret_cast<const acc_real *>(t.p) + 2 * (long long)at + 1);
   }
-  if (lane == 0) {
-    runs[count] = nv;
-    *nruns = count;
-  }
+  return r;
 }
 
-// Asynchronous global -> shared copy of one tap (cp.async: no register staging, so a thread has its
-// whole share of a chunk's taps in flight at once).  Kernel tables are stored in the working
-// precision, so a tap is copied as it is (4, 8 or 16 bytes, aligned to its size).
-template <int BYTES>
-__device__ __forceinline__ void copy_tap_async(void *dst_smem, const void *src) {
-  static_assert(BYTES == 4 || BYTES == 8 || BYTES == 16, "cp.async copies 4, 8 or 16 bytes");
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst_smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(d), "l"(src), "n"(BYTES) : "memory");
-}
-// Waits for this thread's outstanding tap copies; a CTA barrier then publishes them.
-__device__ __forceinline__ void wait_taps() { asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory"); }
-
-// Taps of every valid staged visibility: W column taps, then W + J - 1 row taps, issued as
-// asynchronous copies (the caller runs wait_taps() before the barrier that publishes them).  Thread
-// tid walks (visibility, tap) pairs with a stride of blockDim.x pairs, stepped without division.
-// Rows are stored with strides TUS and TVS (padded to 16 bytes).
-template <int NC, bool WPROJ>
-__device__ __forceinline__ void stage_taps(const GridArgs &a, const VisRec<NC> *recs, int nv, int J, int TUS, int TVS,
-                                           typename TapT<WPROJ>::type *tu, typename TapT<WPROJ>::type *tv) {
-  typedef typename TapT<WPROJ>::type tap_t;
-  typedef typename std::conditional<WPROJ, vis_complex, vis_real>::type stored_t;
-  static_assert(sizeof(stored_t) == sizeof(tap_t), "kernel tables are stored in the working precision");
-  const stored_t *table = reinterpret_cast<const stored_t *>(a.conv_t ? a.conv_t : a.conv);
-  // a caller-owned table (the allocation-free entries) may be only element-part aligned: such a
-  // table is read through registers
-  const bool aligned = (reinterpret_cast<uintptr_t>(table) & (sizeof(tap_t) - 1)) == 0;
-  const int W = a.W;
-  const int per = 2 * W + J - 1;
-  const int tid = threadIdx.x;
-  int vi = tid / per, j = tid - vi * per;
-  const int svi = (int)blockDim.x / per, sj = (int)blockDim.x - svi * per;
-  while (vi < nv) {
-    const int4 h1 = *reinterpret_cast<const int4 *>(&recs[vi].g);  // g, valid, fu, fv
-    if (h1.y) {
-      const bool isv = j >= W;
-      const int js = isv ? j - W : j;  // slot in the staged row
-      int jj = js >= W ? js - W : js;  // repeated leading row taps
-      if (jj >= W) jj = W - 1;
-      const long long idx = a.conv_t ? (long long)(isv ? h1.w : h1.z) + jj
-                                     : (long long)recs[vi].plane * a.K + (isv ? h1.w : h1.z) + (long long)jj * a.os;
-      tap_t *dst = isv ? &tv[vi * TVS + js] : &tu[vi * TUS + js];
-      if (aligned) {
-        copy_tap_async<sizeof(tap_t)>(dst, table + idx);
-      } else {
-        load_tap(table, idx, *dst);
-      }
-    }
-    vi += svi;
-    j += sj;
-    if (j >= per) {
-      j -= per;
-      ++vi;
-    }
-  }
-}
-
-// Tap-copy barrier (mbarrier) of the bulk-copy staging: V arrivals per chunk, one per staging
-// slot, each announcing the bytes of its two row copies.  Waits are bounded.
+// Tap-copy barriers of the record staging.  Waits are bounded.
 __device__ __forceinline__ unsigned smem_addr(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void bar_init(unsigned long long *bar, unsigned count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_addr(bar)), "r"(count) : "memory");
@@ -1296,53 +1295,30 @@ __device__ __forceinline__ void bulk_copy(void *dst, const void *src, unsigned b
                : "memory");
 }
 
-// Bulk-copy staging of a chunk's taps from the support-window table: staging slot tid copies its
-// visibility's column row (TUS taps) and row row (TVS taps, the repeated leading taps included) as
-// two bulk copies and arrives on the barrier with their bytes; an empty slot arrives without bytes.
-template <int NC, bool WPROJ, class Rec>
-__device__ __forceinline__ void stage_taps_bulk(const GridArgs &a, const Rec *recs, int nv, int TUS, int TVS,
-                                                typename TapT<WPROJ>::type *tu, typename TapT<WPROJ>::type *tv,
-                                                unsigned long long *bar) {
-  typedef typename TapT<WPROJ>::type tap_t;
-  const int tid = threadIdx.x;
-  if (tid >= a.V) return;
-  const int4 h1 = *reinterpret_cast<const int4 *>(&recs[tid].g);  // g, valid, fu, fv
-  if (tid < nv && h1.y) {
-    const tap_t *table = reinterpret_cast<const tap_t *>(a.conv_w);
-    const unsigned bu = (unsigned)(sizeof(tap_t) * TUS), bv = (unsigned)(sizeof(tap_t) * TVS);
-    bar_arrive_tx(bar, bu + bv);
-    bulk_copy(tu + tid * TUS, table + h1.z, bu, bar);
-    bulk_copy(tv + tid * TVS, table + h1.w, bv, bar);
-  } else {
-    bar_arrive(bar);
-  }
-}
-
-// Normalisation without precomputed row sums (the allocation-free entry), four lanes per staged
+// Normalisation without precomputed row sums (the allocation-free entries), four lanes per staged
 // visibility: Re(sum_u k_u * sum_v k_v) x weight x flag (loop bounds are warp-uniform so the
 // shuffles always see full warps); lane 4i owns the running sums of staged slot i.
 template <int NC, bool WPROJ>
-__device__ __forceinline__ void norm_from_taps(const GridArgs &a, const VisRec<NC> *recs, int nv, int TUS, int TVS,
-                                               const typename TapT<WPROJ>::type *tu,
-                                               const typename TapT<WPROJ>::type *tv, NormAcc *s_nacc, int *s_ng,
+__device__ __forceinline__ void norm_from_taps(const GridArgs &a, const VisRec<NC> *recs, int nv,
+                                               const TapTable<WPROJ> &table, NormAcc *s_nacc, int *s_ng,
                                                long long fslice) {
   const int W = a.W;
   const int tid = threadIdx.x;
   for (int b4 = tid & ~31; b4 < 4 * nv; b4 += blockDim.x) {
     const int q = b4 + (tid & 31);
     const int vi = q >> 2, part = q & 3;
-    const bool act = vi < nv;
+    const bool act = vi < nv && recs[vi].valid;
     // tap sums in the library's working precision (FP64 units are scarce on this GPU)
     acc_real sur = 0, sui = 0, svr = 0, svi = 0;
     if (act) {
-      if (WPROJ) {
-        const cplx *pu = reinterpret_cast<const cplx *>(tu) + vi * TUS;
-        const cplx *pv = reinterpret_cast<const cplx *>(tv) + vi * TVS;
-        for (int j = part; j < W; j += 4) { sur += pu[j].re; sui += pu[j].im; svr += pv[j].re; svi += pv[j].im; }
-      } else {
-        const acc_real *pu = reinterpret_cast<const acc_real *>(tu) + vi * TUS;
-        const acc_real *pv = reinterpret_cast<const acc_real *>(tv) + vi * TVS;
-        for (int j = part; j < W; j += 4) { sur += pu[j]; svr += pv[j]; }
+      const int fu = recs[vi].fu, fv = recs[vi].fv;
+      for (int j = part; j < W; j += 4) {
+        const typename TapT<WPROJ>::type u = read_tap(table, fu, j), v = read_tap(table, fv, j);
+        if constexpr (WPROJ) {
+          sur += u.re; sui += u.im; svr += v.re; svi += v.im;
+        } else {
+          sur += u; svr += v;
+        }
       }
     }
 #pragma unroll
@@ -1352,7 +1328,7 @@ __device__ __forceinline__ void norm_from_taps(const GridArgs &a, const VisRec<N
       svr += __shfl_xor_sync(0xffffffffu, svr, off);
       svi += __shfl_xor_sync(0xffffffffu, svi, off);
     }
-    if (act && part == 0 && recs[vi].valid) {
+    if (act && part == 0) {
       const VisRec<NC> &r = recs[vi];
       const NormTerm nt = (NormTerm)sur * (NormTerm)svr - (NormTerm)sui * (NormTerm)svi;
       NormAcc *na = s_nacc + vi * NC;
@@ -1372,211 +1348,333 @@ __device__ __forceinline__ void norm_from_taps(const GridArgs &a, const VisRec<N
   }
 }
 
-// Multiply-adds of a staged chunk's runs into an owner thread's cells.  When the footprint moves,
-// the owned cells are recomputed and those that changed are flushed (queued for the warp's
-// compensated flush in single precision; the queue is drained when it fills and at the end of the
-// track).  Every lane of a warp with any owned cell calls this, so the queue drains are
-// warp-uniform.
-template <int NC, bool WPROJ, int J, bool COMP, class Rec>
-__device__ __forceinline__ void grid_runs(const GridArgs &a, const Rec *recs,
-                                          const typename TapT<WPROJ>::type *tu,
-                                          const typename TapT<WPROJ>::type *tv, const int *runs, int nruns,
-                                          int TUS, int TVS, int du, int strip, unsigned rows_mask, long long fbase,
-                                          long long nxy, int gnx, FlushRec<NC> *fq, int *fqn,
-                                          OwnerState<NC, J> &st) {
+// Group starts among slots [32 b, 32 b + 32) of a chunk, merging along u (a group shares its v tap row)
+// and along v, the first slots of runs (one footprint corner and grid group) and the valid slots, as
+// warp masks (whole-warp call).
+struct SlotMasks {
+  unsigned valid, run, along_u, along_v;
+};
+template <class Rec>
+__device__ __forceinline__ SlotMasks slot_masks(const Rec *recs, int nv, int b) {
+  const int t = b * 32 + (threadIdx.x & 31);
+  bool valid = false, run = false, au = false, av = false;
+  if (t < nv) {
+    const int4 c0 = *reinterpret_cast<const int4 *>(&recs[t].u0);
+    const int4 c1 = *reinterpret_cast<const int4 *>(&recs[t].g);
+    valid = c1.y != 0;
+    run = valid;
+    if (valid && t > 0) {
+      const int4 p0 = *reinterpret_cast<const int4 *>(&recs[t - 1].u0);
+      const int4 p1 = *reinterpret_cast<const int4 *>(&recs[t - 1].g);
+      run = !p1.y || p0.x != c0.x || p0.y != c0.y || p1.x != c1.x;
+      au = p1.w != c1.w;
+      av = p1.z != c1.z;
+    }
+    au = valid && (au || run);
+    av = valid && (av || run);
+  }
+  SlotMasks m;
+  m.valid = __ballot_sync(0xffffffffu, valid);
+  m.run = __ballot_sync(0xffffffffu, run);
+  m.along_u = __ballot_sync(0xffffffffu, au);
+  m.along_v = __ballot_sync(0xffffffffu, av);
+  return m;
+}
+
+// A group list entry: first slot (7 bits), visibilities (7 bits), whether a run starts there.
+constexpr int kGroupRun = 1 << 14;
+
+// The groups of a staged chunk, written by every warp into its own list (whole-warp call; all warps
+// find the same groups).  `pick` first decides the merge axis of the item from this chunk: along v
+// when that leaves fewer groups.
+template <class Rec>
+__device__ __forceinline__ int find_groups(const Rec *recs, int nv, bool pick, bool &swap, unsigned short *list) {
+  typedef unsigned long long u64;
+  const SlotMasks m0 = slot_masks(recs, nv, 0);
+  SlotMasks m1{0, 0, 0, 0};
+  if (nv > 32) m1 = slot_masks(recs, nv, 1);
+  if (pick) swap = __popc(m0.along_v) + __popc(m1.along_v) < __popc(m0.along_u) + __popc(m1.along_u);
+  const u64 start = swap ? (u64)m1.along_v << 32 | m0.along_v : (u64)m1.along_u << 32 | m0.along_u;
+  const u64 run = (u64)m1.run << 32 | m0.run;
+  const u64 edge = start | ~((u64)m1.valid << 32 | m0.valid);  // slots that do not continue a group
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int t = lane + 32 * h;
+    if (start >> t & 1) {
+      const u64 rest = t < 63 ? edge >> (t + 1) : 0;
+      const int len = rest ? __ffsll(rest) : 64 - t;
+      list[__popcll(start & ((1ull << t) - 1))] = (unsigned short)(t | len << 7 | ((run >> t & 1) ? kGroupRun : 0));
+    }
+  }
+  __syncwarp();
+  return __popcll(start);
+}
+
+// T(a) and the kb row of groups [g0, g1) of a chunk: thread (column a = ax, part ap of nparts).
+template <int NC, bool WPROJ, class Rec>
+__device__ __forceinline__ void merge_groups(const TapTable<WPROJ> &table, const Rec *recs, const unsigned short *list,
+                                             int g0, int g1, bool swap, int W, int J, int ax, int ap, int nparts,
+                                             typename MergeVec<NC>::type *T, typename TapT<WPROJ>::type *tb) {
   typedef typename TapT<WPROJ>::type tap_t;
-  const int W = a.W;
-  for (int ri = 0; ri < nruns; ++ri) {
-    const int rs = runs[ri], re = runs[ri + 1];
-    const int4 h0 = *reinterpret_cast<const int4 *>(&recs[rs].u0);
-    const int4 h1 = *reinterpret_cast<const int4 *>(&recs[rs].g);
-    if (!h1.y) continue;
-    if (h0.x != st.pu0 || h0.y != st.pv0 || h1.x != st.cg) {
-      // footprint moved: recompute the owned cells, flush those that changed
-      int o = du - h0.z;
-      o += (o < 0) ? W : 0;
-      int nov0 = strip * J - h0.w;
-      nov0 += (nov0 < 0) ? W : 0;
-      if (h0.x + o != st.pu0 + st.ou || h1.x != st.cg) {
-        if (st.dirty) {
+  typedef MergeVec<NC> M;
+  if (ap >= nparts) return;
+  const int TBS = W + J - 1;
+  for (int gi = g0 + ap; gi < g1; gi += nparts) {
+    const int e = list[gi], s = e & 127, end = s + ((e >> 7) & 127);
+    const tap_t kb = read_tap(table, swap ? recs[s].fu : recs[s].fv, ax);
+    cplx t[NC];
 #pragma unroll
-          for (int j = 0; j < J; ++j)
-            if (st.dirty & (1u << j)) {
-              const int oy = st.ov0 + j >= W ? st.ov0 + j - W : st.ov0 + j;
-              if (COMP)
-                queue_cell<NC>(a, fbase + (long long)st.cg * NC * nxy, nxy, gnx, st.pu0 + st.ou, st.pv0 + oy,
-                               st.acc[j], fq, fqn);
-              else
-                flush_cell<NC, false>(a, fbase + (long long)st.cg * NC * nxy, nxy, gnx, st.pu0 + st.ou,
-                                      st.pv0 + oy, st.acc[j]);
-            }
-          st.dirty = 0;
-        }
-        st.cg = h1.x;
+    for (int k = 0; k < NC; ++k) { t[k].re = 0; t[k].im = 0; }
+    // four table loads in flight (past the end: the last one again)
+    for (int v = s; v < end; v += 4) {
+      tap_t ka[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int i = min(v + q, end - 1);
+        ka[q] = read_tap(table, swap ? recs[i].fv : recs[i].fu, ax);
       }
-      if (st.dirty) {
 #pragma unroll
-        for (int j = 0; j < J; ++j) {
-          const int oy = st.ov0 + j >= W ? st.ov0 + j - W : st.ov0 + j;
-          const int ny = nov0 + j >= W ? nov0 + j - W : nov0 + j;
-          if ((st.dirty & (1u << j)) && h0.y + ny != st.pv0 + oy) {
-            if (COMP)
-              queue_cell<NC>(a, fbase + (long long)st.cg * NC * nxy, nxy, gnx, st.pu0 + st.ou, st.pv0 + oy,
-                             st.acc[j], fq, fqn);
-            else
-              flush_cell<NC, false>(a, fbase + (long long)st.cg * NC * nxy, nxy, gnx, st.pu0 + st.ou, st.pv0 + oy,
-                                    st.acc[j]);
-            st.dirty &= ~(1u << j);
+      for (int q = 0; q < 4; ++q)
+        if (v + q < end) {
+          const typename M::type *x = reinterpret_cast<const typename M::type *>(recs[v + q].vis);
+#pragma unroll
+          for (int h = 0; h < M::H; ++h) {
+            const typename M::type y = x[h];
+#pragma unroll
+            for (int n = 0; n < M::N; ++n) mac(t[h * M::N + n], y.v[n], ka[q]);
           }
         }
-      }
-      // columns beyond W (padding lanes) read in-bounds taps and are never flushed
-      st.ou = o < W ? o : W - 1;
-      st.ov0 = nov0 < W ? nov0 : 0;  // lanes past the last strip own nothing: keep their reads in bounds
-      st.pu0 = h0.x;
-      st.pv0 = h0.y;
-      if (COMP) {  // the queue only grows here; the branch is uniform over the warp
-        __syncwarp();
-        if (*fqn >= kDrainAt) drain_queue<NC>(a, nxy, fq, fqn);
-      }
     }
-    // the run's visibilities share the owned cells: a branch-free multiply-add loop over the J
-    // owned rows (offsets modulo W; rows of non-owning lanes stay in bounds and are never flushed)
-#pragma unroll 2
-    for (int vi = rs; vi < re; ++vi) {
-      const tap_t tuv = tu[vi * TUS + st.ou];
-      cplx pre[NC];
 #pragma unroll
-      for (int k = 0; k < NC; ++k) pre[k] = premul(recs[vi].vis[k], tuv);
-      const tap_t *tvrow = tv + vi * TVS + st.ov0;
+    for (int h = 0; h < M::H; ++h) {
+      typename M::type y;
 #pragma unroll
-      for (int j = 0; j < J; ++j) {
-        const tap_t t = tvrow[j];
-#pragma unroll
-        for (int k = 0; k < NC; ++k) mac(st.acc[j][k], pre[k], t);
-      }
+      for (int n = 0; n < M::N; ++n) y.v[n] = t[h * M::N + n];
+      T[((gi - g0) * M::H + h) * W + ax] = y;
     }
-    st.dirty = rows_mask;
+    tap_t *row = tb + (gi - g0) * TBS;
+    row[ax] = kb;
+    for (int j = ax; j < J - 1; j += W) row[W + j] = kb;  // once: J - 1 < W, or the row's own wrap
   }
 }
 
-// One track (facet, channel, rows [r0, r1)) of one CTA: the rows are staged V at a time (prologue,
-// runs, taps) and gridded by the Romein owner threads.  With a tap-copy barrier (`bar`, whose
-// phase parity `phase` carries over from track to track) and the support-window table, a staged
-// visibility's tap rows are two bulk copies; otherwise per-tap asynchronous copies.
+// Multiply-adds of groups [g0, g1) of a chunk into an owner thread's cells.  When the footprint moves,
+// the owned cells are recomputed and those that changed are flushed (queued for the warp's
+// compensated flush in single precision; the queue is drained when it fills and at the end of the
+// track).  Every lane of a warp with any owned cell calls this, so the queue drains are
+// warp-uniform.  Cells lie sa (along a) and sb (along b) elements apart.
+template <int NC, bool WPROJ, int J, bool COMP, class Rec>
+__device__ __forceinline__ void grid_groups(const GridArgs &a, const Rec *recs, const unsigned short *list, int g0, int g1,
+                                            bool swap, const typename MergeVec<NC>::type *T,
+                                            const typename TapT<WPROJ>::type *tb, int du, int strip, unsigned rows_mask,
+                                            long long fbase, long long nxy, int sa, int sb, FlushRec<NC> *fq, int *fqn,
+                                            OwnerState<NC, J> &st) {
+  typedef typename TapT<WPROJ>::type tap_t;
+  typedef MergeVec<NC> M;
+  const int W = a.W, TBS = W + J - 1;
+  for (int gi = g0; gi < g1; ++gi) {
+    const int e = list[gi];
+    if (e & kGroupRun) {
+      const int rs = e & 127;
+      const int4 hr = *reinterpret_cast<const int4 *>(&recs[rs].u0);
+      const int g = recs[rs].g;
+      // corner and residues along (a, b)
+      const int a0 = swap ? hr.y : hr.x, b0 = swap ? hr.x : hr.y, ra = swap ? hr.w : hr.z, rb = swap ? hr.z : hr.w;
+      if (a0 != st.pa0 || b0 != st.pb0 || g != st.cg) {
+        // footprint moved: recompute the owned cells, flush those that changed
+        int o = du - ra;
+        o += (o < 0) ? W : 0;
+        int nob0 = strip * J - rb;
+        nob0 += (nob0 < 0) ? W : 0;
+        if (st.dirty) {
+          const bool all = a0 + o != st.pa0 + st.oa || g != st.cg;
+          const long long slice = fbase + (long long)st.cg * NC * nxy + (long long)(st.pa0 + st.oa) * sa;
+#pragma unroll
+          for (int j = 0; j < J; ++j) {
+            const int ob = st.ob0 + j >= W ? st.ob0 + j - W : st.ob0 + j;
+            const int nb = nob0 + j >= W ? nob0 + j - W : nob0 + j;
+            if ((st.dirty & (1u << j)) && (all || b0 + nb != st.pb0 + ob)) {
+              const long long cell = slice + (long long)(st.pb0 + ob) * sb;
+              if (COMP)
+                queue_cell<NC>(a, cell, nxy, st.acc[j], fq, fqn);
+              else
+                flush_cell<NC, false>(a, cell, nxy, st.acc[j]);
+              st.dirty &= ~(1u << j);
+            }
+          }
+        }
+        st.cg = g;
+        // columns beyond W (padding lanes) read in-bounds values and are never flushed
+        st.oa = o < W ? o : W - 1;
+        st.ob0 = nob0 < W ? nob0 : 0;  // lanes past the last strip own nothing: keep their reads in bounds
+        st.pa0 = a0;
+        st.pb0 = b0;
+        if (COMP) {  // the queue only grows here; the branch is uniform over the warp
+          __syncwarp();
+          if (*fqn >= kDrainAt) drain_queue<NC>(a, nxy, fq, fqn);
+        }
+      }
+    }
+    // branch-free multiply-adds over the J owned rows (offsets modulo W; rows of non-owning lanes stay
+    // in bounds and are never flushed)
+    cplx t[NC];
+#pragma unroll
+    for (int h = 0; h < M::H; ++h) {
+      const typename M::type y = T[((gi - g0) * M::H + h) * W + st.oa];
+#pragma unroll
+      for (int n = 0; n < M::N; ++n) t[h * M::N + n] = y.v[n];
+    }
+    const tap_t *row = tb + (gi - g0) * TBS + st.ob0;
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+      const tap_t k = row[j];
+#pragma unroll
+      for (int c = 0; c < NC; ++c) mac(st.acc[j][c], t[c], k);
+    }
+    st.dirty |= rows_mask;
+  }
+}
+
+// What a CTA keeps for one work item: its shared-memory pieces, owner mapping and facet geometry.
+template <int NC, bool WPROJ>
+struct ItemSetup {
+  typename MergeVec<NC>::type *T;        // [GB][H][W]
+  typename TapT<WPROJ>::type *tb;        // [GB][W + J - 1]
+  unsigned short *list;                  // this warp's group list
+  FlushRec<NC> *fq;                      // this warp's flush queue
+  int *fqn;
+  TapTable<WPROJ> table;
+  int du, strip, ax, ap, nparts, gnx;
+  unsigned rows_mask;
+  bool grids;
+  long long nxy, fbase;
+};
+template <int NC, bool WPROJ, int J, bool COMP, bool WIDE>
+__device__ __forceinline__ void item_setup(const GridArgs &a, int f_local, unsigned char *smem, ItemSetup<NC, WPROJ> &s) {
+  typedef typename MergeVec<NC>::type vec_t;
+  typedef typename TapT<WPROJ>::type tap_t;
+  const int W = a.W, GB = a.GB, tid = threadIdx.x;
+  const int warp_id = tid >> 5, nwarps = (blockDim.x + 31) >> 5;
+  unsigned char *p = smem + stage_head_bytes<NC>(a.V);
+  s.T = reinterpret_cast<vec_t *>(p);
+  p += sizeof(cplx) * NC * (size_t)W * GB;
+  s.tb = reinterpret_cast<tap_t *>(p);
+  p += sizeof(tap_t) * (size_t)(W + J - 1) * GB;
+  p = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(p) + 15) & ~(uintptr_t)15);
+  s.list = reinterpret_cast<unsigned short *>(p) + warp_id * kMaxChunk;
+  p += group_list_bytes(nwarps);
+  s.fq = reinterpret_cast<FlushRec<NC> *>(p) + warp_id * kFlushQueueCap;
+  s.fqn = reinterpret_cast<int *>(p + nwarps * sizeof(FlushRec<NC>) * kFlushQueueCap) + warp_id * 4;
+  if (COMP && (tid & 31) == 0) *s.fqn = 0;
+  s.table = tap_table<WPROJ>(a);
+  bool owner;
+  owner_map<WIDE>(tid, W, J, s.du, s.strip, owner);
+  s.rows_mask = 0;
+#pragma unroll
+  for (int j = 0; j < J; ++j)
+    if (s.strip * J + j < W) s.rows_mask |= 1u << j;
+  if (!owner) s.rows_mask = 0;
+  s.grids = __any_sync(0xffffffffu, s.rows_mask != 0);
+  s.ap = tid / W;
+  s.ax = tid - s.ap * W;
+  s.nparts = (int)blockDim.x / W;
+  const FacetXform &fx = a.facets[f_local];
+  s.gnx = fx.nx;
+  s.nxy = (long long)fx.nx * fx.ny;
+  s.fbase = fx.grid_base;  // element offset of this facet's grid block
+}
+
+// The groups of one staged chunk (block-wide call; ends with the CTA's barrier, after which the
+// records may be overwritten).
+template <int NC, bool WPROJ, int J, bool COMP, class Rec>
+__device__ __forceinline__ void grid_chunk(const GridArgs &a, const Rec *recs, int nv, bool first, bool &swap,
+                                           const ItemSetup<NC, WPROJ> &s, OwnerState<NC, J> &st) {
+  const int ng = find_groups(recs, nv, first, swap, s.list);
+  const int sa = swap ? s.gnx : 1, sb = swap ? 1 : s.gnx;
+  for (int g0 = 0; g0 < ng; g0 += a.GB) {
+    const int g1 = min(ng, g0 + a.GB);
+    merge_groups<NC, WPROJ>(s.table, recs, s.list, g0, g1, swap, a.W, J, s.ax, s.ap, s.nparts, s.T, s.tb);
+    __syncthreads();
+    if (s.grids)
+      grid_groups<NC, WPROJ, J, COMP>(a, recs, s.list, g0, g1, swap, s.T, s.tb, s.du, s.strip, s.rows_mask, s.fbase, s.nxy,
+                                      sa, sb, s.fq, s.fqn, st);
+    __syncthreads();
+  }
+  if (ng == 0) __syncthreads();
+}
+
+// End of a work item: the flush queue is emptied, then the owned cells are flushed.
+template <int NC, bool WPROJ, int J, bool COMP>
+__device__ __forceinline__ void item_flush(const GridArgs &a, const ItemSetup<NC, WPROJ> &s, bool swap,
+                                           OwnerState<NC, J> &st) {
+  const int W = a.W, sa = swap ? s.gnx : 1, sb = swap ? 1 : s.gnx;
+  if (COMP && s.grids) drain_queue<NC>(a, s.nxy, s.fq, s.fqn);
+  if (st.dirty) {
+    const long long slice = s.fbase + (long long)st.cg * NC * s.nxy + (long long)(st.pa0 + st.oa) * sa;
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+      const int ob = st.ob0 + j >= W ? st.ob0 + j - W : st.ob0 + j;
+      if (st.dirty & (1u << j)) flush_cell<NC, COMP>(a, slice + (long long)(st.pb0 + ob) * sb, s.nxy, st.acc[j]);
+    }
+  }
+}
+
+// One track (facet, channel, rows [r0, r1)) of one CTA: the rows are staged V at a time (prologue) and
+// gridded chunk by chunk.
 template <int NC, bool WPROJ, int J, bool COMP, bool WIDE>
 __device__ __forceinline__ void grid_track(const GridArgs &a, const int f_local, const int chan, long long r0,
-                                           long long r1, unsigned long long *bar, unsigned &phase) {
-  typedef typename TapT<WPROJ>::type tap_t;
+                                           long long r1) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int V = a.V, W = a.W;
-  const int TUS = tap_row_u<WPROJ>(W), TVS = tap_row_v<WPROJ>(W, J);  // staged row strides
-  const bool bulk = bar != nullptr && a.conv_w != nullptr;
+  const int V = a.V;
   VisRec<NC> *recs = reinterpret_cast<VisRec<NC> *>(smem_raw);                          // [V]
   NormAcc *s_nacc = reinterpret_cast<NormAcc *>(smem_raw + sizeof(VisRec<NC>) * (size_t)V);  // [V][NC]
   int *s_ng = reinterpret_cast<int *>(s_nacc + (size_t)V * NC);                             // [V]
-  int *s_runs = s_ng + V;                                                                   // [V + 1]
-  tap_t *tu = reinterpret_cast<tap_t *>(smem_raw + stage_head_bytes<NC>(V));               // [V][TUS]
-  tap_t *tv = tu + V * TUS;                                                                 // [V][TVS]
-  // per-warp flush queues follow the taps
-  unsigned char *qbase = reinterpret_cast<unsigned char *>(tv + V * TVS);
-  qbase = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(qbase) + 15) & ~(uintptr_t)15);
-  const int warp_id = threadIdx.x >> 5, nwarps = (blockDim.x + 31) >> 5;
-  FlushRec<NC> *fq = reinterpret_cast<FlushRec<NC> *>(qbase) + warp_id * kFlushQueueCap;
-  int *fqn = reinterpret_cast<int *>(qbase + nwarps * sizeof(FlushRec<NC>) * kFlushQueueCap) + warp_id * 4;
-  if (COMP && (threadIdx.x & 31) == 0) *fqn = 0;
-  __shared__ int s_nruns;
-
-  const FacetXform &fxt = a.facets[f_local];
-  const int gnx = fxt.nx;
-  const long long nxy = (long long)fxt.nx * fxt.ny;
-  const long long fbase = fxt.grid_base;  // element offset of this facet's grid block
+  ItemSetup<NC, WPROJ> s;
+  item_setup<NC, WPROJ, J, COMP, WIDE>(a, f_local, smem_raw, s);
   if (r1 > a.nrows) r1 = a.nrows;
   if (r0 >= r1) return;
-
-  const int tid = threadIdx.x;
-  int du, strip;
-  bool owner;
-  owner_map<WIDE>(tid, W, J, du, strip, owner);
-  unsigned rows_mask = 0;
-#pragma unroll
-  for (int j = 0; j < J; ++j)
-    if (strip * J + j < W) rows_mask |= 1u << j;
-  if (!owner) rows_mask = 0;
-  const bool grids = __any_sync(0xffffffffu, rows_mask != 0);
+  const int tid = threadIdx.x, nt = blockDim.x;
   const long long fslice = (long long)(a.facet_base + f_local) * a.groups;
   const bool want_norm = a.norm != nullptr;
-  if (want_norm && tid < V) {
+  if (want_norm)
+    for (int i = tid; i < V; i += nt) {
 #pragma unroll
-    for (int k = 0; k < NC; ++k) norm_zero(s_nacc[tid * NC + k]);
-    s_ng[tid] = -1;
-  }
-
+      for (int k = 0; k < NC; ++k) norm_zero(s_nacc[i * NC + k]);
+      s_ng[i] = -1;
+    }
   OwnerState<NC, J> st;
-#pragma unroll
-  for (int j = 0; j < J; ++j) {
-#pragma unroll
-    for (int k = 0; k < NC; ++k) { st.acc[j][k].re = 0; st.acc[j][k].im = 0; }
-  }
-  st.dirty = 0;
-  st.cg = -1;
-  st.pu0 = -1;
-  st.pv0 = -1;
-  st.ou = 0;
-  st.ov0 = 0;
+  owner_reset(st);
   ChanCache cc;
   const double plane_scale = WPROJ ? (double)(a.P - 1) / a.wmax : 0.0;
-
+  bool swap = false;
   for (long long base = r0; base < r1; base += V) {
     const int nv = (int)min((long long)V, r1 - base);
-    if (tid < V) stage_slot<NC, WPROJ>(a, f_local, chan, base + tid, tid < nv, tid, recs, cc, plane_scale);
+    for (int i = tid; i < nv; i += nt) stage_slot<NC, WPROJ>(a, f_local, chan, base + i, true, i, recs, cc, plane_scale);
     __syncthreads();
-    if (bulk)
-      stage_taps_bulk<NC, WPROJ>(a, recs, nv, TUS, TVS, tu, tv, bar);
-    else
-      stage_taps<NC, WPROJ>(a, recs, nv, J, TUS, TVS, tu, tv);
-    if (warp_id == 0) find_runs(recs, nv, s_runs, &s_nruns);
-    if (want_norm && a.tap_sums && tid < nv) norm_slot<NC>(a, recs[tid], tid, s_nacc, s_ng, fslice);
-    if (bulk) {
-      // every thread observes the phase (the copies' data is visible to the threads that do);
-      // a wait that runs out is recorded, then waited for once more before the data is used
-      if (!bar_wait(bar, phase)) {
-        atomicOr(a.error, DEV_ERR_WAIT_TIMEOUT);
-        bar_wait(bar, phase);
+    if (want_norm) {
+      if (a.tap_sums) {
+        for (int i = tid; i < nv; i += nt) norm_slot<NC>(a, recs[i], i, s_nacc, s_ng, fslice);
+      } else {
+        norm_from_taps<NC, WPROJ>(a, recs, nv, s.table, s_nacc, s_ng, fslice);
       }
-      phase ^= 1u;
-    } else {
-      wait_taps();
     }
-    __syncthreads();
-    if (want_norm && !a.tap_sums) norm_from_taps<NC, WPROJ>(a, recs, nv, TUS, TVS, tu, tv, s_nacc, s_ng, fslice);
-    if (grids)
-      grid_runs<NC, WPROJ, J, COMP>(a, recs, tu, tv, s_runs, s_nruns, TUS, TVS, du, strip, rows_mask, fbase, nxy, gnx,
-                                    fq, fqn, st);
-    __syncthreads();
+    grid_chunk<NC, WPROJ, J, COMP>(a, recs, nv, base == r0, swap, s, st);
   }
-  // the flush queues carry over from chunk to chunk; empty them before the final flush
-  if (COMP && grids) drain_queue<NC>(a, nxy, fq, fqn);
-  // final flush of owned cells
-  if (st.dirty) {
-#pragma unroll
-    for (int j = 0; j < J; ++j) {
-      const int oy = st.ov0 + j >= W ? st.ov0 + j - W : st.ov0 + j;
-      if (st.dirty & (1u << j))
-        flush_cell<NC, COMP>(a, fbase + (long long)st.cg * NC * nxy, nxy, gnx, st.pu0 + st.ou, st.pv0 + oy, st.acc[j]);
-    }
-  }
+  item_flush<NC, WPROJ, J, COMP>(a, s, swap, st);
   // normalisation: the slots' current partial sums (earlier grid groups went out when the group
   // changed), summed over each warp by shuffles when its slots share one group (one atomic per
   // correlation and warp), added slot by slot otherwise.  The slots' state was last written before
   // the chunk loop's final barrier.
   if (want_norm) {
-    const bool has = tid < V && s_ng[tid] >= 0;
-    const int my_g = has ? s_ng[tid] : -1;
-    const unsigned m = __ballot_sync(0xffffffffu, has);
-    if (m) {
+    for (int b = tid & ~31; b < V; b += nt) {
+      const int i = b + (tid & 31);
+      const bool has = i < V && s_ng[i] >= 0;
+      const int my_g = has ? s_ng[i] : -1;
+      const unsigned m = __ballot_sync(0xffffffffu, has);
+      if (!m) continue;
       const int g0 = __shfl_sync(0xffffffffu, my_g, __ffs(m) - 1);
-      const NormAcc *na = s_nacc + (has ? tid : 0) * NC;
+      const NormAcc *na = s_nacc + (has ? i : 0) * NC;
       if (__all_sync(0xffffffffu, !has || my_g == g0)) {
 #pragma unroll
         for (int k = 0; k < NC; ++k) {
@@ -1596,60 +1694,17 @@ __device__ __forceinline__ void grid_track(const GridArgs &a, const int f_local,
 
 // One work item from precomputed records: its n records (src, 16-byte aligned) are staged V at a
 // time by one bulk copy each into two buffers used in turn, the next chunk's copy in flight while
-// the current chunk's taps arrive and its runs are gridded; the tap rows are bulk copies as in
-// grid_track.  No prologue and no normalisation here (the record kernel did both).  rbar are the
-// two record barriers (one arrival each), rphase their phase parities (bit b for buffer b); a
-// copy is only issued for a chunk of this item, so none is in flight when the item ends.
+// the current chunk is gridded.  No prologue and no normalisation here (the record kernel did both).
+// rbar are the two record barriers (one arrival each), rphase their phase parities (bit b for buffer
+// b); a copy is only issued for a chunk of this item, so none is in flight when the item ends.
 template <int NC, bool WPROJ, int J, bool COMP, bool WIDE>
 __device__ __forceinline__ void grid_track_pre(const GridArgs &a, const int f_local, const GridRec<NC> *src, int n,
-                                               unsigned long long *rbar, unsigned &rphase, unsigned long long *bar,
-                                               unsigned &phase) {
-  typedef typename TapT<WPROJ>::type tap_t;
+                                               unsigned long long *rbar, unsigned &rphase) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int V = a.V, W = a.W;
-  const int TUS = tap_row_u<WPROJ>(W), TVS = tap_row_v<WPROJ>(W, J);
+  const int V = a.V;
   GridRec<NC> *rb = reinterpret_cast<GridRec<NC> *>(smem_raw);  // [2][V]
-  int *s_runs = reinterpret_cast<int *>(rb + 2 * V);             // [V + 1]
-  tap_t *tu = reinterpret_cast<tap_t *>(smem_raw + stage_head_bytes<NC>(V));
-  tap_t *tv = tu + V * TUS;
-  unsigned char *qbase = reinterpret_cast<unsigned char *>(tv + V * TVS);
-  qbase = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(qbase) + 15) & ~(uintptr_t)15);
-  const int warp_id = threadIdx.x >> 5, nwarps = (blockDim.x + 31) >> 5;
-  FlushRec<NC> *fq = reinterpret_cast<FlushRec<NC> *>(qbase) + warp_id * kFlushQueueCap;
-  int *fqn = reinterpret_cast<int *>(qbase + nwarps * sizeof(FlushRec<NC>) * kFlushQueueCap) + warp_id * 4;
-  if (COMP && (threadIdx.x & 31) == 0) *fqn = 0;
-  __shared__ int s_nruns_pre;
   if (n <= 0) return;
-
-  const FacetXform &fxt = a.facets[f_local];
-  const int gnx = fxt.nx;
-  const long long nxy = (long long)fxt.nx * fxt.ny;
-  const long long fbase = fxt.grid_base;
   const int tid = threadIdx.x;
-  int du, strip;
-  bool owner;
-  owner_map<WIDE>(tid, W, J, du, strip, owner);
-  unsigned rows_mask = 0;
-#pragma unroll
-  for (int j = 0; j < J; ++j)
-    if (strip * J + j < W) rows_mask |= 1u << j;
-  if (!owner) rows_mask = 0;
-  const bool grids = __any_sync(0xffffffffu, rows_mask != 0);
-
-  OwnerState<NC, J> st;
-#pragma unroll
-  for (int j = 0; j < J; ++j) {
-#pragma unroll
-    for (int k = 0; k < NC; ++k) { st.acc[j][k].re = 0; st.acc[j][k].im = 0; }
-  }
-  st.dirty = 0;
-  st.cg = -1;
-  st.pu0 = -1;
-  st.pv0 = -1;
-  st.ou = 0;
-  st.ov0 = 0;
-
-  const int nchunks = (n + V - 1) / V;
   if (tid == 0) {
     // the buffers may last have been written by plain stores (an item prepared in place)
     fence_proxy_async();
@@ -1657,6 +1712,12 @@ __device__ __forceinline__ void grid_track_pre(const GridArgs &a, const int f_lo
     bar_arrive_tx(&rbar[0], bytes);
     bulk_copy(rb, src, bytes, &rbar[0]);
   }
+  ItemSetup<NC, WPROJ> s;
+  item_setup<NC, WPROJ, J, COMP, WIDE>(a, f_local, smem_raw, s);
+  OwnerState<NC, J> st;
+  owner_reset(st);
+  bool swap = false;
+  const int nchunks = (n + V - 1) / V;
   int cur = 0;
   for (int c = 0; c < nchunks; ++c, cur ^= 1) {
     const int nv = min(V, n - c * V);
@@ -1666,8 +1727,6 @@ __device__ __forceinline__ void grid_track_pre(const GridArgs &a, const int f_lo
       bar_wait(&rbar[cur], par);
     }
     rphase ^= 1u << cur;
-    const GridRec<NC> *recs = rb + cur * V;
-    stage_taps_bulk<NC, WPROJ>(a, recs, nv, TUS, TVS, tu, tv, bar);
     if (tid == 0 && c + 1 < nchunks) {
       // the other buffer was last read by the previous chunk, which every thread has finished
       const unsigned bytes = (unsigned)(sizeof(GridRec<NC>) * (size_t)min(V, n - (c + 1) * V));
@@ -1675,37 +1734,15 @@ __device__ __forceinline__ void grid_track_pre(const GridArgs &a, const int f_lo
       bar_arrive_tx(&rbar[cur ^ 1], bytes);
       bulk_copy(rb + (cur ^ 1) * V, src + (size_t)(c + 1) * V, bytes, &rbar[cur ^ 1]);
     }
-    if (warp_id == 0) find_runs(recs, nv, s_runs, &s_nruns_pre);
-    if (!bar_wait(bar, phase)) {
-      atomicOr(a.error, DEV_ERR_WAIT_TIMEOUT);
-      bar_wait(bar, phase);
-    }
-    phase ^= 1u;
-    __syncthreads();
-    if (grids)
-      grid_runs<NC, WPROJ, J, COMP>(a, recs, tu, tv, s_runs, s_nruns_pre, TUS, TVS, du, strip, rows_mask, fbase, nxy,
-                                    gnx, fq, fqn, st);
-    __syncthreads();
+    grid_chunk<NC, WPROJ, J, COMP>(a, rb + cur * V, nv, c == 0, swap, s, st);
   }
-  if (COMP && grids) drain_queue<NC>(a, nxy, fq, fqn);
-  if (st.dirty) {
-#pragma unroll
-    for (int j = 0; j < J; ++j) {
-      const int oy = st.ov0 + j >= W ? st.ov0 + j - W : st.ov0 + j;
-      if (st.dirty & (1u << j))
-        flush_cell<NC, COMP>(a, fbase + (long long)st.cg * NC * nxy, nxy, gnx, st.pu0 + st.ou, st.pv0 + oy, st.acc[j]);
-    }
-  }
+  item_flush<NC, WPROJ, J, COMP>(a, s, swap, st);
 }
 
-// Default register budget of the persistent segment kernel: the J = 4 layout (32 accumulator
-// registers) is capped at 80 registers per thread so that more warps stay resident; J = 8 keeps the
-// 128 that 512 threads allow.  The w-projection visibility launches also offer J = 4 builds at 64 and
-// 72 registers to the tuner (different support classes prefer different caps).
+// Register caps of the persistent segment kernel: the J rows' accumulators (8 J values), the merge
+// step's values and the footprint state, without spills in the loops.
 template <int J>
-constexpr int kSegRegs = J == 4 ? 80 : 128;
-// the J = 6 layout of the single-precision w-projection visibility launches
-constexpr int kSegRegs6 = 96;
+constexpr int kSegRegs = J == 4 && sizeof(acc_real) == 4 ? 96 : J == 6 ? 112 : 128;
 
 // One CTA per track: blockIdx -> (facet, baseline slot or row segment, channel).
 template <int NC, bool WPROJ, int J, bool COMP, bool WIDE>
@@ -1723,24 +1760,23 @@ __global__ void __launch_bounds__(512, 1) romein_grid_kernel(const GridArgs a) {
     r0 = (long long)slot * a.seg;
     r1 = min(a.nrows, r0 + a.seg);
   }
-  unsigned phase = 0;
-  grid_track<NC, WPROJ, J, COMP, WIDE>(a, f_local, chan, r0, r1, nullptr, phase);
+  grid_track<NC, WPROJ, J, COMP, WIDE>(a, f_local, chan, r0, r1);
 }
 
 // Persistent form: a fixed grid of CTAs takes (segment, facet) work items from a device counter
 // until the device-side item count is exhausted; every segment is a run of one track's rows
 // whose w planes share this launch's support class (a.W).  Items of one segment are adjacent, so
 // the facets of a segment are gridded while its rows are hot in L2.  The loop ends on the count,
-// never waits on other CTAs.  The tap-copy barrier is set up once (V arrivals per phase).
-template <int NC, bool WPROJ, int J, bool COMP, bool WIDE, int REGS = kSegRegs<J>>
+// never waits on other CTAs.  Two builds share the items of a launch: PRE grids the items that the
+// record kernel had room for, the other build the rest (every item when there are no records); the
+// prologue of the latter would cost the former registers.
+template <int NC, bool WPROJ, int J, bool COMP, bool WIDE, bool PRE, int REGS = kSegRegs<J>>
 __global__ void __launch_bounds__(512, 1) __maxnreg__(REGS) romein_segment_kernel(const GridArgs a, const int nfacets) {
   __shared__ int s_item;
   __shared__ int s_first, s_last;  // unmasked row range of the item (facet row masks)
-  __shared__ __align__(8) unsigned long long s_tap_bar;
   __shared__ __align__(8) unsigned long long s_rec_bar[2];
-  unsigned phase = 0, rphase = 0;
-  if (threadIdx.x == 0) {
-    bar_init(&s_tap_bar, (unsigned)a.V);
+  unsigned rphase = 0;
+  if (PRE && threadIdx.x == 0) {
     bar_init(&s_rec_bar[0], 1);
     bar_init(&s_rec_bar[1], 1);
   }
@@ -1768,48 +1804,46 @@ __global__ void __launch_bounds__(512, 1) __maxnreg__(REGS) romein_segment_kerne
       if (threadIdx.x == 0) atomicOr(a.error, DEV_ERR_GRID_INDEX);
       continue;
     }
-    if (a.records) {
-      // records of this item, when the record kernel had room for its segment: only the item's
-      // first to last valid record (all of them past the range table)
-      const long long len = (long long)sg.y - sg.x;
-      const long long first = a.rec_off[si] * nfacets;
-      if ((a.rec_off[si] + len) * nfacets <= a.rec_capacity) {
-        const long long it = si * nfacets + f_local;
-        int lo = 0, hi = (int)len;
-        if (it < a.range_capacity) {
-          const int2 rg = a.item_range[it];
-          lo = rg.x;
-          hi = rg.y;
-        }
-        if (lo < hi) {
-          const GridRec<NC> *src =
-              reinterpret_cast<const GridRec<NC> *>(a.records) + first + (long long)f_local * len + lo;
-          grid_track_pre<NC, WPROJ, J, COMP, WIDE>(a, f_local, src, hi - lo, s_rec_bar, rphase, &s_tap_bar, phase);
-        }
-        continue;
+    const long long len = (long long)sg.y - sg.x;
+    const bool recorded = a.records && (a.rec_off[si] + len) * nfacets <= a.rec_capacity;
+    if (recorded != PRE) continue;  // the other build's
+    if constexpr (PRE) {
+      // only the item's first to last valid record (all of them past the range table)
+      const long long it = si * nfacets + f_local;
+      int lo = 0, hi = (int)len;
+      if (it < a.range_capacity) {
+        const int2 rg = a.item_range[it];
+        lo = rg.x;
+        hi = rg.y;
       }
-    }
-    long long r0 = sg.x, r1 = sg.y;
-    if (a.facet_row_mask) {
-      // a facet that leaves rows out grids only the item's first to last row it keeps, and skips
-      // the item when it keeps none (the rows in between are still tested in the prologue)
-      const uint8_t *m = a.facet_row_mask + (long long)(a.facet_base + f_local) * a.nrows;
-      int first = 0x7fffffff, last = -1;
-      for (int r = sg.x + (int)threadIdx.x; r < sg.y; r += (int)blockDim.x)
-        if (m[r]) {
-          first = min(first, r);
-          last = max(last, r);
-        }
-      if (last >= 0) {
-        atomicMin(&s_first, first);
-        atomicMax(&s_last, last);
+      if (lo < hi) {
+        const GridRec<NC> *src =
+            reinterpret_cast<const GridRec<NC> *>(a.records) + a.rec_off[si] * nfacets + (long long)f_local * len + lo;
+        grid_track_pre<NC, WPROJ, J, COMP, WIDE>(a, f_local, src, hi - lo, s_rec_bar, rphase);
       }
-      __syncthreads();
-      if (s_last < 0) continue;  // uniform: every thread reads the same shared values
-      r0 = s_first;
-      r1 = (long long)s_last + 1;
+    } else {
+      long long r0 = sg.x, r1 = sg.y;
+      if (a.facet_row_mask) {
+        // a facet that leaves rows out grids only the item's first to last row it keeps, and skips
+        // the item when it keeps none (the rows in between are still tested in the prologue)
+        const uint8_t *m = a.facet_row_mask + (long long)(a.facet_base + f_local) * a.nrows;
+        int first = 0x7fffffff, last = -1;
+        for (int r = sg.x + (int)threadIdx.x; r < sg.y; r += (int)blockDim.x)
+          if (m[r]) {
+            first = min(first, r);
+            last = max(last, r);
+          }
+        if (last >= 0) {
+          atomicMin(&s_first, first);
+          atomicMax(&s_last, last);
+        }
+        __syncthreads();
+        if (s_last < 0) continue;  // uniform: every thread reads the same shared values
+        r0 = s_first;
+        r1 = (long long)s_last + 1;
+      }
+      grid_track<NC, WPROJ, J, COMP, WIDE>(a, f_local, sg.z, r0, r1);
     }
-    grid_track<NC, WPROJ, J, COMP, WIDE>(a, f_local, sg.z, r0, r1, &s_tap_bar, phase);
   }
 }
 

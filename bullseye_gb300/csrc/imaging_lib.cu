@@ -612,9 +612,9 @@ FacetXform bz_facet_xform(double ra0, double dec0, double ra, double dec, bool p
 }
 
 struct LaunchShape {
-  int J, NT, V;
+  int J, NT;
   bool wide;
-  size_t smem;
+  ChunkShape chunk;
 };
 
 // Ownership layout for full support W: J rows per thread; WIDE pads columns to a multiple of 32
@@ -645,8 +645,7 @@ static LaunchShape choose_shape(int W) {
   if (!s.J) s.J = 16;
   const int owners = s.wide ? cols * ((W + s.J - 1) / s.J) : W * ((W + s.J - 1) / s.J);
   s.NT = std::max(32, ((owners + 31) / 32) * 32);
-  s.V = grid_chunk_size<NC, WPROJ>(W, s.NT, s.J);
-  s.smem = grid_smem_bytes<NC, WPROJ>(s.V, W, s.NT, s.J);
+  s.chunk = chunk_shape<NC, WPROJ>(W, s.NT, s.J);
   return s;
 }
 
@@ -662,11 +661,11 @@ static bool launch_j(const GridArgs &a, const LaunchShape &s, long long blocks, 
   (void)comp;  // FP64 accumulation needs no compensation
   kern = romein_grid_kernel<NC, WPROJ, J, false, WIDE>;
 #endif
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem) != cudaSuccess) {
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.chunk.smem) != cudaSuccess) {
     bz_record_error(BZ_ERR_CUDA, "cudaFuncSetAttribute failed");
     return false;
   }
-  kern<<<(unsigned)blocks, s.NT, s.smem, st>>>(a);
+  kern<<<(unsigned)blocks, s.NT, s.chunk.smem, st>>>(a);
   g_ctx.launches++;
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
@@ -683,7 +682,8 @@ static bool launch_nc(GridArgs a, long long blocks, cudaStream_t st, bool comp) 
     bz_record_error(BZ_ERR_UNSUPPORTED, "full support %d is larger than this build supports", a.W);
     return false;
   }
-  a.V = s.V;
+  a.V = s.chunk.V;
+  a.GB = s.chunk.GB;
   if (s.wide) {
     if (s.J == 2) return launch_j<NC, WPROJ, 2, true>(a, s, blocks, st, comp);
     return launch_j<NC, WPROJ, 8, true>(a, s, blocks, st, comp);

@@ -118,9 +118,9 @@ __global__ void noalloc_fold_kernel(vis_complex *__restrict__ grid, const vis_co
 
 // Ownership layout for full support W (same rule as the library's other gridding calls).
 struct Shape {
-  int J, NT, V;
+  int J, NT;
+  ChunkShape chunk;
   bool wide;
-  size_t smem;
 };
 template <bool WPROJ>
 Shape noalloc_shape(int W) {
@@ -138,8 +138,7 @@ Shape noalloc_shape(int W) {
   if (!s.J) s.J = 16;
   const int owners = s.wide ? cols * ((W + s.J - 1) / s.J) : W * ((W + s.J - 1) / s.J);
   s.NT = std::max(32, ((owners + 31) / 32) * 32);
-  s.V = grid_chunk_size<4, WPROJ>(W, s.NT, s.J);
-  s.smem = grid_smem_bytes<4, WPROJ>(s.V, W, s.NT, s.J);
+  s.chunk = chunk_shape<4, WPROJ>(W, s.NT, s.J);
   return s;
 }
 
@@ -150,8 +149,8 @@ bool noalloc_launch(const GridArgs &a, const Shape &s, long long blocks, cudaStr
 #else
   void (*kern)(const GridArgs) = romein_grid_kernel<4, WPROJ, J, false, WIDE>;
 #endif
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.smem) != cudaSuccess) return false;
-  kern<<<(unsigned)blocks, s.NT, s.smem, st>>>(a);
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.chunk.smem) != cudaSuccess) return false;
+  kern<<<(unsigned)blocks, s.NT, s.chunk.smem, st>>>(a);
   return cudaGetLastError() == cudaSuccess;
 }
 
@@ -159,7 +158,8 @@ template <bool WPROJ>
 bool noalloc_dispatch(GridArgs a, long long blocks, cudaStream_t st) {
   Shape s = noalloc_shape<WPROJ>(a.W);
   if (s.NT > 512) return false;
-  a.V = s.V;
+  a.V = s.chunk.V;
+  a.GB = s.chunk.GB;
   if (s.wide) return s.J == 2 ? noalloc_launch<WPROJ, 2, true>(a, s, blocks, st) : noalloc_launch<WPROJ, 8, true>(a, s, blocks, st);
   switch (s.J) {
     case 1: return noalloc_launch<WPROJ, 1, false>(a, s, blocks, st);
