@@ -594,6 +594,10 @@ FacetXform bz_facet_xform(double ra0, double dec0, double ra, double dec, bool p
   // phase_transform_policies.h:110-134 and baseline_transform_policies.h:117-149, in FP64
   FacetXform x;
   std::memset(&x, 0, sizeof x);
+  // at the phase centre both transforms are the identity: a host that contracts the differences of
+  // products below into fused multiply-adds would leave their rounding errors (1e-17), which move a
+  // sample that lies on a cell boundary
+  if (ra == ra0 && dec == dec0) return x;
   const double k = (double)kArcsecToRad;
   double d_ra = (ra - ra0) * k, n_dec = dec * k, o_dec = dec0 * k;
   double c_d_ra = cos(d_ra), s_d_ra = sin(d_ra), c_n = cos(n_dec), s_n = sin(n_dec), c_o = cos(o_dec),
