@@ -118,44 +118,64 @@ __global__ void scan_kernel(const int *__restrict__ in, int *__restrict__ out, i
 // outside the table is left out and reported rather than counted out of bounds.
 __global__ void seg_write_kernel(const size_t *starts, int nslots, int seg_len, long long R, int nchan,
                                  const unsigned char *__restrict__ cls, const int *__restrict__ off,
-                                 int4 *__restrict__ segs, int *__restrict__ class_count, int ncls, int *err) {
+                                 const int *__restrict__ nseg, int4 *__restrict__ segs, int *__restrict__ class_count,
+                                 int ncls, int *err) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= nslots * nchan) return;
   int c;
   long long r0, r1;
   track_rows(t, nchan, nslots, seg_len, R, starts, c, r0, r1);
   const unsigned char *k = cls + (long long)c * R;
-  int o = off[t];
+  // a track's runs in the order that its rows are gridded (last to first for odd channels)
+  const bool back = rows_backwards(c);
+  int o = back ? off[t] + nseg[t] - 1 : off[t];
   long long begin = r0;
   for (long long r = r0; r < r1; ++r) {
     if (r + 1 == r1 || k[r + 1] != k[r]) {
       const int kc = k[r] < ncls ? (int)k[r] : -1;
       if (kc < 0) atomicOr(err, DEV_ERR_GRID_INDEX);
-      segs[o++] = make_int4((int)begin, (int)(r + 1), c, kc);
+      segs[o] = make_int4((int)begin, (int)(r + 1), c, kc);
+      o += back ? -1 : 1;
       if (kc >= 0) atomicAdd(&class_count[kc], 1);
       begin = r + 1;
     }
   }
 }
 
-__global__ void class_offsets_kernel(const int *class_count, int *class_off, int *class_cursor, int ncls) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  int s = 0;
-  for (int k = 0; k < ncls; ++k) {
-    class_off[k] = s;
-    class_cursor[k] = 0;
-    s += class_count[k];
-  }
-}
-
-__global__ void bucket_kernel(const int4 *__restrict__ segs, const int *total, int4 *__restrict__ sorted,
-                              int *class_cursor, const int *class_off) {
+// The runs of class blockIdx.x, in track order, behind those of the classes before it (one block per
+// class; a stable bucketing, so that consecutive runs of a class are neighbouring channels of one
+// baseline: a work item takes several, see romein_segment_kernel).  Also writes the class offsets.
+__global__ void __launch_bounds__(1024) bucket_kernel(const int4 *__restrict__ segs, const int *__restrict__ total,
+                                                      const int *__restrict__ class_count, int4 *__restrict__ sorted,
+                                                      int *__restrict__ class_off) {
+  __shared__ int s_warp[33];
+  const int k = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  int at = 0;
+  for (int i = 0; i < k; ++i) at += class_count[i];
+  if (tid == 0) class_off[k] = at;
+  if (class_count[k] == 0) return;
   const int n = *total;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const int4 s = segs[i];
-    if (s.w < 0) continue;  // reported by seg_write_kernel
-    const int pos = class_off[s.w] + atomicAdd(&class_cursor[s.w], 1);
-    sorted[pos] = s;
+  for (int b = 0; b < n; b += 1024) {
+    const int i = b + tid;
+    const bool mine = i < n && segs[i].w == k;  // (a run without a class was reported by seg_write_kernel)
+    const unsigned m = __ballot_sync(0xffffffffu, mine);
+    if (lane == 0) s_warp[warp] = __popc(m);
+    __syncthreads();
+    if (warp == 0) {
+      const int x = s_warp[lane];
+      int sum = x;
+#pragma unroll
+      for (int off = 1; off < 32; off <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, sum, off);
+        if (lane >= off) sum += y;
+      }
+      s_warp[lane] = sum - x;
+      if (lane == 31) s_warp[32] = sum;
+    }
+    __syncthreads();
+    if (mine) sorted[at + s_warp[warp] + __popc(m & ((1u << lane) - 1))] = segs[i];
+    at += s_warp[32];
+    __syncthreads();
   }
 }
 
@@ -239,6 +259,7 @@ __global__ void __launch_bounds__(kRecordWarps * 32) record_kernel(
       continue;
     }
     const int len = sg.y - sg.x;
+    const bool back = rows_backwards(sg.z);
     if ((rec_off[si] + len) * nfacets > capacity) continue;
     GridRec<NC> *seg_out = out + rec_off[si] * nfacets;
     // residues mod the class width by a multiply-high (exact for corners below 2^26), corrected
@@ -309,7 +330,7 @@ __global__ void __launch_bounds__(kRecordWarps * 32) record_kernel(
 #pragma unroll
               for (int k = 0; k < NC; ++k) g.vis[k].re = g.vis[k].im = 0;
             }
-            seg_out[(long long)f * len + i] = g;
+            seg_out[(long long)f * len + (back ? len - 1 - i : i)] = g;
           }
           const unsigned m = __ballot_sync(0xffffffffu, v);
           if (!m) continue;
@@ -382,7 +403,8 @@ __global__ void __launch_bounds__(kRecordWarps * 32) record_kernel(
       for (int j = lane; j < fb; j += 32) {
         const long long item = (long long)si * nfacets + f0 + j;
         const int2 r = s_rng[j];
-        if (item < range_items) range[item] = r.x == 0x7fffffff ? make_int2(0, 0) : r;
+        if (item < range_items)
+          range[item] = r.x == 0x7fffffff ? make_int2(0, 0) : back ? make_int2(len - r.y, len - r.x) : r;
         if (want_norm && s_ng[j] >= 0) {
           const long long fslice = (long long)(a.facet_base + f0 + j) * a.groups;
 #pragma unroll
@@ -458,7 +480,7 @@ struct BatchedState {
   ClassInfo cls[kMaxClasses];
   DevBuf<int> plane_class, plane_lo;
   DevBuf<unsigned char> row_class;
-  DevBuf<int> nseg, seg_off, seg_total, class_count, class_off, class_cursor, work_next, sample_count;
+  DevBuf<int> nseg, seg_off, seg_total, class_count, class_off, work_next, sample_count;
   DevBuf<int4> segs, sorted;
   DevBuf<FacetXform> facet_table;  // per-facet geometry of bullseye_grid_batched_facets
   DevBuf<vis_real> conv_w;         // support-window table [P][tap_f][conv_w_stride] (plan_classes)
@@ -605,7 +627,7 @@ bool plan_classes() {
   if (!b.plane_class.alloc(P) || !b.plane_lo.alloc(P)) return false;
   BZ_CUDA_TRY_RET(cudaMemcpy(b.plane_class.ptr, pcls.data(), sizeof(int) * P, cudaMemcpyHostToDevice), false);
   BZ_CUDA_TRY_RET(cudaMemcpy(b.plane_lo.ptr, plo.data(), sizeof(int) * P, cudaMemcpyHostToDevice), false);
-  if (!b.class_count.alloc(kMaxClasses) || !b.class_off.alloc(kMaxClasses) || !b.class_cursor.alloc(kMaxClasses) ||
+  if (!b.class_count.alloc(kMaxClasses) || !b.class_off.alloc(kMaxClasses) ||
       !b.work_next.alloc(2 * kMaxClasses) || !b.seg_total.alloc(1) || !b.sample_count.alloc(2 * kMaxClasses))
     return false;
   b.planned = true;
@@ -973,10 +995,10 @@ bool enqueue_schedule(const GridArgs &va, cudaStream_t st, long long r0 = 0, lon
                                                          b.nseg.ptr);
   scan_kernel<<<1, 1024, 0, st>>>(b.nseg.ptr, b.seg_off.ptr, tracks, b.seg_total.ptr);
   seg_write_kernel<<<(tracks + 127) / 128, 128, 0, st>>>(va.starts, va.nslots, va.seg, R, va.nchan, b.row_class.ptr,
-                                                         b.seg_off.ptr, b.segs.ptr, b.class_count.ptr, b.ncls, va.error);
-  class_offsets_kernel<<<1, 1, 0, st>>>(b.class_count.ptr, b.class_off.ptr, b.class_cursor.ptr, b.ncls);
-  bucket_kernel<<<1024, 256, 0, st>>>(b.segs.ptr, b.seg_total.ptr, b.sorted.ptr, b.class_cursor.ptr, b.class_off.ptr);
-  c.launches += 6;
+                                                         b.seg_off.ptr, b.nseg.ptr, b.segs.ptr, b.class_count.ptr, b.ncls,
+                                                         va.error);
+  bucket_kernel<<<b.ncls, 1024, 0, st>>>(b.segs.ptr, b.seg_total.ptr, b.class_count.ptr, b.sorted.ptr, b.class_off.ptr);
+  c.launches += 5;
   BZ_CUDA_TRY_RET(cudaGetLastError(), false);
   return true;
 }
@@ -987,7 +1009,7 @@ void bz_release_batched() {
   BatchedState &b = g_bs;
   b.drop_graphs();
   b.plane_class.release(); b.plane_lo.release(); b.row_class.release(); b.nseg.release(); b.seg_off.release();
-  b.seg_total.release(); b.class_count.release(); b.class_off.release(); b.class_cursor.release();
+  b.seg_total.release(); b.class_count.release(); b.class_off.release();
   b.work_next.release(); b.sample_count.release(); b.segs.release(); b.sorted.release(); b.facet_table.release();
   b.conv_w.release();
   b.conv_w_stride = 0;
@@ -1140,7 +1162,7 @@ int run_batched(const GridArgs &va, const GridArgs *sa, int nfacets, const GridA
   bz_trace_mark("schedule_tune_capture");
   BZ_CUDA_TRY_RET(cudaGraphLaunch(slot->exec, c.stream), BZ_ERR_CUDA);
   const int rec = b.vrec_on && b.vrec.ptr && b.conv_w.ptr ? 2 : 0;  // record offsets + record kernel per build
-  c.launches += 6 + (long long)(b.ncls + rec) * ((vis ? 1 : 0) + (sf ? 1 : 0));
+  c.launches += 5 + (long long)(b.ncls + rec) * ((vis ? 1 : 0) + (sf ? 1 : 0));
   return BZ_OK;
 }
 
@@ -1481,7 +1503,7 @@ __global__ void window_table_kernel(const void *conv, int P, int K, int tap_f, i
 // Workspace layout of the support-aware form (every piece 256-byte aligned).
 struct SupportWs {
   size_t plane_class, plane_lo, plane_w, table, row_class, nseg, seg_off, seg_total, segs, sorted, class_count,
-      class_off, class_cursor, work_next, bytes;
+      class_off, work_next, bytes;
   int L, tap_f;
   long long maxseg;
 };
@@ -1512,7 +1534,6 @@ SupportWs support_ws_layout(long long R, int nchan, int nslots, int P, int os, i
   l.sorted = take(sizeof(int4) * l.maxseg);
   l.class_count = take(sizeof(int) * kMaxClasses);
   l.class_off = take(sizeof(int) * kMaxClasses);
-  l.class_cursor = take(sizeof(int) * kMaxClasses);
   l.work_next = take(sizeof(int) * kMaxClasses);
   l.bytes = off;
   return l;
@@ -1607,7 +1628,6 @@ bool bz_grid_support_aware(const GridArgs &a_in, int nfacets, unsigned char *ws,
   int4 *sorted = reinterpret_cast<int4 *>(ws + l.sorted);
   int *class_count = reinterpret_cast<int *>(ws + l.class_count);
   int *class_off = reinterpret_cast<int *>(ws + l.class_off);
-  int *class_cursor = reinterpret_cast<int *>(ws + l.class_cursor);
   int *work_next = reinterpret_cast<int *>(ws + l.work_next);
   const int P = a_in.P, K = a_in.K;
   const long long R = a_in.nrows;
@@ -1623,9 +1643,8 @@ bool bz_grid_support_aware(const GridArgs &a_in, int nfacets, unsigned char *ws,
                                                          nseg);
   scan_kernel<<<1, 1024, 0, st>>>(nseg, seg_off, tracks, seg_total);
   seg_write_kernel<<<(tracks + 127) / 128, 128, 0, st>>>(a_in.starts, a_in.nslots, a_in.seg, R, a_in.nchan, row_class,
-                                                         seg_off, segs, class_count, cl.n, a_in.error);
-  class_offsets_kernel<<<1, 1, 0, st>>>(class_count, class_off, class_cursor, cl.n);
-  bucket_kernel<<<1024, 256, 0, st>>>(segs, seg_total, sorted, class_cursor, class_off);
+                                                         seg_off, nseg, segs, class_count, cl.n, a_in.error);
+  bucket_kernel<<<cl.n, 1024, 0, st>>>(segs, seg_total, class_count, sorted, class_off);
   if (cudaGetLastError() != cudaSuccess) return false;
   GridArgs a = a_in;
   a.W_full = W;

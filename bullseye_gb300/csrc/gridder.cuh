@@ -1025,26 +1025,27 @@ __device__ __forceinline__ void prologue(const GridArgs &a, int f_local, int cha
 
 // ------------------------------------------------------------------ merged gridding of staged chunks
 //
-// Taps are products: footprint cell (a, b) of a visibility gets vis x ka(a) x kb(b).  Consecutive
+// Taps are products: footprint cell (u, v) of a visibility gets vis x ku(u) x kv(v).  Consecutive
 // visibilities of a track sit a fraction of an oversampling step apart, so a stretch of them often
 // shares the footprint corner and one of the two tap rows.  Such a *group* is summed along the other
-// axis first,
-//     T(a) = sum over the group of vis x ka(a)            (W multiply-adds per visibility)
-//     cell(a, b) += T(a) x kb(b)                            (W^2 multiply-adds per group, not per visibility)
-// which is the same sum with its common factor taken out.  On Earth-rotation tracks sampled every 14 s
-// (27 EVLA antennas, 1024-cell grids 1.4 degrees wide, oversampling 15) groups hold 4.6 visibilities
-// on average when each work item merges along the axis on which its track moves less in tap steps;
-// fixed to one axis they hold 2.3 (u) or 3.9 (v), and merging only identical footprints gives 1.9.
+// axis first; with a common kv,
+//     T(u) = sum over the group of vis x ku(u)            (W multiply-adds per visibility)
+//     cell(u, v) += T(u) x kv(v)                            (W^2 multiply-adds per group, not per visibility)
+// which is the same sum with its common factor taken out (and the other way round with a common ku).
+// On Earth-rotation tracks sampled every 14 s (27 EVLA antennas, 1024-cell grids 1.4 degrees wide,
+// oversampling 15) groups hold 4.6 visibilities on average when each work item merges along the axis on
+// which its track moves more in tap steps; fixed to one axis they hold 2.3 (v) or 3.9 (u), and merging
+// only identical footprints gives 1.9.
 //
 // What the merge and the split of the builds measured (GB300, 27 antennas x 100 times x 64 channels,
 // 16 facets, whole batched call with copy-back): 36.5 -> 27.3 ms in single precision; 64-bit library,
 // 40 times x 16 channels x 4 facets: 28.2 -> 8.1 ms (its FP64 pipe bounded the multiply-adds).
 //
 // A chunk of V records in shared memory is taken in two steps, in batches of GB groups:
-//   merge_groups  thread (a, part) forms T(a) of every nparts-th group of the batch, reading ka from
-//                 the kernel table through L1, and copies the group's kb row;
-//   grid_groups   the Romein owner threads add T(a) x kb(b) to their J cells per column.
-// The item's axes are (a, b) = (u, v), or (v, u) when it merges along v ("swapped").
+//   merge_groups  thread (i, part) forms T(i) of every nparts-th group of the batch, reading the taps
+//                 from the kernel table through L1, and copies the group's common tap row;
+//   grid_groups   the Romein owner threads add T x tap to their J cells per column.  Columns run along
+//                 u whatever the merge axis, so that a warp's flushes are contiguous in the grid.
 
 // Per-warp flush queues (compensated single precision only): nwarps record arrays, then one
 // 16-byte counter slot per warp.
@@ -1082,11 +1083,11 @@ __host__ __device__ inline size_t stage_head_bytes(int V) {
   const size_t pre = 2 * sizeof(GridRec<NC>);
   return ((own > pre ? own : pre) * (size_t)V + 15) / 16 * 16;
 }
-// Merged values and the second axis' tap row (W + J - 1 taps: the first J - 1 repeated after the last,
-// so a thread's J consecutive owned rows read J consecutive taps without a wrap) of one group.
+// Merged values and the common tap row of one group, W + J - 1 of each: the first J - 1 are repeated
+// after the last, so that a thread's J consecutive owned rows read consecutive entries without a wrap.
 template <int NC, bool WPROJ>
 __host__ __device__ inline size_t merge_group_bytes(int W, int J) {
-  return sizeof(cplx) * NC * (size_t)W + sizeof(typename TapT<WPROJ>::type) * (size_t)(W + J - 1);
+  return (sizeof(cplx) * NC + sizeof(typename TapT<WPROJ>::type)) * (size_t)(W + J - 1);
 }
 // One group list per warp.
 __host__ __device__ inline size_t group_list_bytes(int nwarps) { return (size_t)nwarps * kMaxChunk * sizeof(unsigned short); }
@@ -1154,13 +1155,13 @@ __device__ __forceinline__ void owner_map(int tid, int W, int J, int &du, int &s
 }
 
 // Register state of a Romein owner thread: the accumulators of its J cells and the footprint they
-// belong to.  For the last footprint corner (pa0, pb0) the owned cells are
-// (pa0 + oa, pb0 + wrap(ob0 + j)), wrap(i) = i - W when i >= W.
+// belong to.  For the last footprint corner (pu0, pv0) the owned cells are
+// (pu0 + ou, pv0 + wrap(ov0 + j)), wrap(i) = i - W when i >= W.
 template <int NC, int J>
 struct OwnerState {
   cplx acc[J][NC];
   unsigned dirty;
-  int cg, pa0, pb0, oa, ob0;
+  int cg, pu0, pv0, ou, ov0;
 };
 
 template <int NC, int J>
@@ -1172,10 +1173,10 @@ __device__ __forceinline__ void owner_reset(OwnerState<NC, J> &st) {
   }
   st.dirty = 0;
   st.cg = -1;
-  st.pa0 = -1;
-  st.pb0 = -1;
-  st.oa = 0;
-  st.ob0 = 0;
+  st.pu0 = -1;
+  st.pv0 = -1;
+  st.ou = 0;
+  st.ov0 = 0;
 }
 
 // Prologue of one staging slot: the visibility of `row` staged into recs[slot].
@@ -1385,16 +1386,16 @@ __device__ __forceinline__ SlotMasks slot_masks(const Rec *recs, int nv, int b) 
 constexpr int kGroupRun = 1 << 14;
 
 // The groups of a staged chunk, written by every warp into its own list (whole-warp call; all warps
-// find the same groups).  `pick` first decides the merge axis of the item from this chunk: along v
-// when that leaves fewer groups.
+// find the same groups).  `pick` first decides the item's merge axis from this chunk: the one that
+// leaves fewer groups.
 template <class Rec>
-__device__ __forceinline__ int find_groups(const Rec *recs, int nv, bool pick, bool &swap, unsigned short *list) {
+__device__ __forceinline__ int find_groups(const Rec *recs, int nv, bool pick, bool &along_v, unsigned short *list) {
   typedef unsigned long long u64;
   const SlotMasks m0 = slot_masks(recs, nv, 0);
   SlotMasks m1{0, 0, 0, 0};
   if (nv > 32) m1 = slot_masks(recs, nv, 1);
-  if (pick) swap = __popc(m0.along_v) + __popc(m1.along_v) < __popc(m0.along_u) + __popc(m1.along_u);
-  const u64 start = swap ? (u64)m1.along_v << 32 | m0.along_v : (u64)m1.along_u << 32 | m0.along_u;
+  if (pick) along_v = __popc(m0.along_v) + __popc(m1.along_v) < __popc(m0.along_u) + __popc(m1.along_u);
+  const u64 start = along_v ? (u64)m1.along_v << 32 | m0.along_v : (u64)m1.along_u << 32 | m0.along_u;
   const u64 run = (u64)m1.run << 32 | m0.run;
   const u64 edge = start | ~((u64)m1.valid << 32 | m0.valid);  // slots that do not continue a group
   const int lane = threadIdx.x & 31;
@@ -1411,18 +1412,18 @@ __device__ __forceinline__ int find_groups(const Rec *recs, int nv, bool pick, b
   return __popcll(start);
 }
 
-// T(a) and the kb row of groups [g0, g1) of a chunk: thread (column a = ax, part ap of nparts).
+// T and the common tap row of groups [g0, g1) of a chunk: thread (entry i, part of nparts).
 template <int NC, bool WPROJ, class Rec>
 __device__ __forceinline__ void merge_groups(const TapTable<WPROJ> &table, const Rec *recs, const unsigned short *list,
-                                             int g0, int g1, bool swap, int W, int J, int ax, int ap, int nparts,
+                                             int g0, int g1, bool along_v, int W, int J, int i, int part, int nparts,
                                              typename MergeVec<NC>::type *T, typename TapT<WPROJ>::type *tb) {
   typedef typename TapT<WPROJ>::type tap_t;
   typedef MergeVec<NC> M;
-  if (ap >= nparts) return;
-  const int TBS = W + J - 1;
-  for (int gi = g0 + ap; gi < g1; gi += nparts) {
+  if (part >= nparts) return;
+  const int S = W + J - 1;
+  for (int gi = g0 + part; gi < g1; gi += nparts) {
     const int e = list[gi], s = e & 127, end = s + ((e >> 7) & 127);
-    const tap_t kb = read_tap(table, swap ? recs[s].fu : recs[s].fv, ax);
+    const tap_t kb = read_tap(table, along_v ? recs[s].fu : recs[s].fv, i);
     cplx t[NC];
 #pragma unroll
     for (int k = 0; k < NC; ++k) { t[k].re = 0; t[k].im = 0; }
@@ -1431,8 +1432,8 @@ __device__ __forceinline__ void merge_groups(const TapTable<WPROJ> &table, const
       tap_t ka[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        const int i = min(v + q, end - 1);
-        ka[q] = read_tap(table, swap ? recs[i].fv : recs[i].fu, ax);
+        const int r = min(v + q, end - 1);
+        ka[q] = read_tap(table, along_v ? recs[r].fv : recs[r].fu, i);
       }
 #pragma unroll
       for (int q = 0; q < 4; ++q)
@@ -1446,56 +1447,53 @@ __device__ __forceinline__ void merge_groups(const TapTable<WPROJ> &table, const
           }
         }
     }
+    typename M::type *Tg = T + (gi - g0) * M::H * S;
+    tap_t *row = tb + (gi - g0) * S;
 #pragma unroll
     for (int h = 0; h < M::H; ++h) {
       typename M::type y;
 #pragma unroll
       for (int n = 0; n < M::N; ++n) y.v[n] = t[h * M::N + n];
-      T[((gi - g0) * M::H + h) * W + ax] = y;
+      for (int j = i; j < S; j += W) Tg[h * S + j] = y;
     }
-    tap_t *row = tb + (gi - g0) * TBS;
-    row[ax] = kb;
-    for (int j = ax; j < J - 1; j += W) row[W + j] = kb;  // once: J - 1 < W, or the row's own wrap
+    for (int j = i; j < S; j += W) row[j] = kb;
   }
 }
 
 // Multiply-adds of groups [g0, g1) of a chunk into an owner thread's cells.  When the footprint moves,
 // the owned cells are recomputed and those that changed are flushed (queued for the warp's
 // compensated flush in single precision; the queue is drained when it fills and at the end of the
-// track).  Every lane of a warp with any owned cell calls this, so the queue drains are
-// warp-uniform.  Cells lie sa (along a) and sb (along b) elements apart.
+// item).  Every lane of a warp with any owned cell calls this, so the queue drains are warp-uniform.
 template <int NC, bool WPROJ, int J, bool COMP, class Rec>
 __device__ __forceinline__ void grid_groups(const GridArgs &a, const Rec *recs, const unsigned short *list, int g0, int g1,
-                                            bool swap, const typename MergeVec<NC>::type *T,
+                                            bool along_v, const typename MergeVec<NC>::type *T,
                                             const typename TapT<WPROJ>::type *tb, int du, int strip, unsigned rows_mask,
-                                            long long fbase, long long nxy, int sa, int sb, FlushRec<NC> *fq, int *fqn,
+                                            long long fbase, long long nxy, int gnx, FlushRec<NC> *fq, int *fqn,
                                             OwnerState<NC, J> &st) {
   typedef typename TapT<WPROJ>::type tap_t;
   typedef MergeVec<NC> M;
-  const int W = a.W, TBS = W + J - 1;
+  const int W = a.W, S = W + J - 1;
   for (int gi = g0; gi < g1; ++gi) {
     const int e = list[gi];
     if (e & kGroupRun) {
       const int rs = e & 127;
-      const int4 hr = *reinterpret_cast<const int4 *>(&recs[rs].u0);
+      const int4 h = *reinterpret_cast<const int4 *>(&recs[rs].u0);
       const int g = recs[rs].g;
-      // corner and residues along (a, b)
-      const int a0 = swap ? hr.y : hr.x, b0 = swap ? hr.x : hr.y, ra = swap ? hr.w : hr.z, rb = swap ? hr.z : hr.w;
-      if (a0 != st.pa0 || b0 != st.pb0 || g != st.cg) {
+      if (h.x != st.pu0 || h.y != st.pv0 || g != st.cg) {
         // footprint moved: recompute the owned cells, flush those that changed
-        int o = du - ra;
+        int o = du - h.z;
         o += (o < 0) ? W : 0;
-        int nob0 = strip * J - rb;
-        nob0 += (nob0 < 0) ? W : 0;
+        int nov0 = strip * J - h.w;
+        nov0 += (nov0 < 0) ? W : 0;
         if (st.dirty) {
-          const bool all = a0 + o != st.pa0 + st.oa || g != st.cg;
-          const long long slice = fbase + (long long)st.cg * NC * nxy + (long long)(st.pa0 + st.oa) * sa;
+          const bool all = h.x + o != st.pu0 + st.ou || g != st.cg;
+          const long long slice = fbase + (long long)st.cg * NC * nxy + st.pu0 + st.ou;
 #pragma unroll
           for (int j = 0; j < J; ++j) {
-            const int ob = st.ob0 + j >= W ? st.ob0 + j - W : st.ob0 + j;
-            const int nb = nob0 + j >= W ? nob0 + j - W : nob0 + j;
-            if ((st.dirty & (1u << j)) && (all || b0 + nb != st.pb0 + ob)) {
-              const long long cell = slice + (long long)(st.pb0 + ob) * sb;
+            const int ov = st.ov0 + j >= W ? st.ov0 + j - W : st.ov0 + j;
+            const int nv = nov0 + j >= W ? nov0 + j - W : nov0 + j;
+            if ((st.dirty & (1u << j)) && (all || h.y + nv != st.pv0 + ov)) {
+              const long long cell = slice + (long long)(st.pv0 + ov) * gnx;
               if (COMP)
                 queue_cell<NC>(a, cell, nxy, st.acc[j], fq, fqn);
               else
@@ -1506,10 +1504,10 @@ __device__ __forceinline__ void grid_groups(const GridArgs &a, const Rec *recs, 
         }
         st.cg = g;
         // columns beyond W (padding lanes) read in-bounds values and are never flushed
-        st.oa = o < W ? o : W - 1;
-        st.ob0 = nob0 < W ? nob0 : 0;  // lanes past the last strip own nothing: keep their reads in bounds
-        st.pa0 = a0;
-        st.pb0 = b0;
+        st.ou = o < W ? o : W - 1;
+        st.ov0 = nov0 < W ? nov0 : 0;  // lanes past the last strip own nothing: keep their reads in bounds
+        st.pu0 = h.x;
+        st.pv0 = h.y;
         if (COMP) {  // the queue only grows here; the branch is uniform over the warp
           __syncwarp();
           if (*fqn >= kDrainAt) drain_queue<NC>(a, nxy, fq, fqn);
@@ -1518,19 +1516,34 @@ __device__ __forceinline__ void grid_groups(const GridArgs &a, const Rec *recs, 
     }
     // branch-free multiply-adds over the J owned rows (offsets modulo W; rows of non-owning lanes stay
     // in bounds and are never flushed)
-    cplx t[NC];
+    const typename M::type *Tg = T + (gi - g0) * M::H * S;
+    const tap_t *row = tb + (gi - g0) * S;
+    if (along_v) {
+      const tap_t k = row[st.ou];
+      Tg += st.ov0;
 #pragma unroll
-    for (int h = 0; h < M::H; ++h) {
-      const typename M::type y = T[((gi - g0) * M::H + h) * W + st.oa];
+      for (int j = 0; j < J; ++j)
 #pragma unroll
-      for (int n = 0; n < M::N; ++n) t[h * M::N + n] = y.v[n];
-    }
-    const tap_t *row = tb + (gi - g0) * TBS + st.ob0;
+        for (int h = 0; h < M::H; ++h) {
+          const typename M::type y = Tg[h * S + j];
 #pragma unroll
-    for (int j = 0; j < J; ++j) {
-      const tap_t k = row[j];
+          for (int n = 0; n < M::N; ++n) mac(st.acc[j][h * M::N + n], y.v[n], k);
+        }
+    } else {
+      cplx t[NC];
 #pragma unroll
-      for (int c = 0; c < NC; ++c) mac(st.acc[j][c], t[c], k);
+      for (int h = 0; h < M::H; ++h) {
+        const typename M::type y = Tg[h * S + st.ou];
+#pragma unroll
+        for (int n = 0; n < M::N; ++n) t[h * M::N + n] = y.v[n];
+      }
+      row += st.ov0;
+#pragma unroll
+      for (int j = 0; j < J; ++j) {
+        const tap_t k = row[j];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) mac(st.acc[j][c], t[c], k);
+      }
     }
     st.dirty |= rows_mask;
   }
@@ -1539,7 +1552,7 @@ __device__ __forceinline__ void grid_groups(const GridArgs &a, const Rec *recs, 
 // What a CTA keeps for one work item: its shared-memory pieces, owner mapping and facet geometry.
 template <int NC, bool WPROJ>
 struct ItemSetup {
-  typename MergeVec<NC>::type *T;        // [GB][H][W]
+  typename MergeVec<NC>::type *T;        // [GB][H][W + J - 1]
   typename TapT<WPROJ>::type *tb;        // [GB][W + J - 1]
   unsigned short *list;                  // this warp's group list
   FlushRec<NC> *fq;                      // this warp's flush queue
@@ -1558,7 +1571,7 @@ __device__ __forceinline__ void item_setup(const GridArgs &a, int f_local, unsig
   const int warp_id = tid >> 5, nwarps = (blockDim.x + 31) >> 5;
   unsigned char *p = smem + stage_head_bytes<NC>(a.V);
   s.T = reinterpret_cast<vec_t *>(p);
-  p += sizeof(cplx) * NC * (size_t)W * GB;
+  p += sizeof(cplx) * NC * (size_t)(W + J - 1) * GB;
   s.tb = reinterpret_cast<tap_t *>(p);
   p += sizeof(tap_t) * (size_t)(W + J - 1) * GB;
   p = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(p) + 15) & ~(uintptr_t)15);
@@ -1588,100 +1601,163 @@ __device__ __forceinline__ void item_setup(const GridArgs &a, int f_local, unsig
 // The groups of one staged chunk (block-wide call; ends with the CTA's barrier, after which the
 // records may be overwritten).
 template <int NC, bool WPROJ, int J, bool COMP, class Rec>
-__device__ __forceinline__ void grid_chunk(const GridArgs &a, const Rec *recs, int nv, bool first, bool &swap,
+__device__ __forceinline__ void grid_chunk(const GridArgs &a, const Rec *recs, int nv, bool first, bool &along_v,
                                            const ItemSetup<NC, WPROJ> &s, OwnerState<NC, J> &st) {
-  const int ng = find_groups(recs, nv, first, swap, s.list);
-  const int sa = swap ? s.gnx : 1, sb = swap ? 1 : s.gnx;
+  const int ng = find_groups(recs, nv, first, along_v, s.list);
   for (int g0 = 0; g0 < ng; g0 += a.GB) {
     const int g1 = min(ng, g0 + a.GB);
-    merge_groups<NC, WPROJ>(s.table, recs, s.list, g0, g1, swap, a.W, J, s.ax, s.ap, s.nparts, s.T, s.tb);
+    merge_groups<NC, WPROJ>(s.table, recs, s.list, g0, g1, along_v, a.W, J, s.ax, s.ap, s.nparts, s.T, s.tb);
     __syncthreads();
     if (s.grids)
-      grid_groups<NC, WPROJ, J, COMP>(a, recs, s.list, g0, g1, swap, s.T, s.tb, s.du, s.strip, s.rows_mask, s.fbase, s.nxy,
-                                      sa, sb, s.fq, s.fqn, st);
+      grid_groups<NC, WPROJ, J, COMP>(a, recs, s.list, g0, g1, along_v, s.T, s.tb, s.du, s.strip, s.rows_mask, s.fbase,
+                                      s.nxy, s.gnx, s.fq, s.fqn, st);
     __syncthreads();
   }
   if (ng == 0) __syncthreads();
 }
 
-// End of a work item: the flush queue is emptied, then the owned cells are flushed.
+// End of a work item (or of a stretch of its rows): the flush queue is emptied, then the owned cells
+// are flushed and start at zero again, the additions of
+// two cells in flight together (compensated additions return the old value, and one cell at a time a
+// thread waits for the round trip of each; four at a time spill).
 template <int NC, bool WPROJ, int J, bool COMP>
-__device__ __forceinline__ void item_flush(const GridArgs &a, const ItemSetup<NC, WPROJ> &s, bool swap,
-                                           OwnerState<NC, J> &st) {
-  const int W = a.W, sa = swap ? s.gnx : 1, sb = swap ? 1 : s.gnx;
+__device__ __forceinline__ void item_flush(const GridArgs &a, const ItemSetup<NC, WPROJ> &s, OwnerState<NC, J> &st) {
+  const int W = a.W;
   if (COMP && s.grids) drain_queue<NC>(a, s.nxy, s.fq, s.fqn);
-  if (st.dirty) {
-    const long long slice = s.fbase + (long long)st.cg * NC * s.nxy + (long long)(st.pa0 + st.oa) * sa;
+  if (!st.dirty) return;
+  const long long slice = s.fbase + (long long)st.cg * NC * s.nxy + st.pu0 + st.ou;
+  auto cell_of = [&](int j) {
+    const int ov = st.ov0 + j >= W ? st.ov0 + j - W : st.ov0 + j;
+    return slice + (long long)(st.pv0 + ov) * s.gnx;
+  };
+#if defined(BULLSEYE_SINGLE)
+  if constexpr (COMP) {
+    constexpr int B = J < 2 ? J : 2;
 #pragma unroll
-    for (int j = 0; j < J; ++j) {
-      const int ob = st.ob0 + j >= W ? st.ob0 + j - W : st.ob0 + j;
-      if (st.dirty & (1u << j)) flush_cell<NC, COMP>(a, slice + (long long)(st.pb0 + ob) * sb, s.nxy, st.acc[j]);
+    for (int j0 = 0; j0 < J; j0 += B) {
+      float2 old[B][NC];
+#pragma unroll
+      for (int j = 0; j < B; ++j)
+        if (j0 + j < J && (st.dirty & (1u << (j0 + j)))) {
+#pragma unroll
+          for (int k = 0; k < NC; ++k)
+            old[j][k] = atomicAdd(reinterpret_cast<float2 *>(a.grid + cell_of(j0 + j) + k * s.nxy),
+                                  make_float2(st.acc[j0 + j][k].re, st.acc[j0 + j][k].im));
+        }
+#pragma unroll
+      for (int j = 0; j < B; ++j)
+        if (j0 + j < J && (st.dirty & (1u << (j0 + j)))) {
+#pragma unroll
+          for (int k = 0; k < NC; ++k)
+            compensated_add<NC>(a, cell_of(j0 + j) + k * s.nxy, make_float2(st.acc[j0 + j][k].re, st.acc[j0 + j][k].im),
+                                old[j][k]);
+#pragma unroll
+          for (int k = 0; k < NC; ++k) { st.acc[j0 + j][k].re = 0; st.acc[j0 + j][k].im = 0; }
+        }
     }
+    st.dirty = 0;
+    return;
   }
+#endif
+#pragma unroll
+  for (int j = 0; j < J; ++j)
+    if (st.dirty & (1u << j)) flush_cell<NC, false>(a, cell_of(j), s.nxy, st.acc[j]);
+  st.dirty = 0;
 }
 
-// One track (facet, channel, rows [r0, r1)) of one CTA: the rows are staged V at a time (prologue) and
-// gridded chunk by chunk.
+// Rows that an item's segments may add up to before the owned cells go out at a segment's end: cells of
+// slow tracks never leave the footprint, and plain accumulation over ever more channels would lose what
+// the compensated flushes hold (16 segments of 100 rows without it: 3.1e-7 of the grid against 64 bits
+// where one segment at a time has 1.9e-7).
+constexpr int kStayRows = 512;
+
+// Whether the rows of a channel's segments are taken last to first: a work item's segments are
+// consecutive channels of one baseline, and turning round at each channel continues where the channel
+// before it ended, a cell or less away, so that the owned cells stay in registers.
+__device__ __forceinline__ bool rows_backwards(int chan) { return chan & 1; }
+
+// What one CTA grids in place: its running state, and one row range (a channel's rows [r0, r1)) at a
+// time, staged V rows at a time (prologue) and gridded chunk by chunk.
 template <int NC, bool WPROJ, int J, bool COMP, bool WIDE>
-__device__ __forceinline__ void grid_track(const GridArgs &a, const int f_local, const int chan, long long r0,
-                                           long long r1) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int V = a.V;
-  VisRec<NC> *recs = reinterpret_cast<VisRec<NC> *>(smem_raw);                          // [V]
-  NormAcc *s_nacc = reinterpret_cast<NormAcc *>(smem_raw + sizeof(VisRec<NC>) * (size_t)V);  // [V][NC]
-  int *s_ng = reinterpret_cast<int *>(s_nacc + (size_t)V * NC);                             // [V]
+struct InPlace {
+  VisRec<NC> *recs;  // [V]
+  NormAcc *nacc;     // [V][NC]
+  int *ng;           // [V]
   ItemSetup<NC, WPROJ> s;
-  item_setup<NC, WPROJ, J, COMP, WIDE>(a, f_local, smem_raw, s);
-  if (r1 > a.nrows) r1 = a.nrows;
-  if (r0 >= r1) return;
-  const int tid = threadIdx.x, nt = blockDim.x;
-  const long long fslice = (long long)(a.facet_base + f_local) * a.groups;
-  const bool want_norm = a.norm != nullptr;
-  if (want_norm)
-    for (int i = tid; i < V; i += nt) {
-#pragma unroll
-      for (int k = 0; k < NC; ++k) norm_zero(s_nacc[i * NC + k]);
-      s_ng[i] = -1;
-    }
   OwnerState<NC, J> st;
-  owner_reset(st);
-  ChanCache cc;
-  const double plane_scale = WPROJ ? (double)(a.P - 1) / a.wmax : 0.0;
-  bool swap = false;
-  for (long long base = r0; base < r1; base += V) {
-    const int nv = (int)min((long long)V, r1 - base);
-    for (int i = tid; i < nv; i += nt) stage_slot<NC, WPROJ>(a, f_local, chan, base + i, true, i, recs, cc, plane_scale);
-    __syncthreads();
-    if (want_norm) {
-      if (a.tap_sums) {
-        for (int i = tid; i < nv; i += nt) norm_slot<NC>(a, recs[i], i, s_nacc, s_ng, fslice);
-      } else {
-        norm_from_taps<NC, WPROJ>(a, recs, nv, s.table, s_nacc, s_ng, fslice);
+  long long fslice;
+  bool along_v, first;
+  int stay;  // rows since the owned cells last went out
+
+  __device__ __forceinline__ void begin(const GridArgs &a, int f_local) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    recs = reinterpret_cast<VisRec<NC> *>(smem_raw);
+    nacc = reinterpret_cast<NormAcc *>(smem_raw + sizeof(VisRec<NC>) * (size_t)a.V);
+    ng = reinterpret_cast<int *>(nacc + (size_t)a.V * NC);
+    item_setup<NC, WPROJ, J, COMP, WIDE>(a, f_local, smem_raw, s);
+    fslice = (long long)(a.facet_base + f_local) * a.groups;
+    if (a.norm)
+      for (int i = threadIdx.x; i < a.V; i += blockDim.x) {
+#pragma unroll
+        for (int k = 0; k < NC; ++k) norm_zero(nacc[i * NC + k]);
+        ng[i] = -1;
       }
-    }
-    grid_chunk<NC, WPROJ, J, COMP>(a, recs, nv, base == r0, swap, s, st);
+    owner_reset(st);
+    along_v = false;
+    first = true;
+    stay = 0;
   }
-  item_flush<NC, WPROJ, J, COMP>(a, s, swap, st);
-  // normalisation: the slots' current partial sums (earlier grid groups went out when the group
-  // changed), summed over each warp by shuffles when its slots share one group (one atomic per
-  // correlation and warp), added slot by slot otherwise.  The slots' state was last written before
-  // the chunk loop's final barrier.
-  if (want_norm) {
-    for (int b = tid & ~31; b < V; b += nt) {
-      const int i = b + (tid & 31);
-      const bool has = i < V && s_ng[i] >= 0;
-      const int my_g = has ? s_ng[i] : -1;
+
+  __device__ __forceinline__ void rows(const GridArgs &a, int f_local, int chan, long long r0, long long r1) {
+    if (r1 > a.nrows) r1 = a.nrows;
+    const int tid = threadIdx.x, nt = blockDim.x;
+    ChanCache cc;
+    const double plane_scale = WPROJ ? (double)(a.P - 1) / a.wmax : 0.0;
+    const bool back = rows_backwards(chan);
+    for (long long base = r0; base < r1; base += a.V) {
+      const int nv = (int)min((long long)a.V, r1 - base);
+      for (int i = tid; i < nv; i += nt)
+        stage_slot<NC, WPROJ>(a, f_local, chan, back ? r1 - 1 - (base - r0) - i : base + i, true, i, recs, cc, plane_scale);
+      __syncthreads();
+      if (a.norm) {
+        if (a.tap_sums) {
+          for (int i = tid; i < nv; i += nt) norm_slot<NC>(a, recs[i], i, nacc, ng, fslice);
+        } else {
+          norm_from_taps<NC, WPROJ>(a, recs, nv, s.table, nacc, ng, fslice);
+        }
+      }
+      grid_chunk<NC, WPROJ, J, COMP>(a, recs, nv, first, along_v, s, st);
+      first = false;
+    }
+    stay += (int)(r1 - r0);
+  }
+  __device__ __forceinline__ void flush(const GridArgs &a) {
+    item_flush<NC, WPROJ, J, COMP>(a, s, st);
+    stay = 0;
+  }
+
+  // Normalisation, after the last rows.
+  __device__ __forceinline__ void end(const GridArgs &a) {
+    if (!a.norm || first) return;
+    // the slots' current partial sums (earlier grid groups went out when the group
+    // changed), summed over each warp by shuffles when its slots share one group (one atomic per
+    // correlation and warp), added slot by slot otherwise.  The slots' state was last written before
+    // the chunk loop's final barrier.
+    for (int b = threadIdx.x & ~31; b < a.V; b += blockDim.x) {
+      const int i = b + (threadIdx.x & 31);
+      const bool has = i < a.V && ng[i] >= 0;
+      const int my_g = has ? ng[i] : -1;
       const unsigned m = __ballot_sync(0xffffffffu, has);
       if (!m) continue;
       const int g0 = __shfl_sync(0xffffffffu, my_g, __ffs(m) - 1);
-      const NormAcc *na = s_nacc + (has ? i : 0) * NC;
+      const NormAcc *na = nacc + (has ? i : 0) * NC;
       if (__all_sync(0xffffffffu, !has || my_g == g0)) {
 #pragma unroll
         for (int k = 0; k < NC; ++k) {
           double v = has ? norm_value(na[k]) : 0.0;
 #pragma unroll
           for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-          if ((tid & 31) == 0 && v != 0.0) atomicAdd(&a.norm[(fslice + g0) * NC + k], v);
+          if ((threadIdx.x & 31) == 0 && v != 0.0) atomicAdd(&a.norm[(fslice + g0) * NC + k], v);
         }
       } else if (has) {
 #pragma unroll
@@ -1690,35 +1766,55 @@ __device__ __forceinline__ void grid_track(const GridArgs &a, const int f_local,
       }
     }
   }
-}
+};
 
-// One work item from precomputed records: its n records (src, 16-byte aligned) are staged V at a
-// time by one bulk copy each into two buffers used in turn, the next chunk's copy in flight while
-// the current chunk is gridded.  No prologue and no normalisation here (the record kernel did both).
-// rbar are the two record barriers (one arrival each), rphase their phase parities (bit b for buffer
-// b); a copy is only issued for a chunk of this item, so none is in flight when the item ends.
+// Most segments of one work item.
+constexpr int kMaxItemSegs = 16;
+
+// The records of a work item's segments, in the order that they are gridded: piece i holds records
+// [first[i], first[i + 1]) at src[i] (in shared memory, written by the CTA's first warp).
+template <int NC>
+struct RecordPieces {
+  const GridRec<NC> *src[kMaxItemSegs];
+  int first[kMaxItemSegs + 1];
+};
+
+// One work item from precomputed records: its pieces' records are staged V at a time by bulk copies
+// (one per piece that a chunk touches) into two buffers used in turn, the next chunk's copies in flight
+// while the current chunk is gridded.  No prologue and no normalisation here (the record kernel did
+// both).  rbar are the two record barriers (one arrival each), rphase their phase parities (bit b for
+// buffer b); copies are only issued for a chunk of this item, so none is in flight when the item ends.
 template <int NC, bool WPROJ, int J, bool COMP, bool WIDE>
-__device__ __forceinline__ void grid_track_pre(const GridArgs &a, const int f_local, const GridRec<NC> *src, int n,
-                                               unsigned long long *rbar, unsigned &rphase) {
+__device__ __forceinline__ void grid_records(const GridArgs &a, const int f_local, const RecordPieces<NC> &pc, int npieces,
+                                             unsigned long long *rbar, unsigned &rphase) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int V = a.V;
   GridRec<NC> *rb = reinterpret_cast<GridRec<NC> *>(smem_raw);  // [2][V]
+  const int n = pc.first[npieces];
   if (n <= 0) return;
   const int tid = threadIdx.x;
-  if (tid == 0) {
-    // the buffers may last have been written by plain stores (an item prepared in place)
+  int piece = 0;  // thread 0: the piece that the next chunk starts in
+  auto issue = [&](int c, int buf) {
+    const int lo = c * V, hi = min(n, lo + V);
+    // the buffer may last have been written by plain stores (an item prepared in place)
     fence_proxy_async();
-    const unsigned bytes = (unsigned)(sizeof(GridRec<NC>) * (size_t)min(V, n));
-    bar_arrive_tx(&rbar[0], bytes);
-    bulk_copy(rb, src, bytes, &rbar[0]);
-  }
+    bar_arrive_tx(&rbar[buf], (unsigned)(sizeof(GridRec<NC>) * (hi - lo)));
+    GridRec<NC> *dst = rb + buf * V;
+    for (int at = lo; at < hi;) {
+      while (pc.first[piece + 1] <= at) ++piece;
+      const int k = min(hi, pc.first[piece + 1]) - at;
+      bulk_copy(dst + (at - lo), pc.src[piece] + (at - pc.first[piece]), (unsigned)(sizeof(GridRec<NC>) * k), &rbar[buf]);
+      at += k;
+    }
+  };
+  if (tid == 0) issue(0, 0);
   ItemSetup<NC, WPROJ> s;
   item_setup<NC, WPROJ, J, COMP, WIDE>(a, f_local, smem_raw, s);
   OwnerState<NC, J> st;
   owner_reset(st);
-  bool swap = false;
+  bool along_v = false;
   const int nchunks = (n + V - 1) / V;
-  int cur = 0;
+  int cur = 0, stay = 0, last_piece = 0;
   for (int c = 0; c < nchunks; ++c, cur ^= 1) {
     const int nv = min(V, n - c * V);
     const unsigned par = (rphase >> cur) & 1u;
@@ -1727,16 +1823,23 @@ __device__ __forceinline__ void grid_track_pre(const GridArgs &a, const int f_lo
       bar_wait(&rbar[cur], par);
     }
     rphase ^= 1u << cur;
-    if (tid == 0 && c + 1 < nchunks) {
-      // the other buffer was last read by the previous chunk, which every thread has finished
-      const unsigned bytes = (unsigned)(sizeof(GridRec<NC>) * (size_t)min(V, n - (c + 1) * V));
-      fence_proxy_async();
-      bar_arrive_tx(&rbar[cur ^ 1], bytes);
-      bulk_copy(rb + (cur ^ 1) * V, src + (size_t)(c + 1) * V, bytes, &rbar[cur ^ 1]);
+    // the other buffer was last read by the previous chunk, which every thread has finished
+    if (tid == 0 && c + 1 < nchunks) issue(c + 1, cur ^ 1);
+    grid_chunk<NC, WPROJ, J, COMP>(a, rb + cur * V, nv, c == 0, along_v, s, st);
+    // the owned cells go out at the end, and before it once kStayRows rows are in and a segment ended
+    // in the chunk
+    stay += nv;
+    bool out = c + 1 == nchunks;
+    if (!out && stay >= kStayRows) {
+      const int was = last_piece;
+      while (pc.first[last_piece + 1] <= (c + 1) * V) ++last_piece;
+      out = last_piece != was;
     }
-    grid_chunk<NC, WPROJ, J, COMP>(a, rb + cur * V, nv, c == 0, swap, s, st);
+    if (out) {
+      item_flush<NC, WPROJ, J, COMP>(a, s, st);
+      stay = 0;
+    }
   }
-  item_flush<NC, WPROJ, J, COMP>(a, s, swap, st);
 }
 
 // Register caps of the persistent segment kernel: the J rows' accumulators (8 J values), the merge
@@ -1760,89 +1863,132 @@ __global__ void __launch_bounds__(512, 1) romein_grid_kernel(const GridArgs a) {
     r0 = (long long)slot * a.seg;
     r1 = min(a.nrows, r0 + a.seg);
   }
-  grid_track<NC, WPROJ, J, COMP, WIDE>(a, f_local, chan, r0, r1);
+  InPlace<NC, WPROJ, J, COMP, WIDE> work;
+  work.begin(a, f_local);
+  work.rows(a, f_local, chan, r0, r1);
+  work.flush(a);
+  work.end(a);
 }
 
-// Persistent form: a fixed grid of CTAs takes (segment, facet) work items from a device counter
-// until the device-side item count is exhausted; every segment is a run of one track's rows
-// whose w planes share this launch's support class (a.W).  Items of one segment are adjacent, so
-// the facets of a segment are gridded while its rows are hot in L2.  The loop ends on the count,
-// never waits on other CTAs.  Two builds share the items of a launch: PRE grids the items that the
-// record kernel had room for, the other build the rest (every item when there are no records); the
-// prologue of the latter would cost the former registers.
+// Persistent form: a fixed grid of CTAs takes work items from a device counter until the device-side
+// item count is exhausted.  Every segment is a run of one track's rows whose w planes share this
+// launch's support class (a.W), in the order (baseline, channel, rows), the rows of odd channels
+// backwards; an item is a block of consecutive segments in one facet, gridded as one stretch: the owned
+// cells go out when the footprint leaves them, and all of them only at the item's end.  The block is as
+// long as leaves eight items per CTA, kMaxItemSegs at most (gridding 27 antennas x 100 times x 64
+// channels into 16 facets, one segment per item spends a quarter of the class launches on the ends).
+// Items of one block are adjacent, so the facets of a segment are gridded while its rows are hot in L2.
+// The loop ends on the count, never waits on other CTAs.  Two builds share the segments of a launch:
+// PRE grids those that the record kernel had room for, the other build the rest (every segment when
+// there are no records); the prologue of the latter would cost the former registers.
 template <int NC, bool WPROJ, int J, bool COMP, bool WIDE, bool PRE, int REGS = kSegRegs<J>>
 __global__ void __launch_bounds__(512, 1) __maxnreg__(REGS) romein_segment_kernel(const GridArgs a, const int nfacets) {
   __shared__ int s_item;
-  __shared__ int s_first, s_last;  // unmasked row range of the item (facet row masks)
+  __shared__ int s_first, s_last;  // unmasked row range of a segment (facet row masks)
   __shared__ __align__(8) unsigned long long s_rec_bar[2];
+  __shared__ RecordPieces<NC> s_pieces;
   unsigned rphase = 0;
   if (PRE && threadIdx.x == 0) {
     bar_init(&s_rec_bar[0], 1);
     bar_init(&s_rec_bar[1], 1);
   }
   const int count = *a.work_count;
-  const long long total = (long long)count * nfacets;
+  const long long base = *a.segment_base;
+  const int per = (int)max(1ll, min((long long)kMaxItemSegs, (long long)count * nfacets / (8ll * gridDim.x)));
+  const long long total = (long long)((count + per - 1) / per) * nfacets;
+  // a segment of the schedule; false (reported) when it lies outside the schedule or the rows
+  auto segment = [&](long long si, int4 &sg) -> bool {
+    if (si < 0 || si >= a.segment_capacity) {
+      atomicOr(a.error, DEV_ERR_GRID_INDEX);
+      return false;
+    }
+    sg = a.segments[si];
+    if (sg.x < 0 || sg.x > sg.y || (long long)sg.y > a.nrows || sg.z < 0 || sg.z >= a.nchan) {
+      atomicOr(a.error, DEV_ERR_GRID_INDEX);
+      return false;
+    }
+    return true;
+  };
+  auto recorded = [&](long long si, int len) {
+    return a.records && (a.rec_off[si] + len) * nfacets <= a.rec_capacity;
+  };
   for (;;) {
     __syncthreads();
-    if (threadIdx.x == 0) {
-      s_item = atomicAdd(a.work_next, 1);
-      s_first = 0x7fffffff;
-      s_last = -1;
-    }
+    if (threadIdx.x == 0) s_item = atomicAdd(a.work_next, 1);
     __syncthreads();
     const long long item = s_item;
     if (item >= total) break;
-    const int seg = (int)(item / nfacets);
-    const int f_local = (int)(item - (long long)seg * nfacets);
-    const long long si = (long long)*a.segment_base + seg;
-    if (si < 0 || si >= a.segment_capacity) {  // schedule out of range: record and stop
-      if (threadIdx.x == 0) atomicOr(a.error, DEV_ERR_GRID_INDEX);
-      break;
-    }
-    const int4 sg = a.segments[si];
-    if (sg.x < 0 || sg.x > sg.y || (long long)sg.y > a.nrows || sg.z < 0 || sg.z >= a.nchan) {
-      if (threadIdx.x == 0) atomicOr(a.error, DEV_ERR_GRID_INDEX);
-      continue;
-    }
-    const long long len = (long long)sg.y - sg.x;
-    const bool recorded = a.records && (a.rec_off[si] + len) * nfacets <= a.rec_capacity;
-    if (recorded != PRE) continue;  // the other build's
+    const int block = (int)(item / nfacets);
+    const int f_local = (int)(item - (long long)block * nfacets);
+    const long long s0 = base + (long long)block * per;
+    const int nseg = min(per, count - block * per);
     if constexpr (PRE) {
-      // only the item's first to last valid record (all of them past the range table)
-      const long long it = si * nfacets + f_local;
-      int lo = 0, hi = (int)len;
-      if (it < a.range_capacity) {
-        const int2 rg = a.item_range[it];
-        lo = rg.x;
-        hi = rg.y;
-      }
-      if (lo < hi) {
-        const GridRec<NC> *src =
-            reinterpret_cast<const GridRec<NC> *>(a.records) + a.rec_off[si] * nfacets + (long long)f_local * len + lo;
-        grid_track_pre<NC, WPROJ, J, COMP, WIDE>(a, f_local, src, hi - lo, s_rec_bar, rphase);
-      }
-    } else {
-      long long r0 = sg.x, r1 = sg.y;
-      if (a.facet_row_mask) {
-        // a facet that leaves rows out grids only the item's first to last row it keeps, and skips
-        // the item when it keeps none (the rows in between are still tested in the prologue)
-        const uint8_t *m = a.facet_row_mask + (long long)(a.facet_base + f_local) * a.nrows;
-        int first = 0x7fffffff, last = -1;
-        for (int r = sg.x + (int)threadIdx.x; r < sg.y; r += (int)blockDim.x)
-          if (m[r]) {
-            first = min(first, r);
-            last = max(last, r);
+      // one lane per segment: its first to last valid record (all of them past the range table)
+      if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        int n = 0;
+        int4 sg;
+        if (lane < nseg && segment(s0 + lane, sg) && recorded(s0 + lane, sg.y - sg.x)) {
+          const long long si = s0 + lane, it = si * nfacets + f_local;
+          const int len = sg.y - sg.x;
+          int lo = 0, hi = len;
+          if (it < a.range_capacity) {
+            const int2 rg = a.item_range[it];
+            lo = rg.x;
+            hi = rg.y;
           }
-        if (last >= 0) {
-          atomicMin(&s_first, first);
-          atomicMax(&s_last, last);
+          n = max(0, hi - lo);
+          s_pieces.src[lane] = reinterpret_cast<const GridRec<NC> *>(a.records) + a.rec_off[si] * nfacets +
+                               (long long)f_local * len + lo;
         }
-        __syncthreads();
-        if (s_last < 0) continue;  // uniform: every thread reads the same shared values
-        r0 = s_first;
-        r1 = (long long)s_last + 1;
+        int sum = n;
+#pragma unroll
+        for (int off = 1; off < kMaxItemSegs; off <<= 1) {
+          const int x = __shfl_up_sync(0xffffffffu, sum, off);
+          if (lane >= off) sum += x;
+        }
+        if (lane == 0) s_pieces.first[0] = 0;
+        if (lane < nseg) s_pieces.first[lane + 1] = sum;
       }
-      grid_track<NC, WPROJ, J, COMP, WIDE>(a, f_local, sg.z, r0, r1);
+      __syncthreads();
+      grid_records<NC, WPROJ, J, COMP, WIDE>(a, f_local, s_pieces, nseg, s_rec_bar, rphase);
+    } else {
+      InPlace<NC, WPROJ, J, COMP, WIDE> work;
+      work.begin(a, f_local);
+      for (int i = 0;; ++i) {
+        if (i == nseg || work.stay >= kStayRows) work.flush(a);
+        if (i == nseg) break;
+        int4 sg;
+        if (!segment(s0 + i, sg) || recorded(s0 + i, sg.y - sg.x)) continue;
+        long long r0 = sg.x, r1 = sg.y;
+        if (a.facet_row_mask) {
+          // a facet that leaves rows out grids only the segment's first to last row it keeps, and skips
+          // the segment when it keeps none (the rows in between are still tested in the prologue)
+          __syncthreads();
+          if (threadIdx.x == 0) {
+            s_first = 0x7fffffff;
+            s_last = -1;
+          }
+          __syncthreads();
+          const uint8_t *m = a.facet_row_mask + (long long)(a.facet_base + f_local) * a.nrows;
+          int first = 0x7fffffff, last = -1;
+          for (int r = sg.x + (int)threadIdx.x; r < sg.y; r += (int)blockDim.x)
+            if (m[r]) {
+              first = min(first, r);
+              last = max(last, r);
+            }
+          if (last >= 0) {
+            atomicMin(&s_first, first);
+            atomicMax(&s_last, last);
+          }
+          __syncthreads();
+          if (s_last < 0) continue;  // uniform: every thread reads the same shared values
+          r0 = s_first;
+          r1 = (long long)s_last + 1;
+        }
+        work.rows(a, f_local, sg.z, r0, r1);
+      }
+      work.end(a);
     }
   }
 }

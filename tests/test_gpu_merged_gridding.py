@@ -70,3 +70,24 @@ def test_forms_and_correlations(precision, call, form, gpu_libs, oracle_libs):
     finally:
         lib.bullseye_set_visibility_records(1)
         lib.bullseye_set_batched_calls(1)
+
+
+@pytest.mark.parametrize("precision", ["double", "single"])
+@pytest.mark.parametrize("form", ["records", "in_place", "partial"])
+@pytest.mark.parametrize("n_chan,n_facets", [(1, 40), (37, 40)])
+def test_work_items_of_several_segments(precision, form, n_chan, n_facets, gpu_libs, oracle_libs):
+    """Enough (segment, facet) pairs that a work item takes several segments: tracks that change support
+    class, odd channels backwards, rows and channels that are left out, and a record budget that ends
+    inside an item."""
+    lib = gpu_libs[precision]
+    p = _problem(4, 6, 0.05, "u", n_facets, False, nx=65, n_times=41, n_chan=n_chan)
+    enabled = np.ones(n_chan, bool)
+    enabled[1::5] = False
+    p = replace(p, enabled_channels=enabled)
+    lib.bullseye_set_visibility_records(0 if form == "in_place" else 1)
+    lib.bullseye_set_record_budget((1 << 20) if form == "partial" else 0)
+    try:
+        _check(lib, oracle_libs["double"], p, "facet_4_cor", precision)
+    finally:
+        lib.bullseye_set_visibility_records(1)
+        lib.bullseye_set_record_budget(0)
