@@ -78,7 +78,7 @@ struct Context {
   cudaEvent_t ev_g0 = nullptr, ev_g1 = nullptr, ev_i0 = nullptr, ev_i1 = nullptr;
   bool grid_timing_pending = false, inv_timing_pending = false;
   double grid_seconds = 0.0, inv_seconds = 0.0;
-  bool compensated = true;  // FP32: compensated (hi/lo) grid accumulation
+  bool compensated = true;  // FP32: wide grid accumulation, else plain FP32
   bool device_inputs = false;  // row arrays, Jones terms and baseline starts are device pointers
   bool batched_calls = true;   // 4-correlation and sampling-function exports run the batched gridder
   bool jones_time_major = true;  // batched calls: the record kernel reads a time-innermost Jones copy
@@ -134,6 +134,9 @@ struct Context {
   // phase centre as facet centre, phase_transform_policies.h:77-82, so the uv transform is the
   // identity), which is gridded once into sf_acc/sf_lo [sf][ny][nx] and added to every facet.
   DevBuf<vis_complex> grid, grid_lo, sf, sf_acc, sf_lo, scratch, sf_out;
+  // form of grid/grid_lo and of sf_acc/sf_lo (32-bit library): wide (see convert_grid_kernel) after calls
+  // that accumulate wide, narrow after the others
+  bool grid_wide = false, sf_wide = false;
   DevBuf<double> norm;
   DevBuf<int> dev_error;
   std::vector<double> host_norm;  // published through params.normalization_terms

@@ -29,8 +29,9 @@
 //  * tap index = trunc((1 - u + round(u)) * os) + j*os; a visibility is dropped when
 //    disc + W + 2 >= n or disc < 0 (convolution_policies.h:86-97);
 //  * single-precision library: visibilities, taps and the register accumulation are FP32,
-//    the phase is evaluated by sincospif on the argument reduced in FP64 to turns; grid
-//    flushes can be compensated (hi/lo pair, TwoSum on the value returned by the atomic);
+//    the phase is evaluated by sincospif on the argument reduced in FP64 to turns; cells are
+//    added to the grid in FP64 (two FP64 planes in the place of an FP32 grid and its rounding
+//    errors), or in plain FP32 when compensation is off;
 //  * normalisation: sum over taps of the real tap weight times weight x flag
 //    (templated_gridder.h:97 and store_normalization_term), computed per visibility as
 //    Re(sum_j k_u[j] * sum_i k_v[i]) from kernel row sums precomputed in FP64, accumulated per
@@ -105,7 +106,7 @@ struct GridArgs {
   const FacetXform *facets;
   // outputs
   vis_complex *grid;             // slices [(f*groups + g)*NC + k][ny][nx]
-  vis_complex *grid_lo;          // compensation slices (same layout) or null
+  vis_complex *grid_lo;          // second word of the wide accumulation (same layout) or null
   double *norm;                  // [f][groups][NC] or null (sampling function)
   int *error;                    // sticky device error word
   // sizes and scalars
@@ -220,26 +221,41 @@ __device__ __forceinline__ cplx phase_factor(double x) {
 }
 #endif
 
-// Flush one owned cell's register accumulator into the grid (cell: the grid element of correlation 0).  Compensated mode adds with
-// atomics that return the previous value, then recovers each addition's rounding error exactly
-// (TwoSum: s = a + b, e = (a - (s - (s - a))) + (b - (s - a))) and adds it to the lo grid; the
-// final grid is hi + lo.  The NC atomics of a cell are issued before any result is consumed.
-template <int NC, bool COMP>
+// Flush one owned cell's register accumulator into the grid (cell: the grid element of correlation 0).
+//
+// WIDE accumulation (the 32-bit library's default): while a call grids, the 8 bytes of a cell in `grid`
+// hold the FP64 real part of its value and those in `grid_lo` the FP64 imaginary part
+// (kernels_misc.cuh converts).  The additions return nothing, so a thread never waits for
+// one.  Recovering each FP32 addition's rounding error from the value that a returning atomic gives
+// (TwoSum into the second grid) moves the same bytes at about the same rate (coalesced additions into L2:
+// 3.1e11 cells a second here, 3.6e11 there; beyond L2 1.4e11 against 1.2e11), but each flush then waits a
+// round trip, and the registers, queues and instructions around it cost more than the additions.
+#if defined(BULLSEYE_SINGLE)
+// x as FP64, on the integer pipe: the exponent rebiased by 1023 - 127, the fraction moved from 23 to 52
+// bits.  (The conversion instruction runs on the FP64 pipe, at 1/64 of the FP32 rate, and bounded the class
+// launches at 92 % of it.)  Denormals, infinities and NaN take the instruction, under a predicate.
+__device__ __forceinline__ double to_double(float x) {
+  const unsigned u = __float_as_uint(x), t = u & 0x7fffffffu;
+  const int hi = (((int)u >> 3) & (int)0x8fffffff) + 0x38000000;
+  double d = __hiloint2double(t ? hi : (int)u, (int)(u << 29));
+  if (t - 1u < 0x007fffffu || t >= 0x7f800000u) d = (double)x;
+  return d;
+}
+#endif
+
+template <int NC, bool WIDEACC>
 __device__ __forceinline__ void flush_cell(const GridArgs &a, long long cell, long long nxy, cplx (&acc)[NC]) {
 #if defined(BULLSEYE_SINGLE)
-  if (COMP) {
-    float2 old[NC];
+  if (WIDEACC) {
+    double *re = reinterpret_cast<double *>(a.grid) + cell, *im = reinterpret_cast<double *>(a.grid_lo) + cell;
+    unsigned any = 0;
 #pragma unroll
-    for (int k = 0; k < NC; ++k)
-      old[k] = atomicAdd(reinterpret_cast<float2 *>(a.grid + k * nxy + cell), make_float2(acc[k].re, acc[k].im));
+    for (int k = 0; k < NC; ++k) any |= __float_as_uint(acc[k].re) | __float_as_uint(acc[k].im);
+    if (!(any & 0x7fffffffu)) return;  // a zero cell: nothing to add (taps outside a plane's window are zero)
 #pragma unroll
     for (int k = 0; k < NC; ++k) {
-      float s0 = old[k].x + acc[k].re, b0 = s0 - old[k].x;
-      float e0 = (old[k].x - (s0 - b0)) + (acc[k].re - b0);
-      float s1 = old[k].y + acc[k].im, b1 = s1 - old[k].y;
-      float e1 = (old[k].y - (s1 - b1)) + (acc[k].im - b1);
-      if (e0 != 0.0f || e1 != 0.0f)
-        atomicAdd(reinterpret_cast<float2 *>(a.grid_lo + k * nxy + cell), make_float2(e0, e1));
+      atomicAdd(re + k * nxy, to_double(acc[k].re));
+      atomicAdd(im + k * nxy, to_double(acc[k].im));
     }
   } else {
 #pragma unroll
@@ -258,69 +274,6 @@ __device__ __forceinline__ void flush_cell(const GridArgs &a, long long cell, lo
     acc[k].re = 0;
     acc[k].im = 0;
   }
-}
-
-// Compensated flushes go through a per-warp queue in shared memory: a lane that must flush a
-// cell appends (cell, values) and carries on; when a queue holds kDrainAt records the warp drains
-// it with one record per lane, so the atomics' round trips overlap instead of serialising in the
-// lane that owns the cells.
-constexpr int kFlushQueueCap = 64;
-constexpr int kDrainAt = 32;
-
-template <int NC>
-struct FlushRec {
-  long long cell;        // grid element of correlation 0
-  float2 v[NC];
-};
-
-template <int NC>
-__device__ __forceinline__ void compensated_add(const GridArgs &a, long long idx, float2 val, float2 old) {
-  float s0 = old.x + val.x, b0 = s0 - old.x;
-  float e0 = (old.x - (s0 - b0)) + (val.x - b0);
-  float s1 = old.y + val.y, b1 = s1 - old.y;
-  float e1 = (old.y - (s1 - b1)) + (val.y - b1);
-  if (e0 != 0.0f || e1 != 0.0f) atomicAdd(reinterpret_cast<float2 *>(a.grid_lo + idx), make_float2(e0, e1));
-}
-
-// Drain the calling warp's queue (warp-uniform call).
-template <int NC>
-__device__ __forceinline__ void drain_queue(const GridArgs &a, long long nxy, FlushRec<NC> *q, int *qn) {
-#if defined(BULLSEYE_SINGLE)
-  __syncwarp();
-  const int n = min(*qn, kFlushQueueCap);
-  const int lane = threadIdx.x & 31;
-  for (int i = lane; i < n; i += 32) {
-    const FlushRec<NC> r = q[i];
-    float2 old[NC];
-#pragma unroll
-    for (int k = 0; k < NC; ++k) old[k] = atomicAdd(reinterpret_cast<float2 *>(a.grid + r.cell + k * nxy), r.v[k]);
-#pragma unroll
-    for (int k = 0; k < NC; ++k) compensated_add<NC>(a, r.cell + k * nxy, r.v[k], old[k]);
-  }
-  __syncwarp();
-  if (lane == 0) *qn = 0;
-  __syncwarp();
-#endif
-}
-
-// Queue one owned cell's accumulator (falls back to a direct flush when the queue is full).
-template <int NC>
-__device__ __forceinline__ void queue_cell(const GridArgs &a, long long cell, long long nxy, cplx (&acc)[NC],
-                                           FlushRec<NC> *q, int *qn) {
-#if defined(BULLSEYE_SINGLE)
-  const int slot = atomicAdd(qn, 1);
-  if (slot < kFlushQueueCap) {
-    FlushRec<NC> r;
-    r.cell = cell;
-#pragma unroll
-    for (int k = 0; k < NC; ++k) r.v[k] = make_float2(acc[k].re, acc[k].im);
-    q[slot] = r;
-#pragma unroll
-    for (int k = 0; k < NC; ++k) { acc[k].re = 0; acc[k].im = 0; }
-  } else {
-    flush_cell<NC, true>(a, cell, nxy, acc);
-  }
-#endif
 }
 
 // Per-visibility normalisation partial sums of a staged chunk (8 bytes per correlation either way).
@@ -1028,14 +981,21 @@ __device__ __forceinline__ void prologue(const GridArgs &a, int f_local, int cha
 // Taps are products: footprint cell (u, v) of a visibility gets vis x ku(u) x kv(v).  Consecutive
 // visibilities of a track sit a fraction of an oversampling step apart, so a stretch of them often
 // shares the footprint corner and one of the two tap rows.  Such a *group* is summed along the other
-// axis first; with a common kv,
-//     T(u) = sum over the group of vis x ku(u)            (W multiply-adds per visibility)
-//     cell(u, v) += T(u) x kv(v)                            (W^2 multiply-adds per group, not per visibility)
-// which is the same sum with its common factor taken out (and the other way round with a common ku).
+// axis first; with a common ku,
+//     T(v) = sum over the group of vis x kv(v)            (W multiply-adds per visibility)
+//     cell(u, v) += ku(u) x T(v)                            (W^2 multiply-adds per group, not per visibility)
+// which is the same sum with its common factor taken out (and the other way round with a common kv).
 // On Earth-rotation tracks sampled every 14 s (27 EVLA antennas, 1024-cell grids 1.4 degrees wide,
 // oversampling 15) groups hold 4.6 visibilities on average when each work item merges along the axis on
 // which its track moves more in tap steps; fixed to one axis they hold 2.3 (v) or 3.9 (u), and merging
 // only identical footprints gives 1.9.
+//
+// An item's axes are (a, b): b is the merge axis, (a, b) = (u, v) or (v, u).  A warp's lanes own columns
+// along a, a thread's J rows run along b, so that the frequent moves (along b) flush one row of a strip
+// with all its lanes.  A chunk of V records in shared memory is taken in two steps, in batches of GB groups:
+//   merge_groups  thread (i, part) forms T(i) of every nparts-th group of the batch, reading the taps
+//                 from the kernel table through L1, and copies the group's common tap row;
+//   grid_groups   the Romein owner threads add their column's tap x T(row) to their J cells.
 //
 // What the merge and the split of the builds measured (GB300, 27 antennas x 100 times x 64 channels,
 // 16 facets, whole batched call with copy-back): 36.5 -> 27.3 ms in single precision; 64-bit library,
@@ -1046,18 +1006,6 @@ __device__ __forceinline__ void prologue(const GridArgs &a, int f_local, int cha
 //                 from the kernel table through L1, and copies the group's common tap row;
 //   grid_groups   the Romein owner threads add T x tap to their J cells per column.  Columns run along
 //                 u whatever the merge axis, so that a warp's flushes are contiguous in the grid.
-
-// Per-warp flush queues (compensated single precision only): nwarps record arrays, then one
-// 16-byte counter slot per warp.
-template <int NC>
-__host__ __device__ inline size_t flush_queue_bytes(int nwarps) {
-#if defined(BULLSEYE_SINGLE)
-  return (size_t)nwarps * (sizeof(FlushRec<NC>) * kFlushQueueCap + 16);
-#else
-  (void)nwarps;
-  return 0;
-#endif
-}
 
 // Most records of a chunk: group lists are built from 64-bit masks.
 constexpr int kMaxChunk = 64;
@@ -1083,14 +1031,17 @@ __host__ __device__ inline size_t stage_head_bytes(int V) {
   const size_t pre = 2 * sizeof(GridRec<NC>);
   return ((own > pre ? own : pre) * (size_t)V + 15) / 16 * 16;
 }
-// Merged values and the common tap row of one group, W + J - 1 of each: the first J - 1 are repeated
-// after the last, so that a thread's J consecutive owned rows read consecutive entries without a wrap.
+// Merged values (W + J - 1: the first J - 1 are repeated after the last, so that a thread's J consecutive
+// owned rows read consecutive entries without a wrap) and the common tap row of one group.
 template <int NC, bool WPROJ>
 __host__ __device__ inline size_t merge_group_bytes(int W, int J) {
-  return (sizeof(cplx) * NC + sizeof(typename TapT<WPROJ>::type)) * (size_t)(W + J - 1);
+  return sizeof(cplx) * NC * (size_t)(W + J - 1) + sizeof(typename TapT<WPROJ>::type) * (size_t)W;
 }
-// One group list per warp.
-__host__ __device__ inline size_t group_list_bytes(int nwarps) { return (size_t)nwarps * kMaxChunk * sizeof(unsigned short); }
+// Per warp: the group list, and one column's values (flush_column).
+template <int NC>
+__host__ __device__ inline size_t warp_scratch_bytes(int J) {
+  return kMaxChunk * sizeof(unsigned short) + sizeof(cplx) * NC * (size_t)J;
+}
 
 // Staged records V, groups per batch GB and dynamic shared memory of a launch.
 struct ChunkShape {
@@ -1105,7 +1056,7 @@ struct ChunkShape {
 template <int NC, bool WPROJ>
 __host__ inline ChunkShape chunk_shape(int W, int nthreads, int J, int regs = 128) {
   const int nwarps = (nthreads + 31) / 32;
-  const size_t fixed = flush_queue_bytes<NC>(nwarps) + group_list_bytes(nwarps) + 64;
+  const size_t fixed = warp_scratch_bytes<NC>(J) * nwarps + 64;
   const size_t per = merge_group_bytes<NC, WPROJ>(W, J);
   ChunkShape s{32, 1, 0};
   for (int ctas = std::max(1, std::min(24, 65536 / (nthreads * regs)));; --ctas) {
@@ -1155,13 +1106,13 @@ __device__ __forceinline__ void owner_map(int tid, int W, int J, int &du, int &s
 }
 
 // Register state of a Romein owner thread: the accumulators of its J cells and the footprint they
-// belong to.  For the last footprint corner (pu0, pv0) the owned cells are
-// (pu0 + ou, pv0 + wrap(ov0 + j)), wrap(i) = i - W when i >= W.
+// belong to.  For the last footprint corner (pa0, pb0) the owned cells are
+// (pa0 + oa, pb0 + wrap(ob0 + j)), wrap(i) = i - W when i >= W.
 template <int NC, int J>
 struct OwnerState {
   cplx acc[J][NC];
   unsigned dirty;
-  int cg, pu0, pv0, ou, ov0;
+  int cg, pa0, pb0, oa, ob0;
 };
 
 template <int NC, int J>
@@ -1173,10 +1124,10 @@ __device__ __forceinline__ void owner_reset(OwnerState<NC, J> &st) {
   }
   st.dirty = 0;
   st.cg = -1;
-  st.pu0 = -1;
-  st.pv0 = -1;
-  st.ou = 0;
-  st.ov0 = 0;
+  st.pa0 = -1;
+  st.pb0 = -1;
+  st.oa = 0;
+  st.ob0 = 0;
 }
 
 // Prologue of one staging slot: the visibility of `row` staged into recs[slot].
@@ -1423,17 +1374,17 @@ __device__ __forceinline__ void merge_groups(const TapTable<WPROJ> &table, const
   const int S = W + J - 1;
   for (int gi = g0 + part; gi < g1; gi += nparts) {
     const int e = list[gi], s = e & 127, end = s + ((e >> 7) & 127);
-    const tap_t kb = read_tap(table, along_v ? recs[s].fu : recs[s].fv, i);
+    const tap_t ka0 = read_tap(table, along_v ? recs[s].fu : recs[s].fv, i);
     cplx t[NC];
 #pragma unroll
     for (int k = 0; k < NC; ++k) { t[k].re = 0; t[k].im = 0; }
     // four table loads in flight (past the end: the last one again)
     for (int v = s; v < end; v += 4) {
-      tap_t ka[4];
+      tap_t kb[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const int r = min(v + q, end - 1);
-        ka[q] = read_tap(table, along_v ? recs[r].fv : recs[r].fu, i);
+        kb[q] = read_tap(table, along_v ? recs[r].fv : recs[r].fu, i);
       }
 #pragma unroll
       for (int q = 0; q < 4; ++q)
@@ -1443,12 +1394,11 @@ __device__ __forceinline__ void merge_groups(const TapTable<WPROJ> &table, const
           for (int h = 0; h < M::H; ++h) {
             const typename M::type y = x[h];
 #pragma unroll
-            for (int n = 0; n < M::N; ++n) mac(t[h * M::N + n], y.v[n], ka[q]);
+            for (int n = 0; n < M::N; ++n) mac(t[h * M::N + n], y.v[n], kb[q]);
           }
         }
     }
     typename M::type *Tg = T + (gi - g0) * M::H * S;
-    tap_t *row = tb + (gi - g0) * S;
 #pragma unroll
     for (int h = 0; h < M::H; ++h) {
       typename M::type y;
@@ -1456,19 +1406,67 @@ __device__ __forceinline__ void merge_groups(const TapTable<WPROJ> &table, const
       for (int n = 0; n < M::N; ++n) y.v[n] = t[h * M::N + n];
       for (int j = i; j < S; j += W) Tg[h * S + j] = y;
     }
-    for (int j = i; j < S; j += W) row[j] = kb;
+    tb[(gi - g0) * W + i] = ka0;
   }
 }
 
-// Multiply-adds of groups [g0, g1) of a chunk into an owner thread's cells.  When the footprint moves,
-// the owned cells are recomputed and those that changed are flushed (queued for the warp's
-// compensated flush in single precision; the queue is drained when it fills and at the end of the
-// item).  Every lane of a warp with any owned cell calls this, so the queue drains are warp-uniform.
+// Adds one real component (part 0 real, 1 imaginary) of correlation k of a cell.
+template <bool COMP>
+__device__ __forceinline__ void add_component(const GridArgs &a, long long at, int part, acc_real x) {
+#if defined(BULLSEYE_SINGLE)
+  if (COMP)
+    atomicAdd(reinterpret_cast<double *>(part ? a.grid_lo : a.grid) + at, to_double(x));
+  else
+    atomicAdd(reinterpret_cast<float *>(a.grid + at) + part, x);
+#else
+  atomicAdd(reinterpret_cast<double *>(a.grid + at) + part, x);
+#endif
+}
+
+// Flushes the J cells of lane l of the calling warp (whole-warp call): the lane puts them in shared
+// memory and the warp's lanes add one component each.  By itself the lane would add its 2 NC J components
+// one after the other while the warp waits, which took a third of the class launches.  cell0: the grid
+// element of correlation 0 at row coordinate 0 of the lane's column.
+template <int NC, int J, bool COMP>
+__device__ __forceinline__ void flush_column(const GridArgs &a, int l, int W, long long cell0, long long nxy, int sb,
+                                             cplx *buf, OwnerState<NC, J> &st) {
+  const int lane = threadIdx.x & 31;
+  const unsigned dirty = __shfl_sync(0xffffffffu, st.dirty, l);
+  const int ob0 = __shfl_sync(0xffffffffu, st.ob0, l);
+  cell0 = __shfl_sync(0xffffffffu, cell0, l);
+  if (lane == l) {
+#pragma unroll
+    for (int j = 0; j < J; ++j)
+#pragma unroll
+      for (int k = 0; k < NC; ++k) {
+        buf[j * NC + k] = st.acc[j][k];
+        st.acc[j][k].re = 0;
+        st.acc[j][k].im = 0;
+      }
+    st.dirty = 0;
+  }
+  __syncwarp();
+#pragma unroll
+  for (int c0 = 0; c0 < J * NC * 2; c0 += 32) {
+    const int c = c0 + lane, j = c / (2 * NC), k = (c >> 1) % NC;
+    if (c < J * NC * 2 && (dirty >> j & 1)) {
+      const int ob = ob0 + j >= W ? ob0 + j - W : ob0 + j;
+      add_component<COMP>(a, cell0 + (long long)(st.pb0 + ob) * sb + k * nxy, c & 1,
+                          reinterpret_cast<const acc_real *>(buf)[c]);
+    }
+  }
+  __syncwarp();
+}
+
+// Multiply-adds of groups [g0, g1) of a chunk into an owner thread's cells (whole-warp call).  When the
+// footprint moves, the owned cells are recomputed and those that changed are flushed: rows that moved by
+// every lane of their strip, one or two columns that moved by flush_column.  Cells lie sa (along a) and
+// sb (along b) elements apart.
 template <int NC, bool WPROJ, int J, bool COMP, class Rec>
 __device__ __forceinline__ void grid_groups(const GridArgs &a, const Rec *recs, const unsigned short *list, int g0, int g1,
                                             bool along_v, const typename MergeVec<NC>::type *T,
                                             const typename TapT<WPROJ>::type *tb, int du, int strip, unsigned rows_mask,
-                                            long long fbase, long long nxy, int gnx, FlushRec<NC> *fq, int *fqn,
+                                            long long fbase, long long nxy, int gnx, cplx *col_buf,
                                             OwnerState<NC, J> &st) {
   typedef typename TapT<WPROJ>::type tap_t;
   typedef MergeVec<NC> M;
@@ -1479,72 +1477,51 @@ __device__ __forceinline__ void grid_groups(const GridArgs &a, const Rec *recs, 
       const int rs = e & 127;
       const int4 h = *reinterpret_cast<const int4 *>(&recs[rs].u0);
       const int g = recs[rs].g;
-      if (h.x != st.pu0 || h.y != st.pv0 || g != st.cg) {
-        // footprint moved: recompute the owned cells, flush those that changed
-        int o = du - h.z;
+      const int a0 = along_v ? h.x : h.y, b0 = along_v ? h.y : h.x;
+      if (a0 != st.pa0 || b0 != st.pb0 || g != st.cg) {
+        const int sa = along_v ? 1 : gnx, sb = along_v ? gnx : 1;
+        int o = du - (along_v ? h.z : h.w);
         o += (o < 0) ? W : 0;
-        int nov0 = strip * J - h.w;
-        nov0 += (nov0 < 0) ? W : 0;
+        int nob0 = strip * J - (along_v ? h.w : h.z);
+        nob0 += (nob0 < 0) ? W : 0;
+        const long long cell0 = fbase + (long long)st.cg * NC * nxy + (long long)(st.pa0 + st.oa) * sa;
+        bool out = st.dirty && (a0 + o != st.pa0 + st.oa || g != st.cg);  // the column moved
+        const unsigned m = __ballot_sync(0xffffffffu, out);
+        if (m && __popc(m) <= 2) {
+          flush_column<NC, J, COMP>(a, __ffs(m) - 1, W, cell0, nxy, sb, col_buf, st);
+          if (m & (m - 1)) flush_column<NC, J, COMP>(a, 31 - __clz(m), W, cell0, nxy, sb, col_buf, st);
+        }
         if (st.dirty) {
-          const bool all = h.x + o != st.pu0 + st.ou || g != st.cg;
-          const long long slice = fbase + (long long)st.cg * NC * nxy + st.pu0 + st.ou;
 #pragma unroll
           for (int j = 0; j < J; ++j) {
-            const int ov = st.ov0 + j >= W ? st.ov0 + j - W : st.ov0 + j;
-            const int nv = nov0 + j >= W ? nov0 + j - W : nov0 + j;
-            if ((st.dirty & (1u << j)) && (all || h.y + nv != st.pv0 + ov)) {
-              const long long cell = slice + (long long)(st.pv0 + ov) * gnx;
-              if (COMP)
-                queue_cell<NC>(a, cell, nxy, st.acc[j], fq, fqn);
-              else
-                flush_cell<NC, false>(a, cell, nxy, st.acc[j]);
+            const int ob = st.ob0 + j >= W ? st.ob0 + j - W : st.ob0 + j;
+            const int nb = nob0 + j >= W ? nob0 + j - W : nob0 + j;
+            if ((st.dirty & (1u << j)) && (out || b0 + nb != st.pb0 + ob)) {
+              flush_cell<NC, COMP>(a, cell0 + (long long)(st.pb0 + ob) * sb, nxy, st.acc[j]);
               st.dirty &= ~(1u << j);
             }
           }
         }
         st.cg = g;
         // columns beyond W (padding lanes) read in-bounds values and are never flushed
-        st.ou = o < W ? o : W - 1;
-        st.ov0 = nov0 < W ? nov0 : 0;  // lanes past the last strip own nothing: keep their reads in bounds
-        st.pu0 = h.x;
-        st.pv0 = h.y;
-        if (COMP) {  // the queue only grows here; the branch is uniform over the warp
-          __syncwarp();
-          if (*fqn >= kDrainAt) drain_queue<NC>(a, nxy, fq, fqn);
-        }
+        st.oa = o < W ? o : W - 1;
+        st.ob0 = nob0 < W ? nob0 : 0;  // lanes past the last strip own nothing: keep their reads in bounds
+        st.pa0 = a0;
+        st.pb0 = b0;
       }
     }
     // branch-free multiply-adds over the J owned rows (offsets modulo W; rows of non-owning lanes stay
     // in bounds and are never flushed)
-    const typename M::type *Tg = T + (gi - g0) * M::H * S;
-    const tap_t *row = tb + (gi - g0) * S;
-    if (along_v) {
-      const tap_t k = row[st.ou];
-      Tg += st.ov0;
+    const typename M::type *Tg = T + (gi - g0) * M::H * S + st.ob0;
+    const tap_t k = tb[(gi - g0) * W + st.oa];
 #pragma unroll
-      for (int j = 0; j < J; ++j)
-#pragma unroll
-        for (int h = 0; h < M::H; ++h) {
-          const typename M::type y = Tg[h * S + j];
-#pragma unroll
-          for (int n = 0; n < M::N; ++n) mac(st.acc[j][h * M::N + n], y.v[n], k);
-        }
-    } else {
-      cplx t[NC];
+    for (int j = 0; j < J; ++j)
 #pragma unroll
       for (int h = 0; h < M::H; ++h) {
-        const typename M::type y = Tg[h * S + st.ou];
+        const typename M::type y = Tg[h * S + j];
 #pragma unroll
-        for (int n = 0; n < M::N; ++n) t[h * M::N + n] = y.v[n];
+        for (int n = 0; n < M::N; ++n) mac(st.acc[j][h * M::N + n], y.v[n], k);
       }
-      row += st.ov0;
-#pragma unroll
-      for (int j = 0; j < J; ++j) {
-        const tap_t k = row[j];
-#pragma unroll
-        for (int c = 0; c < NC; ++c) mac(st.acc[j][c], t[c], k);
-      }
-    }
     st.dirty |= rows_mask;
   }
 }
@@ -1553,10 +1530,9 @@ __device__ __forceinline__ void grid_groups(const GridArgs &a, const Rec *recs, 
 template <int NC, bool WPROJ>
 struct ItemSetup {
   typename MergeVec<NC>::type *T;        // [GB][H][W + J - 1]
-  typename TapT<WPROJ>::type *tb;        // [GB][W + J - 1]
+  typename TapT<WPROJ>::type *tb;        // [GB][W]
   unsigned short *list;                  // this warp's group list
-  FlushRec<NC> *fq;                      // this warp's flush queue
-  int *fqn;
+  cplx *col_buf;                         // this warp's column buffer [J][NC]
   TapTable<WPROJ> table;
   int du, strip, ax, ap, nparts, gnx;
   unsigned rows_mask;
@@ -1568,18 +1544,16 @@ __device__ __forceinline__ void item_setup(const GridArgs &a, int f_local, unsig
   typedef typename MergeVec<NC>::type vec_t;
   typedef typename TapT<WPROJ>::type tap_t;
   const int W = a.W, GB = a.GB, tid = threadIdx.x;
-  const int warp_id = tid >> 5, nwarps = (blockDim.x + 31) >> 5;
+  const int warp_id = tid >> 5;
   unsigned char *p = smem + stage_head_bytes<NC>(a.V);
   s.T = reinterpret_cast<vec_t *>(p);
   p += sizeof(cplx) * NC * (size_t)(W + J - 1) * GB;
   s.tb = reinterpret_cast<tap_t *>(p);
-  p += sizeof(tap_t) * (size_t)(W + J - 1) * GB;
+  p += sizeof(tap_t) * (size_t)W * GB;
   p = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(p) + 15) & ~(uintptr_t)15);
-  s.list = reinterpret_cast<unsigned short *>(p) + warp_id * kMaxChunk;
-  p += group_list_bytes(nwarps);
-  s.fq = reinterpret_cast<FlushRec<NC> *>(p) + warp_id * kFlushQueueCap;
-  s.fqn = reinterpret_cast<int *>(p + nwarps * sizeof(FlushRec<NC>) * kFlushQueueCap) + warp_id * 4;
-  if (COMP && (tid & 31) == 0) *s.fqn = 0;
+  p += warp_scratch_bytes<NC>(J) * warp_id;
+  s.col_buf = reinterpret_cast<cplx *>(p);
+  s.list = reinterpret_cast<unsigned short *>(s.col_buf + J * NC);
   s.table = tap_table<WPROJ>(a);
   bool owner;
   owner_map<WIDE>(tid, W, J, s.du, s.strip, owner);
@@ -1610,64 +1584,30 @@ __device__ __forceinline__ void grid_chunk(const GridArgs &a, const Rec *recs, i
     __syncthreads();
     if (s.grids)
       grid_groups<NC, WPROJ, J, COMP>(a, recs, s.list, g0, g1, along_v, s.T, s.tb, s.du, s.strip, s.rows_mask, s.fbase,
-                                      s.nxy, s.gnx, s.fq, s.fqn, st);
+                                      s.nxy, s.gnx, s.col_buf, st);
     __syncthreads();
   }
   if (ng == 0) __syncthreads();
 }
 
-// End of a work item (or of a stretch of its rows): the flush queue is emptied, then the owned cells
-// are flushed and start at zero again, the additions of
-// two cells in flight together (compensated additions return the old value, and one cell at a time a
-// thread waits for the round trip of each; four at a time spill).
+// End of a work item (or of a stretch of its rows): the owned cells are flushed and start at zero again.
 template <int NC, bool WPROJ, int J, bool COMP>
-__device__ __forceinline__ void item_flush(const GridArgs &a, const ItemSetup<NC, WPROJ> &s, OwnerState<NC, J> &st) {
-  const int W = a.W;
-  if (COMP && s.grids) drain_queue<NC>(a, s.nxy, s.fq, s.fqn);
+__device__ __forceinline__ void item_flush(const GridArgs &a, const ItemSetup<NC, WPROJ> &s, bool along_v,
+                                           OwnerState<NC, J> &st) {
   if (!st.dirty) return;
-  const long long slice = s.fbase + (long long)st.cg * NC * s.nxy + st.pu0 + st.ou;
-  auto cell_of = [&](int j) {
-    const int ov = st.ov0 + j >= W ? st.ov0 + j - W : st.ov0 + j;
-    return slice + (long long)(st.pv0 + ov) * s.gnx;
-  };
-#if defined(BULLSEYE_SINGLE)
-  if constexpr (COMP) {
-    constexpr int B = J < 2 ? J : 2;
+  const int sa = along_v ? 1 : s.gnx, sb = along_v ? s.gnx : 1;
+  const long long cell0 = s.fbase + (long long)st.cg * NC * s.nxy + (long long)(st.pa0 + st.oa) * sa;
 #pragma unroll
-    for (int j0 = 0; j0 < J; j0 += B) {
-      float2 old[B][NC];
-#pragma unroll
-      for (int j = 0; j < B; ++j)
-        if (j0 + j < J && (st.dirty & (1u << (j0 + j)))) {
-#pragma unroll
-          for (int k = 0; k < NC; ++k)
-            old[j][k] = atomicAdd(reinterpret_cast<float2 *>(a.grid + cell_of(j0 + j) + k * s.nxy),
-                                  make_float2(st.acc[j0 + j][k].re, st.acc[j0 + j][k].im));
-        }
-#pragma unroll
-      for (int j = 0; j < B; ++j)
-        if (j0 + j < J && (st.dirty & (1u << (j0 + j)))) {
-#pragma unroll
-          for (int k = 0; k < NC; ++k)
-            compensated_add<NC>(a, cell_of(j0 + j) + k * s.nxy, make_float2(st.acc[j0 + j][k].re, st.acc[j0 + j][k].im),
-                                old[j][k]);
-#pragma unroll
-          for (int k = 0; k < NC; ++k) { st.acc[j0 + j][k].re = 0; st.acc[j0 + j][k].im = 0; }
-        }
-    }
-    st.dirty = 0;
-    return;
+  for (int j = 0; j < J; ++j) {
+    const int ob = st.ob0 + j >= a.W ? st.ob0 + j - a.W : st.ob0 + j;
+    if (st.dirty & (1u << j)) flush_cell<NC, COMP>(a, cell0 + (long long)(st.pb0 + ob) * sb, s.nxy, st.acc[j]);
   }
-#endif
-#pragma unroll
-  for (int j = 0; j < J; ++j)
-    if (st.dirty & (1u << j)) flush_cell<NC, false>(a, cell_of(j), s.nxy, st.acc[j]);
   st.dirty = 0;
 }
 
 // Rows that an item's segments may add up to before the owned cells go out at a segment's end: cells of
 // slow tracks never leave the footprint, and plain accumulation over ever more channels would lose what
-// the compensated flushes hold (16 segments of 100 rows without it: 3.1e-7 of the grid against 64 bits
+// the wide flushes hold (16 segments of 100 rows without it: 3.1e-7 of the grid against 64 bits
 // where one segment at a time has 1.9e-7).
 constexpr int kStayRows = 512;
 
@@ -1732,7 +1672,7 @@ struct InPlace {
     stay += (int)(r1 - r0);
   }
   __device__ __forceinline__ void flush(const GridArgs &a) {
-    item_flush<NC, WPROJ, J, COMP>(a, s, st);
+    item_flush<NC, WPROJ, J, COMP>(a, s, along_v, st);
     stay = 0;
   }
 
@@ -1836,7 +1776,7 @@ __device__ __forceinline__ void grid_records(const GridArgs &a, const int f_loca
       out = last_piece != was;
     }
     if (out) {
-      item_flush<NC, WPROJ, J, COMP>(a, s, st);
+      item_flush<NC, WPROJ, J, COMP>(a, s, along_v, st);
       stay = 0;
     }
   }
@@ -1994,3 +1934,9 @@ __global__ void __launch_bounds__(512, 1) __maxnreg__(REGS) romein_segment_kerne
 }
 
 }  // namespace bz
+
+// Queues the conversion of n cells of a narrow grid to the wide form of the 32-bit library's accumulation
+// (have_lo: its second word holds a value; else it is written), and back, in place or to `out` as one word
+// (kernels_misc.cuh); no work in the 64-bit library.
+bool bz_widen_grid(vis_complex *hi, vis_complex *lo, long long n, bool have_lo, cudaStream_t st);
+bool bz_narrow_grid(vis_complex *hi, vis_complex *lo, vis_complex *out, long long n, cudaStream_t st);

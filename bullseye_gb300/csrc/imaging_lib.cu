@@ -262,7 +262,7 @@ extern "C" double bullseye_fp32_fma_tflops(int iters) {
   return ms > 0 ? flops / (ms * 1e-3) / 1e12 : 0.0;
 }
 
-// Zero the device-resident grids, compensation grids and normalisation sums (a fresh image
+// Zero the device-resident grids (zero in either form) and normalisation sums (a fresh image
 // without reallocating; the caller's host buffers are untouched).
 extern "C" void bullseye_zero_grids() {
   Context &c = g_ctx;
@@ -465,6 +465,7 @@ extern "C" void initLibrary(gridding_parameters *pp) {
   if (!c.grid_lo.alloc(ng)) return;
   BZ_CUDA_TRY(cudaMemset(c.grid_lo.ptr, 0, sizeof(vis_complex) * ng));
 #endif
+  c.grid_wide = c.sf_wide = false;
   if (c.want_sf) {
     const size_t ns = c.F * c.sf_count * nxy;
     if (!c.sf.alloc(ns)) return;
@@ -727,8 +728,43 @@ static void device_tracks(const gridding_parameters &p, int &nslots, int &seg, c
 }
 
 bool bz_check_ready(const char *fn) { return check_ready(fn); }
+bool bz_widen_grid(vis_complex *hi, vis_complex *lo, long long n, bool have_lo, cudaStream_t st) {
+#if defined(BULLSEYE_SINGLE)
+  if (have_lo)
+    convert_grid_kernel<true><<<152 * 8, 256, 0, st>>>(hi, lo, n);
+  else
+    widen_grid_new_kernel<<<2048, 256, 0, st>>>(hi, lo, n);
+#endif
+  return cudaGetLastError() == cudaSuccess;
+}
+bool bz_narrow_grid(vis_complex *hi, vis_complex *lo, vis_complex *out, long long n, cudaStream_t st) {
+#if defined(BULLSEYE_SINGLE)
+  if (out)
+    resolve_grid_kernel<<<2048, 256, 0, st>>>(hi, lo, true, out, n);
+  else
+    convert_grid_kernel<false><<<152 * 8, 256, 0, st>>>(hi, lo, n);
+#endif
+  return cudaGetLastError() == cudaSuccess;
+}
+
+// The library's grid (or sampling grid) in the form that the next call adds to.
+static bool grid_form(bool sampling, bool wide) {
+  Context &c = g_ctx;
+  bool &now = sampling ? c.sf_wide : c.grid_wide;
+  if (now == wide) return true;
+  vis_complex *hi = sampling ? c.sf_acc.ptr : c.grid.ptr, *lo = sampling ? c.sf_lo.ptr : c.grid_lo.ptr;
+  const long long n = (long long)((sampling ? c.sf_count : c.F * c.cube * c.C) * c.nx * c.ny);
+  if (!(wide ? bz_widen_grid(hi, lo, n, true, c.stream) : bz_narrow_grid(hi, lo, nullptr, n, c.stream))) {
+    bz_record_error(BZ_ERR_CUDA, "grid conversion failed to launch");
+    return false;
+  }
+  c.launches++;
+  now = wide;
+  return true;
+}
+
 void bz_copy_back_grids(gridding_parameters &p, bool sampling);
-// Final-chunk copy-back, queued without waiting: the resolved grids (hi + lo) and the normalisation
+// Final-chunk copy-back, queued without waiting: the resolved grids and the normalisation
 // sums are copied to the caller's buffers on the copy stream, overlapping whatever the library
 // stream does next (the sampling-function call of the chunk); gridding_barrier waits for them and
 // publishes the normalisation terms.  A copy-back buffer is rewritten only after its previous copy.
@@ -738,7 +774,7 @@ static void copy_back_grids(gridding_parameters &p, bool sampling) {
   if (!sampling) {
     const size_t n = c.F * c.cube * c.C * nxy;
     BZ_CUDA_TRY(cudaStreamWaitEvent(c.stream, c.ev_copied_vis, 0));
-    resolve_compensated_kernel<<<1024, 256, 0, c.stream>>>(c.grid.ptr, c.grid_lo.ptr, c.scratch.ptr, (long long)n);
+    resolve_grid_kernel<<<1024, 256, 0, c.stream>>>(c.grid.ptr, c.grid_lo.ptr, c.grid_wide, c.scratch.ptr, (long long)n);
     c.launches++;
     BZ_CUDA_TRY(cudaEventRecord(c.ev_ready_vis, c.stream));
     BZ_CUDA_TRY(cudaStreamWaitEvent(c.copy_stream, c.ev_ready_vis, 0));
@@ -752,7 +788,7 @@ static void copy_back_grids(gridding_parameters &p, bool sampling) {
   } else {
     const size_t n = c.F * c.sf_count * nxy;
     BZ_CUDA_TRY(cudaStreamWaitEvent(c.stream, c.ev_copied_sf, 0));
-    broadcast_add_kernel<<<1024, 256, 0, c.stream>>>(c.sf.ptr, c.sf_acc.ptr, c.sf_lo.ptr, c.sf_out.ptr,
+    broadcast_add_kernel<<<1024, 256, 0, c.stream>>>(c.sf.ptr, c.sf_acc.ptr, c.sf_lo.ptr, c.sf_wide, c.sf_out.ptr,
                                                     (long long)(c.sf_count * nxy), (long long)c.F);
     c.launches++;
     BZ_CUDA_TRY(cudaEventRecord(c.ev_ready_sf, c.stream));
@@ -921,6 +957,7 @@ bool bz_prepare_grid_args(const gridding_parameters &p, int nc, int mode, bool f
   a.grid_lo = nullptr;
 #if defined(BULLSEYE_SINGLE)
   if (c.compensated) a.grid_lo = sampling ? c.sf_lo.ptr : c.grid_lo.ptr;
+  if (!grid_form(sampling, c.compensated)) return false;
 #endif
   a.norm = sampling ? nullptr : c.norm.ptr;
   a.error = c.dev_error.ptr;

@@ -1,4 +1,4 @@
-// Small device kernels around the gridder: Jones inversion, compensated-grid resolution,
+// Small device kernels around the gridder: Jones inversion, the grids' two forms,
 // and the finalize (shift / real-part packing / gridding correction) passes.
 #pragma once
 #include "common.h"
@@ -66,33 +66,118 @@ __global__ void invert_jones_kernel(const vis_complex *__restrict__ in, vis_comp
   if (o2) { o2[0] = r0; o2[1] = r1; o2[2] = r2; o2[3] = r3; }
 }
 
-// out = hi + lo (compensated grid resolution), element-wise over complex values.
-__global__ void resolve_compensated_kernel(const vis_complex *__restrict__ hi, const vis_complex *__restrict__ lo,
-                                           vis_complex *__restrict__ out, long long n) {
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    vis_complex h = hi[i];
-    if (lo) {
-      vis_complex l = lo[i];
-      h.re += l.re;
-      h.im += l.im;
+#if defined(BULLSEYE_SINGLE)
+// The two forms of a single-precision grid: *narrow*, a value is hi + lo of two FP32 complex words, and
+// *wide*, the form that the wide accumulation adds to: the 8 bytes of hi hold the FP64 real part, those of
+// lo the imaginary part.  A conversion works in place, on both words of a cell at once.  A zero cell has
+// the same bits in both forms and is left alone: most of a grid is zero (the tracks of a bench facet
+// cover 6 % of it), the kernels then read 16 bytes a cell (HBM), and the FP64 pipe is kept for the rest.
+__device__ __forceinline__ bool widen_cell(uint2 &h, uint2 &l) {
+  if ((h.x | h.y | l.x | l.y) == 0) return false;
+  const double re = (double)__uint_as_float(h.x) + (double)__uint_as_float(l.x);
+  const double im = (double)__uint_as_float(h.y) + (double)__uint_as_float(l.y);
+  h = make_uint2((unsigned)__double2loint(re), (unsigned)__double2hiint(re));
+  l = make_uint2((unsigned)__double2loint(im), (unsigned)__double2hiint(im));
+  return true;
+}
+__device__ __forceinline__ bool narrow_cell(uint2 &h, uint2 &l) {
+  if ((h.x | h.y | l.x | l.y) == 0) return false;
+  const double re = __hiloint2double((int)h.y, (int)h.x), im = __hiloint2double((int)l.y, (int)l.x);
+  const float a = (float)re, b = (float)im;
+  h = make_uint2(__float_as_uint(a), __float_as_uint(b));
+  l = make_uint2(__float_as_uint((float)(re - (double)a)), __float_as_uint((float)(im - (double)b)));
+  return true;
+}
+// Both directions over n cells, eight cells per thread in flight (16-byte loads of two cells when both
+// buffers allow them, cell by cell otherwise).
+template <bool WIDEN>
+__global__ void __launch_bounds__(256) convert_grid_kernel(vis_complex *hi, vis_complex *lo, long long n) {
+  const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x, nt = (long long)gridDim.x * blockDim.x;
+  auto one = [](uint2 &h, uint2 &l) { return WIDEN ? widen_cell(h, l) : narrow_cell(h, l); };
+  long long done = 0;
+  if (((reinterpret_cast<uintptr_t>(hi) | reinterpret_cast<uintptr_t>(lo)) & 15) == 0) {
+    uint4 *ph = reinterpret_cast<uint4 *>(hi), *pl = reinterpret_cast<uint4 *>(lo);
+    const long long pairs = n / 2;
+    for (long long i = tid; i < pairs; i += 4 * nt) {
+      uint4 h[4], l[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (i + q * nt < pairs) {
+          h[q] = ph[i + q * nt];
+          l[q] = pl[i + q * nt];
+        } else {
+          h[q] = l[q] = make_uint4(0, 0, 0, 0);
+        }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        uint2 h0 = make_uint2(h[q].x, h[q].y), h1 = make_uint2(h[q].z, h[q].w);
+        uint2 l0 = make_uint2(l[q].x, l[q].y), l1 = make_uint2(l[q].z, l[q].w);
+        const bool c0 = one(h0, l0), c1 = one(h1, l1);
+        if (c0 || c1) {
+          ph[i + q * nt] = make_uint4(h0.x, h0.y, h1.x, h1.y);
+          pl[i + q * nt] = make_uint4(l0.x, l0.y, l1.x, l1.y);
+        }
+      }
     }
-    out[i] = h;
+    done = 2 * pairs;
+  }
+  for (long long i = done + tid; i < n; i += nt) {
+    uint2 h = reinterpret_cast<uint2 *>(hi)[i], l = reinterpret_cast<uint2 *>(lo)[i];
+    if (one(h, l)) {
+      reinterpret_cast<uint2 *>(hi)[i] = h;
+      reinterpret_cast<uint2 *>(lo)[i] = l;
+    }
   }
 }
+// The same for a grid without a second word yet (lo is written).
+__global__ void widen_grid_new_kernel(vis_complex *hi, vis_complex *lo, long long n) {
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    const uint2 h = reinterpret_cast<const uint2 *>(hi)[i];
+    double im = 0.0;
+    if (h.x | h.y) {
+      reinterpret_cast<double *>(hi)[i] = (double)__uint_as_float(h.x);
+      im = (double)__uint_as_float(h.y);
+    }
+    reinterpret_cast<double *>(lo)[i] = im;
+  }
+}
+#endif
 
-// out[f][i] = init[f][i] + hi[i] + lo[i] for f < nf, i < per: a facet-invariant accumulated
+// The value of cell i of an accumulated grid: hi + lo, or the rounded wide value.
+__device__ __forceinline__ vis_complex grid_value(const vis_complex *hi, const vis_complex *lo, bool wide, long long i) {
+  vis_complex h;
+#if defined(BULLSEYE_SINGLE)
+  if (wide) {
+    uint2 a = reinterpret_cast<const uint2 *>(hi)[i], b = reinterpret_cast<const uint2 *>(lo)[i];
+    narrow_cell(a, b);
+    h.re = __uint_as_float(a.x) + __uint_as_float(b.x);
+    h.im = __uint_as_float(a.y) + __uint_as_float(b.y);
+    return h;
+  }
+#endif
+  h = hi[i];
+  if (lo) {
+    h.re += lo[i].re;
+    h.im += lo[i].im;
+  }
+  return h;
+}
+
+// out = the accumulated grid's values (out may be hi).
+__global__ void resolve_grid_kernel(const vis_complex *hi, const vis_complex *lo, bool wide,
+                                    vis_complex *out, long long n) {
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+    out[i] = grid_value(hi, lo, wide, i);
+}
+
+// out[f][i] = init[f][i] + the accumulated value of cell i, for f < nf, i < per: a facet-invariant
 // contribution added to every facet's initial grid.
 __global__ void broadcast_add_kernel(const vis_complex *__restrict__ init, const vis_complex *__restrict__ hi,
-                                     const vis_complex *__restrict__ lo, vis_complex *__restrict__ out, long long per,
-                                     long long nf) {
+                                     const vis_complex *__restrict__ lo, bool wide, vis_complex *__restrict__ out,
+                                     long long per, long long nf) {
   const long long total = per * nf;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const long long r = i % per;
-    vis_complex h = hi[r];
-    if (lo) {
-      h.re += lo[r].re;
-      h.im += lo[r].im;
-    }
+    const vis_complex h = grid_value(hi, lo, wide, i % per);
     vis_complex o = init[i];
     o.re += h.re;
     o.im += h.im;

@@ -9,7 +9,8 @@
 // fixed, file-scope device scratch array of this library (g_noalloc_scratch below); it calls no
 // cudaMalloc, cudaFree or allocating library routine.
 //
-// The scratch array holds the compensation (lo) half of the single-precision grid accumulation,
+// The scratch array holds the second word of the single-precision library's wide grid accumulation
+// (while a call grids, a cell's FP64 real part lies in the caller's grid and its imaginary part here),
 // the per-facet transform table and an error word.  It is BZ_NOALLOC_SCRATCH_BYTES bytes (40 MiB
 // for the compensation grid, so at most 40 MiB / 8 bytes = 5,242,880 complex cells over
 // facets x cube x 4 correlations x ny x nx, plus 64 KiB for the table), and every GPU that loads
@@ -106,14 +107,6 @@ __global__ void noalloc_invert_kernel(vis_complex *m, long long n, int *err) {
   m[4 * i + 1] = mul(b, -ir, -ii);
   m[4 * i + 2] = mul(c, -ir, -ii);
   m[4 * i + 3] = mul(a, ir, ii);
-}
-
-__global__ void noalloc_fold_kernel(vis_complex *__restrict__ grid, const vis_complex *__restrict__ lo, long long n) {
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    vis_complex l = lo[i];
-    grid[i].re += l.re;
-    grid[i].im += l.im;
-  }
 }
 
 // Ownership layout for full support W (same rule as the library's other gridding calls).
@@ -285,7 +278,9 @@ int grid_4cor_jones(const gridding_parameters &p, const Workspace &ws, void *str
   // launches
   cudaStream_t st = static_cast<cudaStream_t>(stream);
 #if defined(BULLSEYE_SINGLE)
-  if (cudaMemsetAsync(ws.lo, 0, grid_elems * sizeof(vis_complex), st) != cudaSuccess) return BZ_ERR_CUDA;
+  if (p.row_count > 0 &&
+      !bz_widen_grid(p.output_buffer, ws.lo, (long long)grid_elems, false, st))
+    return BZ_ERR_CUDA;
 #endif
   if (cudaMemsetAsync(ws.err, 0, sizeof(int), st) != cudaSuccess) return BZ_ERR_CUDA;
   noalloc_facet_table_kernel<<<(unsigned)((F + 127) / 128), 128, 0, st>>>(
@@ -304,8 +299,7 @@ int grid_4cor_jones(const gridding_parameters &p, const Workspace &ws, void *str
     return BZ_ERR_CUDA;
   }
 #if defined(BULLSEYE_SINGLE)
-  noalloc_fold_kernel<<<1024, 256, 0, st>>>(p.output_buffer, ws.lo, (long long)grid_elems);
-  if (cudaGetLastError() != cudaSuccess) return BZ_ERR_CUDA;
+  if (!bz_narrow_grid(p.output_buffer, ws.lo, p.output_buffer, (long long)grid_elems, st)) return BZ_ERR_CUDA;
 #endif
   return BZ_OK;
 }
