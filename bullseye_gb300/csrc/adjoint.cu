@@ -26,10 +26,22 @@
 //   V'  = D (w >= 0) or conj(D) (w < 0),   M = e^{-i phi_f} V'
 //   V  += J_p M J_q^H   (the gains applied forward; no weights, no flags), summed over facets.
 //
-// Work layout: a warp takes 32 (row, channel) items; each lane resolves its own item's Jones terms
-// and geometry, the warp gathers the footprints item by item with every lane, and shuffles reduce
-// each item's sums into its lane.  The visibility result (summed over facets) is written once;
-// Jones gradients are accumulated with atomics because every antenna appears on many baselines.
+// Work layout: a warp takes 32 consecutive rows of one channel; each lane resolves its own row's Jones
+// terms and geometry.  Rows are consecutive times of a baseline when they come baseline by baseline, so
+// stretches of them share the footprint corner, the w plane and the row taps kv: such a *group* gathers the
+// grid once,
+//   R(u) = sum over v of g_G(u, v) conj(kv(v))      (W^2 grid reads per group, lanes along u),
+//   D    = sum over u of R(u) conj(ku(u))            (W per visibility, reduced over the warp),
+// which is each visibility's footprint sum with its common factor taken out.  EVLA tracks with 14 s samples
+// (oversampling 15) give 3.9 visibilities per group.  Rows in any other order give groups of one.
+//
+// Prediction with w kernels keeps every visibility's own order of additions: its model grids come from
+// images divided by the taper, whose large edge values cancel in each footprint sum by factors of 1e3 and
+// more, so that sums taken in another order differ by as much as they are off.  There, up to four
+// visibilities of a stretch that shares corner, w plane and grid (a *run*, 14 visibilities on the tracks
+// above) read each grid cell once and keep their own products and sums.
+// The visibility result (summed over facets) is written once; Jones gradients are accumulated with
+// atomics because every antenna appears on many baselines.
 #include <cufft.h>
 
 #include <cstring>
@@ -66,15 +78,25 @@ struct AdjointArgs {
   long long nrows;
   int nchan, nspw, nant, ntimes, nfacets, cube, nx, ny, W, os, K, P, faceting;
   int normalise;  // prediction: divide each facet's gathered value by the real part of its tap sum
+  int row_bytes;  // shared memory of a warp's staged kernel row, 0: taps are read from the table
   int grid_interleaved;  // prediction from its own model grids: a cell's 4 correlations are adjacent
   unsigned imaging_field;
   double u_scale, v_scale, gcx, gcy, wmax, ra0, dec0;
 };
 
 // Dynamic shared memory of the gather kernel: the facet transforms, the w planes' windows, then
-// (16-byte aligned) each warp's staged taps.
-__host__ __device__ inline size_t degrid_taps_offset(int nfacets, int P) {
+// (16-byte aligned) per warp the rows' sums [32][8] and, when there is room, one plane's kernel row [K].
+__host__ __device__ inline size_t degrid_warps_offset(int nfacets, int P) {
   return (sizeof(FacetXform) * (size_t)nfacets + sizeof(int2) * (size_t)P + 15) / 16 * 16;
+}
+constexpr int kDegridWarps = 4;
+constexpr size_t kDegridSums = 32 * 9 * sizeof(acc_real);  // 8 components and the tap sum per row
+// The kernel row is staged up to this size per warp (with four warps per CTA, four CTAs on an SM).
+constexpr size_t kDegridRowMax = 11 * 1024;
+template <bool WPROJ>
+__host__ __device__ inline size_t degrid_row_bytes(int K) {
+  const size_t b = (sizeof(typename TapT<WPROJ>::type) * (size_t)K + 15) / 16 * 16;
+  return b <= kDegridRowMax ? b : 0;
 }
 
 // The 4 adjacent correlations of one cell (32 bytes in single precision, 16-byte aligned): two
@@ -134,18 +156,102 @@ __device__ __forceinline__ bool inv2(cplx *m) {
   return true;
 }
 
-template <bool WPROJ>
-__device__ __forceinline__ cplx tap_at(const void *conv, long long idx) {
+__device__ __forceinline__ acc_real tap_at(const void *conv, long long idx, acc_real) {
+  return (acc_real)((const vis_real *)conv)[idx];
+}
+__device__ __forceinline__ cplx tap_at(const void *conv, long long idx, cplx) {
+  const vis_complex c = ((const vis_complex *)conv)[idx];
   cplx t;
-  if (WPROJ) {
-    const vis_complex c = ((const vis_complex *)conv)[idx];
-    t.re = (acc_real)c.re;
-    t.im = (acc_real)c.im;
-  } else {
-    t.re = (acc_real)((const vis_real *)conv)[idx];
-    t.im = 0;
-  }
+  t.re = (acc_real)c.re;
+  t.im = (acc_real)c.im;
   return t;
+}
+__device__ __forceinline__ bool tap_zero(acc_real t) { return t == (acc_real)0; }
+__device__ __forceinline__ bool tap_zero(cplx t) { return t.re == (acc_real)0 && t.im == (acc_real)0; }
+// acc += g conj(t)
+__device__ __forceinline__ void mac_conj(cplx &acc, cplx g, acc_real t) {
+  acc.re = fma(g.re, t, acc.re);
+  acc.im = fma(g.im, t, acc.im);
+}
+__device__ __forceinline__ void mac_conj(cplx &acc, cplx g, cplx t) {
+  acc.re = fma(g.re, t.re, acc.re);
+  acc.re = fma(g.im, t.im, acc.re);
+  acc.im = fma(g.im, t.re, acc.im);
+  acc.im = fma(-g.re, t.im, acc.im);
+}
+__device__ __forceinline__ cplx tap_value(acc_real t) { cplx c; c.re = t; c.im = 0; return c; }
+__device__ __forceinline__ cplx tap_value(cplx t) { return t; }
+
+// The footprint sums of B visibilities of one run (each in the order of a visibility by itself: lane l takes
+// cells l, l + 32, ... of the window, then a butterfly over the lanes), cells read once.  fu, fv: the
+// visibilities' first taps in the window.
+template <int B, class Tap, class Cell>
+__device__ __forceinline__ void gather_run(const int (&fu)[B], const int (&fv)[B], int ww, int os, long long nx,
+                                           const Tap &tap, const Cell &cell, acc_real (&v)[B][8], acc_real (&ts)[B]) {
+  cplx D[B][4];
+#pragma unroll
+  for (int b = 0; b < B; ++b) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) { D[b][k].re = 0; D[b][k].im = 0; }
+    ts[b] = 0;
+  }
+  const int lane = threadIdx.x & 31;
+  const int ncell = ww * ww, sju = 32 % ww, sjv = 32 / ww;
+  int ru = lane % ww, rv = lane / ww;
+  long long off = (long long)rv * nx + ru;
+  const long long step = (long long)sjv * nx + sju, wrap = nx - ww;
+#pragma unroll(B > 1 ? 1 : 2)
+  for (int idx = lane; idx < ncell; idx += 32) {
+    cplx gc[4];
+    cell(off, gc);
+#pragma unroll
+    for (int b = 0; b < B; ++b) {
+      const cplx t = cmul(tap_value(tap(fu[b] + ru * os)), tap_value(tap(fv[b] + rv * os)));
+      const cplx ct = cconj(t);
+      ts[b] += t.re;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) D[b][k] = cadd(D[b][k], cmul(gc[k], ct));
+    }
+    ru += sju;
+    rv += sjv;
+    off += step;
+    if (ru >= ww) {  // one wrap at most: sju < ww, or ww > 32 and sju = 32
+      ru -= ww;
+      ++rv;
+      off += wrap;
+    }
+  }
+#pragma unroll
+  for (int b = 0; b < B; ++b)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      v[b][2 * k] = D[b][k].re;
+      v[b][2 * k + 1] = D[b][k].im;
+    }
+}
+
+// Sums eight values over the warp; lane l returns the sum of value l >> 2 (in each group of four lanes).
+// Each of the first three steps halves the values a lane carries: 9 shuffles, not 40.
+__device__ __forceinline__ acc_real warp_sum8(const acc_real (&v)[8]) {
+  const int lane = threadIdx.x & 31;
+  acc_real a[4], b[2], c;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const acc_real send = (lane & 16) ? v[i] : v[i + 4], keep = (lane & 16) ? v[i + 4] : v[i];
+    a[i] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const acc_real send = (lane & 8) ? a[i] : a[i + 2], keep = (lane & 8) ? a[i + 2] : a[i];
+    b[i] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
+  }
+  {
+    const acc_real send = (lane & 4) ? b[0] : b[1], keep = (lane & 4) ? b[1] : b[0];
+    c = keep + __shfl_xor_sync(0xffffffffu, send, 4);
+  }
+  c += __shfl_xor_sync(0xffffffffu, c, 2);
+  c += __shfl_xor_sync(0xffffffffu, c, 1);
+  return c;
 }
 
 __device__ __forceinline__ void atomic_add_c(vis_complex *dst, cplx v) {
@@ -156,7 +262,8 @@ __device__ __forceinline__ void atomic_add_c(vis_complex *dst, cplx v) {
 // PREDICT = false: the adjoint (grad_grid -> grad_vis, grad_jones).  PREDICT = true: prediction
 // (model grids in grad_grid -> visibilities in grad_vis).
 template <bool WPROJ, bool PREDICT>
-__global__ void __launch_bounds__(256) degrid_adjoint_kernel(const AdjointArgs a) {
+__global__ void __launch_bounds__(kDegridWarps * 32, sizeof(acc_real) == 4 ? 4 : 3) degrid_adjoint_kernel(const AdjointArgs a) {
+  typedef typename TapT<WPROJ>::type tap_t;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   FacetXform *fx = reinterpret_cast<FacetXform *>(smem_raw);
   for (int f = threadIdx.x; f < a.nfacets; f += blockDim.x) {
@@ -192,8 +299,7 @@ __global__ void __launch_bounds__(256) degrid_adjoint_kernel(const AdjointArgs a
     for (int pl = wid; pl < a.P; pl += nw) {
       int lo = 0x7fffffff, hi = -1;
       for (int i = ln; i < a.K; i += 32) {
-        const cplx t = tap_at<WPROJ>(a.conv, (long long)pl * a.K + i);
-        if (t.re != (acc_real)0 || t.im != (acc_real)0) {
+        if (!tap_zero(tap_at(a.conv, (long long)pl * a.K + i, tap_t()))) {
           lo = min(lo, i);
           hi = max(hi, i);
         }
@@ -215,9 +321,11 @@ __global__ void __launch_bounds__(256) degrid_adjoint_kernel(const AdjointArgs a
   }
   __syncthreads();
   const int lane = threadIdx.x & 31;
-  // this warp's staged column and row taps of the item it gathers ([2][W])
-  cplx *s_taps = reinterpret_cast<cplx *>(smem_raw + degrid_taps_offset(a.nfacets, a.P)) +
-                 (size_t)(threadIdx.x >> 5) * 2 * a.W;
+  const size_t row_bytes = (size_t)a.row_bytes;
+  unsigned char *mine = smem_raw + degrid_warps_offset(a.nfacets, a.P) + (kDegridSums + row_bytes) * (threadIdx.x >> 5);
+  acc_real *s_sum = reinterpret_cast<acc_real *>(mine);              // [32][8], then [32] tap sums
+  tap_t *s_row = reinterpret_cast<tap_t *>(mine + kDegridSums);      // the kernel row of plane staged
+  int staged = -1;
   const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
   const int W = a.W;
@@ -225,22 +333,20 @@ __global__ void __launch_bounds__(256) degrid_adjoint_kernel(const AdjointArgs a
   const double plane_scale = WPROJ ? (double)(a.P - 1) / a.wmax : 0.0;
   const bool jones_vec = vec16(a.jones);  // 16-byte loads of the 2x2 terms (every term starts at 4 x 8 bytes)
 
-  // Each warp takes 32 consecutive (row, channel) items at a time.  Lane i does the scalar work
-  // of item i: its loads, the FP64 geometry, the Jones inverses and the chain rule.  FP64 and the
-  // 2x2 algebra therefore run 32 items per instruction, not one (GB300 issues FP64 at 1/64 of
-  // FP32).  The warp then gathers the footprints one item at a time with every lane, and each
-  // item's sums land in its own lane.
-  const long long total = a.nrows * a.nchan;
-  for (long long base0 = warp * 32; base0 < total; base0 += nwarps * 32) {
-    const long long item = base0 + lane;
-    bool live = item < total;
-    long long row = 0, sc = 0;
-    int c = 0;
+  // Each warp takes 32 consecutive rows of one channel at a time (the channels of a row block by
+  // neighbouring warps).  Lane i does the scalar work of row i: its loads, the FP64 geometry, the Jones
+  // inverses and the chain rule, so that FP64 and the 2x2 algebra run 32 rows per instruction (GB300
+  // issues FP64 at 1/64 of FP32).  The warp then gathers the footprints group by group with every lane,
+  // and each row's sums land in its own lane.
+  const long long blocks = (a.nrows + 31) / 32, total = blocks * a.nchan;
+  for (long long task = warp; task < total; task += nwarps) {
+    const int c = (int)(task % a.nchan);
+    const long long row = task / a.nchan * 32 + lane;
+    bool live = row < a.nrows;
+    long long sc = 0;
     unsigned spw = 0;
     size_t g = 0;
     if (live) {
-      row = item / a.nchan;
-      c = (int)(item - row * a.nchan);
       spw = a.spw[row];
       live = spw < (unsigned)a.nspw;
     }
@@ -293,92 +399,185 @@ __global__ void __launch_bounds__(256) degrid_adjoint_kernel(const AdjointArgs a
       if (ok)
         ok = choose_cells<WPROJ>(um, vm, wm, cc, fx[f], a.faceting != 0, a.faceting != 0, a.u_scale, a.v_scale,
                                  plane_scale, a.gcx, a.gcy, a.nx, a.ny, W, a.P, a.os, ph, cell);
-      // gather, item by item: D_k = sum over the footprint of g_G conj(tap)
-      cplx myD[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) { myD[k].re = 0; myD[k].im = 0; }
-      acc_real myTS = 0;  // prediction: real part of the item's tap sum
+      // gather, group by group: D_k = sum over the footprint of g_G conj(tap)
       const bool want_ts = PREDICT && a.normalise;
-      unsigned todo = __ballot_sync(0xffffffffu, ok);
+      int prev_fv = __shfl_up_sync(0xffffffffu, cell.fv, 1), prev_u = __shfl_up_sync(0xffffffffu, cell.du, 1);
+      int prev_v = __shfl_up_sync(0xffffffffu, cell.dv, 1), prev_pl = __shfl_up_sync(0xffffffffu, cell.plane, 1);
+      const int gi = (int)g, prev_g = __shfl_up_sync(0xffffffffu, gi, 1);
+      const unsigned oks = __ballot_sync(0xffffffffu, ok);
+      constexpr bool kRuns = PREDICT && WPROJ;  // see the work layout above
+      const bool begins = ok && !(lane > 0 && (oks >> (lane - 1) & 1) && (kRuns || prev_fv == cell.fv) &&
+                                  prev_u == cell.du && prev_v == cell.dv && prev_pl == cell.plane && prev_g == gi);
+      const unsigned starts = __ballot_sync(0xffffffffu, begins);
+      unsigned todo = starts;
+      __syncwarp();  // every lane has read the previous facet's sums
       while (todo) {
         const int it = __ffs(todo) - 1;
         todo &= todo - 1;
+        // the group's rows [it, end): up to the next group or row without a footprint
+        const unsigned edge = (starts | ~oks) & (it < 31 ? ~0u << (it + 1) : 0u);
+        const int end = edge ? __ffs(edge) - 1 : 32;
         const int u0 = __shfl_sync(0xffffffffu, cell.du, it), v0 = __shfl_sync(0xffffffffu, cell.dv, it);
-        const int plane = __shfl_sync(0xffffffffu, cell.plane, it);
-        const long long fu = (long long)plane * a.K + __shfl_sync(0xffffffffu, cell.fu, it);
-        const long long fv = (long long)plane * a.K + __shfl_sync(0xffffffffu, cell.fv, it);
-        const long long git = __shfl_sync(0xffffffffu, (long long)g, it);
+        const int plane = __shfl_sync(0xffffffffu, cell.plane, it), fv = __shfl_sync(0xffffffffu, cell.fv, it);
+        const long long git = __shfl_sync(0xffffffffu, gi, it);
         const long long slice0 = ((long long)f * a.cube + git) * 4;
         const long long cube0 = ((long long)f * a.cube + git) * nxy;  // interleaved layout
-        // lane walks the cells lane, lane + 32, ... of the plane's nonzero window as (ju, jv)
-        // without division
         const int2 w2 = win[plane];
         const int ww = w2.y - w2.x + 1;
-        if (ww <= 0) continue;  // an all-zero kernel row: the item's sums stay zero
-        // the item's W column taps and W row taps, once per item instead of once per cell
-        for (int j = lane; j < ww; j += 32) {
-          s_taps[j] = tap_at<WPROJ>(a.conv, fu + (long long)(w2.x + j) * a.os);
-          s_taps[a.W + j] = tap_at<WPROJ>(a.conv, fv + (long long)(w2.x + j) * a.os);
+        // the plane's kernel row (the w plane does not depend on the facet: it changes once or twice in
+        // a warp's rows)
+        if (row_bytes && staged != plane) {
+          __syncwarp();
+          for (int i = lane; i < a.K; i += 32) s_row[i] = tap_at(a.conv, (long long)plane * a.K + i, tap_t());
+          __syncwarp();
+          staged = plane;
         }
-        __syncwarp();
-        cplx D[4];
+        auto tap = [&](int at) { return row_bytes ? s_row[at] : tap_at(a.conv, (long long)plane * a.K + at, tap_t()); };
+        if (ww <= 0) {  // an all-zero kernel row: the sums are zero
+          for (int i = it * 8 + lane; i < end * 8; i += 32) s_sum[i] = 0;
+          if (want_ts && lane >= it && lane < end) s_sum[256 + lane] = 0;
+          continue;
+        }
+        if constexpr (kRuns) {
+          const long long corner = (long long)(v0 + w2.x) * a.nx + (u0 + w2.x);
+          const int w0 = w2.x * a.os;
+          const bool packed = a.grid_interleaved != 0;
+          const vis_complex *p = packed ? a.grad_grid + (cube0 + corner) * 4 : a.grad_grid + slice0 * nxy + corner;
+          auto cells = [&](long long off, cplx (&gc)[4]) {
+            if (packed) {
+              load_cell4(p + off * 4, gc);
+            } else {
 #pragma unroll
-        for (int k = 0; k < 4; ++k) { D[k].re = 0; D[k].im = 0; }
-        acc_real TS = 0;
-        // (ru, rv): the lane's cell relative to the window corner; off: its offset in the grid.
-        // The trip count is fixed before the loop, so prediction's loads of consecutive cells
-        // overlap (two cells per iteration); the adjoint's four strided slices run one cell at a time.
-        const int ncell = ww * ww, sju = 32 % ww, sjv = 32 / ww;
-        int ru = lane % ww, rv = lane / ww;
+              for (int k = 0; k < 4; ++k) {
+                const vis_complex gg = p[k * nxy + off];
+                gc[k].re = gg.re;
+                gc[k].im = gg.im;
+              }
+            }
+          };
+          auto some = [&](auto nb, int i0) {
+            constexpr int B = decltype(nb)::value;
+            int fus[B], fvs[B];
+            acc_real v[B][8], ts[B];
+#pragma unroll
+            for (int b = 0; b < B; ++b) {
+              fus[b] = __shfl_sync(0xffffffffu, cell.fu, i0 + b) + w0;
+              fvs[b] = __shfl_sync(0xffffffffu, cell.fv, i0 + b) + w0;
+            }
+            gather_run<B>(fus, fvs, ww, a.os, a.nx, tap, cells, v, ts);
+#pragma unroll
+            for (int b = 0; b < B; ++b) {
+              const acc_real sum = warp_sum8(v[b]);
+              if ((lane & 3) == 0) s_sum[(i0 + b) * 8 + (lane >> 2)] = sum;
+              if (want_ts) {
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) ts[b] += __shfl_xor_sync(0xffffffffu, ts[b], o);
+                if (lane == 0) s_sum[256 + i0 + b] = ts[b];
+              }
+            }
+          };
+          int i = it;
+          for (; i + 4 <= end; i += 4) some(std::integral_constant<int, 4>{}, i);
+          if (i + 2 <= end) {
+            some(std::integral_constant<int, 2>{}, i);
+            i += 2;
+          }
+          if (i < end) some(std::integral_constant<int, 1>{}, i);
+          continue;
+        }
+        // lanes along u (32 columns at a time); a narrow window's rows are dealt to 32 / xw lane sets
+        const int xw = ww > 16 ? 32 : ww > 8 ? 16 : 8, ys = 32 / xw, y0 = lane / xw;
         const long long corner = (long long)(v0 + w2.x) * a.nx + (u0 + w2.x);
-        long long off = (long long)rv * a.nx + ru;
-        const long long step = (long long)sjv * a.nx + sju, wrap = (long long)a.nx - ww;
-#pragma unroll(PREDICT ? 2 : 1)
-        for (int idx = lane; idx < ncell; idx += 32) {
-          const cplx tap = cmul(s_taps[ru], s_taps[a.W + rv]);
-          const cplx ct = cconj(tap);
-          if (want_ts) TS += tap.re;
-          const long long cidx = corner + off;
-          cplx gc[4];
-          if (PREDICT && a.grid_interleaved) {
-            load_cell4(a.grad_grid + (cube0 + cidx) * 4, gc);
-          } else {
+        const int fvw = fv + w2.x * a.os;
+        for (int xb = 0; xb < ww; xb += 32) {
+          const int xl = xb + (lane & (xw - 1));
+          const bool in = xl < ww;
+          const int x = in ? xl : ww - 1;  // lanes past the window read its last column and count zero
+          cplx R[4];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              const vis_complex gg = a.grad_grid[(slice0 + k) * nxy + cidx];
-              gc[k].re = gg.re;
-              gc[k].im = gg.im;
+          for (int k = 0; k < 4; ++k) { R[k].re = 0; R[k].im = 0; }
+          if (PREDICT && a.grid_interleaved) {
+            const vis_complex *p = a.grad_grid + (cube0 + corner + x) * 4;
+#pragma unroll 4
+            for (int y = y0; y < ww; y += ys) {
+              cplx gc[4];
+              load_cell4(p + (long long)y * a.nx * 4, gc);
+              const tap_t t = tap(fvw + y * a.os);
+#pragma unroll
+              for (int k = 0; k < 4; ++k) mac_conj(R[k], gc[k], t);
+            }
+          } else {
+            const vis_complex *p = a.grad_grid + slice0 * nxy + corner + x;
+#pragma unroll 2
+            for (int y = y0; y < ww; y += ys) {
+              cplx gc[4];
+#pragma unroll
+              for (int k = 0; k < 4; ++k) {
+                const vis_complex gg = p[k * nxy + (long long)y * a.nx];
+                gc[k].re = gg.re;
+                gc[k].im = gg.im;
+              }
+              const tap_t t = tap(fvw + y * a.os);
+#pragma unroll
+              for (int k = 0; k < 4; ++k) mac_conj(R[k], gc[k], t);
             }
           }
+          for (int i = it; i < end; ++i) {
+            const int at = __shfl_sync(0xffffffffu, cell.fu, i) + (w2.x + x) * a.os;
+            tap_t t = tap(at);
+            cplx D[4];
 #pragma unroll
-          for (int k = 0; k < 4; ++k) D[k] = cadd(D[k], cmul(gc[k], ct));
-          ru += sju;
-          rv += sjv;
-          off += step;
-          if (ru >= ww) {  // one wrap at most: sju < ww, or ww > 32 and sju = 32
-            ru -= ww;
-            ++rv;
-            off += wrap;
-          }
-        }
+            for (int k = 0; k < 4; ++k) {
+              D[k].re = 0;
+              D[k].im = 0;
+              mac_conj(D[k], R[k], t);
+            }
+            acc_real v[8];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-#pragma unroll
-          for (int off = 16; off > 0; off >>= 1) {
-            D[k].re += __shfl_xor_sync(0xffffffffu, D[k].re, off);
-            D[k].im += __shfl_xor_sync(0xffffffffu, D[k].im, off);
+            for (int k = 0; k < 4; ++k) {
+              v[2 * k] = in ? D[k].re : (acc_real)0;
+              v[2 * k + 1] = in ? D[k].im : (acc_real)0;
+            }
+            const acc_real sum = warp_sum8(v);
+            if ((lane & 3) == 0) {
+              acc_real *d = s_sum + i * 8 + (lane >> 2);
+              *d = xb ? *d + sum : sum;
+            }
           }
         }
         if (want_ts) {
+          // real part of each row's tap sum, Re(sum of ku x sum of kv)
+          cplx sv = tap_value(tap_t()), su;
+          sv.re = sv.im = 0;
+          for (int y = lane; y < ww; y += 32) sv = cadd(sv, tap_value(tap(fvw + y * a.os)));
 #pragma unroll
-          for (int off = 16; off > 0; off >>= 1) TS += __shfl_xor_sync(0xffffffffu, TS, off);
-        }
-        if (lane == it) {
+          for (int off = 16; off > 0; off >>= 1) {
+            sv.re += __shfl_xor_sync(0xffffffffu, sv.re, off);
+            sv.im += __shfl_xor_sync(0xffffffffu, sv.im, off);
+          }
+          for (int i = it; i < end; ++i) {
+            const int at = __shfl_sync(0xffffffffu, cell.fu, i) + w2.x * a.os;
+            su.re = su.im = 0;
+            for (int x = lane; x < ww; x += 32) su = cadd(su, tap_value(tap(at + x * a.os)));
 #pragma unroll
-          for (int k = 0; k < 4; ++k) myD[k] = D[k];
-          myTS = TS;
+            for (int off = 16; off > 0; off >>= 1) {
+              su.re += __shfl_xor_sync(0xffffffffu, su.re, off);
+              su.im += __shfl_xor_sync(0xffffffffu, su.im, off);
+            }
+            if (lane == i) s_sum[256 + i] = su.re * sv.re - su.im * sv.im;
+          }
         }
-        __syncwarp();  // every lane has read the staged taps before the next item's
+      }
+      __syncwarp();
+      cplx myD[4];
+      acc_real myTS = 0;
+      if (ok) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          myD[k].re = s_sum[lane * 8 + 2 * k];
+          myD[k].im = s_sum[lane * 8 + 2 * k + 1];
+        }
+        if (want_ts) myTS = s_sum[256 + lane];
       }
       if (!ok) continue;
       if (PREDICT) {
@@ -505,43 +704,83 @@ AdjointArgs degrid_args(const gridding_parameters &p, int faceting) {
   return a;
 }
 
-// Zeroes the output, then one persistent-style launch of the gather (32 items per warp pass).
+// Zeroes the output, then one persistent-style launch of the gather (32 rows of a channel per warp pass).
 template <bool PREDICT>
-int launch_degrid(const AdjointArgs &a, bool wproj, cudaStream_t st) {
-  const size_t smem = degrid_taps_offset(a.nfacets, a.P) + (size_t)8 * 2 * a.W * sizeof(cplx);  // 8 warps
-  if (smem > 200 * 1024) return BZ_ERR_UNSUPPORTED;
+int launch_degrid(AdjointArgs a, bool wproj, cudaStream_t st) {
+  const size_t head = degrid_warps_offset(a.nfacets, a.P);
+  if (head + (size_t)8 * 2 * a.W * sizeof(cplx) > 200 * 1024) return BZ_ERR_UNSUPPORTED;  // facets and planes
+  const size_t row = wproj ? degrid_row_bytes<true>(a.K) : degrid_row_bytes<false>(a.K);
+  a.row_bytes = head + kDegridWarps * (kDegridSums + row) <= 200 * 1024 ? (int)row : 0;
+  const size_t smem = head + kDegridWarps * (kDegridSums + (size_t)a.row_bytes);
   if (cudaMemsetAsync(a.grad_vis, 0, sizeof(vis_complex) * (size_t)a.nrows * a.nchan * 4, st) != cudaSuccess) return BZ_ERR_CUDA;
   if (a.nrows == 0) return BZ_OK;
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const long long warps_needed = (a.nrows * a.nchan + 31) / 32;  // 32 items per warp pass
-  const long long blocks = std::min<long long>((warps_needed + 7) / 8, (long long)sms * 16);
+  const long long warps_needed = (a.nrows + 31) / 32 * a.nchan;  // 32 rows of a channel per warp pass
+  const long long blocks = std::min<long long>((warps_needed + kDegridWarps - 1) / kDegridWarps, (long long)sms * 32);
   auto kern = wproj ? degrid_adjoint_kernel<true, PREDICT> : degrid_adjoint_kernel<false, PREDICT>;
   if (smem > 48 * 1024 && cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     return BZ_ERR_CUDA;
-  kern<<<(unsigned)blocks, 256, smem, st>>>(a);
+  kern<<<(unsigned)blocks, kDegridWarps * 32, smem, st>>>(a);
   return cudaGetLastError() == cudaSuccess ? BZ_OK : BZ_ERR_CUDA;
 }
 
+// v / c for the single-precision library with c's reciprocal as a pair of floats (r = hi + lo, 48 bits):
+// v r in error-free FP32 steps, the FP64 quotient's rounding but for ties.  FP64 divisions, two per value at
+// 1/64 of the FP32 rate, took 5.6 ms for 64 slices of 1024^2 (0.16 ms of HBM time).  Values whose product
+// is not well inside the normal range are divided in FP64.
+#if defined(BULLSEYE_SINGLE)
+__device__ __forceinline__ float taper_divide(float v, double c, float hi, float lo, bool pair) {
+  const float p = __fmul_rn(v, hi);
+  const float m = fabsf(p);
+  if (pair && m > 1e-25f && m < 1e37f) return __fadd_rn(p, fmaf(v, lo, fmaf(v, hi, -p)));
+  if (v == 0.0f && pair) return p;
+  return (float)((double)v / c);
+}
+#endif
+
 // Model images -> the FFT input: dst[s][y][x] = img[s][(y+ny/2)%ny][(x+nx/2)%nx] / (taper_x[x'] taper_y[y'])
 // at the source pixel (x', y') (numpy's ifftshift; the tapers are the gridding correction c(l) c(m)
-// that finalize divides by, or null).
-__global__ void predict_taper_shift_kernel(const vis_complex *__restrict__ img, vis_complex *__restrict__ dst, int nx,
-                                           int ny, long long slices, const double *__restrict__ taper_x,
-                                           const double *__restrict__ taper_y) {
-  const long long nxy = (long long)nx * ny, total = nxy * slices;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const long long s = i / nxy, r = i - s * nxy;
+// that finalize divides by, or null).  A thread takes one pixel of blockIdx.y's slices: its taper once.
+__global__ void __launch_bounds__(256) predict_taper_shift_kernel(const vis_complex *__restrict__ img,
+                                                                  vis_complex *__restrict__ dst, int nx, int ny,
+                                                                  long long slices, const double *__restrict__ taper_x,
+                                                                  const double *__restrict__ taper_y) {
+  const long long nxy = (long long)nx * ny;
+  const long long per = (slices + gridDim.y - 1) / gridDim.y, s0 = blockIdx.y * per, s1 = min(slices, s0 + per);
+  for (long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r < nxy; r += (long long)gridDim.x * blockDim.x) {
     const int y = (int)(r / nx), x = (int)(r - (long long)y * nx);
     const int sy = (y + ny / 2) % ny, sx = (x + nx / 2) % nx;
-    vis_complex v = img[s * nxy + (long long)sy * nx + sx];
+    const vis_complex *in = img + (long long)sy * nx + sx;
+    double c = 1.0;
+#if defined(BULLSEYE_SINGLE)
+    float hi = 1.f, lo = 0.f;
+    bool pair = false;
+#endif
     if (taper_x) {
-      const double c = taper_x[sx] * taper_y[sy];
-      v.re = (vis_real)((double)v.re / c);
-      v.im = (vis_real)((double)v.im / c);
+      c = taper_x[sx] * taper_y[sy];
+#if defined(BULLSEYE_SINGLE)
+      const double q = 1.0 / c;
+      hi = (float)q;
+      lo = (float)(q - (double)hi);
+      pair = fabs(q) > 1e-12 && fabs(q) < 1e12;
+#endif
     }
-    dst[i] = v;
+#pragma unroll 4
+    for (long long s = s0; s < s1; ++s) {
+      vis_complex v = in[s * nxy];
+      if (taper_x) {
+#if defined(BULLSEYE_SINGLE)
+        v.re = taper_divide(v.re, c, hi, lo, pair);
+        v.im = taper_divide(v.im, c, hi, lo, pair);
+#else
+        v.re = v.re / c;
+        v.im = v.im / c;
+#endif
+      }
+      dst[s * nxy + r] = v;
+    }
   }
 }
 
@@ -671,7 +910,11 @@ extern "C" int bullseye_predict(const gridding_parameters *params, const void *m
   if (!from_grid) {
     vis_complex *buf = static_cast<vis_complex *>(workspace);
     vis_complex *out = buf + (size_t)slices * p.nx * p.ny;
-    predict_taper_shift_kernel<<<2048, 256, 0, st>>>(grids, buf, (int)p.nx, (int)p.ny, slices, taper_x, taper_y);
+    // about 300 K threads: pixels, and the slices in as many parts as small images leave room for
+    const long long nxy = (long long)p.nx * (long long)p.ny;
+    const unsigned pixels = (unsigned)std::min<long long>((nxy + 255) / 256, 4096);
+    const unsigned parts = (unsigned)std::max<long long>(1, std::min<long long>(slices, 1216 / pixels));
+    predict_taper_shift_kernel<<<dim3(pixels, parts), 256, 0, st>>>(grids, buf, (int)p.nx, (int)p.ny, slices, taper_x, taper_y);
     int rc = cudaGetLastError() == cudaSuccess ? BZ_OK : BZ_ERR_CUDA;
     if (rc == BZ_OK) rc = forward_fft(buf, (int)p.nx, (int)p.ny, (int)slices, st);
     if (rc == BZ_OK) {
