@@ -1050,9 +1050,12 @@ struct ChunkShape {
 };
 
 // The chunk shape for CTAs of nthreads with regs registers per thread: as many CTAs per SM as the
-// register file allows, with about 28 KB of the SM left to L1 for the kernel table, fewer when a batch
-// of six groups does not fit.  64 records per chunk where they take at most half of the CTA's share (a
+// register file allows within 195 KB (the next split between shared memory and L1 is 196 KB, which
+// leaves 60 KB to the kernel table; 199 KB and the 28 KB of the last split cost 1 % of a batched call of 27
+// antennas x 300 times x 64 channels, and 163 KB with shorter batches 6 % of a 64-antenna snapshot step),
+// fewer when a batch of six groups does not fit.  64 records per chunk where they take at most half of the CTA's share (a
 // chunk's end also ends a group), 32 otherwise.
+constexpr size_t kStaticSmem = 640;  // at most, of the segment kernel
 template <int NC, bool WPROJ>
 __host__ inline ChunkShape chunk_shape(int W, int nthreads, int J, int regs = 128) {
   const int nwarps = (nthreads + 31) / 32;
@@ -1060,7 +1063,7 @@ __host__ inline ChunkShape chunk_shape(int W, int nthreads, int J, int regs = 12
   const size_t per = merge_group_bytes<NC, WPROJ>(W, J);
   ChunkShape s{32, 1, 0};
   for (int ctas = std::max(1, std::min(24, 65536 / (nthreads * regs)));; --ctas) {
-    const size_t budget = std::min<size_t>(200 * 1024, (size_t)(227 - 28) * 1024 / ctas - 1024);
+    const size_t budget = std::min<size_t>(200 * 1024, (size_t)195 * 1024 / ctas - 1024 - kStaticSmem);
     for (int V : {64, 32}) {
       const size_t head = stage_head_bytes<NC>(V) + fixed;
       if (V > 32 && 2 * head > budget) continue;
@@ -1336,9 +1339,8 @@ __device__ __forceinline__ SlotMasks slot_masks(const Rec *recs, int nv, int b) 
 // A group list entry: first slot (7 bits), visibilities (7 bits), whether a run starts there.
 constexpr int kGroupRun = 1 << 14;
 
-// The groups of a staged chunk, written by every warp into its own list (whole-warp call; all warps
-// find the same groups).  `pick` first decides the item's merge axis from this chunk: the one that
-// leaves fewer groups.
+// The groups of a staged chunk, written by the calling warp (whole-warp call; any warp finds the same
+// groups).  `pick` first decides the item's merge axis from this chunk: the one that leaves fewer groups.
 template <class Rec>
 __device__ __forceinline__ int find_groups(const Rec *recs, int nv, bool pick, bool &along_v, unsigned short *list) {
   typedef unsigned long long u64;
@@ -1572,22 +1574,23 @@ __device__ __forceinline__ void item_setup(const GridArgs &a, int f_local, unsig
   s.fbase = fx.grid_base;  // element offset of this facet's grid block
 }
 
-// The groups of one staged chunk (block-wide call; ends with the CTA's barrier, after which the
-// records may be overwritten).
-template <int NC, bool WPROJ, int J, bool COMP, class Rec>
-__device__ __forceinline__ void grid_chunk(const GridArgs &a, const Rec *recs, int nv, bool first, bool &along_v,
-                                           const ItemSetup<NC, WPROJ> &s, OwnerState<NC, J> &st) {
-  const int ng = find_groups(recs, nv, first, along_v, s.list);
-  for (int g0 = 0; g0 < ng; g0 += a.GB) {
+// The ng groups of one staged chunk (block-wide call; ends with the CTA's barrier, after which the
+// records may be overwritten).  Before that barrier, next() prepares what follows the chunk.
+template <int NC, bool WPROJ, int J, bool COMP, class Rec, class Next>
+__device__ __forceinline__ void grid_chunk(const GridArgs &a, const Rec *recs, const unsigned short *list, int ng,
+                                           bool along_v, const ItemSetup<NC, WPROJ> &s, OwnerState<NC, J> &st, Next next) {
+  int g0 = 0;
+  do {
     const int g1 = min(ng, g0 + a.GB);
-    merge_groups<NC, WPROJ>(s.table, recs, s.list, g0, g1, along_v, a.W, J, s.ax, s.ap, s.nparts, s.T, s.tb);
+    merge_groups<NC, WPROJ>(s.table, recs, list, g0, g1, along_v, a.W, J, s.ax, s.ap, s.nparts, s.T, s.tb);
     __syncthreads();
     if (s.grids)
-      grid_groups<NC, WPROJ, J, COMP>(a, recs, s.list, g0, g1, along_v, s.T, s.tb, s.du, s.strip, s.rows_mask, s.fbase,
+      grid_groups<NC, WPROJ, J, COMP>(a, recs, list, g0, g1, along_v, s.T, s.tb, s.du, s.strip, s.rows_mask, s.fbase,
                                       s.nxy, s.gnx, s.col_buf, st);
+    if (g1 == ng) next();
     __syncthreads();
-  }
-  if (ng == 0) __syncthreads();
+    g0 = g1;
+  } while (g0 < ng);
 }
 
 // End of a work item (or of a stretch of its rows): the owned cells are flushed and start at zero again.
@@ -1666,7 +1669,8 @@ struct InPlace {
           norm_from_taps<NC, WPROJ>(a, recs, nv, s.table, nacc, ng, fslice);
         }
       }
-      grid_chunk<NC, WPROJ, J, COMP>(a, recs, nv, first, along_v, s, st);
+      const int ngroups = find_groups(recs, nv, first, along_v, s.list);  // every warp its own list
+      grid_chunk<NC, WPROJ, J, COMP>(a, recs, s.list, ngroups, along_v, s, st, [] {});
       first = false;
     }
     stay += (int)(r1 - r0);
@@ -1754,18 +1758,43 @@ __device__ __forceinline__ void grid_records(const GridArgs &a, const int f_loca
   owner_reset(st);
   bool along_v = false;
   const int nchunks = (n + V - 1) / V;
+  // Where the strips are long (J > 4), the group lists of chunks after the first are found by the last warp
+  // (it has the fewest owners) for the CTA while the other warps still grid the chunk before; found by
+  // every warp ahead of the chunk's merge they cost 2 % of a batched call of 27 antennas x 300 times x 64
+  // channels.  The first chunk's list has nothing to hide behind, and the launches with J = 4 (small
+  // supports, few warps) lost 3 % of a 16-time snapshot's class launches by it.
+  constexpr bool kOneFinder = J > 4;
+  __shared__ unsigned short s_list[2][kMaxChunk];
+  __shared__ int s_ngroups[2];
+  auto landed = [&](int buf) {
+    const unsigned par = (rphase >> buf) & 1u;
+    if (!bar_wait(&rbar[buf], par)) {
+      atomicOr(a.error, DEV_ERR_WAIT_TIMEOUT);
+      bar_wait(&rbar[buf], par);
+    }
+  };
   int cur = 0, stay = 0, last_piece = 0;
   for (int c = 0; c < nchunks; ++c, cur ^= 1) {
     const int nv = min(V, n - c * V);
-    const unsigned par = (rphase >> cur) & 1u;
-    if (!bar_wait(&rbar[cur], par)) {
-      atomicOr(a.error, DEV_ERR_WAIT_TIMEOUT);
-      bar_wait(&rbar[cur], par);
-    }
+    landed(cur);
     rphase ^= 1u << cur;
     // the other buffer was last read by the previous chunk, which every thread has finished
     if (tid == 0 && c + 1 < nchunks) issue(c + 1, cur ^ 1);
-    grid_chunk<NC, WPROJ, J, COMP>(a, rb + cur * V, nv, c == 0, along_v, s, st);
+    const unsigned short *list = s.list;
+    int ng;
+    if (kOneFinder && c > 0) {
+      list = s_list[cur];
+      ng = s_ngroups[cur];
+    } else {
+      ng = find_groups(rb + cur * V, nv, c == 0, along_v, s.list);
+    }
+    grid_chunk<NC, WPROJ, J, COMP>(a, rb + cur * V, list, ng, along_v, s, st, [&] {
+      if (kOneFinder && c + 1 < nchunks && threadIdx.x >= blockDim.x - 32) {
+        landed(cur ^ 1);
+        const int found = find_groups(rb + (cur ^ 1) * V, min(V, n - (c + 1) * V), false, along_v, s_list[cur ^ 1]);
+        if ((tid & 31) == 0) s_ngroups[cur ^ 1] = found;
+      }
+    });
     // the owned cells go out at the end, and before it once kStayRows rows are in and a segment ended
     // in the chunk
     stay += nv;

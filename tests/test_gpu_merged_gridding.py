@@ -91,3 +91,26 @@ def test_work_items_of_several_segments(precision, form, n_chan, n_facets, gpu_l
     finally:
         lib.bullseye_set_visibility_records(1)
         lib.bullseye_set_record_budget(0)
+
+
+@pytest.mark.parametrize("precision", ["double", "single"])
+@pytest.mark.parametrize("s", [3, 11, 19])
+@pytest.mark.parametrize("n_times", [31, 33, 63, 64, 65, 128, 129])
+def test_chunk_edges(precision, s, n_times, gpu_libs, oracle_libs):
+    """Segments that end on, one before and one after a staged chunk's end (32 or 64 records), at supports
+    whose launches find the next chunk's groups in one warp and at one whose launches do so in every warp."""
+    p = _problem(s, 3, 0.05, "u", 2, False, n_times=n_times, n_chan=2)
+    _check(gpu_libs[precision], oracle_libs["double"], p, "facet_4_cor", precision)
+
+
+@pytest.mark.parametrize("call", ["facet_4_cor", "grid_duel_pol"])
+def test_compensation_switched_between_calls(call, gpu_libs, oracle_libs):
+    """Each call starts from what the one before left, with and without the second word of its cells."""
+    lib = gpu_libs["single"]
+    p = _problem(5, 4, 0.1, "v", 2 if call.startswith("facet") else 0, False)
+    try:
+        for on in (1, 0, 1):
+            lib.bullseye_set_compensated(on)
+            _check(lib, oracle_libs["double"], p, call, "single")
+    finally:
+        lib.bullseye_set_compensated(1)
