@@ -179,10 +179,41 @@ __global__ void __launch_bounds__(1024) bucket_kernel(const int4 *__restrict__ s
   }
 }
 
-// Exclusive scan of the scheduled segments' row counts by one block: rec_off[i] = rows of the
-// segments before i (in class order), rec_off[n] = all rows; n = the segments of every class.
-__global__ void rec_offsets_kernel(const int4 *__restrict__ sorted, const int *__restrict__ class_count, int ncls,
-                                   long long *__restrict__ rec_off) {
+// Per-call constants of the record kernel (single precision): 1 / lambda of every (spw, channel), then the
+// double-float facet constants of every (spw, channel, facet).  Made by every segment for itself they kept
+// the FP64 pipe (1/64 of the FP32 rate) busy for 61 % of the record kernel of a 16-time snapshot in 8 facets
+// (1.46 million FP64 instructions; 0.45 million and 19 % with the table): 136 -> 115 us there with
+// kRecordItems, and 1813 -> 1725 us for the record kernels of 27 antennas x 100 times x 64 channels in 16 facets.
+size_t record_const_bytes(long long nsc, int nfacets) {
+  return (size_t)nsc * (sizeof(double) + (size_t)nfacets * sizeof(DfFacet));
+}
+// Most bytes kept for them; past it the segments make their own.
+constexpr size_t kRecordConstBytes = 64u << 20;
+
+// Exclusive scan of the scheduled segments' row counts by the first block: rec_off[i] = rows of the
+// segments before i (in class order), rec_off[n] = all rows; n = the segments of every class.  The
+// other blocks write the record kernel's constants (consts: record_const_bytes, or null), each FP64-bound
+// warp's entries on another block.
+__global__ void __launch_bounds__(1024) rec_offsets_kernel(
+    const int4 *__restrict__ sorted, const int *__restrict__ class_count, int ncls, long long *__restrict__ rec_off,
+    const FacetXform *__restrict__ facets, const vis_real *__restrict__ wavelengths, int nsc, int nfacets, int os,
+    double *__restrict__ consts) {
+  if (blockIdx.x > 0) {
+#if defined(BULLSEYE_SINGLE)
+    DfFacet *df = reinterpret_cast<DfFacet *>(consts + nsc);
+    const int nb = (int)gridDim.x - 1, nw = (int)blockDim.x >> 5;
+    const long long total = (long long)nsc * nfacets;
+    for (long long w = (long long)(threadIdx.x >> 5) * nb + blockIdx.x - 1; w * 32 < total; w += (long long)nb * nw) {
+      const long long e = w * 32 + (threadIdx.x & 31);
+      if (e >= total) continue;
+      const int sc = (int)(e / nfacets), f = (int)(e - (long long)sc * nfacets);
+      const double inv = 1.0 / (double)wavelengths[sc];
+      if (f == 0) consts[sc] = inv;
+      df_facet(facets[f], inv, os, df[e]);
+    }
+#endif
+    return;
+  }
   __shared__ long long part[1024];
   int n = 0;
   for (int k = 0; k < ncls; ++k) n += class_count[k];
@@ -211,25 +242,32 @@ __global__ void rec_offsets_kernel(const int4 *__restrict__ sorted, const int *_
 // memory); more facets are taken in blocks, each block reloading the segment's rows.
 constexpr int kRecordFacetBlock = 32;
 constexpr int kRecordWarps = 8;
+constexpr int kRecordItems = 8;
 
 template <int NC>
 constexpr size_t record_smem_bytes() {
   return (size_t)kRecordWarps * kRecordFacetBlock * (NC * sizeof(double) + sizeof(int2) + sizeof(int) + sizeof(DfFacet));
 }
 
-// Visibility records of every scheduled segment, one warp per segment taking segments from a
-// counter.  Each lane loads one row of the segment (load_row) and writes its record for every
-// facet (facet_record: the in-place gridder's prologue, so the same cells, taps, corrections and
+// Visibility records of every scheduled segment, one warp per (segment, block of facets) taking them
+// from a counter.  Each lane loads one row of the segment (load_row) and writes its record for the block's
+// facets (facet_record: the in-place gridder's prologue, so the same cells, taps, corrections and
 // weights) at rec_off[si] x F + f x len + row, with the footprint residues for the segment's class
 // width.  Per facet the warp keeps, in shared memory, the first and last valid row (the work item's
 // range) and the normalisation sums of the current grid group (added to the global sums when the
 // group changes and when the segment ends).  A segment whose records would pass `capacity` is left
 // to the segment kernel's in-place prologue.
+//
+// An item is a chain of dependent loads (segment, rows, cells, kernel row sums) at 16 warps per SM, so few
+// segments leave the SMs waiting: a block holds all facets only when that leaves kRecordItems items per
+// resident warp (each block reads the rows once more).  The snapshot's record kernel takes 128, 129, 125, 115
+// and 128 us at 1, 2, 4, 8 and 16.  More warps by fewer registers (80 or 96 instead of 128) spill and lose.
 template <int NC, bool WPROJ>
 __global__ void __launch_bounds__(kRecordWarps * 32) record_kernel(
     const GridArgs a, const int4 *__restrict__ sorted, const int *__restrict__ class_count, int ncls,
     const long long *__restrict__ rec_off, const int *__restrict__ widths, int nfacets, GridRec<NC> *__restrict__ out,
-    long long capacity, int2 *__restrict__ range, long long range_items, int *next) {
+    long long capacity, int2 *__restrict__ range, long long range_items, int *next, int least_items,
+    const double *__restrict__ consts) {
   extern __shared__ __align__(16) unsigned char rk_smem[];
   constexpr int FB = kRecordFacetBlock;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -247,10 +285,15 @@ __global__ void __launch_bounds__(kRecordWarps * 32) record_kernel(
   for (int k = 0; k < ncls; ++k) nseg += class_count[k];
   const double plane_scale = WPROJ ? (double)(a.P - 1) / a.wmax : 0.0;
   const bool want_norm = a.norm != nullptr;
+  // facets per item: halved while there are too few items
+  int fper = nfacets;
+  while (fper > 1 && (long long)nseg * ((nfacets + fper - 1) / fper) < least_items) fper = (fper + 1) / 2;
+  const int nblocks = (nfacets + fper - 1) / fper;
   for (;;) {
-    int si = 0;
-    if (lane == 0) si = atomicAdd(next, 1);
-    si = __shfl_sync(0xffffffffu, si, 0);
+    int item = 0;
+    if (lane == 0) item = atomicAdd(next, 1);
+    item = __shfl_sync(0xffffffffu, item, 0);
+    const int si = item / nblocks, facet0 = (item - si * nblocks) * fper, facet1 = min(nfacets, facet0 + fper);
     if (si >= nseg) break;
     const int4 sg = sorted[si];
     if (sg.x < 0 || sg.x > sg.y || (long long)sg.y > a.nrows || sg.z < 0 || sg.z >= a.nchan || sg.w < 0 ||
@@ -273,26 +316,35 @@ __global__ void __launch_bounds__(kRecordWarps * 32) record_kernel(
       const unsigned s0 = a.spw[sg.x];
       if (len > 0 && s0 < (unsigned)a.nspw) {
         dspw = s0;
-        dinv = 1.0 / (double)a.wavelengths[(long long)s0 * a.nchan + sg.z];
+        const long long sc = (long long)s0 * a.nchan + sg.z;
+        dinv = consts ? consts[sc] : 1.0 / (double)a.wavelengths[sc];
       }
     }
 #else
     (void)dinv;  // the 64-bit library keeps the FP64 cell choice
 #endif
-    for (int f0 = 0; f0 < nfacets; f0 += FB) {
-      const int fb = min(FB, nfacets - f0);
+    for (int f0 = facet0; f0 < facet1; f0 += FB) {
+      const int fb = min(FB, facet1 - f0);
       for (int j = lane; j < fb; j += 32) {
         s_rng[j] = make_int2(0x7fffffff, 0);
         s_ng[j] = -1;
 #pragma unroll
         for (int k = 0; k < NC; ++k) s_norm[j * NC + k] = 0.0;
 #if defined(BULLSEYE_SINGLE)
-        if (dspw != 0xffffffffu) df_facet(a.facets[f0 + j], dinv, a.os, s_df[j]);
+        if (dspw != 0xffffffffu && !consts) df_facet(a.facets[f0 + j], dinv, a.os, s_df[j]);
 #endif
       }
+#if defined(BULLSEYE_SINGLE)
+      if (dspw != 0xffffffffu && consts) {
+        const DfFacet *df = reinterpret_cast<const DfFacet *>(consts + (long long)a.nspw * a.nchan);
+        const int *src = reinterpret_cast<const int *>(df + ((long long)dspw * a.nchan + sg.z) * nfacets + f0);
+        for (int j = lane; j < fb * (int)(sizeof(DfFacet) / sizeof(int)); j += 32)
+          reinterpret_cast<int *>(s_df)[j] = __ldg(src + j);
+      }
+#endif
       __syncwarp();
-      unsigned cspw = 0xffffffffu;
-      double inv = 0.0;
+      unsigned cspw = dspw;
+      double inv = dinv;
       for (int b = 0; b < len; b += 32) {
         const int i = b + lane;
         RowInputs<NC> ri;
@@ -305,7 +357,7 @@ __global__ void __launch_bounds__(kRecordWarps * 32) record_kernel(
         const bool use_df = ri.use && ri.spw == dspw;
         int plane_df = 0;
         if (WPROJ && use_df) {
-          const double pl = rint(fabs(ri.wm) * (inv * plane_scale));
+          const double pl = rint(fabs((double)ri.uvw_in[2]) * (inv * plane_scale));
           plane_df = (pl >= 0.0 && pl < (double)a.P) ? (int)pl : -1;
         }
         for (int fj = 0; fj < fb; ++fj) {
@@ -525,6 +577,7 @@ struct BatchedState {
   DevBuf<int2> vrec_range;
   long long vrec_range_items = 0;
   DevBuf<int> cls_width, vrec_next;
+  DevBuf<unsigned char> vrec_const;  // record_const_bytes, or none
 };
 BatchedState g_bs;
 
@@ -691,7 +744,7 @@ bool ensure_records(int nfacets, long long rows, int nchan, long long segments) 
   }
   const size_t budget = b.vrec_budget ? b.vrec_budget : tot / 10 * 3;
   const double need = (double)std::max(nfacets, 1) * (double)rows * nchan * sizeof(GridRec<4>);
-  const void *before[3] = {b.vrec.ptr, b.vrec_off.ptr, b.vrec_range.ptr};
+  const void *before[4] = {b.vrec.ptr, b.vrec_off.ptr, b.vrec_range.ptr, b.vrec_const.ptr};
   const double room = (double)b.vrec.n + (double)fr * 0.8;
   const size_t want = (size_t)(std::min(need, std::min((double)budget, room)) / 256) * 256;
   if (want > b.vrec.n && want >= (1u << 20)) {
@@ -706,7 +759,22 @@ bool ensure_records(int nfacets, long long rows, int nchan, long long segments) 
     b.vrec_range_items = items;
   }
   if (!b.vrec_next.ptr && !b.vrec_next.alloc(1)) return false;
-  if (before[0] != b.vrec.ptr || before[1] != b.vrec_off.ptr || before[2] != b.vrec_range.ptr) b.drop_graphs();
+#if defined(BULLSEYE_SINGLE)
+  // a failed allocation is no error: the segments make their own constants then
+  const size_t cb = record_const_bytes((long long)g_ctx.nspw * nchan, std::max(nfacets, 1));
+  if (cb > b.vrec_const.n && cb <= kRecordConstBytes) {
+    b.vrec_const.release();
+    if (bz_dev_alloc((void **)&b.vrec_const.ptr, cb)) {
+      b.vrec_const.n = cb;
+    } else {
+      b.vrec_const.ptr = nullptr;
+      cudaGetLastError();
+    }
+  }
+#endif
+  if (before[0] != b.vrec.ptr || before[1] != b.vrec_off.ptr || before[2] != b.vrec_range.ptr ||
+      before[3] != b.vrec_const.ptr)
+    b.drop_graphs();
   return true;
 }
 
@@ -742,12 +810,23 @@ bool launch_records(const GridArgs &base, int nfacets, cudaStream_t st, GridArgs
     if (sms <= 0) sms = 1;
   }
   BZ_CUDA_TRY_RET(cudaMemsetAsync(b.vrec_next.ptr, 0, sizeof(int), st), false);
-  rec_offsets_kernel<<<1, 1024, 0, st>>>(b.sorted.ptr, b.class_count.ptr, b.ncls, b.vrec_off.ptr);
+  double *consts = nullptr;
+  int const_blocks = 0;
+#if defined(BULLSEYE_SINGLE)
+  if (b.vrec_const.ptr && record_const_bytes((long long)a.nspw * a.nchan, nfacets) <= b.vrec_const.n) {
+    consts = reinterpret_cast<double *>(b.vrec_const.ptr);
+    const_blocks = (int)std::min<long long>(2 * sms, ((long long)a.nspw * a.nchan * nfacets + 31) / 32);
+  }
+#endif
+  rec_offsets_kernel<<<1 + const_blocks, 1024, 0, st>>>(b.sorted.ptr, b.class_count.ptr, b.ncls, b.vrec_off.ptr, a.facets,
+                                                        a.wavelengths, a.nspw * a.nchan, nfacets, a.os, consts);
+  // two CTAs of 128-register threads per SM are resident
+  const int least_items = sms * 2 * kRecordWarps * kRecordItems;
   record_kernel<NC, WPROJ><<<sms * 4, kRecordWarps * 32, record_smem_bytes<NC>(), st>>>(
       a, b.sorted.ptr, b.class_count.ptr, b.ncls, b.vrec_off.ptr,
                                                     b.cls_width.ptr, nfacets, reinterpret_cast<GridRec<NC> *>(b.vrec.ptr),
                                                     (long long)(b.vrec.n / sizeof(GridRec<NC>)), b.vrec_range.ptr,
-                                                    b.vrec_range_items, b.vrec_next.ptr);
+                                                    b.vrec_range_items, b.vrec_next.ptr, least_items, consts);
   g_ctx.launches += 2;
   BZ_CUDA_TRY_RET(cudaGetLastError(), false);
   set_record_args<NC>(out);
@@ -1019,6 +1098,7 @@ void bz_release_batched() {
   b.conv_w.release();
   b.conv_w_stride = 0;
   b.vrec.release(); b.vrec_off.release(); b.vrec_range.release(); b.cls_width.release(); b.vrec_next.release();
+  b.vrec_const.release();
   b.vrec_range_items = 0;
   b.rows_cap = b.tracks_cap = b.segs_cap = 0;
   b.planned = false;

@@ -629,7 +629,6 @@ struct RowInputs {
   long long sc;        // spw x nchan + channel
   long long jt1, jt2;  // Jones rows t x nant + antenna; with jones_inv_t, ((antenna x S + spw) x Ch + channel) x F
   long long tt;        // the row's time index (with jones_inv_t)
-  double um, vm, wm;
   vis_real uvw_in[3];  // as stored (the double-float cell choice starts from them)
   cplx vis[NC];
   acc_real wt[NC];
@@ -659,9 +658,6 @@ __device__ __forceinline__ void load_row(const GridArgs &a, int chan, long long 
   ri.uvw_in[0] = a.uvw[3 * row];
   ri.uvw_in[1] = a.uvw[3 * row + 1];
   ri.uvw_in[2] = a.uvw[3 * row + 2];
-  ri.um = (double)ri.uvw_in[0];
-  ri.vm = (double)ri.uvw_in[1];
-  ri.wm = (double)ri.uvw_in[2];
   ri.row_ok = !a.flagged_rows[row] && (a.field[row] == a.imaging_field);
   const long long base = ((long long)row * a.nchan + c) * a.npol;
   if (a.mode == CORR_SAMPLING) {
@@ -773,7 +769,7 @@ __device__ __forceinline__ void facet_record(const GridArgs &a, int f_local, int
     cc.su = inv * fx.u_scale;
     cc.sv = inv * fx.v_scale;
     cc.sw = inv * plane_scale;
-    if (!choose_cells<WPROJ>(ri.um, ri.vm, ri.wm, cc, fx, a.phase != 0, a.uvx != 0, fx.u_scale, fx.v_scale,
+    if (!choose_cells<WPROJ>((double)ri.uvw_in[0], (double)ri.uvw_in[1], (double)ri.uvw_in[2], cc, fx, a.phase != 0, a.uvx != 0, fx.u_scale, fx.v_scale,
                              plane_scale, fx.gcx, fx.gcy, fx.nx, fx.ny, a.W_full ? a.W_full : a.W, a.P, a.os, ph, cell))
       return;
   }
