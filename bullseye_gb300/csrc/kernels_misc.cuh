@@ -98,7 +98,11 @@ __global__ void __launch_bounds__(256) convert_grid_kernel(vis_complex *hi, vis_
   if (((reinterpret_cast<uintptr_t>(hi) | reinterpret_cast<uintptr_t>(lo)) & 15) == 0) {
     uint4 *ph = reinterpret_cast<uint4 *>(hi), *pl = reinterpret_cast<uint4 *>(lo);
     const long long pairs = n / 2;
-    for (long long i = tid; i < pairs; i += 4 * nt) {
+    // whole warps stay in the loop: a stretch whose cells are all zero is passed by on a vote (on each lane's
+    // own test the FP64 path was evaluated ahead of it, 6 FP64 operations for every zero cell: 28.5 us for the
+    // 2 million cells of a snapshot's facets, 12.5 for the way back)
+    for (long long i0 = tid - (threadIdx.x & 31); i0 < pairs; i0 += 4 * nt) {
+      const long long i = i0 + (threadIdx.x & 31);
       uint4 h[4], l[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q)
@@ -110,6 +114,8 @@ __global__ void __launch_bounds__(256) convert_grid_kernel(vis_complex *hi, vis_
         }
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
+        const unsigned bits = h[q].x | h[q].y | h[q].z | h[q].w | l[q].x | l[q].y | l[q].z | l[q].w;
+        if (!__any_sync(0xffffffffu, bits != 0)) continue;
         uint2 h0 = make_uint2(h[q].x, h[q].y), h1 = make_uint2(h[q].z, h[q].w);
         uint2 l0 = make_uint2(l[q].x, l[q].y), l1 = make_uint2(l[q].z, l[q].w);
         const bool c0 = one(h0, l0), c1 = one(h1, l1);
@@ -163,11 +169,49 @@ __device__ __forceinline__ vis_complex grid_value(const vis_complex *hi, const v
   return h;
 }
 
-// out = the accumulated grid's values (out may be hi).
-__global__ void resolve_grid_kernel(const vis_complex *hi, const vis_complex *lo, bool wide,
-                                    vis_complex *out, long long n) {
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    out[i] = grid_value(hi, lo, wide, i);
+// out = the accumulated grid's values (out may be hi).  Wide grids go two cells per load, eight in flight,
+// and pass by the FP64 path where a warp's cells are all zero (cell by cell, with the conversions evaluated
+// for zero cells too, the 16 facets of 1024^2 cells x 4 correlations took 546 us; 239 so, the HBM time).
+__global__ void __launch_bounds__(256) resolve_grid_kernel(const vis_complex *hi, const vis_complex *lo, bool wide,
+                                                           vis_complex *out, long long n) {
+  const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x, nt = (long long)gridDim.x * blockDim.x;
+  long long done = 0;
+#if defined(BULLSEYE_SINGLE)
+  if (wide && ((reinterpret_cast<uintptr_t>(hi) | reinterpret_cast<uintptr_t>(lo) | reinterpret_cast<uintptr_t>(out)) &
+               15) == 0) {
+    const long long pairs = n / 2;
+    for (long long i0 = tid - (threadIdx.x & 31); i0 < pairs; i0 += 4 * nt) {
+      const long long i = i0 + (threadIdx.x & 31);
+      uint4 h[4], l[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        h[q] = l[q] = make_uint4(0, 0, 0, 0);
+        if (i + q * nt < pairs) {
+          h[q] = reinterpret_cast<const uint4 *>(hi)[i + q * nt];
+          l[q] = reinterpret_cast<const uint4 *>(lo)[i + q * nt];
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        uint4 r = make_uint4(0, 0, 0, 0);
+        const unsigned bits = h[q].x | h[q].y | h[q].z | h[q].w | l[q].x | l[q].y | l[q].z | l[q].w;
+        if (__any_sync(0xffffffffu, bits != 0)) {
+          uint2 h0 = make_uint2(h[q].x, h[q].y), h1 = make_uint2(h[q].z, h[q].w);
+          uint2 l0 = make_uint2(l[q].x, l[q].y), l1 = make_uint2(l[q].z, l[q].w);
+          narrow_cell(h0, l0);
+          narrow_cell(h1, l1);
+          r = make_uint4(__float_as_uint(__uint_as_float(h0.x) + __uint_as_float(l0.x)),
+                         __float_as_uint(__uint_as_float(h0.y) + __uint_as_float(l0.y)),
+                         __float_as_uint(__uint_as_float(h1.x) + __uint_as_float(l1.x)),
+                         __float_as_uint(__uint_as_float(h1.y) + __uint_as_float(l1.y)));
+        }
+        if (i + q * nt < pairs) reinterpret_cast<uint4 *>(out)[i + q * nt] = r;
+      }
+    }
+    done = 2 * pairs;
+  }
+#endif
+  for (long long i = done + tid; i < n; i += nt) out[i] = grid_value(hi, lo, wide, i);
 }
 
 // out[f][i] = init[f][i] + the accumulated value of cell i, for f < nf, i < per: a facet-invariant
