@@ -13,8 +13,9 @@
 //   seg_count    per track (baseline, channel): number of runs of one class;
 //   scan         track offsets;
 //   seg_write    the runs {row_begin, row_end, channel, class};
-//   bucket       runs ordered by class;
-//   per class    one persistent Romein launch (romein_segment_kernel) over (run, facet) items,
+//   bucket       runs ordered by class, each class in (baseline, channel, rows) order;
+//   records      every run's prologue, one record per row and facet (record_kernel);
+//   per class    one persistent Romein launch (romein_segment_kernel) over (consecutive runs, facet) items,
 //                with the thread layout chosen for that class width by the autotuner; then the
 //                same for the sampling function (facet-invariant, gridded once).
 #include <algorithm>
@@ -643,9 +644,8 @@ bool plan_classes() {
   std::vector<int> pcls(P);
   for (int p = 0; p < P; ++p) pcls[p] = (int)(std::find(widths.begin(), widths.end(), pw[p]) - widths.begin());
   // Support-window table: row (plane p, tap offset f) holds the taps s = plo[p] + j,
-  // j < pw[p] (conv[p][f + s os]), then its first 7 taps again (the J - 1 <= 7 repeated leading
-  // row taps of a Romein strip), zero-padded to a multiple of 16 bytes.  A staged tap row is then
-  // one 16-byte aligned bulk copy from the row start.
+  // j < pw[p] (conv[p][f + s os]), then its first 7 taps again, zero-padded to a multiple of 16 bytes.
+  // The merge step reads a row's taps by consecutive lanes.
   {
     const size_t ncomp = wproj ? 2 : 1;
     const int E = (int)(16 / (ncomp * sizeof(vis_real)));
@@ -910,8 +910,7 @@ bool tune_class(const GridArgs &base, int k, int nfacets, Variant &out, int host
   auto key = std::make_tuple(W, NC, (int)WPROJ, (int)COMP);
   auto it = b.tuned.find(key);
   std::vector<Variant> cands;
-  // J = 6 (single precision, four correlations, w-projection): 48 accumulator registers, the
-  // column tap shared by 6 rows
+  // J = 6 (single precision, four correlations, w-projection): 48 accumulator registers
   const bool six = BZ_PRECISION_BITS == 32 && NC == 4 && WPROJ;
   for (int J : {8, 6, 4})
     for (bool wide : {true, false}) {

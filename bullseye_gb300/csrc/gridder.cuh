@@ -996,12 +996,6 @@ __device__ __forceinline__ void prologue(const GridArgs &a, int f_local, int cha
 // What the merge and the split of the builds measured (GB300, 27 antennas x 100 times x 64 channels,
 // 16 facets, whole batched call with copy-back): 36.5 -> 27.3 ms in single precision; 64-bit library,
 // 40 times x 16 channels x 4 facets: 28.2 -> 8.1 ms (its FP64 pipe bounded the multiply-adds).
-//
-// A chunk of V records in shared memory is taken in two steps, in batches of GB groups:
-//   merge_groups  thread (i, part) forms T(i) of every nparts-th group of the batch, reading the taps
-//                 from the kernel table through L1, and copies the group's common tap row;
-//   grid_groups   the Romein owner threads add T x tap to their J cells per column.  Columns run along
-//                 u whatever the merge axis, so that a warp's flushes are contiguous in the grid.
 
 // Most records of a chunk: group lists are built from 64-bit masks.
 constexpr int kMaxChunk = 64;
@@ -1048,7 +1042,7 @@ struct ChunkShape {
 // The chunk shape for CTAs of nthreads with regs registers per thread: as many CTAs per SM as the
 // register file allows within 195 KB (the next split between shared memory and L1 is 196 KB, which
 // leaves 60 KB to the kernel table; 199 KB and the 28 KB of the last split cost 1 % of a batched call of 27
-// antennas x 300 times x 64 channels, and 163 KB with shorter batches 6 % of a 64-antenna snapshot step),
+// antennas x 400 times x 64 channels, and 163 KB with shorter batches 6 % of a 64-antenna snapshot step),
 // fewer when a batch of six groups does not fit.  64 records per chunk where they take at most half of the CTA's share (a
 // chunk's end also ends a group), 32 otherwise.
 constexpr size_t kStaticSmem = 640;  // at most, of the segment kernel
@@ -1201,7 +1195,7 @@ __device__ __forceinline__ cplx read_tap(const TapTable<true> &t, int first, int
   return r;
 }
 
-// Tap-copy barriers of the record staging.  Waits are bounded.
+// Barriers of the record staging.  Waits are bounded.
 __device__ __forceinline__ unsigned smem_addr(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void bar_init(unsigned long long *bar, unsigned count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_addr(bar)), "r"(count) : "memory");
@@ -1756,7 +1750,7 @@ __device__ __forceinline__ void grid_records(const GridArgs &a, const int f_loca
   const int nchunks = (n + V - 1) / V;
   // Where the strips are long (J > 4), the group lists of chunks after the first are found by the last warp
   // (it has the fewest owners) for the CTA while the other warps still grid the chunk before; found by
-  // every warp ahead of the chunk's merge they cost 2 % of a batched call of 27 antennas x 300 times x 64
+  // every warp ahead of the chunk's merge they cost 2 % of a batched call of 27 antennas x 400 times x 64
   // channels.  The first chunk's list has nothing to hide behind, and the launches with J = 4 (small
   // supports, few warps) lost 3 % of a 16-time snapshot's class launches by it.
   constexpr bool kOneFinder = J > 4;

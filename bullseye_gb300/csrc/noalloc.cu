@@ -313,7 +313,7 @@ int report_device_error(int h, const char *name) {
     bz_record_error(BZ_ERR_INVALID_ARGUMENT, "%s: channel grid index, spw or schedule entry out of range", name);
   if (h & DEV_ERR_JONES_INDEX)
     bz_record_error(BZ_ERR_INVALID_ARGUMENT, "%s: timestamp or antenna id out of range of the Jones terms", name);
-  if (h & DEV_ERR_WAIT_TIMEOUT) bz_record_error(BZ_ERR_CUDA, "%s: a bounded wait for staged kernel taps ran out", name);
+  if (h & DEV_ERR_WAIT_TIMEOUT) bz_record_error(BZ_ERR_CUDA, "%s: a bounded wait for staged records ran out", name);
   if (h & DEV_ERR_SINGULAR) return BZ_ERR_SINGULAR_JONES;
   if (h & (DEV_ERR_GRID_INDEX | DEV_ERR_JONES_INDEX)) return BZ_ERR_INVALID_ARGUMENT;
   return BZ_ERR_CUDA;

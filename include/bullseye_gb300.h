@@ -92,7 +92,8 @@ int bullseye_last_error(char *buf, size_t n);
 void bullseye_clear_error(void);
 /* 32 or 64: the data precision of the loaded library. */
 int bullseye_precision_bits(void);
-/* 32-bit library: compensated (hi/lo TwoSum) grid accumulation on (1, default) or off (0). */
+/* 32-bit library: grid accumulation in FP64 (flushed cells are added to a second word beside each cell) on
+ * (1, default) or plain FP32 (0). */
 void bullseye_set_compensated(int on);
 /* When on, the row arrays, jones_terms and baseline_starting_indexes in gridding_parameters are
  * device pointers in baseline-major order and gridding calls copy nothing from the host. */
@@ -167,8 +168,9 @@ int bullseye_grid_batched(gridding_parameters *params, int call, int with_sampli
  * support-aware persistent schedule and graph replay as bullseye_grid_batched, over `nfacets`
  * facets described by `facets` (host array), accumulated into CALLER-OWNED device buffers:
  * grids (complex, each facet's block at its grid_offset), grid_lo (the 32-bit library's
- * compensation buffer, same size as grids and zeroed by the caller, or null for plain FP32
- * accumulation; a cell's value is then grids + grid_lo; ignored by the 64-bit library) and norms
+ * second words, same size as grids and zeroed by the caller, or null for plain FP32 accumulation; a
+ * cell's value is then grids + grid_lo, and while a call's work runs the two words of a cell hold an FP64
+ * pair; ignored by the 64-bit library) and norms
  * (float64 [nfacets][cube][4]).  Work is queued on the library stream (bullseye_get_stream).
  * row_mask, if not null, is a device array [nfacets][row_count] of bytes (device-resident inputs
  * only, bullseye_set_device_inputs; rejected with BZ_ERR_UNSUPPORTED otherwise): 0 leaves that row out of
@@ -186,7 +188,7 @@ int bullseye_grid_batched_facets(gridding_parameters *params, const bullseye_fac
 void bullseye_set_batched_profiling(int on);
 /* The last profiled call's class launches: support width, correlations (4 visibilities, 1
  * sampling function), layout (J rows per thread; `wide` bit 0 = WIDE, bits 1.. = the build's register
- * cap), (track run, facet) work items and
+ * cap), (track run, facet) pairs and
  * milliseconds, up to max entries; returns the number of launches recorded. */
 int bullseye_batched_profile(int *width, int *nc, int *J, int *wide, int *items, float *ms, int max);
 /* Support-class width the batched gridder uses for every w plane (the plane's nonzero window,
