@@ -136,15 +136,19 @@ __global__ void __launch_bounds__(256) convert_grid_kernel(vis_complex *hi, vis_
   }
 }
 // The same for a grid without a second word yet (lo is written).
-__global__ void widen_grid_new_kernel(vis_complex *hi, vis_complex *lo, long long n) {
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const uint2 h = reinterpret_cast<const uint2 *>(hi)[i];
+__global__ void __launch_bounds__(256) widen_grid_new_kernel(vis_complex *hi, vis_complex *lo, long long n) {
+  const int lane = threadIdx.x & 31;
+  for (long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x - lane; i0 < n;
+       i0 += (long long)gridDim.x * blockDim.x) {
+    const long long i = i0 + lane;
+    uint2 h = make_uint2(0, 0);
+    if (i < n) h = reinterpret_cast<const uint2 *>(hi)[i];
     double im = 0.0;
-    if (h.x | h.y) {
+    if (__any_sync(0xffffffffu, (h.x | h.y) != 0) && (h.x | h.y)) {
       reinterpret_cast<double *>(hi)[i] = (double)__uint_as_float(h.x);
       im = (double)__uint_as_float(h.y);
     }
-    reinterpret_cast<double *>(lo)[i] = im;
+    if (i < n) reinterpret_cast<double *>(lo)[i] = im;
   }
 }
 #endif
