@@ -74,8 +74,10 @@ __global__ void invert_jones_kernel(const vis_complex *__restrict__ in, vis_comp
 // cover 6 % of it), the kernels then read 16 bytes a cell (HBM), and the FP64 pipe is kept for the rest.
 __device__ __forceinline__ bool widen_cell(uint2 &h, uint2 &l) {
   if ((h.x | h.y | l.x | l.y) == 0) return false;
-  const double re = (double)__uint_as_float(h.x) + (double)__uint_as_float(l.x);
-  const double im = (double)__uint_as_float(h.y) + (double)__uint_as_float(l.y);
+  // (-0 + 0 is +0: a cell without a second word keeps its sign)
+  double re = (double)__uint_as_float(h.x), im = (double)__uint_as_float(h.y);
+  if (l.x) re += (double)__uint_as_float(l.x);
+  if (l.y) im += (double)__uint_as_float(l.y);
   h = make_uint2((unsigned)__double2loint(re), (unsigned)__double2hiint(re));
   l = make_uint2((unsigned)__double2loint(im), (unsigned)__double2hiint(im));
   return true;
@@ -84,8 +86,11 @@ __device__ __forceinline__ bool narrow_cell(uint2 &h, uint2 &l) {
   if ((h.x | h.y | l.x | l.y) == 0) return false;
   const double re = __hiloint2double((int)h.y, (int)h.x), im = __hiloint2double((int)l.y, (int)l.x);
   const float a = (float)re, b = (float)im;
+  // what is not finite has no second word: inf - inf would turn an infinity that lies in the grid into NaN
+  const float a2 = isfinite(a) ? (float)(re - (double)a) : 0.f;
+  const float b2 = isfinite(b) ? (float)(im - (double)b) : 0.f;
   h = make_uint2(__float_as_uint(a), __float_as_uint(b));
-  l = make_uint2(__float_as_uint((float)(re - (double)a)), __float_as_uint((float)(im - (double)b)));
+  l = make_uint2(__float_as_uint(a2), __float_as_uint(b2));
   return true;
 }
 // Both directions over n cells, eight cells per thread in flight (16-byte loads of two cells when both
