@@ -272,21 +272,8 @@ __global__ void __launch_bounds__(kDegridWarps * 32, sizeof(acc_real) == 4 ? 4 :
       ra = (double)a.facet_centres[2 * f];
       dec = (double)a.facet_centres[2 * f + 1];
     }
-    // same constants as the gridder (phase_transform_policies.h:110-134, baseline_transform_policies.h:117-149)
-    const double k = (double)kArcsecToRad;
-    double d_ra = (ra - a.ra0) * k, n_dec = dec * k, o_dec = a.dec0 * k;
-    double c_d_ra = cos(d_ra), s_d_ra = sin(d_ra), c_n = cos(n_dec), s_n = sin(n_dec), c_o = cos(o_dec), s_o = sin(o_dec);
-    FacetXform x;
-    memset(&x, 0, sizeof x);
-    if (a.faceting) {
-      double li0 = c_n * s_d_ra, mi0 = s_n * c_o - c_n * s_o * c_d_ra, ni0 = s_n * s_o + c_n * c_o * c_d_ra;
-      x.u_term = li0 / ni0;
-      x.v_term = mi0 / ni0;
-      x.dl = -c_n * s_d_ra;
-      x.dm = -(s_n * c_o - c_n * s_o * c_d_ra);
-      x.dn = 1.0 - sqrt(1.0 - x.dl * x.dl - x.dm * x.dm);
-    }
-    fx[f] = x;
+    // the gridder's own transform, so that a sample takes the same cells
+    fx[f] = facet_transform(a.ra0, a.dec0, ra, dec, a.faceting != 0, a.faceting != 0);
   }
   // nonzero window [lo, hi] of every w plane's kernel row, one warp per plane: a footprint cell s
   // reads sample fu + s*os with fu in [floor(os/2), floor(3 os/2)] (w-projection, round to nearest)

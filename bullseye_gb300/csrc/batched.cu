@@ -1456,7 +1456,7 @@ extern "C" int bullseye_grid_batched_facets(gridding_parameters *pp, const bulls
   const double ra0 = (double)p.phase_centre_ra, dec0 = (double)p.phase_centre_dec;
   for (int f = 0; f < nfacets; ++f) {
     const bullseye_facet &d = facets[f];
-    fx[f] = bz_facet_xform(ra0, dec0, faceting ? d.ra : ra0, faceting ? d.dec : dec0, faceting, faceting);
+    fx[f] = facet_transform(ra0, dec0, faceting ? d.ra : ra0, faceting ? d.dec : dec0, faceting, faceting);
     fx[f].nx = (int)d.nx;
     fx[f].ny = (int)d.ny;
     fx[f].u_scale = (double)d.nx * d.cell_x * (double)kArcsecToRad;

@@ -63,7 +63,7 @@ __device__ __forceinline__ cplx cmul(cplx a, cplx b) {
 
 enum CorrMode { CORR_SINGLE = 0, CORR_DUAL = 1, CORR_QUAD = 2, CORR_QUAD_JONES = 3, CORR_SAMPLING = 4 };
 
-// Per-facet transform constants, evaluated on the host in FP64
+// Per-facet transform constants in FP64
 // (phase_transform_policies.h:110-134, baseline_transform_policies.h:117-149).
 struct FacetXform {
   double u_term, v_term;  // planar uv transform: u -= w u_term, v -= w v_term
@@ -74,6 +74,31 @@ struct FacetXform {
   long long grid_base;
   int nx, ny;
 };
+
+// The transform to a facet centre (arcsec), with its phase rotation and its uv transform each on or off: the
+// one place where host and device code form it.  At the phase centre both are exactly the identity: where
+// multiply-adds are contracted the differences of products below would leave their rounding errors (1e-17),
+// which move a sample that lies on a cell boundary.
+__host__ __device__ inline FacetXform facet_transform(double ra0, double dec0, double ra, double dec, bool phase,
+                                                      bool uvx) {
+  FacetXform x = {};
+  if (ra == ra0 && dec == dec0) return x;
+  const double k = (double)kArcsecToRad;
+  const double d_ra = (ra - ra0) * k, n_dec = dec * k, o_dec = dec0 * k;
+  const double c_d_ra = cos(d_ra), s_d_ra = sin(d_ra), c_n = cos(n_dec), s_n = sin(n_dec), c_o = cos(o_dec),
+               s_o = sin(o_dec);
+  if (uvx) {
+    const double li0 = c_n * s_d_ra, mi0 = s_n * c_o - c_n * s_o * c_d_ra, ni0 = s_n * s_o + c_n * c_o * c_d_ra;
+    x.u_term = li0 / ni0;
+    x.v_term = mi0 / ni0;
+  }
+  if (phase) {
+    x.dl = -c_n * s_d_ra;
+    x.dm = -(s_n * c_o - c_n * s_o * c_d_ra);
+    x.dn = 1.0 - sqrt(1.0 - x.dl * x.dl - x.dm * x.dm);
+  }
+  return x;
+}
 
 struct GridArgs {
   // row inputs (device)

@@ -675,31 +675,6 @@ extern "C" void repack_input_data(gridding_parameters *pp) {
 }
 
 // ---------------------------------------------------------------- gridding launch
-FacetXform bz_facet_xform(double ra0, double dec0, double ra, double dec, bool phase, bool uvx) {
-  // phase_transform_policies.h:110-134 and baseline_transform_policies.h:117-149, in FP64
-  FacetXform x;
-  std::memset(&x, 0, sizeof x);
-  // at the phase centre both transforms are the identity: a host that contracts the differences of
-  // products below into fused multiply-adds would leave their rounding errors (1e-17), which move a
-  // sample that lies on a cell boundary
-  if (ra == ra0 && dec == dec0) return x;
-  const double k = (double)kArcsecToRad;
-  double d_ra = (ra - ra0) * k, n_dec = dec * k, o_dec = dec0 * k;
-  double c_d_ra = cos(d_ra), s_d_ra = sin(d_ra), c_n = cos(n_dec), s_n = sin(n_dec), c_o = cos(o_dec),
-         s_o = sin(o_dec);
-  if (uvx) {
-    double li0 = c_n * s_d_ra, mi0 = s_n * c_o - c_n * s_o * c_d_ra, ni0 = s_n * s_o + c_n * c_o * c_d_ra;
-    x.u_term = li0 / ni0;
-    x.v_term = mi0 / ni0;
-  }
-  if (phase) {
-    x.dl = -c_n * s_d_ra;
-    x.dm = -(s_n * c_o - c_n * s_o * c_d_ra);
-    x.dn = 1.0 - sqrt(1.0 - x.dl * x.dl - x.dm * x.dm);
-  }
-  return x;
-}
-
 struct LaunchShape {
   int J, NT;
   bool wide;
@@ -999,7 +974,7 @@ bool bz_prepare_grid_args(const gridding_parameters &p, int nc, int mode, bool f
     }
     // the sampling-function policy reports the phase centre as facet centre
     // (phase_transform_policies.h:77-82), so its uv transform is the identity
-    fx[f] = bz_facet_xform(ra0, dec0, ra, dec, phase, faceting);
+    fx[f] = facet_transform(ra0, dec0, ra, dec, phase, faceting);
     // every facet shares the library's grid size: u_scale = nx * cell * ARCSEC_TO_RAD,
     // v_scale = -(ny * cell * ARCSEC_TO_RAD) (templated_gridder.h:23-24)
     fx[f].nx = (int)c.nx;

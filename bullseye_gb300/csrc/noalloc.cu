@@ -53,24 +53,14 @@ static std::mutex g_noalloc_resolve_mutex;
 
 namespace {
 
-// Per-facet transform constants (FP64) from device-resident facet centres (arcsec):
-// phase_transform_policies.h:110-134 and baseline_transform_policies.h:117-149.
+// Per-facet transform constants (FP64) from device-resident facet centres (arcsec).
 __global__ void noalloc_facet_table_kernel(FacetXform *out, const vis_real *centres, int nf, double ra0, double dec0,
                                            int nx, int ny, double u_scale, double v_scale, double gcx, double gcy,
                                            long long facet_elems) {
   int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= nf) return;
-  const double k = (double)kArcsecToRad;
   const double ra = centres ? (double)centres[2 * f] : ra0, dec = centres ? (double)centres[2 * f + 1] : dec0;
-  double d_ra = (ra - ra0) * k, n_dec = dec * k, o_dec = dec0 * k;
-  double c_d_ra = cos(d_ra), s_d_ra = sin(d_ra), c_n = cos(n_dec), s_n = sin(n_dec), c_o = cos(o_dec), s_o = sin(o_dec);
-  FacetXform x;
-  double li0 = c_n * s_d_ra, mi0 = s_n * c_o - c_n * s_o * c_d_ra, ni0 = s_n * s_o + c_n * c_o * c_d_ra;
-  x.u_term = li0 / ni0;
-  x.v_term = mi0 / ni0;
-  x.dl = -c_n * s_d_ra;
-  x.dm = -(s_n * c_o - c_n * s_o * c_d_ra);
-  x.dn = 1.0 - sqrt(1.0 - x.dl * x.dl - x.dm * x.dm);
+  FacetXform x = facet_transform(ra0, dec0, ra, dec, true, true);
   x.nx = nx;
   x.ny = ny;
   x.u_scale = u_scale;
