@@ -170,8 +170,9 @@ struct Workspace {
 };
 
 // Every rejection happens before the first launch, so a rejected call leaves the caller's arrays
-// (jones_terms included) untouched.  Only a launch failure reported by the runtime after the Jones
-// inversion was queued (the device is then unusable anyway) returns with the terms inverted.
+// (jones_terms included) untouched.  Only a launch failure that the runtime reports after the Jones
+// inversion was queued returns with the terms inverted; the caller's grid then holds its earlier values, plus
+// what the launches before the failure added.
 int grid_4cor_jones(const gridding_parameters &p, const Workspace &ws, void *stream, const char *name) {
   const size_t F = p.num_facet_centres ? p.num_facet_centres : 1;
   const size_t nxy = p.nx * p.ny;
@@ -267,11 +268,6 @@ int grid_4cor_jones(const gridding_parameters &p, const Workspace &ws, void *str
 
   // launches
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-#if defined(BULLSEYE_SINGLE)
-  if (p.row_count > 0 &&
-      !bz_widen_grid(p.output_buffer, ws.lo, (long long)grid_elems, false, st))
-    return BZ_ERR_CUDA;
-#endif
   if (cudaMemsetAsync(ws.err, 0, sizeof(int), st) != cudaSuccess) return BZ_ERR_CUDA;
   noalloc_facet_table_kernel<<<(unsigned)((F + 127) / 128), 128, 0, st>>>(
       ws.table, p.facet_centres, (int)F, (double)p.phase_centre_ra, (double)p.phase_centre_dec, (int)p.nx, (int)p.ny,
@@ -281,17 +277,22 @@ int grid_4cor_jones(const gridding_parameters &p, const Workspace &ws, void *str
   if (nj > 0) noalloc_invert_kernel<<<(unsigned)((nj + 255) / 256), 256, 0, st>>>(p.jones_terms, nj, ws.err);
   if (cudaGetLastError() != cudaSuccess) return BZ_ERR_CUDA;
   if (p.row_count == 0) return BZ_OK;
+  // the caller's grid is in the wide form only between these two conversions, whatever fails there
+#if defined(BULLSEYE_SINGLE)
+  if (!bz_widen_grid(p.output_buffer, ws.lo, (long long)grid_elems, false, st)) return BZ_ERR_CUDA;
+#endif
+  int rc = BZ_OK;
   if (ws.sched) {
     // workspace entry: support-aware (each w plane's nonzero window only; the same grids)
-    if (!bz_grid_support_aware(a, (int)F, ws.sched, ws.sched_bytes, st)) return bz_error_code() ? bz_error_code() : BZ_ERR_CUDA;
+    if (!bz_grid_support_aware(a, (int)F, ws.sched, ws.sched_bytes, st)) rc = bz_error_code() ? bz_error_code() : BZ_ERR_CUDA;
   } else if (!(wproj ? noalloc_dispatch<true>(a, blocks, st) : noalloc_dispatch<false>(a, blocks, st))) {
     bz_record_error(BZ_ERR_CUDA, "%s: gridder launch failed", name);
-    return BZ_ERR_CUDA;
+    rc = BZ_ERR_CUDA;
   }
 #if defined(BULLSEYE_SINGLE)
-  if (!bz_narrow_grid(p.output_buffer, ws.lo, p.output_buffer, (long long)grid_elems, st)) return BZ_ERR_CUDA;
+  if (!bz_narrow_grid(p.output_buffer, ws.lo, p.output_buffer, (long long)grid_elems, st) && rc == BZ_OK) rc = BZ_ERR_CUDA;
 #endif
-  return BZ_OK;
+  return rc;
 }
 
 // Maps the error bits of a call's error word to the library's sticky error (as the regular entry
