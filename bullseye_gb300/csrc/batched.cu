@@ -119,8 +119,7 @@ __global__ void scan_kernel(const int *__restrict__ in, int *__restrict__ out, i
 // outside the table is left out and reported rather than counted out of bounds.
 __global__ void seg_write_kernel(const size_t *starts, int nslots, int seg_len, long long R, int nchan,
                                  const unsigned char *__restrict__ cls, const int *__restrict__ off,
-                                 const int *__restrict__ nseg, int4 *__restrict__ segs, int *__restrict__ class_count,
-                                 int ncls, int *err) {
+                                 const int *__restrict__ nseg, int4 *__restrict__ segs, int ncls, int *err) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= nslots * nchan) return;
   int c;
@@ -137,46 +136,98 @@ __global__ void seg_write_kernel(const size_t *starts, int nslots, int seg_len, 
       if (kc < 0) atomicOr(err, DEV_ERR_GRID_INDEX);
       segs[o] = make_int4((int)begin, (int)(r + 1), c, kc);
       o += back ? -1 : 1;
-      if (kc >= 0) atomicAdd(&class_count[kc], 1);
       begin = r + 1;
     }
   }
 }
 
-// The runs of class blockIdx.x, in track order, behind those of the classes before it (one block per
-// class; a stable bucketing, so that consecutive runs of a class are neighbouring channels of one
-// baseline: a work item takes several, see romein_segment_kernel).  Also writes the class offsets.
+// Stable bucketing by class: the runs of a class in track order, so that consecutive runs of a class are
+// neighbouring channels of one baseline (a work item takes several, see romein_segment_kernel).  Block b takes
+// the runs [b per, (b + 1) per): a first launch counts their classes, a second one places them behind the
+// earlier classes and blocks.  (With one block per class that passes over all runs by itself a call of 10
+// million visibilities in time order took 64.5 ms, 62.4 so.)
+constexpr int kBucketRuns = 4096;    // runs per block, more past kBucketBlocks blocks
+constexpr int kBucketBlocks = 1024;
+static_assert(kMaxClasses == 32, "a lane or warp per class");
+struct BucketShape {
+  int blocks, per;
+};
+inline BucketShape bucket_shape(long long maxseg) {
+  BucketShape s;
+  s.per = (int)std::max<long long>(kBucketRuns, (maxseg + kBucketBlocks - 1) / kBucketBlocks);
+  s.blocks = (int)std::max<long long>(1, (maxseg + s.per - 1) / s.per);
+  return s;
+}
+
+__global__ void __launch_bounds__(1024) bucket_count_kernel(const int4 *__restrict__ segs, const int *__restrict__ total,
+                                                            int per, int *__restrict__ block_count,
+                                                            int *__restrict__ class_count) {
+  __shared__ int s_count[kMaxClasses];
+  const int tid = threadIdx.x;
+  const long long n = *total, lo = (long long)blockIdx.x * per, hi = min(n, lo + per);
+  if (lo >= n) return;
+  if (tid < kMaxClasses) s_count[tid] = 0;
+  __syncthreads();
+  for (long long i0 = lo; i0 < hi; i0 += 1024) {
+    const long long i = i0 + tid;
+    const int k = i < hi ? segs[i].w : -1;  // (a run without a class was reported by seg_write_kernel)
+    const unsigned m = __match_any_sync(0xffffffffu, k);
+    if (k >= 0 && (tid & 31) == __ffs(m) - 1) atomicAdd(&s_count[k], __popc(m));
+  }
+  __syncthreads();
+  if (tid < kMaxClasses) {
+    block_count[blockIdx.x * kMaxClasses + tid] = s_count[tid];
+    if (s_count[tid]) atomicAdd(&class_count[tid], s_count[tid]);
+  }
+}
+
 __global__ void __launch_bounds__(1024) bucket_kernel(const int4 *__restrict__ segs, const int *__restrict__ total,
+                                                      int per, int ncls, const int *__restrict__ block_count,
                                                       const int *__restrict__ class_count, int4 *__restrict__ sorted,
                                                       int *__restrict__ class_off) {
-  __shared__ int s_warp[33];
-  const int k = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  int at = 0;
-  for (int i = 0; i < k; ++i) at += class_count[i];
-  if (tid == 0) class_off[k] = at;
-  if (class_count[k] == 0) return;
-  const int n = *total;
-  for (int b = 0; b < n; b += 1024) {
-    const int i = b + tid;
-    const bool mine = i < n && segs[i].w == k;  // (a run without a class was reported by seg_write_kernel)
-    const unsigned m = __ballot_sync(0xffffffffu, mine);
-    if (lane == 0) s_warp[warp] = __popc(m);
-    __syncthreads();
-    if (warp == 0) {
-      const int x = s_warp[lane];
-      int sum = x;
+  __shared__ int s_base[kMaxClasses];
+  __shared__ int s_at[32][kMaxClasses + 1];  // [warp][class]: first the warp's runs, then its first place
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const long long n = *total, lo = (long long)blockIdx.x * per, hi = min(n, lo + per);
+  if (blockIdx.x > 0 && lo >= n) return;
+  if (warp == 0) {
+    const int x = lane < ncls ? class_count[lane] : 0;
+    int sum = x;
 #pragma unroll
-      for (int off = 1; off < 32; off <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, sum, off);
-        if (lane >= off) sum += y;
-      }
-      s_warp[lane] = sum - x;
-      if (lane == 31) s_warp[32] = sum;
+    for (int off = 1; off < 32; off <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, sum, off);
+      if (lane >= off) sum += y;
     }
+    s_base[lane] = sum - x;
+    if (blockIdx.x == 0 && lane < ncls) class_off[lane] = sum - x;
+  }
+  __syncthreads();
+  int before = 0;  // runs of class `lane` in a warp's share of the earlier blocks
+  for (int b = warp; b < (int)blockIdx.x; b += 32) before += block_count[b * kMaxClasses + lane];
+  if (before) atomicAdd(&s_base[lane], before);
+  __syncthreads();
+  int base = s_base[warp];  // warp k: the next place of class k
+  for (long long i0 = lo; i0 < hi; i0 += 1024) {
+    const long long i = i0 + tid;
+    int4 sg = make_int4(0, 0, 0, -1);
+    if (i < hi) sg = segs[i];
+    const unsigned m = __match_any_sync(0xffffffffu, sg.w);
+    s_at[warp][lane] = 0;
+    __syncwarp();
+    if (sg.w >= 0 && lane == __ffs(m) - 1) s_at[warp][sg.w] = __popc(m);
     __syncthreads();
-    if (mine) sorted[at + s_warp[warp] + __popc(m & ((1u << lane) - 1))] = segs[i];
-    at += s_warp[32];
+    const int x = s_at[lane][warp];
+    int sum = x;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, sum, off);
+      if (lane >= off) sum += y;
+    }
+    s_at[lane][warp] = base + sum - x;
+    base += __shfl_sync(0xffffffffu, sum, 31);
     __syncthreads();
+    if (sg.w >= 0) sorted[s_at[warp][sg.w] + __popc(m & ((1u << lane) - 1))] = sg;
+    __syncwarp();
   }
 }
 
@@ -536,7 +587,7 @@ struct BatchedState {
   ClassInfo cls[kMaxClasses];
   DevBuf<int> plane_class, plane_lo;
   DevBuf<unsigned char> row_class;
-  DevBuf<int> nseg, seg_off, seg_total, class_count, class_off, work_next, sample_count;
+  DevBuf<int> nseg, seg_off, seg_total, class_count, bucket_count, class_off, work_next, sample_count;
   DevBuf<int4> segs, sorted;
   DevBuf<FacetXform> facet_table;  // per-facet geometry of bullseye_grid_batched_facets
   DevBuf<vis_real> conv_w;         // support-window table [P][tap_f][conv_w_stride] (plan_classes)
@@ -685,7 +736,8 @@ bool plan_classes() {
   if (!b.plane_class.alloc(P) || !b.plane_lo.alloc(P)) return false;
   BZ_CUDA_TRY_RET(cudaMemcpy(b.plane_class.ptr, pcls.data(), sizeof(int) * P, cudaMemcpyHostToDevice), false);
   BZ_CUDA_TRY_RET(cudaMemcpy(b.plane_lo.ptr, plo.data(), sizeof(int) * P, cudaMemcpyHostToDevice), false);
-  if (!b.class_count.alloc(kMaxClasses) || !b.class_off.alloc(kMaxClasses) ||
+  if (!b.class_count.alloc(kMaxClasses) || !b.bucket_count.alloc((size_t)kBucketBlocks * kMaxClasses) ||
+      !b.class_off.alloc(kMaxClasses) ||
       !b.work_next.alloc(2 * kMaxClasses) || !b.seg_total.alloc(1) || !b.sample_count.alloc(2 * kMaxClasses))
     return false;
   b.planned = true;
@@ -1078,10 +1130,13 @@ bool enqueue_schedule(const GridArgs &va, cudaStream_t st, long long r0 = 0, lon
                                                          b.nseg.ptr);
   scan_kernel<<<1, 1024, 0, st>>>(b.nseg.ptr, b.seg_off.ptr, tracks, b.seg_total.ptr);
   seg_write_kernel<<<(tracks + 127) / 128, 128, 0, st>>>(va.starts, va.nslots, va.seg, R, va.nchan, b.row_class.ptr,
-                                                         b.seg_off.ptr, b.nseg.ptr, b.segs.ptr, b.class_count.ptr, b.ncls,
-                                                         va.error);
-  bucket_kernel<<<b.ncls, 1024, 0, st>>>(b.segs.ptr, b.seg_total.ptr, b.class_count.ptr, b.sorted.ptr, b.class_off.ptr);
-  c.launches += 5;
+                                                         b.seg_off.ptr, b.nseg.ptr, b.segs.ptr, b.ncls, va.error);
+  const BucketShape bs = bucket_shape(n * va.nchan);
+  bucket_count_kernel<<<bs.blocks, 1024, 0, st>>>(b.segs.ptr, b.seg_total.ptr, bs.per, b.bucket_count.ptr,
+                                                  b.class_count.ptr);
+  bucket_kernel<<<bs.blocks, 1024, 0, st>>>(b.segs.ptr, b.seg_total.ptr, bs.per, b.ncls, b.bucket_count.ptr,
+                                            b.class_count.ptr, b.sorted.ptr, b.class_off.ptr);
+  c.launches += 6;
   BZ_CUDA_TRY_RET(cudaGetLastError(), false);
   return true;
 }
@@ -1092,7 +1147,7 @@ void bz_release_batched() {
   BatchedState &b = g_bs;
   b.drop_graphs();
   b.plane_class.release(); b.plane_lo.release(); b.row_class.release(); b.nseg.release(); b.seg_off.release();
-  b.seg_total.release(); b.class_count.release(); b.class_off.release();
+  b.seg_total.release(); b.class_count.release(); b.bucket_count.release(); b.class_off.release();
   b.work_next.release(); b.sample_count.release(); b.segs.release(); b.sorted.release(); b.facet_table.release();
   b.conv_w.release();
   b.conv_w_stride = 0;
@@ -1246,7 +1301,7 @@ int run_batched(const GridArgs &va, const GridArgs *sa, int nfacets, const GridA
   bz_trace_mark("schedule_tune_capture");
   BZ_CUDA_TRY_RET(cudaGraphLaunch(slot->exec, c.stream), BZ_ERR_CUDA);
   const int rec = b.vrec_on && b.vrec.ptr && b.conv_w.ptr ? 2 : 0;  // record offsets + record kernel per build
-  c.launches += 5 + (long long)(b.ncls + rec) * ((vis ? 1 : 0) + (sf ? 1 : 0));
+  c.launches += 6 + (long long)(b.ncls + rec) * ((vis ? 1 : 0) + (sf ? 1 : 0));
   return BZ_OK;
 }
 
@@ -1753,8 +1808,13 @@ bool bz_grid_support_aware(const GridArgs &a_in, int nfacets, unsigned char *ws,
                                                          nseg);
   scan_kernel<<<1, 1024, 0, st>>>(nseg, seg_off, tracks, seg_total);
   seg_write_kernel<<<(tracks + 127) / 128, 128, 0, st>>>(a_in.starts, a_in.nslots, a_in.seg, R, a_in.nchan, row_class,
-                                                         seg_off, nseg, segs, class_count, cl.n, a_in.error);
-  bucket_kernel<<<cl.n, 1024, 0, st>>>(segs, seg_total, class_count, sorted, class_off);
+                                                         seg_off, nseg, segs, cl.n, a_in.error);
+  // the rows' classes are read for the last time above: the blocks' counts take their place (128 bytes per block
+  // of at least 4,096 runs, against a byte per row and channel)
+  const BucketShape bs = bucket_shape(l.maxseg);
+  int *bucket_count = reinterpret_cast<int *>(row_class);
+  bucket_count_kernel<<<bs.blocks, 1024, 0, st>>>(segs, seg_total, bs.per, bucket_count, class_count);
+  bucket_kernel<<<bs.blocks, 1024, 0, st>>>(segs, seg_total, bs.per, cl.n, bucket_count, class_count, sorted, class_off);
   if (cudaGetLastError() != cudaSuccess) return false;
   GridArgs a = a_in;
   a.W_full = W;
