@@ -593,8 +593,13 @@ struct BatchedState {
   DevBuf<vis_real> conv_w;         // support-window table [P][tap_f][conv_w_stride] (plan_classes)
   int conv_w_stride = 0;
   size_t rows_cap = 0, tracks_cap = 0, segs_cap = 0;
-  // tuning decisions, by (class width, NC, WPROJ, COMP)
-  std::map<std::tuple<int, int, int, int>, std::tuple<int, int>> tuned;  // -> (J, wide)
+  // layout decisions, by (class width, NC, WPROJ, COMP): timed, or a default of a class that had nothing to time
+  // on (no work, or no records) and is timed by the first call that has
+  struct Layout {
+    int J;
+    bool wide, timed;
+  };
+  std::map<std::tuple<int, int, int, int>, Layout> tuned;
   // captured graphs, by launch arguments (two slots: the reference's exports alternate between
   // the visibilities and the sampling function); least recently used is replaced
   struct GraphSlot {
@@ -952,7 +957,7 @@ bool launch_class(const GridArgs &base, int k, const Variant &v, int nfacets, co
   return launch_build<NC, WPROJ, COMP>(base, k, in, true, nfacets, count, next, st);
 }
 
-// Autotuner: time every valid layout of a class on a sample of its own work items, gridding into
+// Autotuner: time every valid layout of a class on a sample of its own work items, gridding their records into
 // scratch grids, and keep the fastest.  Decisions are cached by (width, NC, WPROJ, COMP).
 template <int NC, bool WPROJ, bool COMP>
 bool tune_class(const GridArgs &base, int k, int nfacets, Variant &out, int host_count) {
@@ -974,16 +979,18 @@ bool tune_class(const GridArgs &base, int k, int nfacets, Variant &out, int host
     bz_record_error(BZ_ERR_UNSUPPORTED, "batched: no layout for support class %d", W);
     return false;
   }
-  if (it != b.tuned.end()) {
+  // launches without records have one fixed layout (inplace_variant): nothing to time there
+  const bool can_time = cands.size() > 1 && host_count > 0 && base.records;
+  if (it != b.tuned.end() && (it->second.timed || !can_time)) {
     for (auto &v : cands)
-      if (v.J == std::get<0>(it->second) && (int)v.wide == std::get<1>(it->second)) {
+      if (v.J == it->second.J && v.wide == it->second.wide) {
         out = v;
         return true;
       }
   }
-  if (cands.size() == 1 || host_count == 0) {
+  if (!can_time) {
     out = cands[0];
-    b.tuned[key] = std::make_tuple(out.J, (int)out.wide);
+    b.tuned[key] = {out.J, out.wide, cands.size() == 1};
     return true;
   }
   // Each candidate grids a quarter of the class's runs (at least 4096, when there are that many)
@@ -1003,10 +1010,10 @@ bool tune_class(const GridArgs &base, int k, int nfacets, Variant &out, int host
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
   for (auto &v : cands) {
-    if (!launch_class<NC, WPROJ, COMP>(a, k, v, nfacets, b.sample_count.ptr + 2 * k, b.work_next.ptr + k, c.stream))
+    if (!launch_build<NC, WPROJ, COMP>(a, k, v, false, nfacets, b.sample_count.ptr + 2 * k, b.work_next.ptr + k, c.stream))
       break;
     cudaEventRecord(e0, c.stream);
-    launch_class<NC, WPROJ, COMP>(a, k, v, nfacets, b.sample_count.ptr + 2 * k + 1, b.work_next.ptr + k, c.stream);
+    launch_build<NC, WPROJ, COMP>(a, k, v, false, nfacets, b.sample_count.ptr + 2 * k + 1, b.work_next.ptr + k, c.stream);
     cudaEventRecord(e1, c.stream);
     cudaEventSynchronize(e1);
     float ms = 0;
@@ -1019,8 +1026,9 @@ bool tune_class(const GridArgs &base, int k, int nfacets, Variant &out, int host
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   BZ_CUDA_TRY_RET(cudaMemsetAsync(c.scratch.ptr, 0, sizeof(vis_complex) * c.scratch.n, c.stream), false);
-  b.tuned[key] = std::make_tuple(out.J, (int)out.wide);
-  return bz_error_code() == BZ_OK;
+  if (bz_error_code() != BZ_OK) return false;
+  b.tuned[key] = {out.J, out.wide, true};
+  return true;
 }
 
 template <int NC, bool WPROJ, bool COMP>
@@ -1028,8 +1036,10 @@ bool tune_all(const GridArgs &base, int nfacets, bool sampling, const std::vecto
   // records for the timing runs only when some class has work and no layout decided yet (a
   // decided class takes its layout without launching)
   bool timing = false;
-  for (int k = 0; k < g_bs.ncls; ++k)
-    if (counts[k] > 0 && !g_bs.tuned.count(std::make_tuple(g_bs.cls[k].width, NC, (int)WPROJ, (int)COMP))) timing = true;
+  for (int k = 0; k < g_bs.ncls; ++k) {
+    const auto it = g_bs.tuned.find(std::make_tuple(g_bs.cls[k].width, NC, (int)WPROJ, (int)COMP));
+    if (counts[k] > 0 && (it == g_bs.tuned.end() || !it->second.timed)) timing = true;
+  }
   GridArgs tb = base, rb = base;
   tb.norm = nullptr;  // tuning launches leave the normalisation alone
   if (timing && !launch_records<NC, WPROJ>(tb, nfacets, g_ctx.stream, rb)) return false;
@@ -1079,7 +1089,11 @@ bool launch_all(const GridArgs &base_in, int nfacets, bool sampling, cudaStream_
       cudaEventElapsedTime(&ms, e0, e1);
       cudaEventDestroy(e0);
       cudaEventDestroy(e1);
-      b.records.push_back({b.cls[k].width, NC, v.J, (int)v.wide | (seg_regs(v.J) << 1), counts ? (*counts)[k] * nfacets : 0, ms});
+      // the build that ran: without records it is the in-place one
+      Variant ran = v;
+      if (!base.records) inplace_variant<NC, WPROJ, COMP>(b.cls[k].width, ran);
+      const int regs = !base.records && ran.J == 4 ? kInPlaceRegs : seg_regs(ran.J);
+      b.records.push_back({b.cls[k].width, NC, ran.J, (int)ran.wide | (regs << 1), counts ? (*counts)[k] * nfacets : 0, ms});
     }
     if (!ok) return false;
   }
