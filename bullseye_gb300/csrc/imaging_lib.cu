@@ -539,13 +539,13 @@ extern "C" void releaseLibrary() {
 }
 
 // ---------------------------------------------------------------- host loops
-// fn(lo, hi) over [0, n), on one thread per 32 MB of touched memory, eight at most: where another pool's
+// fn(lo, hi) over [0, n), on one thread per 32 MB of touched memory, 64 at most: where another pool's
 // threads still hold the cores (the caller's own loops), a thread takes milliseconds to start and join, and
 // uniform weighting of one 1024^2 facet (75 MB) takes 0.9 ms on three threads, 3.0 on one.  What cannot be started
 // runs here.
 template <typename Fn>
 static void parallel_for(size_t n, double bytes, Fn fn) {
-  const size_t most = std::min<size_t>(8, std::max(1u, std::thread::hardware_concurrency()));
+  const size_t most = std::min<size_t>(64, std::max(1u, std::thread::hardware_concurrency()));
   const size_t nt = std::min({most, n, (size_t)(bytes / 32e6) + 1});
   if (nt <= 1) {
     fn((size_t)0, n);
