@@ -537,6 +537,9 @@ using SegKernel = void (*)(const GridArgs, const int);
 template <int NC, bool WPROJ, bool COMP, bool WIDE>
 SegKernel<NC, WPROJ, COMP> seg_kernel_of(int J) {
   if (J == 8) return romein_segment_kernel<NC, WPROJ, 8, COMP, WIDE, true>;
+  if constexpr (!WIDE) {
+    if (J == 2) return romein_segment_kernel<NC, WPROJ, 2, COMP, WIDE, true>;
+  }
 #if defined(BULLSEYE_SINGLE)
   if constexpr (NC == 4 && WPROJ) {
     if (J == 6) return romein_segment_kernel<NC, WPROJ, 6, COMP, WIDE, true>;
@@ -557,11 +560,18 @@ constexpr int kInPlaceRegs = 128;
 template <int NC, bool WPROJ, bool COMP>
 SegKernel<NC, WPROJ, COMP> inplace_kernel(int J, bool wide) {
   if (wide) return romein_segment_kernel<NC, WPROJ, 8, COMP, true, false>;
+  if (J == 2) return romein_segment_kernel<NC, WPROJ, 2, COMP, false, false, kInPlaceRegs>;
   return J == 8 ? romein_segment_kernel<NC, WPROJ, 8, COMP, false, false>
                 : romein_segment_kernel<NC, WPROJ, 4, COMP, false, false, kInPlaceRegs>;
 }
 
-constexpr int seg_regs(int J) { return J == 4 ? kSegRegs<4> : J == 6 ? kSegRegs<6> : kSegRegs<8>; }
+constexpr int seg_regs(int J) { return J == 2 ? kSegRegs<2> : J == 4 ? kSegRegs<4> : J == 6 ? kSegRegs<6> : kSegRegs<8>; }
+
+// Supports whose cells one warp owns with two rows per thread (W = 7: 28 lanes, 14 with four rows).  Where each
+// sample moves the whole footprint the launches issue flushes, and half the lanes idled: gridding with its gradients,
+// W = 7, 64 antennas x 38 times x 45 channels at 0.67 degrees a sample 6.30 -> 4.83 ms, 64 x 60 x 16 with rows in time
+// order 5.66 -> 4.20; slow tracks 2.07 -> 1.84.
+constexpr bool narrow_support(int W) { return W * ((W + 1) / 2) <= 32; }
 
 template <int NC, bool WPROJ>
 bool make_variant(int W, int J, bool wide, Variant &v) {
@@ -937,8 +947,10 @@ bool finish_variant(Variant &v, bool inplace = false) {
 // threads).
 template <int NC, bool WPROJ, bool COMP>
 bool inplace_variant(int W, Variant &v) {
-  for (int J : {4, 8})
+  for (int J : {2, 4, 8}) {
+    if (J == 2 && !narrow_support(W)) continue;
     if (make_variant<NC, WPROJ>(W, J, false, v) && finish_variant<NC, WPROJ, COMP>(v, true)) return true;
+  }
   return make_variant<NC, WPROJ>(W, 8, true, v) && finish_variant<NC, WPROJ, COMP>(v, true);
 }
 
@@ -969,9 +981,9 @@ bool tune_class(const GridArgs &base, int k, int nfacets, Variant &out, int host
   std::vector<Variant> cands;
   // J = 6 (single precision, four correlations, w-projection): 48 accumulator registers
   const bool six = BZ_PRECISION_BITS == 32 && NC == 4 && WPROJ;
-  for (int J : {8, 6, 4})
+  for (int J : {8, 6, 4, 2})
     for (bool wide : {true, false}) {
-      if (J == 6 && !six) continue;
+      if ((J == 6 && !six) || (J == 2 && (wide || !narrow_support(W)))) continue;
       Variant v;
       if (make_variant<NC, WPROJ>(W, J, wide, v) && finish_variant<NC, WPROJ, COMP>(v)) cands.push_back(v);
     }
@@ -1092,7 +1104,7 @@ bool launch_all(const GridArgs &base_in, int nfacets, bool sampling, cudaStream_
       // the build that ran: without records it is the in-place one
       Variant ran = v;
       if (!base.records) inplace_variant<NC, WPROJ, COMP>(b.cls[k].width, ran);
-      const int regs = !base.records && ran.J == 4 ? kInPlaceRegs : seg_regs(ran.J);
+      const int regs = !base.records && ran.J <= 4 ? kInPlaceRegs : seg_regs(ran.J);
       b.records.push_back({b.cls[k].width, NC, ran.J, (int)ran.wide | (regs << 1), counts ? (*counts)[k] * nfacets : 0, ms});
     }
     if (!ok) return false;

@@ -1829,7 +1829,7 @@ __device__ __forceinline__ void grid_records(const GridArgs &a, const int f_loca
 // Register caps of the persistent segment kernel: the J rows' accumulators (8 J values), the merge
 // step's values and the footprint state, without spills in the loops.
 template <int J>
-constexpr int kSegRegs = J == 4 && sizeof(acc_real) == 4 ? 96 : J == 6 ? 112 : 128;
+constexpr int kSegRegs = J <= 4 && sizeof(acc_real) == 4 ? 96 : J == 6 ? 112 : 128;
 
 // One CTA per track: blockIdx -> (facet, baseline slot or row segment, channel).
 template <int NC, bool WPROJ, int J, bool COMP, bool WIDE>
