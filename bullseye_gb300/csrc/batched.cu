@@ -530,39 +530,42 @@ struct Variant {
   ChunkShape chunk{0, 0, 0};
 };
 
-template <int NC, bool WPROJ, bool COMP>
+template <int NC, bool WPROJ, int ACC>
 using SegKernel = void (*)(const GridArgs, const int);
 
 // Launches from visibility records (the tuner's candidates).
-template <int NC, bool WPROJ, bool COMP, bool WIDE>
-SegKernel<NC, WPROJ, COMP> seg_kernel_of(int J) {
-  if (J == 8) return romein_segment_kernel<NC, WPROJ, 8, COMP, WIDE, true>;
+template <int NC, bool WPROJ, int ACC, bool WIDE>
+SegKernel<NC, WPROJ, ACC> seg_kernel_of(int J) {
+  if (J == 8) return romein_segment_kernel<NC, WPROJ, 8, ACC, WIDE, true>;
   if constexpr (!WIDE) {
-    if (J == 2) return romein_segment_kernel<NC, WPROJ, 2, COMP, WIDE, true>;
+    if (J == 2) return romein_segment_kernel<NC, WPROJ, 2, ACC, WIDE, true>;
   }
 #if defined(BULLSEYE_SINGLE)
   if constexpr (NC == 4 && WPROJ) {
-    if (J == 6) return romein_segment_kernel<NC, WPROJ, 6, COMP, WIDE, true>;
+    if (J == 6) return romein_segment_kernel<NC, WPROJ, 6, ACC, WIDE, true>;
   }
 #endif
-  return romein_segment_kernel<NC, WPROJ, 4, COMP, WIDE, true>;
+  return romein_segment_kernel<NC, WPROJ, 4, ACC, WIDE, true>;
 }
 
-template <int NC, bool WPROJ, bool COMP>
-SegKernel<NC, WPROJ, COMP> seg_kernel(int J, bool wide) {
-  return wide ? seg_kernel_of<NC, WPROJ, COMP, true>(J) : seg_kernel_of<NC, WPROJ, COMP, false>(J);
+template <int NC, bool WPROJ, int ACC>
+SegKernel<NC, WPROJ, ACC> seg_kernel(int J, bool wide) {
+  if constexpr (ACC != ACC_PAIR) {  // (small calls: two layouts do)
+    if (wide) return seg_kernel_of<NC, WPROJ, ACC, true>(J);
+  }
+  return seg_kernel_of<NC, WPROJ, ACC, false>(J);
 }
 
 // Launches that prepare their visibilities in place (no records, or past the record budget).  The prologue
 // needs registers beside the accumulators: 128 for the J = 4 layout (1.58 ms for a differentiable step's
 // class launches, 1.69 at 96).
 constexpr int kInPlaceRegs = 128;
-template <int NC, bool WPROJ, bool COMP>
-SegKernel<NC, WPROJ, COMP> inplace_kernel(int J, bool wide) {
-  if (wide) return romein_segment_kernel<NC, WPROJ, 8, COMP, true, false>;
-  if (J == 2) return romein_segment_kernel<NC, WPROJ, 2, COMP, false, false, kInPlaceRegs>;
-  return J == 8 ? romein_segment_kernel<NC, WPROJ, 8, COMP, false, false>
-                : romein_segment_kernel<NC, WPROJ, 4, COMP, false, false, kInPlaceRegs>;
+template <int NC, bool WPROJ, int ACC>
+SegKernel<NC, WPROJ, ACC> inplace_kernel(int J, bool wide) {
+  if (wide) return romein_segment_kernel<NC, WPROJ, 8, ACC, true, false>;
+  if (J == 2) return romein_segment_kernel<NC, WPROJ, 2, ACC, false, false, kInPlaceRegs>;
+  return J == 8 ? romein_segment_kernel<NC, WPROJ, 8, ACC, false, false>
+                : romein_segment_kernel<NC, WPROJ, 4, ACC, false, false, kInPlaceRegs>;
 }
 
 constexpr int seg_regs(int J) { return J == 2 ? kSegRegs<2> : J == 4 ? kSegRegs<4> : J == 6 ? kSegRegs<6> : kSegRegs<8>; }
@@ -603,7 +606,7 @@ struct BatchedState {
   DevBuf<vis_real> conv_w;         // support-window table [P][tap_f][conv_w_stride] (plan_classes)
   int conv_w_stride = 0;
   size_t rows_cap = 0, tracks_cap = 0, segs_cap = 0;
-  // layout decisions, by (class width, NC, WPROJ, COMP): timed, or a default of a class that had nothing to time
+  // layout decisions, by (class width, NC, WPROJ, ACC): timed, or a default of a class that had nothing to time
   // on (no work, or no records) and is timed by the first call that has
   struct Layout {
     int J;
@@ -900,7 +903,7 @@ bool launch_records(const GridArgs &base, int nfacets, cudaStream_t st, GridArgs
   return true;
 }
 
-template <int NC, bool WPROJ, bool COMP>
+template <int NC, bool WPROJ, int ACC>
 bool launch_build(const GridArgs &base, int k, const Variant &v, bool inplace, int nfacets, const int *count, int *next,
                   cudaStream_t st) {
   GridArgs a = base;
@@ -919,7 +922,7 @@ bool launch_build(const GridArgs &base, int k, const Variant &v, bool inplace, i
     bz_record_error(BZ_ERR_CUDA, "batched: no layout chosen for support class %d", a.W);
     return false;
   }
-  auto kern = inplace ? inplace_kernel<NC, WPROJ, COMP>(v.J, v.wide) : seg_kernel<NC, WPROJ, COMP>(v.J, v.wide);
+  auto kern = inplace ? inplace_kernel<NC, WPROJ, ACC>(v.J, v.wide) : seg_kernel<NC, WPROJ, ACC>(v.J, v.wide);
   if (!open_smem(kern)) {
     bz_record_error(BZ_ERR_CUDA, "batched: cudaFuncSetAttribute failed");
     return false;
@@ -931,9 +934,9 @@ bool launch_build(const GridArgs &base, int k, const Variant &v, bool inplace, i
   return true;
 }
 
-template <int NC, bool WPROJ, bool COMP>
+template <int NC, bool WPROJ, int ACC>
 bool finish_variant(Variant &v, bool inplace = false) {
-  auto kern = inplace ? inplace_kernel<NC, WPROJ, COMP>(v.J, v.wide) : seg_kernel<NC, WPROJ, COMP>(v.J, v.wide);
+  auto kern = inplace ? inplace_kernel<NC, WPROJ, ACC>(v.J, v.wide) : seg_kernel<NC, WPROJ, ACC>(v.J, v.wide);
   if (!open_smem(kern)) return false;
   int per_sm = 0, dev = 0, sms = 0;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, v.NT, v.chunk.smem) != cudaSuccess || per_sm < 1) return false;
@@ -945,38 +948,38 @@ bool finish_variant(Variant &v, bool inplace = false) {
 
 // The layout of launches that prepare in place: J = 4 (J = 8 where the J = 4 layout needs more than 512
 // threads).
-template <int NC, bool WPROJ, bool COMP>
+template <int NC, bool WPROJ, int ACC>
 bool inplace_variant(int W, Variant &v) {
   for (int J : {2, 4, 8}) {
     if (J == 2 && !narrow_support(W)) continue;
-    if (make_variant<NC, WPROJ>(W, J, false, v) && finish_variant<NC, WPROJ, COMP>(v, true)) return true;
+    if (make_variant<NC, WPROJ>(W, J, false, v) && finish_variant<NC, WPROJ, ACC>(v, true)) return true;
   }
-  return make_variant<NC, WPROJ>(W, 8, true, v) && finish_variant<NC, WPROJ, COMP>(v, true);
+  return make_variant<NC, WPROJ>(W, 8, true, v) && finish_variant<NC, WPROJ, ACC>(v, true);
 }
 
 // One support class: from records, and in place where there are none or they may not hold every item.
-template <int NC, bool WPROJ, bool COMP>
+template <int NC, bool WPROJ, int ACC>
 bool launch_class(const GridArgs &base, int k, const Variant &v, int nfacets, const int *count, int *next,
                   cudaStream_t st) {
   const bool all = base.records && (double)base.nrows * base.nchan * nfacets <= (double)base.rec_capacity;
-  if (base.records && !launch_build<NC, WPROJ, COMP>(base, k, v, false, nfacets, count, next, st)) return false;
+  if (base.records && !launch_build<NC, WPROJ, ACC>(base, k, v, false, nfacets, count, next, st)) return false;
   if (all) return true;
   Variant in;
-  if (!inplace_variant<NC, WPROJ, COMP>(g_bs.cls[k].width, in)) {
+  if (!inplace_variant<NC, WPROJ, ACC>(g_bs.cls[k].width, in)) {
     bz_record_error(BZ_ERR_UNSUPPORTED, "batched: no layout for support class %d", g_bs.cls[k].width);
     return false;
   }
-  return launch_build<NC, WPROJ, COMP>(base, k, in, true, nfacets, count, next, st);
+  return launch_build<NC, WPROJ, ACC>(base, k, in, true, nfacets, count, next, st);
 }
 
 // Autotuner: time every valid layout of a class on a sample of its own work items, gridding their records into
-// scratch grids, and keep the fastest.  Decisions are cached by (width, NC, WPROJ, COMP).
-template <int NC, bool WPROJ, bool COMP>
+// scratch grids, and keep the fastest.  Decisions are cached by (width, NC, WPROJ, ACC).
+template <int NC, bool WPROJ, int ACC>
 bool tune_class(const GridArgs &base, int k, int nfacets, Variant &out, int host_count) {
   BatchedState &b = g_bs;
   Context &c = g_ctx;
   const int W = b.cls[k].width;
-  auto key = std::make_tuple(W, NC, (int)WPROJ, (int)COMP);
+  auto key = std::make_tuple(W, NC, (int)WPROJ, ACC);
   auto it = b.tuned.find(key);
   std::vector<Variant> cands;
   // J = 6 (single precision, four correlations, w-projection): 48 accumulator registers
@@ -985,7 +988,7 @@ bool tune_class(const GridArgs &base, int k, int nfacets, Variant &out, int host
     for (bool wide : {true, false}) {
       if ((J == 6 && !six) || (J == 2 && (wide || !narrow_support(W)))) continue;
       Variant v;
-      if (make_variant<NC, WPROJ>(W, J, wide, v) && finish_variant<NC, WPROJ, COMP>(v)) cands.push_back(v);
+      if (make_variant<NC, WPROJ>(W, J, wide, v) && finish_variant<NC, WPROJ, ACC>(v)) cands.push_back(v);
     }
   if (cands.empty()) {
     bz_record_error(BZ_ERR_UNSUPPORTED, "batched: no layout for support class %d", W);
@@ -1014,7 +1017,7 @@ bool tune_class(const GridArgs &base, int k, int nfacets, Variant &out, int host
   BZ_CUDA_TRY_RET(cudaStreamSynchronize(c.stream), false);
   GridArgs a = base;
   a.grid = c.scratch.ptr;
-  a.grid_lo = COMP ? c.scratch.ptr : nullptr;
+  a.grid_lo = ACC != ACC_PLAIN ? c.scratch.ptr : nullptr;
   a.norm = nullptr;
   BZ_CUDA_TRY_RET(cudaStreamWaitEvent(c.stream, c.ev_copied_vis, 0), false);  // a copy-back may read the scratch grid
   float best = 1e30f;
@@ -1022,10 +1025,10 @@ bool tune_class(const GridArgs &base, int k, int nfacets, Variant &out, int host
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
   for (auto &v : cands) {
-    if (!launch_build<NC, WPROJ, COMP>(a, k, v, false, nfacets, b.sample_count.ptr + 2 * k, b.work_next.ptr + k, c.stream))
+    if (!launch_build<NC, WPROJ, ACC>(a, k, v, false, nfacets, b.sample_count.ptr + 2 * k, b.work_next.ptr + k, c.stream))
       break;
     cudaEventRecord(e0, c.stream);
-    launch_build<NC, WPROJ, COMP>(a, k, v, false, nfacets, b.sample_count.ptr + 2 * k + 1, b.work_next.ptr + k, c.stream);
+    launch_build<NC, WPROJ, ACC>(a, k, v, false, nfacets, b.sample_count.ptr + 2 * k + 1, b.work_next.ptr + k, c.stream);
     cudaEventRecord(e1, c.stream);
     cudaEventSynchronize(e1);
     float ms = 0;
@@ -1043,13 +1046,13 @@ bool tune_class(const GridArgs &base, int k, int nfacets, Variant &out, int host
   return true;
 }
 
-template <int NC, bool WPROJ, bool COMP>
+template <int NC, bool WPROJ, int ACC>
 bool tune_all(const GridArgs &base, int nfacets, bool sampling, const std::vector<int> &counts) {
   // records for the timing runs only when some class has work and no layout decided yet (a
   // decided class takes its layout without launching)
   bool timing = false;
   for (int k = 0; k < g_bs.ncls; ++k) {
-    const auto it = g_bs.tuned.find(std::make_tuple(g_bs.cls[k].width, NC, (int)WPROJ, (int)COMP));
+    const auto it = g_bs.tuned.find(std::make_tuple(g_bs.cls[k].width, NC, (int)WPROJ, ACC));
     if (counts[k] > 0 && (it == g_bs.tuned.end() || !it->second.timed)) timing = true;
   }
   GridArgs tb = base, rb = base;
@@ -1057,12 +1060,12 @@ bool tune_all(const GridArgs &base, int nfacets, bool sampling, const std::vecto
   if (timing && !launch_records<NC, WPROJ>(tb, nfacets, g_ctx.stream, rb)) return false;
   for (int k = 0; k < g_bs.ncls; ++k) {
     Variant &v = sampling ? g_bs.cls[k].sf : g_bs.cls[k].vis;
-    if (!tune_class<NC, WPROJ, COMP>(rb, k, nfacets, v, counts[k])) return false;
+    if (!tune_class<NC, WPROJ, ACC>(rb, k, nfacets, v, counts[k])) return false;
   }
   return true;
 }
 
-template <int NC, bool WPROJ, bool COMP>
+template <int NC, bool WPROJ, int ACC>
 bool launch_all(const GridArgs &base_in, int nfacets, bool sampling, cudaStream_t st, const std::vector<int> *counts) {
   BatchedState &b = g_bs;
   GridArgs base;
@@ -1092,7 +1095,7 @@ bool launch_all(const GridArgs &base_in, int nfacets, bool sampling, cudaStream_
       cudaEventCreate(&e1);
       cudaEventRecord(e0, st);
     }
-    const bool ok = launch_class<NC, WPROJ, COMP>(base, k, v, nfacets, b.class_count.ptr + k,
+    const bool ok = launch_class<NC, WPROJ, ACC>(base, k, v, nfacets, b.class_count.ptr + k,
                                                   b.work_next.ptr + (sampling ? kMaxClasses : 0) + k, st);
     if (b.profile) {
       cudaEventRecord(e1, st);
@@ -1103,7 +1106,7 @@ bool launch_all(const GridArgs &base_in, int nfacets, bool sampling, cudaStream_
       cudaEventDestroy(e1);
       // the build that ran: without records it is the in-place one
       Variant ran = v;
-      if (!base.records) inplace_variant<NC, WPROJ, COMP>(b.cls[k].width, ran);
+      if (!base.records) inplace_variant<NC, WPROJ, ACC>(b.cls[k].width, ran);
       const int regs = !base.records && ran.J <= 4 ? kInPlaceRegs : seg_regs(ran.J);
       b.records.push_back({b.cls[k].width, NC, ran.J, (int)ran.wide | (regs << 1), counts ? (*counts)[k] * nfacets : 0, ms});
     }
@@ -1114,31 +1117,38 @@ bool launch_all(const GridArgs &base_in, int nfacets, bool sampling, cudaStream_
 
 // vis = false launches (and tunes) only the sampling function's classes; va then only feeds the
 // schedule.
-template <bool WPROJ, bool COMP>
+template <bool WPROJ, int ACC>
 bool dispatch(const GridArgs &va, const GridArgs *sa, int nfacets, bool tune, const std::vector<int> &counts,
               cudaStream_t st, bool vis) {
   if (tune) {
-    if (vis && !tune_all<4, WPROJ, COMP>(va, nfacets, false, counts)) return false;
-    if (sa && !tune_all<1, WPROJ, COMP>(*sa, 1, true, counts)) return false;
+    if (vis && !tune_all<4, WPROJ, ACC>(va, nfacets, false, counts)) return false;
+    if constexpr (ACC != ACC_PAIR) {  // (caller-owned grids: no sampling function)
+      if (sa && !tune_all<1, WPROJ, ACC>(*sa, 1, true, counts)) return false;
+    }
     return true;
   }
-  if (vis && !launch_all<4, WPROJ, COMP>(va, nfacets, false, st, &counts)) return false;
-  if (sa && !launch_all<1, WPROJ, COMP>(*sa, 1, true, st, &counts)) return false;
+  if (vis && !launch_all<4, WPROJ, ACC>(va, nfacets, false, st, &counts)) return false;
+  if constexpr (ACC != ACC_PAIR) {
+    if (sa && !launch_all<1, WPROJ, ACC>(*sa, 1, true, st, &counts)) return false;
+  }
   return true;
 }
 
-bool run_dispatch(const GridArgs &va, const GridArgs *sa, bool wproj, bool comp, bool tune, const std::vector<int> &counts,
+bool run_dispatch(const GridArgs &va, const GridArgs *sa, bool wproj, Acc acc, bool tune, const std::vector<int> &counts,
                   cudaStream_t st, int nfacets, bool vis) {
   const int F = nfacets > 0 ? nfacets : (int)g_ctx.F;
 #if defined(BULLSEYE_SINGLE)
-  if (comp)
-    return wproj ? dispatch<true, true>(va, sa, F, tune, counts, st, vis)
-                 : dispatch<false, true>(va, sa, F, tune, counts, st, vis);
+  if (acc == ACC_WIDE)
+    return wproj ? dispatch<true, ACC_WIDE>(va, sa, F, tune, counts, st, vis)
+                 : dispatch<false, ACC_WIDE>(va, sa, F, tune, counts, st, vis);
+  if (acc == ACC_PAIR)
+    return wproj ? dispatch<true, ACC_PAIR>(va, nullptr, F, tune, counts, st, vis)
+                 : dispatch<false, ACC_PAIR>(va, nullptr, F, tune, counts, st, vis);
 #else
-  (void)comp;
+  (void)acc;
 #endif
-  return wproj ? dispatch<true, false>(va, sa, F, tune, counts, st, vis)
-               : dispatch<false, false>(va, sa, F, tune, counts, st, vis);
+  return wproj ? dispatch<true, ACC_PLAIN>(va, sa, F, tune, counts, st, vis)
+               : dispatch<false, ACC_PLAIN>(va, sa, F, tune, counts, st, vis);
 }
 
 // The schedule-building kernels (everything before the per-class launches), for the tracks of
@@ -1257,7 +1267,7 @@ namespace {
 // in profiling mode.  vis = false grids only the sampling function (sa), with va feeding the
 // schedule.
 int run_batched(const GridArgs &va, const GridArgs *sa, int nfacets, const GridArgs &ta, int tune_facets, bool wproj,
-                bool comp, const char *name, bool vis = true) {
+                Acc acc, const char *name, bool vis = true) {
   Context &c = g_ctx;
   BatchedState &b = g_bs;
   const bool sf = sa != nullptr;
@@ -1266,7 +1276,7 @@ int run_batched(const GridArgs &va, const GridArgs *sa, int nfacets, const GridA
   std::memcpy(key.data(), &va, sizeof(GridArgs));
   if (sf) std::memcpy(key.data() + sizeof(GridArgs), sa, sizeof(GridArgs));
   key[sizeof(GridArgs) * 2] = (unsigned char)sf;
-  key[sizeof(GridArgs) * 2 + 1] = (unsigned char)comp;
+  key[sizeof(GridArgs) * 2 + 1] = (unsigned char)acc;
   key[sizeof(GridArgs) * 2 + 2] = (unsigned char)vis;
   std::memcpy(key.data() + sizeof(GridArgs) * 2 + 4, &nfacets, sizeof(int));
 
@@ -1284,9 +1294,9 @@ int run_batched(const GridArgs &va, const GridArgs *sa, int nfacets, const GridA
   if (b.profile) {
     std::vector<int> counts(kMaxClasses, 0);
     if (!schedule_counts(counts)) return bz_error_code() ? bz_error_code() : BZ_ERR_CUDA;
-    if (!run_dispatch(ta, sa, wproj, comp, true, counts, c.stream, tune_facets, vis)) return bz_error_code();
+    if (!run_dispatch(ta, sa, wproj, acc, true, counts, c.stream, tune_facets, vis)) return bz_error_code();
     b.records.clear();
-    if (!run_dispatch(va, sa, wproj, comp, false, counts, c.stream, nfacets, vis)) return bz_error_code();
+    if (!run_dispatch(va, sa, wproj, acc, false, counts, c.stream, nfacets, vis)) return bz_error_code();
     return BZ_OK;
   }
   BatchedState::GraphSlot *slot = nullptr;
@@ -1300,14 +1310,14 @@ int run_batched(const GridArgs &va, const GridArgs *sa, int nfacets, const GridA
       if (g.used < slot->used) slot = &g;
     std::vector<int> counts(kMaxClasses, 0);
     if (!schedule_counts(counts)) return bz_error_code() ? bz_error_code() : BZ_ERR_CUDA;
-    if (!run_dispatch(ta, sa, wproj, comp, true, counts, c.stream, tune_facets, vis)) return bz_error_code();
+    if (!run_dispatch(ta, sa, wproj, acc, true, counts, c.stream, tune_facets, vis)) return bz_error_code();
     if (slot->exec) cudaGraphExecDestroy(slot->exec);
     slot->exec = nullptr;
     slot->key.clear();
     cudaGraph_t graph;
     BZ_CUDA_TRY_RET(cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeThreadLocal), BZ_ERR_CUDA);
     const long long launches0 = c.launches;
-    bool ok = enqueue_schedule(va, c.stream) && run_dispatch(va, sa, wproj, comp, false, counts, c.stream, nfacets, vis);
+    bool ok = enqueue_schedule(va, c.stream) && run_dispatch(va, sa, wproj, acc, false, counts, c.stream, nfacets, vis);
     cudaError_t ce = cudaStreamEndCapture(c.stream, &graph);
     if (!ok || ce != cudaSuccess) {
       bz_record_error(BZ_ERR_CUDA, "%s: graph capture failed (%s)", name, cudaGetErrorString(ce));
@@ -1331,6 +1341,14 @@ int run_batched(const GridArgs &va, const GridArgs *sa, int nfacets, const GridA
   return BZ_OK;
 }
 
+// Whether a call that grids `pairs` (visibility, facet) pairs into `cells` caller-owned cells accumulates in pairs of
+// words.  The wide form reads every cell's 16 bytes twice more (to it and back), the pair form waits for the
+// values that its additions return.  Whole calls with the caller's own clearing, wide and pair: 12,000 cells per pair
+// (27 antennas, one time, 4 facets of 4096^2) 3115 and 1843 us, 120 per pair 2491 and 1897, 15 per pair 6687 and
+// 6318, 12.7 per pair 1993 and 2042, 1.9 per pair 7331 and 7524.
+constexpr long long kPairCells = 14;
+bool pair_accumulation(long long pairs, long long cells) { return cells > kPairCells * std::max(1ll, pairs); }
+
 bool call_mode(int call, int &mode, bool &faceting, const char *name) {
   switch (call) {
     case 0: mode = CORR_QUAD_JONES; faceting = true; return true;  // facet_4_cor_corrections
@@ -1343,9 +1361,9 @@ bool call_mode(int call, int &mode, bool &faceting, const char *name) {
 }
 
 // Whether every support class has a tuned layout for these visibility launches.
-bool classes_tuned(int nc, bool wproj, bool comp) {
+bool classes_tuned(int nc, bool wproj, Acc acc) {
   for (int k = 0; k < g_bs.ncls; ++k)
-    if (!g_bs.tuned.count(std::make_tuple(g_bs.cls[k].width, nc, (int)wproj, (int)comp))) return false;
+    if (!g_bs.tuned.count(std::make_tuple(g_bs.cls[k].width, nc, (int)wproj, (int)acc))) return false;
   return true;
 }
 
@@ -1357,7 +1375,8 @@ bool classes_tuned(int nc, bool wproj, bool comp) {
 // a launch tail.
 bool stream_visibilities(gridding_parameters &p, const GridArgs &va, int nfacets, bool jones, const char *name) {
   Context &c = g_ctx;
-  const bool wproj = va.P > 1, comp = va.grid_lo != nullptr;
+  const bool wproj = va.P > 1;
+  const Acc acc = acc_form(va.grid_lo != nullptr);
   RowsPlan plan;
   if (!bz_plan_rows(p, plan)) return false;
   if (!ensure_capacity(p.row_count, (size_t)plan.chunks * plan.slots * c.nchan)) return false;
@@ -1368,7 +1387,7 @@ bool stream_visibilities(gridding_parameters &p, const GridArgs &va, int nfacets
       return false;
     }
     bz_trace_mark("vis.rows_sorted");
-    return run_batched(va, nullptr, nfacets, va, nfacets, wproj, comp, name, true) == BZ_OK;
+    return run_batched(va, nullptr, nfacets, va, nfacets, wproj, acc, name, true) == BZ_OK;
   }
   std::vector<int> counts(kMaxClasses, 0);
   if (!ensure_records(nfacets, (long long)p.row_count, (int)c.nchan, 0)) return false;
@@ -1384,14 +1403,14 @@ bool stream_visibilities(gridding_parameters &p, const GridArgs &va, int nfacets
     if (k0 == 0) {
       // every call sets its classes' layouts up for this build (NC, w-projection, compensation) from
       // the tuned decisions; classes without a decision yet are timed on this group's runs
-      if (!classes_tuned(4, wproj, comp)) {
+      if (!classes_tuned(4, wproj, acc)) {
         BZ_CUDA_TRY_RET(cudaMemcpyAsync(counts.data(), g_bs.class_count.ptr, sizeof(int) * kMaxClasses,
                                         cudaMemcpyDeviceToHost, c.stream), false);
         BZ_CUDA_TRY_RET(cudaStreamSynchronize(c.stream), false);
       }
-      if (!run_dispatch(vk, nullptr, wproj, comp, true, counts, c.stream, nfacets, true)) return false;
+      if (!run_dispatch(vk, nullptr, wproj, acc, true, counts, c.stream, nfacets, true)) return false;
     }
-    const bool ok = run_dispatch(vk, nullptr, wproj, comp, false, counts, c.stream, nfacets, true);
+    const bool ok = run_dispatch(vk, nullptr, wproj, acc, false, counts, c.stream, nfacets, true);
     bz_trace_mark("vis.group_grid");
     k0 = k + 1;
     return ok;
@@ -1422,15 +1441,16 @@ bool bz_grid_batched_call(gridding_parameters &p, int mode, bool faceting, const
     if (!bz_error_code()) bz_record_error(BZ_ERR_CUDA, "%s: support-class planning failed", name);
     return false;
   }
-  const bool wproj = p.wplanes > 1, comp = a.grid_lo != nullptr;
+  const bool wproj = p.wplanes > 1;
+  const Acc acc = acc_form(a.grid_lo != nullptr);
   if (stream) {
     const bool ok = stream_visibilities(p, a, (int)c.F, mode == CORR_QUAD_JONES, name);
     bz_trace_mark("vis.grid");
     return ok;
   }
   if (!ensure_capacity(p.row_count, (size_t)nslots * c.nchan)) return false;
-  const int rc = sampling ? run_batched(a, &a, 1, a, 1, wproj, comp, name, false)
-                          : run_batched(a, nullptr, (int)c.F, a, (int)c.F, wproj, comp, name, true);
+  const int rc = sampling ? run_batched(a, &a, 1, a, 1, wproj, acc, name, false)
+                          : run_batched(a, nullptr, (int)c.F, a, (int)c.F, wproj, acc, name, true);
   bz_trace_mark(sampling ? "sf.grid" : "vis.grid");
   return rc == BZ_OK;
 }
@@ -1466,7 +1486,7 @@ extern "C" int bullseye_grid_batched(gridding_parameters *pp, int call, int with
     if (sf) {
       if (!bz_prepare_grid_args(p, 1, CORR_SAMPLING, faceting, sa, nslots_sf, "bullseye_grid_batched")) return bz_error_code();
       if (!ensure_capacity(p.row_count, (size_t)nslots_sf * c.nchan)) return bz_error_code();
-      const int rc = run_batched(sa, &sa, 1, sa, 1, p.wplanes > 1, sa.grid_lo != nullptr, "bullseye_grid_batched", false);
+      const int rc = run_batched(sa, &sa, 1, sa, 1, p.wplanes > 1, acc_form(sa.grid_lo != nullptr), "bullseye_grid_batched", false);
       if (rc != BZ_OK) return rc;
     }
   } else {
@@ -1474,7 +1494,7 @@ extern "C" int bullseye_grid_batched(gridding_parameters *pp, int call, int with
     if (sf && !bz_prepare_grid_args(p, 1, CORR_SAMPLING, faceting, sa, nslots_sf, "bullseye_grid_batched", false))
       return bz_error_code();
     if (!ensure_capacity(p.row_count, (size_t)nslots * c.nchan)) return bz_error_code();
-    const int rc = run_batched(va, sf ? &sa : nullptr, (int)c.F, va, (int)c.F, p.wplanes > 1, va.grid_lo != nullptr,
+    const int rc = run_batched(va, sf ? &sa : nullptr, (int)c.F, va, (int)c.F, p.wplanes > 1, acc_form(va.grid_lo != nullptr),
                                "bullseye_grid_batched");
     if (rc != BZ_OK) return rc;
   }
@@ -1564,8 +1584,7 @@ extern "C" int bullseye_grid_batched_facets(gridding_parameters *pp, const bulls
   va.norm = norms;
   if (!b.planned && !plan_classes()) return bz_error_code() ? bz_error_code() : BZ_ERR_CUDA;
   if (!ensure_capacity(p.row_count, (size_t)nslots * c.nchan)) return bz_error_code();
-  // wide accumulation: the caller's grids go to the wide form and back around the call, each cell once
-  // (facets may share cells: the union of their blocks, as disjoint ranges)
+  // the caller's cells, each once (facets may share some: the union of their blocks, as disjoint ranges)
   std::vector<std::pair<long long, long long>> cells;
   if (va.grid_lo) {
     for (int f = 0; f < nfacets; ++f) {
@@ -1580,10 +1599,20 @@ extern "C" int bullseye_grid_batched_facets(gridding_parameters *pp, const bulls
     }
     cells.resize(n);
   }
+  Acc acc = acc_form(va.grid_lo != nullptr);
+  if (acc == ACC_WIDE) {
+    long long n = 0;
+    for (const auto &r : cells) n += r.second - r.first;
+    if (pair_accumulation((long long)p.row_count * (long long)c.nchan * nfacets, n)) {
+      acc = ACC_PAIR;
+      cells.clear();
+    }
+  }
+  // wide accumulation: the caller's grids go to the wide form and back around the call
   bool ok = true;
   for (const auto &r : cells)
     ok = bz_widen_grid(va.grid + r.first, va.grid_lo + r.first, r.second - r.first, true, c.stream) && ok;
-  const int rc = run_batched(va, nullptr, nfacets, ta, 1, p.wplanes > 1, va.grid_lo != nullptr, name);
+  const int rc = run_batched(va, nullptr, nfacets, ta, 1, p.wplanes > 1, acc, name);
   for (const auto &r : cells)
     ok = bz_narrow_grid(va.grid + r.first, va.grid_lo + r.first, nullptr, r.second - r.first, c.stream) && ok;
   c.launches += 2 * (long long)cells.size();
@@ -1730,26 +1759,27 @@ SupportWs support_ws_layout(long long R, int nchan, int nslots, int P, int os, i
   return l;
 }
 
-template <bool WPROJ, bool COMP>
+template <bool WPROJ, int ACC>
 bool support_aware_layouts(const ClassList &cl, Variant *vs) {
   for (int k = 0; k < cl.n; ++k)
-    if (!inplace_variant<4, WPROJ, COMP>(cl.w[k], vs[k])) {
+    if (!inplace_variant<4, WPROJ, ACC>(cl.w[k], vs[k])) {
       bz_record_error(BZ_ERR_UNSUPPORTED, "support-aware gridding: no layout for class width %d", cl.w[k]);
       return false;
     }
   return true;
 }
 
-bool support_aware_layouts(const ClassList &cl, bool wproj, bool comp, Variant *vs) {
+bool support_aware_layouts(const ClassList &cl, bool wproj, Acc acc, Variant *vs) {
 #if defined(BULLSEYE_SINGLE)
-  if (comp) return wproj ? support_aware_layouts<true, true>(cl, vs) : support_aware_layouts<false, true>(cl, vs);
+  if (acc == ACC_WIDE)
+    return wproj ? support_aware_layouts<true, ACC_WIDE>(cl, vs) : support_aware_layouts<false, ACC_WIDE>(cl, vs);
 #else
-  (void)comp;
+  (void)acc;
 #endif
-  return wproj ? support_aware_layouts<true, false>(cl, vs) : support_aware_layouts<false, false>(cl, vs);
+  return wproj ? support_aware_layouts<true, ACC_PLAIN>(cl, vs) : support_aware_layouts<false, ACC_PLAIN>(cl, vs);
 }
 
-template <bool WPROJ, bool COMP>
+template <bool WPROJ, int ACC>
 bool support_aware_launches(const GridArgs &a, const ClassList &cl, const Variant *vs, int nfacets, int *class_count,
                             int *class_off, int *work_next, cudaStream_t st) {
   for (int k = 0; k < cl.n; ++k) {
@@ -1761,7 +1791,7 @@ bool support_aware_launches(const GridArgs &a, const ClassList &cl, const Varian
     ak.segment_base = class_off + k;
     ak.work_count = class_count + k;
     ak.work_next = work_next + k;
-    auto kern = inplace_kernel<4, WPROJ, COMP>(v.J, v.wide);
+    auto kern = inplace_kernel<4, WPROJ, ACC>(v.J, v.wide);
     if (cudaMemsetAsync(work_next + k, 0, sizeof(int), st) != cudaSuccess) return false;
     kern<<<v.grid, v.NT, v.chunk.smem, st>>>(ak, nfacets);
     if (cudaGetLastError() != cudaSuccess) return false;
@@ -1792,7 +1822,7 @@ bool bz_support_aware_check(const GridArgs &a, size_t bytes) {
   }
   const ClassList cl = candidate_classes(a.W);
   Variant vs[kMaxClasses];
-  return support_aware_layouts(cl, wproj, a.grid_lo != nullptr, vs);
+  return support_aware_layouts(cl, wproj, acc_form(a.grid_lo != nullptr), vs);
 }
 
 bool bz_grid_support_aware(const GridArgs &a_in, int nfacets, unsigned char *ws, size_t bytes, cudaStream_t st) {
@@ -1805,8 +1835,8 @@ bool bz_grid_support_aware(const GridArgs &a_in, int nfacets, unsigned char *ws,
   }
   const ClassList cl = candidate_classes(W);
   Variant vs[kMaxClasses];
-  const bool comp = a_in.grid_lo != nullptr;
-  if (!support_aware_layouts(cl, wproj, comp, vs)) return false;
+  const Acc acc = acc_form(a_in.grid_lo != nullptr);
+  if (!support_aware_layouts(cl, wproj, acc, vs)) return false;
   int *plane_class = reinterpret_cast<int *>(ws + l.plane_class);
   int *plane_lo = reinterpret_cast<int *>(ws + l.plane_lo);
   int *plane_w = reinterpret_cast<int *>(ws + l.plane_w);
@@ -1851,10 +1881,10 @@ bool bz_grid_support_aware(const GridArgs &a_in, int nfacets, unsigned char *ws,
   a.segments = sorted;
   a.segment_capacity = l.maxseg;
 #if defined(BULLSEYE_SINGLE)
-  if (comp)
-    return wproj ? support_aware_launches<true, true>(a, cl, vs, nfacets, class_count, class_off, work_next, st)
-                 : support_aware_launches<false, true>(a, cl, vs, nfacets, class_count, class_off, work_next, st);
+  if (acc == ACC_WIDE)
+    return wproj ? support_aware_launches<true, ACC_WIDE>(a, cl, vs, nfacets, class_count, class_off, work_next, st)
+                 : support_aware_launches<false, ACC_WIDE>(a, cl, vs, nfacets, class_count, class_off, work_next, st);
 #endif
-  return wproj ? support_aware_launches<true, false>(a, cl, vs, nfacets, class_count, class_off, work_next, st)
-               : support_aware_launches<false, false>(a, cl, vs, nfacets, class_count, class_off, work_next, st);
+  return wproj ? support_aware_launches<true, ACC_PLAIN>(a, cl, vs, nfacets, class_count, class_off, work_next, st)
+               : support_aware_launches<false, ACC_PLAIN>(a, cl, vs, nfacets, class_count, class_off, work_next, st);
 }

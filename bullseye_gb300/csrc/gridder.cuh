@@ -268,20 +268,57 @@ __device__ __forceinline__ double to_double(float x) {
 }
 #endif
 
-template <int NC, bool WIDEACC>
+// PAIR accumulation (the 32-bit library's form for caller-owned grids that are large for the call, see
+// pair_accumulation): a cell keeps its FP32 value in `grid`, and what an addition rounded off goes to `grid_lo` (TwoSum
+// of the value that the returning addition gives).  It converts nothing around the call.
+enum Acc { ACC_PLAIN = 0, ACC_WIDE = 1, ACC_PAIR = 2 };
+
+// The form of a call with or without second words (FP64 accumulation needs none).
+inline Acc acc_form(bool second_words) {
+#if defined(BULLSEYE_SINGLE)
+  return second_words ? ACC_WIDE : ACC_PLAIN;
+#else
+  (void)second_words;
+  return ACC_PLAIN;
+#endif
+}
+
+#if defined(BULLSEYE_SINGLE)
+__device__ __forceinline__ float2 pair_add(const GridArgs &a, long long at, cplx x) {
+  return atomicAdd(reinterpret_cast<float2 *>(a.grid + at), make_float2(x.re, x.im));
+}
+__device__ __forceinline__ void pair_rest(const GridArgs &a, long long at, cplx x, float2 old) {
+  const float s0 = __fadd_rn(old.x, x.re), b0 = __fsub_rn(s0, old.x);
+  const float s1 = __fadd_rn(old.y, x.im), b1 = __fsub_rn(s1, old.y);
+  const float e0 = __fadd_rn(__fsub_rn(old.x, __fsub_rn(s0, b0)), __fsub_rn(x.re, b0));
+  const float e1 = __fadd_rn(__fsub_rn(old.y, __fsub_rn(s1, b1)), __fsub_rn(x.im, b1));
+  const bool r0 = e0 != 0.f && isfinite(s0), r1 = e1 != 0.f && isfinite(s1);  // (an infinity has no second word)
+  if (r0 || r1) atomicAdd(reinterpret_cast<float2 *>(a.grid_lo + at), make_float2(r0 ? e0 : 0.f, r1 ? e1 : 0.f));
+}
+#endif
+
+template <int NC, int ACC>
 __device__ __forceinline__ void flush_cell(const GridArgs &a, long long cell, long long nxy, cplx (&acc)[NC]) {
 #if defined(BULLSEYE_SINGLE)
-  if (WIDEACC) {
-    double *re = reinterpret_cast<double *>(a.grid) + cell, *im = reinterpret_cast<double *>(a.grid_lo) + cell;
+  if (ACC != ACC_PLAIN) {
     unsigned any = 0;
 #pragma unroll
     for (int k = 0; k < NC; ++k) any |= __float_as_uint(acc[k].re) | __float_as_uint(acc[k].im);
     if (!(any & 0x7fffffffu)) return;  // a zero cell: nothing to add (taps outside a plane's window are zero)
+  }
+  if (ACC == ACC_WIDE) {
+    double *re = reinterpret_cast<double *>(a.grid) + cell, *im = reinterpret_cast<double *>(a.grid_lo) + cell;
 #pragma unroll
     for (int k = 0; k < NC; ++k) {
       atomicAdd(re + k * nxy, to_double(acc[k].re));
       atomicAdd(im + k * nxy, to_double(acc[k].im));
     }
+  } else if (ACC == ACC_PAIR) {
+    float2 old[NC];
+#pragma unroll
+    for (int k = 0; k < NC; ++k) old[k] = pair_add(a, cell + k * nxy, acc[k]);
+#pragma unroll
+    for (int k = 0; k < NC; ++k) pair_rest(a, cell + k * nxy, acc[k], old[k]);
   } else {
 #pragma unroll
     for (int k = 0; k < NC; ++k)
@@ -1428,10 +1465,10 @@ __device__ __forceinline__ void merge_groups(const TapTable<WPROJ> &table, const
 }
 
 // Adds one real component (part 0 real, 1 imaginary) of correlation k of a cell.
-template <bool COMP>
+template <int ACC>
 __device__ __forceinline__ void add_component(const GridArgs &a, long long at, int part, acc_real x) {
 #if defined(BULLSEYE_SINGLE)
-  if (COMP)
+  if (ACC == ACC_WIDE)
     atomicAdd(reinterpret_cast<double *>(part ? a.grid_lo : a.grid) + at, to_double(x));
   else
     atomicAdd(reinterpret_cast<float *>(a.grid + at) + part, x);
@@ -1444,7 +1481,7 @@ __device__ __forceinline__ void add_component(const GridArgs &a, long long at, i
 // memory and the warp's lanes add one component each.  By itself the lane would add its 2 NC J components
 // one after the other while the warp waits, which took a third of the class launches.  cell0: the grid
 // element of correlation 0 at row coordinate 0 of the lane's column.
-template <int NC, int J, bool COMP>
+template <int NC, int J, int ACC>
 __device__ __forceinline__ void flush_column(const GridArgs &a, int l, int W, long long cell0, long long nxy, int sb,
                                              cplx *buf, OwnerState<NC, J> &st) {
   const int lane = threadIdx.x & 31;
@@ -1463,12 +1500,28 @@ __device__ __forceinline__ void flush_column(const GridArgs &a, int l, int W, lo
     st.dirty = 0;
   }
   __syncwarp();
+#if defined(BULLSEYE_SINGLE)
+  if constexpr (ACC == ACC_PAIR) {  // whole cells: both components come back with one addition
+#pragma unroll
+    for (int c0 = 0; c0 < J * NC; c0 += 32) {
+      const int c = c0 + lane, j = c / NC, k = c % NC;
+      if (c < J * NC && (dirty >> j & 1)) {
+        const cplx x = buf[c];
+        const int ob = ob0 + j >= W ? ob0 + j - W : ob0 + j;
+        const long long at = cell0 + (long long)(st.pb0 + ob) * sb + k * nxy;
+        if (x.re != 0.f || x.im != 0.f) pair_rest(a, at, x, pair_add(a, at, x));
+      }
+    }
+    __syncwarp();
+    return;
+  }
+#endif
 #pragma unroll
   for (int c0 = 0; c0 < J * NC * 2; c0 += 32) {
     const int c = c0 + lane, j = c / (2 * NC), k = (c >> 1) % NC;
     if (c < J * NC * 2 && (dirty >> j & 1)) {
       const int ob = ob0 + j >= W ? ob0 + j - W : ob0 + j;
-      add_component<COMP>(a, cell0 + (long long)(st.pb0 + ob) * sb + k * nxy, c & 1,
+      add_component<ACC>(a, cell0 + (long long)(st.pb0 + ob) * sb + k * nxy, c & 1,
                           reinterpret_cast<const acc_real *>(buf)[c]);
     }
   }
@@ -1479,7 +1532,7 @@ __device__ __forceinline__ void flush_column(const GridArgs &a, int l, int W, lo
 // footprint moves, the owned cells are recomputed and those that changed are flushed: rows that moved by
 // every lane of their strip, one or two columns that moved by flush_column.  Cells lie sa (along a) and
 // sb (along b) elements apart.
-template <int NC, bool WPROJ, int J, bool COMP, class Rec>
+template <int NC, bool WPROJ, int J, int ACC, class Rec>
 __device__ __forceinline__ void grid_groups(const GridArgs &a, const Rec *recs, const unsigned short *list, int g0, int g1,
                                             bool along_v, const typename MergeVec<NC>::type *T,
                                             const typename TapT<WPROJ>::type *tb, int du, int strip, unsigned rows_mask,
@@ -1505,8 +1558,8 @@ __device__ __forceinline__ void grid_groups(const GridArgs &a, const Rec *recs, 
         bool out = st.dirty && (a0 + o != st.pa0 + st.oa || g != st.cg);  // the column moved
         const unsigned m = __ballot_sync(0xffffffffu, out);
         if (m && __popc(m) <= 2) {
-          flush_column<NC, J, COMP>(a, __ffs(m) - 1, W, cell0, nxy, sb, col_buf, st);
-          if (m & (m - 1)) flush_column<NC, J, COMP>(a, 31 - __clz(m), W, cell0, nxy, sb, col_buf, st);
+          flush_column<NC, J, ACC>(a, __ffs(m) - 1, W, cell0, nxy, sb, col_buf, st);
+          if (m & (m - 1)) flush_column<NC, J, ACC>(a, 31 - __clz(m), W, cell0, nxy, sb, col_buf, st);
         }
         if (st.dirty) {
 #pragma unroll
@@ -1514,7 +1567,7 @@ __device__ __forceinline__ void grid_groups(const GridArgs &a, const Rec *recs, 
             const int ob = st.ob0 + j >= W ? st.ob0 + j - W : st.ob0 + j;
             const int nb = nob0 + j >= W ? nob0 + j - W : nob0 + j;
             if ((st.dirty & (1u << j)) && (out || b0 + nb != st.pb0 + ob)) {
-              flush_cell<NC, COMP>(a, cell0 + (long long)(st.pb0 + ob) * sb, nxy, st.acc[j]);
+              flush_cell<NC, ACC>(a, cell0 + (long long)(st.pb0 + ob) * sb, nxy, st.acc[j]);
               st.dirty &= ~(1u << j);
             }
           }
@@ -1556,7 +1609,7 @@ struct ItemSetup {
   bool grids;
   long long nxy, fbase;
 };
-template <int NC, bool WPROJ, int J, bool COMP, bool WIDE>
+template <int NC, bool WPROJ, int J, int ACC, bool WIDE>
 __device__ __forceinline__ void item_setup(const GridArgs &a, int f_local, unsigned char *smem, ItemSetup<NC, WPROJ> &s) {
   typedef typename MergeVec<NC>::type vec_t;
   typedef typename TapT<WPROJ>::type tap_t;
@@ -1591,7 +1644,7 @@ __device__ __forceinline__ void item_setup(const GridArgs &a, int f_local, unsig
 
 // The ng groups of one staged chunk (block-wide call; ends with the CTA's barrier, after which the
 // records may be overwritten).  Before that barrier, next() prepares what follows the chunk.
-template <int NC, bool WPROJ, int J, bool COMP, class Rec, class Next>
+template <int NC, bool WPROJ, int J, int ACC, class Rec, class Next>
 __device__ __forceinline__ void grid_chunk(const GridArgs &a, const Rec *recs, const unsigned short *list, int ng,
                                            bool along_v, const ItemSetup<NC, WPROJ> &s, OwnerState<NC, J> &st, Next next) {
   int g0 = 0;
@@ -1600,7 +1653,7 @@ __device__ __forceinline__ void grid_chunk(const GridArgs &a, const Rec *recs, c
     merge_groups<NC, WPROJ>(s.table, recs, list, g0, g1, along_v, a.W, J, s.ax, s.ap, s.nparts, s.T, s.tb);
     __syncthreads();
     if (s.grids)
-      grid_groups<NC, WPROJ, J, COMP>(a, recs, list, g0, g1, along_v, s.T, s.tb, s.du, s.strip, s.rows_mask, s.fbase,
+      grid_groups<NC, WPROJ, J, ACC>(a, recs, list, g0, g1, along_v, s.T, s.tb, s.du, s.strip, s.rows_mask, s.fbase,
                                       s.nxy, s.gnx, s.col_buf, st);
     if (g1 == ng) next();
     __syncthreads();
@@ -1609,7 +1662,7 @@ __device__ __forceinline__ void grid_chunk(const GridArgs &a, const Rec *recs, c
 }
 
 // End of a work item (or of a stretch of its rows): the owned cells are flushed and start at zero again.
-template <int NC, bool WPROJ, int J, bool COMP>
+template <int NC, bool WPROJ, int J, int ACC>
 __device__ __forceinline__ void item_flush(const GridArgs &a, const ItemSetup<NC, WPROJ> &s, bool along_v,
                                            OwnerState<NC, J> &st) {
   if (!st.dirty) return;
@@ -1618,7 +1671,7 @@ __device__ __forceinline__ void item_flush(const GridArgs &a, const ItemSetup<NC
 #pragma unroll
   for (int j = 0; j < J; ++j) {
     const int ob = st.ob0 + j >= a.W ? st.ob0 + j - a.W : st.ob0 + j;
-    if (st.dirty & (1u << j)) flush_cell<NC, COMP>(a, cell0 + (long long)(st.pb0 + ob) * sb, s.nxy, st.acc[j]);
+    if (st.dirty & (1u << j)) flush_cell<NC, ACC>(a, cell0 + (long long)(st.pb0 + ob) * sb, s.nxy, st.acc[j]);
   }
   st.dirty = 0;
 }
@@ -1636,7 +1689,7 @@ __device__ __forceinline__ bool rows_backwards(int chan) { return chan & 1; }
 
 // What one CTA grids in place: its running state, and one row range (a channel's rows [r0, r1)) at a
 // time, staged V rows at a time (prologue) and gridded chunk by chunk.
-template <int NC, bool WPROJ, int J, bool COMP, bool WIDE>
+template <int NC, bool WPROJ, int J, int ACC, bool WIDE>
 struct InPlace {
   VisRec<NC> *recs;  // [V]
   NormAcc *nacc;     // [V][NC]
@@ -1652,7 +1705,7 @@ struct InPlace {
     recs = reinterpret_cast<VisRec<NC> *>(smem_raw);
     nacc = reinterpret_cast<NormAcc *>(smem_raw + sizeof(VisRec<NC>) * (size_t)a.V);
     ng = reinterpret_cast<int *>(nacc + (size_t)a.V * NC);
-    item_setup<NC, WPROJ, J, COMP, WIDE>(a, f_local, smem_raw, s);
+    item_setup<NC, WPROJ, J, ACC, WIDE>(a, f_local, smem_raw, s);
     fslice = (long long)(a.facet_base + f_local) * a.groups;
     if (a.norm)
       for (int i = threadIdx.x; i < a.V; i += blockDim.x) {
@@ -1685,13 +1738,13 @@ struct InPlace {
         }
       }
       const int ngroups = find_groups(recs, nv, first, along_v, s.list);  // every warp its own list
-      grid_chunk<NC, WPROJ, J, COMP>(a, recs, s.list, ngroups, along_v, s, st, [] {});
+      grid_chunk<NC, WPROJ, J, ACC>(a, recs, s.list, ngroups, along_v, s, st, [] {});
       first = false;
     }
     stay += (int)(r1 - r0);
   }
   __device__ __forceinline__ void flush(const GridArgs &a) {
-    item_flush<NC, WPROJ, J, COMP>(a, s, along_v, st);
+    item_flush<NC, WPROJ, J, ACC>(a, s, along_v, st);
     stay = 0;
   }
 
@@ -1743,7 +1796,7 @@ struct RecordPieces {
 // while the current chunk is gridded.  No prologue and no normalisation here (the record kernel did
 // both).  rbar are the two record barriers (one arrival each), rphase their phase parities (bit b for
 // buffer b); copies are only issued for a chunk of this item, so none is in flight when the item ends.
-template <int NC, bool WPROJ, int J, bool COMP, bool WIDE>
+template <int NC, bool WPROJ, int J, int ACC, bool WIDE>
 __device__ __forceinline__ void grid_records(const GridArgs &a, const int f_local, const RecordPieces<NC> &pc, int npieces,
                                              unsigned long long *rbar, unsigned &rphase) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1768,7 +1821,7 @@ __device__ __forceinline__ void grid_records(const GridArgs &a, const int f_loca
   };
   if (tid == 0) issue(0, 0);
   ItemSetup<NC, WPROJ> s;
-  item_setup<NC, WPROJ, J, COMP, WIDE>(a, f_local, smem_raw, s);
+  item_setup<NC, WPROJ, J, ACC, WIDE>(a, f_local, smem_raw, s);
   OwnerState<NC, J> st;
   owner_reset(st);
   bool along_v = false;
@@ -1803,7 +1856,7 @@ __device__ __forceinline__ void grid_records(const GridArgs &a, const int f_loca
     } else {
       ng = find_groups(rb + cur * V, nv, c == 0, along_v, s.list);
     }
-    grid_chunk<NC, WPROJ, J, COMP>(a, rb + cur * V, list, ng, along_v, s, st, [&] {
+    grid_chunk<NC, WPROJ, J, ACC>(a, rb + cur * V, list, ng, along_v, s, st, [&] {
       if (kOneFinder && c + 1 < nchunks && threadIdx.x >= blockDim.x - 32) {
         landed(cur ^ 1);
         const int found = find_groups(rb + (cur ^ 1) * V, min(V, n - (c + 1) * V), false, along_v, s_list[cur ^ 1]);
@@ -1820,7 +1873,7 @@ __device__ __forceinline__ void grid_records(const GridArgs &a, const int f_loca
       out = last_piece != was;
     }
     if (out) {
-      item_flush<NC, WPROJ, J, COMP>(a, s, along_v, st);
+      item_flush<NC, WPROJ, J, ACC>(a, s, along_v, st);
       stay = 0;
     }
   }
@@ -1832,7 +1885,7 @@ template <int J>
 constexpr int kSegRegs = J <= 4 && sizeof(acc_real) == 4 ? 96 : J == 6 ? 112 : 128;
 
 // One CTA per track: blockIdx -> (facet, baseline slot or row segment, channel).
-template <int NC, bool WPROJ, int J, bool COMP, bool WIDE>
+template <int NC, bool WPROJ, int J, int ACC, bool WIDE>
 __global__ void __launch_bounds__(512, 1) romein_grid_kernel(const GridArgs a) {
   long long track = blockIdx.x;
   const int chan = (int)(track % a.nchan);
@@ -1847,7 +1900,7 @@ __global__ void __launch_bounds__(512, 1) romein_grid_kernel(const GridArgs a) {
     r0 = (long long)slot * a.seg;
     r1 = min(a.nrows, r0 + a.seg);
   }
-  InPlace<NC, WPROJ, J, COMP, WIDE> work;
+  InPlace<NC, WPROJ, J, ACC, WIDE> work;
   work.begin(a, f_local);
   work.rows(a, f_local, chan, r0, r1);
   work.flush(a);
@@ -1865,7 +1918,7 @@ __global__ void __launch_bounds__(512, 1) romein_grid_kernel(const GridArgs a) {
 // The loop ends on the count, never waits on other CTAs.  Two builds share the segments of a launch:
 // PRE grids those that the record kernel had room for, the other build the rest (every segment when
 // there are no records); the prologue of the latter would cost the former registers.
-template <int NC, bool WPROJ, int J, bool COMP, bool WIDE, bool PRE, int REGS = kSegRegs<J>>
+template <int NC, bool WPROJ, int J, int ACC, bool WIDE, bool PRE, int REGS = kSegRegs<J>>
 __global__ void __launch_bounds__(512, 1) __maxnreg__(REGS) romein_segment_kernel(const GridArgs a, const int nfacets) {
   __shared__ int s_item;
   __shared__ int s_first, s_last;  // unmasked row range of a segment (facet row masks)
@@ -1935,9 +1988,9 @@ __global__ void __launch_bounds__(512, 1) __maxnreg__(REGS) romein_segment_kerne
         if (lane < nseg) s_pieces.first[lane + 1] = sum;
       }
       __syncthreads();
-      grid_records<NC, WPROJ, J, COMP, WIDE>(a, f_local, s_pieces, nseg, s_rec_bar, rphase);
+      grid_records<NC, WPROJ, J, ACC, WIDE>(a, f_local, s_pieces, nseg, s_rec_bar, rphase);
     } else {
-      InPlace<NC, WPROJ, J, COMP, WIDE> work;
+      InPlace<NC, WPROJ, J, ACC, WIDE> work;
       work.begin(a, f_local);
       for (int i = 0;; ++i) {
         if (i == nseg || work.stay >= kStayRows) work.flush(a);

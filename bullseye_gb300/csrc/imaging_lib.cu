@@ -714,16 +714,12 @@ static LaunchShape choose_shape(int W) {
 }
 
 template <int NC, bool WPROJ, int J, bool WIDE>
-static bool launch_j(const GridArgs &a, const LaunchShape &s, long long blocks, cudaStream_t st, bool comp) {
-  void (*kern)(const GridArgs);
+static bool launch_j(const GridArgs &a, const LaunchShape &s, long long blocks, cudaStream_t st, Acc acc) {
+  void (*kern)(const GridArgs) = romein_grid_kernel<NC, WPROJ, J, ACC_PLAIN, WIDE>;
 #if defined(BULLSEYE_SINGLE)
-  if (comp)
-    kern = romein_grid_kernel<NC, WPROJ, J, true, WIDE>;
-  else
-    kern = romein_grid_kernel<NC, WPROJ, J, false, WIDE>;
+  if (acc == ACC_WIDE) kern = romein_grid_kernel<NC, WPROJ, J, ACC_WIDE, WIDE>;
 #else
-  (void)comp;  // FP64 accumulation needs no compensation
-  kern = romein_grid_kernel<NC, WPROJ, J, false, WIDE>;
+  (void)acc;
 #endif
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.chunk.smem) != cudaSuccess) {
     bz_record_error(BZ_ERR_CUDA, "cudaFuncSetAttribute failed");
@@ -740,7 +736,7 @@ static bool launch_j(const GridArgs &a, const LaunchShape &s, long long blocks, 
 }
 
 template <int NC, bool WPROJ>
-static bool launch_nc(GridArgs a, long long blocks, cudaStream_t st, bool comp) {
+static bool launch_nc(GridArgs a, long long blocks, cudaStream_t st, Acc acc) {
   LaunchShape s = choose_shape<NC, WPROJ>(a.W);
   if (s.NT > 512) {
     bz_record_error(BZ_ERR_UNSUPPORTED, "full support %d is larger than this build supports", a.W);
@@ -749,27 +745,27 @@ static bool launch_nc(GridArgs a, long long blocks, cudaStream_t st, bool comp) 
   a.V = s.chunk.V;
   a.GB = s.chunk.GB;
   if (s.wide) {
-    if (s.J == 2) return launch_j<NC, WPROJ, 2, true>(a, s, blocks, st, comp);
-    return launch_j<NC, WPROJ, 8, true>(a, s, blocks, st, comp);
+    if (s.J == 2) return launch_j<NC, WPROJ, 2, true>(a, s, blocks, st, acc);
+    return launch_j<NC, WPROJ, 8, true>(a, s, blocks, st, acc);
   }
   switch (s.J) {
-    case 1: return launch_j<NC, WPROJ, 1, false>(a, s, blocks, st, comp);
-    case 2: return launch_j<NC, WPROJ, 2, false>(a, s, blocks, st, comp);
-    case 4: return launch_j<NC, WPROJ, 4, false>(a, s, blocks, st, comp);
-    case 8: return launch_j<NC, WPROJ, 8, false>(a, s, blocks, st, comp);
-    default: return launch_j<NC, WPROJ, 16, false>(a, s, blocks, st, comp);
+    case 1: return launch_j<NC, WPROJ, 1, false>(a, s, blocks, st, acc);
+    case 2: return launch_j<NC, WPROJ, 2, false>(a, s, blocks, st, acc);
+    case 4: return launch_j<NC, WPROJ, 4, false>(a, s, blocks, st, acc);
+    case 8: return launch_j<NC, WPROJ, 8, false>(a, s, blocks, st, acc);
+    default: return launch_j<NC, WPROJ, 16, false>(a, s, blocks, st, acc);
   }
 }
 
-static bool launch_gridder(const GridArgs &a, int nc, bool wproj, long long blocks, cudaStream_t st, bool comp) {
+static bool launch_gridder(const GridArgs &a, int nc, bool wproj, long long blocks, cudaStream_t st, Acc acc) {
   if (blocks <= 0) return true;
   if (blocks > 0x7fffffffLL) {
     bz_record_error(BZ_ERR_UNSUPPORTED, "too many gridding work items in one chunk");
     return false;
   }
-  if (nc == 1) return wproj ? launch_nc<1, true>(a, blocks, st, comp) : launch_nc<1, false>(a, blocks, st, comp);
-  if (nc == 2) return wproj ? launch_nc<2, true>(a, blocks, st, comp) : launch_nc<2, false>(a, blocks, st, comp);
-  return wproj ? launch_nc<4, true>(a, blocks, st, comp) : launch_nc<4, false>(a, blocks, st, comp);
+  if (nc == 1) return wproj ? launch_nc<1, true>(a, blocks, st, acc) : launch_nc<1, false>(a, blocks, st, acc);
+  if (nc == 2) return wproj ? launch_nc<2, true>(a, blocks, st, acc) : launch_nc<2, false>(a, blocks, st, acc);
+  return wproj ? launch_nc<4, true>(a, blocks, st, acc) : launch_nc<4, false>(a, blocks, st, acc);
 }
 
 // Track setup of device-resident inputs (bullseye_set_device_inputs): the caller's baseline starts
@@ -1071,7 +1067,8 @@ static void grid_common(gridding_parameters *pp, int nc, int mode, bool faceting
   const long long blocks = (long long)(sampling ? 1 : c.F) * nslots * (long long)c.nchan;
   settle_kernel_timing();
   cudaEventRecord(c.ev_k0, c.stream);
-  if (p.row_count > 0 && !launch_gridder(a, nc_launch, p.wplanes > 1, blocks, c.stream, a.grid_lo != nullptr)) return;
+  if (p.row_count > 0 && !launch_gridder(a, nc_launch, p.wplanes > 1, blocks, c.stream, acc_form(a.grid_lo != nullptr)))
+    return;
   cudaEventRecord(c.ev_k1, c.stream);
   c.kernel_timing_pending = true;
   c.kernel_timing_kind = sampling ? 1 : 0;

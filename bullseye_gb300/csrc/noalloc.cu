@@ -128,9 +128,9 @@ Shape noalloc_shape(int W) {
 template <bool WPROJ, int J, bool WIDE>
 bool noalloc_launch(const GridArgs &a, const Shape &s, long long blocks, cudaStream_t st) {
 #if defined(BULLSEYE_SINGLE)
-  void (*kern)(const GridArgs) = romein_grid_kernel<4, WPROJ, J, true, WIDE>;
+  void (*kern)(const GridArgs) = romein_grid_kernel<4, WPROJ, J, ACC_WIDE, WIDE>;
 #else
-  void (*kern)(const GridArgs) = romein_grid_kernel<4, WPROJ, J, false, WIDE>;
+  void (*kern)(const GridArgs) = romein_grid_kernel<4, WPROJ, J, ACC_PLAIN, WIDE>;
 #endif
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s.chunk.smem) != cudaSuccess) return false;
   kern<<<(unsigned)blocks, s.NT, s.chunk.smem, st>>>(a);

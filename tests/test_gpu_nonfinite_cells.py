@@ -45,14 +45,16 @@ def _same(got, want, bits):
         assert np.array_equal(g[~nan], w[~nan])
 
 
+@pytest.mark.parametrize("n_times", [10, 60])  # few and many visibilities for the blocks' cells: either form
 @pytest.mark.parametrize("wplanes", [1, 4])
-def test_caller_blocks(wplanes, gpu_required, built_libraries):
+def test_caller_blocks(wplanes, n_times, gpu_required, built_libraries):
     import torch
     from bullseye_gb300.abi import BullseyeFacet
     from bullseye_gb300.library import check, load_library
     torch.cuda.set_device(0)
     lib = load_library("GPU", "single")
-    p = _problem("single", wplanes)
+    p = synth.small_problem("single", nx=96, n_ant=7, n_times=n_times, n_chan=3, n_facets=3, jones=False, s=4, os=9,
+                            wplanes=wplanes, min_support=5 if wplanes > 1 else None, seed=31)
     n = 90
     size = p.cube * 4 * n * n
     table = (BullseyeFacet * 2)()
