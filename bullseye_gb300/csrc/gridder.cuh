@@ -1676,11 +1676,21 @@ __device__ __forceinline__ void item_flush(const GridArgs &a, const ItemSetup<NC
   st.dirty = 0;
 }
 
-// Rows that an item's segments may add up to before the owned cells go out at a segment's end: cells of
-// slow tracks never leave the footprint, and plain accumulation over ever more channels would lose what
-// the wide flushes hold (16 segments of 100 rows without it: 3.1e-7 of the grid against 64 bits
-// where one segment at a time has 1.9e-7).
-constexpr int kStayRows = 512;
+// How long the owned cells of an item may stay in registers, over segments: cells of slow tracks never leave the
+// footprint, and plain accumulation over ever more channels would lose what the flushes hold.  `segs`
+// segments with `rows` rows in `groups` merged groups are in; one more may follow while that makes four at most, no
+// more than the visibilities per group (each group is one addition to a cell, so that a cell takes no more
+// additions than it has visibilities in one segment), and one per 30 rows of a segment (short segments end
+// their groups early).  The bar is the error against 64 bits of a segment gridded visibility by visibility and
+// flushed without loss at its end.  Parts of it with 1, 2, 3 and 4 segments in every stay: 100 rows of 14 s 0.51 0.63 0.69
+// 0.80, 200 rows 0.42 0.53 0.63 0.72; 16 rows 0.87 1.00 1.09 1.14; 100 fast rows (0.8 degrees each, groups of one or two)
+// 0.80 1.02 1.17 1.37.  (With stays of 512 rows whatever the track, arrays of ten antennas were 1.2 to 2.3 times past
+// it.)  The rule costs 27 antennas x 100 times x 64 channels in 16 facets 19.7 -> 21.6 ms, 400 times 61.1 -> 61.8, a
+// snapshot of 16 times 632 -> 723 us.
+constexpr int kStaySegs = 4, kStayRows = 30;
+__device__ __forceinline__ bool may_stay(int segs, int rows, int groups) {
+  return segs < kStaySegs && (segs + 1) * groups <= rows && (segs + 1) * segs * kStayRows <= rows;
+}
 
 // Whether the rows of a channel's segments are taken last to first: a work item's segments are
 // consecutive channels of one baseline, and turning round at each channel continues where the channel
@@ -1698,7 +1708,7 @@ struct InPlace {
   OwnerState<NC, J> st;
   long long fslice;
   bool along_v, first;
-  int stay;  // rows since the owned cells last went out
+  int segs, stay, groups;  // since the owned cells last went out: segments, their rows and groups
 
   __device__ __forceinline__ void begin(const GridArgs &a, int f_local) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1716,7 +1726,7 @@ struct InPlace {
     owner_reset(st);
     along_v = false;
     first = true;
-    stay = 0;
+    segs = stay = groups = 0;
   }
 
   __device__ __forceinline__ void rows(const GridArgs &a, int f_local, int chan, long long r0, long long r1) {
@@ -1740,12 +1750,14 @@ struct InPlace {
       const int ngroups = find_groups(recs, nv, first, along_v, s.list);  // every warp its own list
       grid_chunk<NC, WPROJ, J, ACC>(a, recs, s.list, ngroups, along_v, s, st, [] {});
       first = false;
+      groups += ngroups;
     }
     stay += (int)(r1 - r0);
+    ++segs;
   }
   __device__ __forceinline__ void flush(const GridArgs &a) {
     item_flush<NC, WPROJ, J, ACC>(a, s, along_v, st);
-    stay = 0;
+    segs = stay = groups = 0;
   }
 
   // Normalisation, after the last rows.
@@ -1805,27 +1817,48 @@ __device__ __forceinline__ void grid_records(const GridArgs &a, const int f_loca
   const int n = pc.first[npieces];
   if (n <= 0) return;
   const int tid = threadIdx.x;
-  int piece = 0;  // thread 0: the piece that the next chunk starts in
-  auto issue = [&](int c, int buf) {
-    const int lo = c * V, hi = min(n, lo + V);
+  // Chunks hold V records.  Where not even two segments may stay in registers together (see may_stay) they end with
+  // their segments, so that the cells go out exactly there: a chunk that runs on into the next segment adds its
+  // rows to cells that have taken a whole segment already (64 records over segments of 45 rows: grids 1.2 times
+  // as far off).  The first chunk ends with its segment; its groups tell for the next ones.  Thread 0 keeps the
+  // books in shared memory, where they cost the owner threads no registers.
+  __shared__ struct {
+    int count[2], last[2];         // the staged chunks' records; whether no other chunk follows
+    int at, piece, brief, cut;     // the next chunk's first record, and the piece that the one before it started in
+    int ended, segs, stay, groups;  // pieces that ended; since the cells last went out: segments, rows and groups
+    int out;                       // the cells go out after this chunk
+  } s_ck;
+  auto issue = [&](int buf) {
+    const int lo = s_ck.at;
+    int p = s_ck.piece;
+    while (pc.first[p + 1] <= lo) ++p;
+    s_ck.piece = p;
+    const int hi = min(min(n, lo + V), s_ck.cut ? pc.first[p + 1] : n);
+    s_ck.at = hi;
+    s_ck.count[buf] = hi - lo;
+    s_ck.last[buf] = hi == n;
     // the buffer may last have been written by plain stores (an item prepared in place)
     fence_proxy_async();
-    bar_arrive_tx(&rbar[buf], (unsigned)(sizeof(GridRec<NC>) * (hi - lo)));
+    bar_arrive_tx(&rbar[buf], (unsigned)(sizeof(GridRec<NC>) * (hi - lo)));  // (and publishes the above)
     GridRec<NC> *dst = rb + buf * V;
     for (int at = lo; at < hi;) {
-      while (pc.first[piece + 1] <= at) ++piece;
-      const int k = min(hi, pc.first[piece + 1]) - at;
-      bulk_copy(dst + (at - lo), pc.src[piece] + (at - pc.first[piece]), (unsigned)(sizeof(GridRec<NC>) * k), &rbar[buf]);
+      while (pc.first[p + 1] <= at) ++p;
+      const int k = min(hi, pc.first[p + 1]) - at;
+      bulk_copy(dst + (at - lo), pc.src[p] + (at - pc.first[p]), (unsigned)(sizeof(GridRec<NC>) * k), &rbar[buf]);
       at += k;
     }
   };
-  if (tid == 0) issue(0, 0);
+  if (tid == 0) {
+    s_ck.at = s_ck.piece = s_ck.ended = s_ck.segs = s_ck.stay = s_ck.groups = 0;
+    s_ck.brief = n < 2 * kStayRows * npieces;
+    s_ck.cut = 1;
+    issue(0);
+  }
   ItemSetup<NC, WPROJ> s;
   item_setup<NC, WPROJ, J, ACC, WIDE>(a, f_local, smem_raw, s);
   OwnerState<NC, J> st;
   owner_reset(st);
   bool along_v = false;
-  const int nchunks = (n + V - 1) / V;
   // Where the strips are long (J > 4), the group lists of chunks after the first are found by the last warp
   // (it has the fewest owners) for the CTA while the other warps still grid the chunk before; found by
   // every warp ahead of the chunk's merge they cost 2 % of a batched call of 27 antennas x 400 times x 64
@@ -1841,41 +1874,57 @@ __device__ __forceinline__ void grid_records(const GridArgs &a, const int f_loca
       bar_wait(&rbar[buf], par);
     }
   };
-  int cur = 0, stay = 0, last_piece = 0;
-  for (int c = 0; c < nchunks; ++c, cur ^= 1) {
-    const int nv = min(V, n - c * V);
+  bool first = true;
+  for (int cur = 0;; cur ^= 1) {
     landed(cur);
     rphase ^= 1u << cur;
-    // the other buffer was last read by the previous chunk, which every thread has finished
-    if (tid == 0 && c + 1 < nchunks) issue(c + 1, cur ^ 1);
+    const int nv = s_ck.count[cur];
+    const bool last = s_ck.last[cur];
     const unsigned short *list = s.list;
-    int ng;
-    if (kOneFinder && c > 0) {
-      list = s_list[cur];
-      ng = s_ngroups[cur];
-    } else {
-      ng = find_groups(rb + cur * V, nv, c == 0, along_v, s.list);
+    int ng = 0;
+    if (first) {
+      ng = find_groups(rb + cur * V, nv, true, along_v, s.list);
+      if (tid == 0) s_ck.cut = s_ck.brief || 2 * ng > nv;
     }
+    // the other buffer was last read by the previous chunk, which every thread has finished
+    if (tid == 0 && !last) issue(cur ^ 1);
+    if (!first) {
+      if (kOneFinder) {
+        list = s_list[cur];
+        ng = s_ngroups[cur];
+      } else {
+        ng = find_groups(rb + cur * V, nv, false, along_v, s.list);
+      }
+    }
+    first = false;
     grid_chunk<NC, WPROJ, J, ACC>(a, rb + cur * V, list, ng, along_v, s, st, [&] {
-      if (kOneFinder && c + 1 < nchunks && threadIdx.x >= blockDim.x - 32) {
+      if (kOneFinder && !last && threadIdx.x >= blockDim.x - 32) {
         landed(cur ^ 1);
-        const int found = find_groups(rb + (cur ^ 1) * V, min(V, n - (c + 1) * V), false, along_v, s_list[cur ^ 1]);
+        const int found = find_groups(rb + (cur ^ 1) * V, s_ck.count[cur ^ 1], false, along_v, s_list[cur ^ 1]);
         if ((tid & 31) == 0) s_ngroups[cur ^ 1] = found;
       }
+      // the owned cells go out at the end, and before it when a segment ended in the chunk and may_stay says so
+      if (tid == 0) {
+        const int stay = s_ck.stay + nv, groups = s_ck.groups + ng;
+        int segs = s_ck.segs, out = last;
+        if (!last) {
+          const int hi = s_ck.at - s_ck.count[cur ^ 1], was = segs;
+          int e = s_ck.ended;
+          for (; pc.first[e + 1] <= hi; ++e) segs += pc.first[e + 1] > pc.first[e];
+          s_ck.ended = e;
+          if (segs != was) {
+            out = !may_stay(segs, stay, groups);
+            s_ck.cut = s_ck.brief || 2 * groups > stay;
+          }
+        }
+        s_ck.segs = out ? 0 : segs;
+        s_ck.stay = out ? 0 : stay;
+        s_ck.groups = out ? 0 : groups;
+        s_ck.out = out;
+      }
     });
-    // the owned cells go out at the end, and before it once kStayRows rows are in and a segment ended
-    // in the chunk
-    stay += nv;
-    bool out = c + 1 == nchunks;
-    if (!out && stay >= kStayRows) {
-      const int was = last_piece;
-      while (pc.first[last_piece + 1] <= (c + 1) * V) ++last_piece;
-      out = last_piece != was;
-    }
-    if (out) {
-      item_flush<NC, WPROJ, J, ACC>(a, s, along_v, st);
-      stay = 0;
-    }
+    if (s_ck.out) item_flush<NC, WPROJ, J, ACC>(a, s, along_v, st);
+    if (last) break;
   }
 }
 
@@ -1911,9 +1960,11 @@ __global__ void __launch_bounds__(512, 1) romein_grid_kernel(const GridArgs a) {
 // item count is exhausted.  Every segment is a run of one track's rows whose w planes share this
 // launch's support class (a.W), in the order (baseline, channel, rows), the rows of odd channels
 // backwards; an item is a block of consecutive segments in one facet, gridded as one stretch: the owned
-// cells go out when the footprint leaves them, and all of them only at the item's end.  The block is as
-// long as leaves eight items per CTA, kMaxItemSegs at most (gridding 27 antennas x 100 times x 64
-// channels into 16 facets, one segment per item spends a quarter of the class launches on the ends).
+// cells go out when the footprint leaves them, and all of them only where may_stay ends a stay.  The block is
+// as long as leaves eight items per CTA, kMaxItemSegs at most (gridding 27 antennas x 100 times x 64
+// channels into 16 facets, one segment per item spends a quarter of the class launches on the ends).  From
+// records without w kernels it is one segment (supports of 7 and 15, 8 facets: 200 slow times 2678 -> 2651 and 4383 ->
+// 4398 us, fast tracks 4724 -> 4494 and 8274 -> 7759, and errors below those of several).
 // Items of one block are adjacent, so the facets of a segment are gridded while its rows are hot in L2.
 // The loop ends on the count, never waits on other CTAs.  Two builds share the segments of a launch:
 // PRE grids those that the record kernel had room for, the other build the rest (every segment when
@@ -1931,7 +1982,8 @@ __global__ void __launch_bounds__(512, 1) __maxnreg__(REGS) romein_segment_kerne
   }
   const int count = *a.work_count;
   const long long base = *a.segment_base;
-  const int per = (int)max(1ll, min((long long)kMaxItemSegs, (long long)count * nfacets / (8ll * gridDim.x)));
+  int per = (int)max(1ll, min((long long)kMaxItemSegs, (long long)count * nfacets / (8ll * gridDim.x)));
+  if (PRE && !WPROJ) per = 1;
   const long long total = (long long)((count + per - 1) / per) * nfacets;
   // a segment of the schedule; false (reported) when it lies outside the schedule or the rows
   auto segment = [&](long long si, int4 &sg) -> bool {
@@ -1993,7 +2045,7 @@ __global__ void __launch_bounds__(512, 1) __maxnreg__(REGS) romein_segment_kerne
       InPlace<NC, WPROJ, J, ACC, WIDE> work;
       work.begin(a, f_local);
       for (int i = 0;; ++i) {
-        if (i == nseg || work.stay >= kStayRows) work.flush(a);
+        if (i == nseg || (work.segs && !may_stay(work.segs, work.stay, work.groups))) work.flush(a);
         if (i == nseg) break;
         int4 sg;
         if (!segment(s0 + i, sg) || recorded(s0 + i, sg.y - sg.x)) continue;
