@@ -180,6 +180,8 @@ __device__ __forceinline__ void mac_conj(cplx &acc, cplx g, cplx t) {
 }
 __device__ __forceinline__ cplx tap_value(acc_real t) { cplx c; c.re = t; c.im = 0; return c; }
 __device__ __forceinline__ cplx tap_value(cplx t) { return t; }
+__device__ __forceinline__ acc_real real_part(acc_real t) { return t; }
+__device__ __forceinline__ acc_real real_part(cplx t) { return t.re; }
 
 // The footprint sums of B visibilities of one run (each in the order of a visibility by itself: lane l takes
 // cells l, l + 32, ... of the window, then a butterfly over the lanes), cells read once.  fu, fv: the
@@ -251,6 +253,27 @@ __device__ __forceinline__ acc_real warp_sum8(const acc_real (&v)[8]) {
   c += __shfl_xor_sync(0xffffffffu, c, 2);
   c += __shfl_xor_sync(0xffffffffu, c, 1);
   return c;
+}
+
+// A value as the sum of two words: the tap sum that prediction divides by, so that the quotient is rounded once
+// (summed and divided in single words it is off by as much again as the gathered value: 1.19e-7 against 0.89e-7;
+// products of taps that are summed as they are gathered share their roundings with it, 1.07e-7).
+struct Pair {
+  acc_real hi, lo;
+};
+__device__ __forceinline__ void pair_add(Pair &s, acc_real x) {
+  const acc_real t = s.hi + x, b = t - s.hi;
+  s.lo += (s.hi - (t - b)) + (x - b);
+  s.hi = t;
+}
+__device__ __forceinline__ Pair pair_product(Pair a, Pair b) {
+  const acc_real p = a.hi * b.hi;
+  return Pair{p, fma(a.hi, b.hi, -p) + fma(a.hi, b.lo, a.lo * b.hi)};
+}
+// v / d, inv = 1 / d.hi
+__device__ __forceinline__ acc_real pair_quotient(acc_real v, Pair d, acc_real inv) {
+  const acc_real q = v * inv, r = fma(fma(-q, d.lo, fma(-q, d.hi, v)), inv, q);
+  return r == r ? r : q;  // (an infinity's remainder is not a number)
 }
 
 __device__ __forceinline__ void atomic_add_c(vis_complex *dst, cplx v) {
@@ -531,28 +554,6 @@ __global__ void __launch_bounds__(kDegridWarps * 32, sizeof(acc_real) == 4 ? 4 :
             }
           }
         }
-        if (want_ts) {
-          // real part of each row's tap sum, Re(sum of ku x sum of kv)
-          cplx sv = tap_value(tap_t()), su;
-          sv.re = sv.im = 0;
-          for (int y = lane; y < ww; y += 32) sv = cadd(sv, tap_value(tap(fvw + y * a.os)));
-#pragma unroll
-          for (int off = 16; off > 0; off >>= 1) {
-            sv.re += __shfl_xor_sync(0xffffffffu, sv.re, off);
-            sv.im += __shfl_xor_sync(0xffffffffu, sv.im, off);
-          }
-          for (int i = it; i < end; ++i) {
-            const int at = __shfl_sync(0xffffffffu, cell.fu, i) + w2.x * a.os;
-            su.re = su.im = 0;
-            for (int x = lane; x < ww; x += 32) su = cadd(su, tap_value(tap(at + x * a.os)));
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) {
-              su.re += __shfl_xor_sync(0xffffffffu, su.re, off);
-              su.im += __shfl_xor_sync(0xffffffffu, su.im, off);
-            }
-            if (lane == i) s_sum[256 + i] = su.re * sv.re - su.im * sv.im;
-          }
-        }
       }
       __syncwarp();
       cplx myD[4];
@@ -563,7 +564,21 @@ __global__ void __launch_bounds__(kDegridWarps * 32, sizeof(acc_real) == 4 ? 4 :
           myD[k].re = s_sum[lane * 8 + 2 * k];
           myD[k].im = s_sum[lane * 8 + 2 * k + 1];
         }
-        if (want_ts) myTS = s_sum[256 + lane];
+        if (kRuns && want_ts) myTS = s_sum[256 + lane];
+      }
+      Pair ts{0, 0};
+      if (PREDICT && !kRuns && want_ts && ok) {
+        // sum of ku x sum of kv of the lane's own row (real taps, one plane: w kernels are predicted by runs)
+        const int2 w2 = win[cell.plane];
+        Pair su{0, 0}, sv{0, 0};
+        for (int s = w2.x; s <= w2.y; ++s) {
+          const int u = cell.fu + s * a.os, v = cell.fv + s * a.os;
+          const long long row0 = (long long)cell.plane * a.K;
+          pair_add(su, real_part(row_bytes ? s_row[u] : tap_at(a.conv, row0 + u, tap_t())));
+          pair_add(sv, real_part(row_bytes ? s_row[v] : tap_at(a.conv, row0 + v, tap_t())));
+        }
+        ts = pair_product(su, sv);
+        myTS = ts.hi;
       }
       if (!ok) continue;
       if (PREDICT) {
@@ -574,8 +589,13 @@ __global__ void __launch_bounds__(kDegridWarps * 32, sizeof(acc_real) == 4 ? 4 :
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           cplx v = cell.flip ? cconj(myD[k]) : myD[k];
-          v.re *= inv;
-          v.im *= inv;
+          if (kRuns || !want_ts || myTS == (acc_real)0) {  // (runs keep every visibility's own operations)
+            v.re *= inv;
+            v.im *= inv;
+          } else {
+            v.re = pair_quotient(v.re, ts, inv);
+            v.im = pair_quotient(v.im, ts, inv);
+          }
           X[k] = cmul(cph, v);
         }
         if (a.jones) {
