@@ -783,10 +783,19 @@ static void device_tracks(const gridding_parameters &p, int &nslots, int &seg, c
 }
 
 bool bz_check_ready(const char *fn) { return check_ready(fn); }
+#if defined(BULLSEYE_SINGLE)
+// Blocks of a conversion: eight of 256 threads are resident on an SM.
+static int convert_blocks() {
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return std::max(1, sms) * 8;
+}
+#endif
 bool bz_widen_grid(vis_complex *hi, vis_complex *lo, long long n, bool have_lo, cudaStream_t st) {
 #if defined(BULLSEYE_SINGLE)
   if (have_lo)
-    convert_grid_kernel<true><<<152 * 8, 256, 0, st>>>(hi, lo, n);
+    convert_grid_kernel<true><<<convert_blocks(), 256, 0, st>>>(hi, lo, n);
   else
     widen_grid_new_kernel<<<2048, 256, 0, st>>>(hi, lo, n);
 #endif
@@ -797,7 +806,7 @@ bool bz_narrow_grid(vis_complex *hi, vis_complex *lo, vis_complex *out, long lon
   if (out)
     resolve_grid_kernel<<<2048, 256, 0, st>>>(hi, lo, true, out, n);
   else
-    convert_grid_kernel<false><<<152 * 8, 256, 0, st>>>(hi, lo, n);
+    convert_grid_kernel<false><<<convert_blocks(), 256, 0, st>>>(hi, lo, n);
 #endif
   return cudaGetLastError() == cudaSuccess;
 }
