@@ -54,7 +54,7 @@ def _f32(a):
 def test_gradients_with_w_kernels(gpu_required, built_libraries):
     import torch
     from bullseye_gb300 import autograd
-    p = _problem(4, 11, 24)
+    p = _problem(4, 11, 40)
     geom = autograd.FacetGeometry.from_problem(p)
     rng = np.random.default_rng(4)
     grad = (rng.normal(size=(1, 1, 4, p.ny, p.nx)) + 1j * rng.normal(size=(1, 1, 4, p.ny, p.nx))).astype(np.complex64)
