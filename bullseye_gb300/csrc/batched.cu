@@ -713,13 +713,13 @@ bool plan_classes() {
   std::vector<int> pcls(P);
   for (int p = 0; p < P; ++p) pcls[p] = (int)(std::find(widths.begin(), widths.end(), pw[p]) - widths.begin());
   // Support-window table: row (plane p, tap offset f) holds the taps s = plo[p] + j,
-  // j < pw[p] (conv[p][f + s os]), then its first 7 taps again, zero-padded to a multiple of 16 bytes.
+  // j < pw[p] (conv[p][f + s os]), zero-padded to a multiple of 16 bytes.
   // The merge step reads a row's taps by consecutive lanes.
   {
     const size_t ncomp = wproj ? 2 : 1;
     const int E = (int)(16 / (ncomp * sizeof(vis_real)));
     const int pwmax = *std::max_element(pw.begin(), pw.end());
-    const int L = (pwmax + 7 + E - 1) / E * E;
+    const int L = (pwmax + E - 1) / E * E;
     const size_t tf = c.tap_f;
     std::vector<vis_real> tab(ncomp * (size_t)P * tf * L, (vis_real)0);
     for (int p = 0; p < P; ++p)
@@ -730,8 +730,6 @@ bool plan_classes() {
           if (i >= (size_t)K) break;
           for (size_t q = 0; q < ncomp; ++q) row[ncomp * j + q] = c.conv_host[ncomp * ((size_t)p * K + i) + q];
         }
-        for (int j = pw[p]; j < pw[p] + 7; ++j)
-          for (size_t q = 0; q < ncomp; ++q) row[ncomp * j + q] = row[ncomp * (j - pw[p]) + q];
       }
     if (!b.conv_w.alloc(tab.size())) return false;
     BZ_CUDA_TRY_RET(cudaMemcpy(b.conv_w.ptr, tab.data(), sizeof(vis_real) * tab.size(), cudaMemcpyHostToDevice), false);
@@ -1697,10 +1695,9 @@ __global__ void window_table_kernel(const void *conv, int P, int K, int tap_f, i
     const long long pf = e / L;
     const int f = (int)(pf % tap_f), p = (int)(pf / tap_f);
     const int pw = plane_w[p];
-    const int jj = j < pw ? j : (j < pw + 7 ? j - pw : -1);
     vis_real re = 0, im = 0;
-    if (jj >= 0) {
-      const long long i = f + (long long)(plane_lo[p] + jj) * os;
+    if (j < pw) {
+      const long long i = f + (long long)(plane_lo[p] + j) * os;
       if (i < K) {
         if (wproj) {
           const vis_complex t = ((const vis_complex *)conv)[(long long)p * K + i];
@@ -1732,7 +1729,7 @@ SupportWs support_ws_layout(long long R, int nchan, int nslots, int P, int os, i
   SupportWs l;
   const size_t ncomp = wproj ? 2 : 1;
   const int E = (int)(16 / (ncomp * sizeof(vis_real)));
-  l.L = (W + 7 + E - 1) / E * E;
+  l.L = (W + E - 1) / E * E;
   l.tap_f = 2 * os + 1;
   l.maxseg = std::max<long long>(1, R * nchan);
   const long long tracks = std::max<long long>(1, (long long)nslots * nchan);

@@ -125,7 +125,7 @@ struct GridArgs {
   int tap_f;
   const void *conv_t;            // kernel regrouped by tap offset [P][tap_f][W], or null
   const void *conv_w;            // support-window rows [P][tap_f][conv_w_stride], or null (see
-                                 // the batched planner): a staged tap row is one bulk copy
+                                 // the batched planner)
   int conv_w_stride;
   const uint8_t *facet_row_mask; // [facets][rows]: 0 leaves the row out of that facet, or null
   const FacetXform *facets;
@@ -168,7 +168,7 @@ enum DeviceError {
   DEV_ERR_JONES_INDEX = 2,
   DEV_ERR_SINGULAR = 4,
   DEV_ERR_POL_INDEX = 8,
-  DEV_ERR_WAIT_TIMEOUT = 16,  // a bounded wait on the tap-copy barrier ran out
+  DEV_ERR_WAIT_TIMEOUT = 16,  // a bounded wait for staged records ran out
   DEV_ERR_ANTENNA = 32        // an antenna pair outside baseline_count (row sort)
 };
 
@@ -202,24 +202,6 @@ struct __align__(16) GridRec {
   int g, valid, fu, fv;    // grid group, validity, support-window table rows
   cplx vis[NC];            // weighted, corrected, rotated visibility
 };
-
-__device__ __forceinline__ void load_tap(const void *conv, long long idx, acc_real &t) {
-  t = (acc_real)((const vis_real *)conv)[idx];
-}
-__device__ __forceinline__ void load_tap(const void *conv, long long idx, cplx &t) {
-  vis_complex c = ((const vis_complex *)conv)[idx];
-  t.re = (acc_real)c.re;
-  t.im = (acc_real)c.im;
-}
-
-__device__ __forceinline__ cplx tap_mul(acc_real a, acc_real b, cplx v) {
-  acc_real t = a * b;
-  cplx r;
-  r.re = v.re * t;
-  r.im = v.im * t;
-  return r;
-}
-__device__ __forceinline__ cplx tap_mul(cplx a, cplx b, cplx v) { return cmul(v, cmul(a, b)); }
 
 // 2x2 complex products on row-major [a b; c d] stored as 4 cplx
 __device__ __forceinline__ void jmul(const cplx *A, const cplx *B, cplx *O) {
