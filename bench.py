@@ -17,12 +17,13 @@ Lines printed (rank 0, one JSON line):
   e2e       the same metric through the reference-facing C-ABI with host buffers: initLibrary,
             facet_4_cor_corrections + facet_sampling_function (pinned host inputs, final-chunk
             copy-back), weight_uniformly, normalize, finalize, releaseLibrary every step;
-  roofline  the gridder kernel against the measured FP32 FMA rate of this GPU (the gridder is
-            FP32-issue bound; HBM traffic is reported alongside);
+  roofline  the direct sum's operations (every visibility's footprint by itself) against the measured
+            FP32 FMA rate of this GPU.  The gridder sums visibilities that share a tap row first and
+            executes fewer: the fraction is a rate of results.  HBM traffic is reported alongside;
   cpu_baseline  the oracle port of the reference CPU library (OpenMP over facets) on a bounded
             sample of rows, on this machine's host cores;
   precision the precision form: per-facet max / RMS relative dirty-image error of the FP32
-            library (compensated and plain flushes) against the FP64 library, config 3 (80 km,
+            library (FP64 and plain FP32 accumulation) against the FP64 library, config 3 (80 km,
             4 facets of 4096^2).
 
 With N ranks (torchrun) each rank grids its own 16 facets of a 16 N-facet field (facet sharding,
@@ -55,11 +56,11 @@ WORKLOAD = ("facet_4_cor_corrections+facet_sampling_function, 27 ant x 2000 t x 
 
 
 # DRAM traffic of one batched step (dram__bytes_read.sum + dram__bytes_write.sum, every launch of
-# the step), captured with ncu on the 16-channel, 4-facet cut of this workload (11.20 GB for
+# the step), captured with ncu on the 16-channel, 4-facet cut of this workload (10.46 GB for
 # 44.93 M vis-facet pairs, visibility records included) and scaled by vis-facet pairs: an upper
 # estimate for the full step, where 16 facets rather than 4 share each row's loads.
-TRAFFIC_BYTES_PER_PAIR = 11.20e9 / 44928000
-TRAFFIC_SOURCE = ("ncu dram bytes of one eager step of the 16-channel 4-facet case (11.20 GB / 44.93 M pairs, "
+TRAFFIC_BYTES_PER_PAIR = 10.46e9 / 44928000
+TRAFFIC_SOURCE = ("ncu dram bytes of one eager step of the 16-channel 4-facet case (10.46 GB / 44.93 M pairs, "
                   "visibility records written and read once), scaled by vis-facet pairs (upper estimate: more "
                   "facets share each row's loads)")
 
@@ -74,7 +75,7 @@ def parse():
     ap.add_argument("--no-e2e", action="store_true")
     ap.add_argument("--no-cpu", action="store_true")
     ap.add_argument("--cpu-seconds", type=float, default=12.0)
-    ap.add_argument("--no-comp", action="store_true", help="plain (uncompensated) FP32 grid flushes")
+    ap.add_argument("--no-comp", action="store_true", help="plain FP32 grid accumulation")
     ap.add_argument("--chans", type=int, default=0, help="override the channel count (profiling cases)")
     ap.add_argument("--form", default="batched", choices=["batched", "plain"],
                     help="batched: bullseye_grid_batched; plain: the per-call drop-in ABI path")
@@ -195,7 +196,7 @@ def class_profile(lib, step, counts, plane_width):
         rows.append({"width": int(width[i]), "corr": int(nc[i]), "J": int(J[i]), "wide": bool(wide[i] & 1),
                      "registers": int(wide[i]) >> 1,
                      "work_items": int(items[i]), "vis": vis, "ms": float(ms[i]),
-                     "executed_tflops": flops / (float(ms[i]) * 1e-3) / 1e12 if ms[i] > 0 else None})
+                     "direct_sum_tflops": flops / (float(ms[i]) * 1e-3) / 1e12 if ms[i] > 0 else None})
     return rows
 
 
@@ -483,7 +484,7 @@ def dirty(grid):
 def parity_check(lib32, geo, conv1d, smp):
     """The batched FP32 path against the FP64 oracle on the row sample: the same reference exports
     through the C-ABI (host inputs; the exports run the support-aware batched gridder with the
-    tuned class layouts and compensated FP32) and the oracle port in double precision on the same
+    tuned class layouts and FP32 accumulated in FP64) and the oracle port in double precision on the same
     values, both followed by weight_uniformly and normalize.  Per facet: max and RMS relative error
     of the weighted, normalised grids and of the dirty images."""
     from bullseye_gb300.filters import outer_stack
@@ -507,7 +508,7 @@ def parity_check(lib32, geo, conv1d, smp):
     return {"against": "oracle port of the reference CPU library in FP64 (same input values, 2-D w-kernel stack "
                        "of the FP32 1-D stack), weight_uniformly + normalize on both",
             "form": "reference exports facet_4_cor_corrections + facet_sampling_function on the batched "
-                    "support-aware gridder (tuned class layouts, compensated FP32)",
+                    "support-aware gridder (tuned class layouts, FP32 accumulated in FP64)",
             "sample": f"{smp['starts'].size - 1} whole baselines, {smp['uvw'].shape[0]} rows x {N_CHAN} ch x "
                       f"{N_FACETS} facets",
             "max_rel": worst, "rms_rel": max(x["image_rms_rel"] for x in facets),
@@ -522,8 +523,8 @@ def precision_report():
     The config-1 observation on an 80 km disc, 4 facets of 4096^2 (0.25 arcsec) at l offsets of
     0, 0.5, 1 and 2 deg, facet_4_cor + normalize + finalize through the C-ABI.  Both libraries get
     the same input values (the single-precision arrays, widened for the FP64 run), so the figures
-    are the arithmetic error of the FP32 path: compensated (the precision form) and plain FP32
-    flushes.  max_rel = max|I32 - I64| / max|I64|, rms_rel = rms(I32 - I64) / rms(I64), on the XX
+    are the arithmetic error of the FP32 path: accumulated in FP64 (the precision form) and
+    plain FP32.  max_rel = max|I32 - I64| / max|I64|, rms_rel = rms(I32 - I64) / rms(I64), on the XX
     image of each facet.
     """
     from bullseye_gb300 import synth
@@ -711,7 +712,7 @@ def uneven_main(args):
                                    f"(log-uniform), 5 arcsec cells, per-facet baseline/time flagging masks keeping "
                                    f"1e5..5e7 visibilities per facet (log-uniform), "
                                    f"27 ant x {UNEVEN_TIMES} t x {N_CHAN} ch ({R * N_CHAN / 1e6:.1f}M vis), w-proj "
-                                   f"{WPLANES} planes support {MIN_SUPPORT}-{2 * S_HALF + 1}, facet_4_cor, compensated FP32",
+                                   f"{WPLANES} planes support {MIN_SUPPORT}-{2 * S_HALF + 1}, facet_4_cor, FP32 accumulated in FP64",
                        "facet_vis_min": int(kept_rows.min()) * N_CHAN, "facet_vis_max": int(kept_rows.max()) * N_CHAN,
                        "grid_cells": off, "vis_facet_pairs_per_step": pairs_per_step,
                        "form": "bullseye_grid_batched_facets (persistent per-class launches, CUDA graph replay)"},
@@ -817,7 +818,7 @@ def uneven_parity(lib, geo, conv1d, sizes, fl, fm, masks, d, torch, no_comp, nbl
     worst = max(x["image_max_rel"] for x in per_facet)
     parity = {"against": "oracle port of the reference CPU library in FP64 on each facet's own grid (masked rows "
                          "flagged), 2-D stack of the FP32 1-D w kernels",
-              "form": "bullseye_grid_batched_facets over the sampled facets (device inputs, compensated FP32)",
+              "form": "bullseye_grid_batched_facets over the sampled facets (device inputs, FP32 accumulated in FP64)",
               "sample": f"{pick.size} whole baselines ({R} rows x {N_CHAN} ch), facets {sel}",
               "max_rel": worst, "tolerance": 1e-5, "pass": worst <= 1e-5, "per_facet": per_facet,
               "seconds": time.perf_counter() - t0}
@@ -1316,12 +1317,12 @@ def main():
         # the visibility gridder launch (CUDA events around it in the library), padded W = 63
         launch_ms = vis_kernel_ms / n_vis_launch
         step_flops = true_taps * N_FACETS * 8 * 4 + pairs_per_step * (6 * 4 + 128)  # visibility launch only
-        executed_taps = float(counts.sum()) * W * W
+        class_taps_sum = float(counts.sum()) * W * W
         kernel_name = "romein_grid_kernel<4,wproj,J=8,wide> (visibilities, padded W=63)"
     else:
         # batched: the per-class persistent launches make up the step (timed whole)
         launch_ms = ms_per_step
-        executed_taps = sum(t for _, t in class_taps(counts, plane_width).values()) if plane_width is not None else None
+        class_taps_sum = sum(t for _, t in class_taps(counts, plane_width).values()) if plane_width is not None else None
         kernel_name = "romein_segment_kernel per support class (whole batched step)"
     achieved = step_flops / (launch_ms * 1e-3) / 1e12
     hbm_gbs = pairs_per_step * bytes_per_pair / (launch_ms * 1e-3) / 1e9
@@ -1482,8 +1483,8 @@ def main():
             "config": {"workload": WORKLOAD, "rows": R, "channels": N_CHAN, "facets": N_FACETS,
                        "vis_facet_pairs_per_step": pairs_per_step, "l2": "inputs 4.2 GB per step > 129 MB L2",
                        "form": ("batched: bullseye_grid_batched (support-aware, persistent per-class launches, "
-                                "CUDA graph, compensated FP32)" if args.form == "batched" else
-                                "plain: per-call drop-in ABI path (padded support, compensated FP32)")},
+                                "CUDA graph, FP32 accumulated in FP64)" if args.form == "batched" else
+                                "plain: per-call drop-in ABI path (padded support, FP32 accumulated in FP64)")},
             "other_form": None if other_ms is None else {
                 "form": "plain" if args.form == "batched" else "batched", "ms_per_step": other_ms,
                 "value": pairs_per_step * world / (other_ms * 1e-3) / 1e6, "unit": "Mvis/s"},
@@ -1500,8 +1501,9 @@ def main():
                          "kernel": kernel_name, "launch_ms": launch_ms,
                          "flops_per_pair": flops_per_pair,
                          "flops_rule": "8 x 4 corr x W_p^2 per (vis, facet) with W_p the visibility's w-plane "
-                                       "support (+ sampling function once, + 152 for phase and Jones)",
-                         "executed_taps_per_vis": executed_taps / float(counts.sum()) if executed_taps else None,
+                                       "support (+ sampling function once, + 152 for phase and Jones): the direct "
+                                       "sum, of which merged groups execute a part",
+                         "class_taps_per_vis": class_taps_sum / float(counts.sum()) if class_taps_sum else None,
                          "true_taps_per_vis": true_taps / float(counts.sum()),
                          "hbm_gbs": hbm_gbs,
                          "hbm_frac_of_measured": hbm_gbs / peaks["hbm_gbs"] if peaks.get("hbm_gbs") else None,

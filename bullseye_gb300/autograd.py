@@ -10,7 +10,7 @@ baseline_transform_policies.h:117-149).  The forward pass runs the library's wor
 and returns dL/dV and dL/dJ in PyTorch's complex-gradient convention (dL = Re sum conj(g) dz).
 
 Both passes are the CUDA library: there is no PyTorch or CPU implementation here, and a missing
-library raises.  ``complex64`` inputs run the 32-bit library (compensated FP32 gridding),
+library raises.  ``complex64`` inputs run the 32-bit library (FP32 gridding, accumulated in FP64),
 ``complex128`` the 64-bit one.
 """
 from __future__ import annotations

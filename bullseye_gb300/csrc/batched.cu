@@ -1399,7 +1399,7 @@ bool stream_visibilities(gridding_parameters &p, const GridArgs &va, int nfacets
     vk.nslots = (k - k0 + 1) * (int)plan.slots;
     if (!enqueue_schedule(vk, c.stream, g_r0, r1 - g_r0)) return false;
     if (k0 == 0) {
-      // every call sets its classes' layouts up for this build (NC, w-projection, compensation) from
+      // every call sets its classes' layouts up for this build (NC, w-projection, accumulation) from
       // the tuned decisions; classes without a decision yet are timed on this group's runs
       if (!classes_tuned(4, wproj, acc)) {
         BZ_CUDA_TRY_RET(cudaMemcpyAsync(counts.data(), g_bs.class_count.ptr, sizeof(int) * kMaxClasses,

@@ -1038,8 +1038,8 @@ __device__ __forceinline__ void prologue(const GridArgs &a, int f_local, int cha
 //   grid_groups   the Romein owner threads add their column's tap x T(row) to their J cells.
 //
 // What the merge and the split of the builds measured (GB300, 27 antennas x 100 times x 64 channels,
-// 16 facets, whole batched call with copy-back): 36.5 -> 27.3 ms in single precision; 64-bit library,
-// 40 times x 16 channels x 4 facets: 28.2 -> 8.1 ms (its FP64 pipe bounded the multiply-adds).
+// 16 facets, whole batched call with copy-back): 36.0 -> 27.2 ms in single precision; 64-bit library,
+// 40 times x 16 channels x 4 facets: 27.3 -> 7.7 ms (its FP64 pipe bounded the multiply-adds).
 
 // Most records of a chunk: group lists are built from 64-bit masks.
 constexpr int kMaxChunk = 64;

@@ -12,7 +12,7 @@
 // The scratch array holds the second word of the single-precision library's wide grid accumulation
 // (while a call grids, a cell's FP64 real part lies in the caller's grid and its imaginary part here),
 // the per-facet transform table and an error word.  It is BZ_NOALLOC_SCRATCH_BYTES bytes (40 MiB
-// for the compensation grid, so at most 40 MiB / 8 bytes = 5,242,880 complex cells over
+// for the second words, so at most 40 MiB / 8 bytes = 5,242,880 complex cells over
 // facets x cube x 4 correlations x ny x nx, plus 64 KiB for the table), and every GPU that loads
 // the library keeps it until the process exits.  All calls share it and it keeps the last call's
 // contents: each call clears the parts that must start at zero, and calls whose work overlaps on
@@ -157,7 +157,7 @@ bool noalloc_dispatch(GridArgs a, long long blocks, cudaStream_t st) {
 
 namespace {
 
-// Device scratch of one gridding call: the compensation grid (single precision), the facet table
+// Device scratch of one gridding call: the second words (single precision), the facet table
 // and an error word, with the capacities the call checks its sizes against.
 struct Workspace {
   vis_complex *lo;
@@ -198,7 +198,7 @@ int grid_4cor_jones(const gridding_parameters &p, const Workspace &ws, void *str
 #if defined(BULLSEYE_SINGLE)
   if (grid_elems * sizeof(vis_complex) > ws.lo_bytes) {
     bz_record_error(BZ_ERR_UNSUPPORTED,
-                    "%s: %zu grid cells need %zu bytes of compensation scratch, more than the %zu bytes available "
+                    "%s: %zu grid cells need %zu bytes of scratch for second words, more than the %zu bytes available "
                     "(the fixed scratch array of the allocation-free entry)",
                     name, grid_elems, grid_elems * sizeof(vis_complex), ws.lo_bytes);
     return BZ_ERR_UNSUPPORTED;
@@ -391,7 +391,7 @@ extern "C" size_t bullseye_facet_4_cor_corrections_ws_bytes(const gridding_param
   return ws_lo_bytes(*params) + ws_table_bytes(*params) + 256 + ws_sched_bytes(*params);
 }
 
-// Workspace pieces of bullseye_facet_4_cor_corrections_ws: compensation grid, facet table, error
+// Workspace pieces of bullseye_facet_4_cor_corrections_ws: second words, facet table, error
 // word, support-aware schedule.
 static Workspace caller_workspace(const gridding_parameters &p, unsigned char *w) {
   Workspace ws;

@@ -142,7 +142,7 @@ void bullseye_set_max_stage_bytes(size_t bytes);
  * record per (row, facet, channel) of its work (footprint corner, tap rows, grid group, and the
  * weighted, Jones-corrected, phase-rotated visibility, 64 bytes in single precision) and its
  * normalisation sums, by a kernel that takes every row in parallel; the class launches then stage
- * records and tap rows by bulk copies only.  The records take at most the record budget (0: the
+ * records by bulk copies and read the kernel table through L1.  The records take at most the record budget (0: the
  * default, 30 % of the device's memory) and the free memory; work past it is prepared in place, as
  * with records off.  Results are the same either way. */
 void bullseye_set_visibility_records(int on);
@@ -169,7 +169,7 @@ int bullseye_grid_batched(gridding_parameters *params, int call, int with_sampli
  * facets described by `facets` (host array), accumulated into CALLER-OWNED device buffers:
  * grids (complex, each facet's block at its grid_offset), grid_lo (the 32-bit library's
  * second words, same size as grids and zeroed by the caller, or null for plain FP32 accumulation; a
- * cell's value is then grids + grid_lo, and while a call's work runs the two words of a cell hold an FP64
+ * cell's value is then grids + grid_lo, and while a call's work runs the two words of a cell may hold an FP64
  * pair; ignored by the 64-bit library) and norms
  * (float64 [nfacets][cube][4]).  Work is queued on the library stream (bullseye_get_stream).
  * row_mask, if not null, is a device array [nfacets][row_count] of bytes (device-resident inputs
@@ -249,7 +249,7 @@ int bullseye_facet_4_cor_corrections_noalloc(const gridding_parameters *params, 
  * device and the visibilities are gridded by persistent per-support-class launches over a run
  * schedule built in the workspace (the same grids as the full padded support).  The workspace must
  * be 256-byte aligned and at least bullseye_facet_4_cor_corrections_ws_bytes(params) bytes (the
- * 32-bit library's compensation grid, the facet table, an error word, and the support windows,
+ * 32-bit library's second words, the facet table, an error word, and the support windows,
  * window table and run schedule: about 33 bytes per (row, channel)); its contents need not be
  * initialised.  jones_terms is inverted in place.  No counterpart in the reference. */
 size_t bullseye_facet_4_cor_corrections_ws_bytes(const gridding_parameters *params);
